@@ -326,6 +326,13 @@ int nla3d_probe_fma_peak(int fp64, double* flops);
  *   nla3d_mlp_column_sum      out[c] = sum_r X[r, c] (row-major rows x cols)
  *   nla3d_mlp_adam    Adam step on FP32 master weights (step >= 1), refreshing
  *                     the BF16 copy w_bf16 when non-NULL
+ *   nla3d_mlp_layer_grads  dW[o,i] = sum_b dY[b,o] X[b,i] and db[o] = sum_b
+ *                     dY[b,o] in one launch (row-major, contiguous)
+ *   nla3d_mlp_input_grad   dX[b,i] = (sum_o dY[b,o] W[o,i]) (1 - Y[b,i]^2), W
+ *                     BF16 (n_out x n_in), Y the layer's tanh input (NULL:
+ *                     without the factor)
+ *   nla3d_mlp_adam_multi   nla3d_mlp_adam on `count` tensors; w_bf16[t] may be
+ *                     NULL; the arrays are host arrays, read by the call
  *   nla3d_mlp_mse_grad dY = scale * (Y - T)
  *   nla3d_mlp_to_bf16 round-to-nearest-even FP32 -> BF16 */
 int nla3d_mlp_gemm(int M, int N, int K, const void* A, int a_bf16, int64_t lda_m, int64_t lda_k,
@@ -335,6 +342,13 @@ int nla3d_mlp_tanh_backward(const float* Y, float* dY, int64_t n, void* stream);
 int nla3d_mlp_column_sum(const float* X, int64_t rows, int64_t cols, float* out, void* stream);
 int nla3d_mlp_adam(float* w, const float* g, float* m, float* v, int64_t n, float lr, float beta1,
                    float beta2, float eps, int step, uint16_t* w_bf16, void* stream);
+int nla3d_mlp_layer_grads(int batch, int n_out, int n_in, const float* dY, const float* X,
+                          float* dW, float* db, void* stream);
+int nla3d_mlp_input_grad(int batch, int n_out, int n_in, const float* dY, const uint16_t* W_bf16,
+                         const float* Y, float* dX, void* stream);
+int nla3d_mlp_adam_multi(int count, float* const* w, const float* const* g, float* const* m,
+                         float* const* v, const int64_t* n, uint16_t* const* w_bf16, float lr,
+                         float beta1, float beta2, float eps, int step, void* stream);
 int nla3d_mlp_mse_grad(const float* Y, const float* T, float* dY, int64_t n, float scale,
                        void* stream);
 int nla3d_mlp_to_bf16(const float* x, uint16_t* y, int64_t n, void* stream);

@@ -20,25 +20,33 @@ namespace {
 
 // ---- C = act(A B + bias) on the tensor cores (tcgen05.mma kind::f16, BF16) ----
 //
-// One CTA (256 threads) per 128 x 128 tile of C, K in chunks of 32.  Both
-// operands are staged in shared memory as BF16 in the canonical K-major
-// layout without swizzle (8-row x 16-byte core matrices; K-adjacent cores
-// 128 B apart, 8-row groups 512 B apart): A as its 128 rows m, B as its 128
-// columns n (the MMA computes D[m][n] = sum_k A[m][k] B'[n][k]).  An FP32
+// One CTA (512 threads) per 128 x 32 tile of C, K in chunks of 128, two
+// shared-memory stages.  Both operands are staged as BF16 in the canonical
+// K-major layout without swizzle (8-row x 16-byte core matrices; K-adjacent
+// cores 128 B apart, 8-row groups 2 KB apart): A as its 128 rows m, B as its
+// 32 columns n (the MMA computes D[m][n] = sum_k A[m][k] B'[n][k]).  An FP32
 // operand (activations, gradients) is split into a BF16 high part and the
 // BF16 rounding of the remainder, x = hi + lo + O(2^-16 |x|); a BF16 operand
 // (the weights) is exact as it is.  One thread issues, per 16-wide K step,
 // hi.hi, then hi.lo and lo.hi where an operand has a low part (BF16 x BF16
-// products are exact in FP32), accumulating in FP32 in 128 TMEM columns, and
-// commits them to an mbarrier; the next chunk is staged once they have
-// released the buffers.  The epilogue reads TMEM (warp w: lanes 32 (w % 4)
-// .. +31 = rows, columns 64 (w / 4) .. +63), adds the bias, applies the
-// activation and stores FP32.  Every wait is bounded: on a timeout the
-// tile's outputs are set to NaN and g_mlp_timeouts is incremented.
-constexpr int kTcM = 128, kTcN = 128, kTcK = 32;
-constexpr int kThreads = 256;
-constexpr uint32_t kTileElems = kTcM * kTcK;                      // one 128 x 32 operand
-constexpr size_t kTcSmem = 4 * kTileElems * sizeof(__nv_bfloat16) + 64;
+// products are exact in FP32), accumulating in FP32 in 32 TMEM columns, and
+// commits them to the stage's mbarrier; a stage is refilled once its MMAs
+// have released it, and a chunk's loads are issued before that wait.  The
+// epilogue reads TMEM (warp w: lanes 32 (w % 4) .. +31 = rows, columns
+// 8 (w / 4) .. +7), adds the bias, applies the activation and stores FP32.
+// Every wait is bounded: on a timeout the tile's outputs are set to NaN and
+// g_mlp_timeouts is incremented.
+//
+// The network's products (batch x 256 x 256) are far below the chip: what
+// bounds one is the latency of its serial chunks.  128 x 128 tiles with
+// 32-wide chunks ran 4 CTAs x 8 serial load-convert-multiply rounds, 51 us a
+// product at batch 256 (ncu, cold); 128 x 32 tiles with 128-wide chunks run
+// 16 CTAs x 2 rounds, each with all of a chunk's loads in flight, 14 us.
+constexpr int kTcM = 128, kTcN = 32, kTcK = 128;
+constexpr int kThreads = 512;
+constexpr uint32_t kATile = kTcM * kTcK, kBTile = kTcN * kTcK;      // elements per operand part
+constexpr uint32_t kStageElems = 2 * (kATile + kBTile);             // A hi, A lo, B hi, B lo
+constexpr size_t kTcSmem = 2 * kStageElems * sizeof(__nv_bfloat16) + 64;
 // instruction descriptor: D F32 (bit 4), A and B BF16 (bits 7, 10), both
 // K-major, N / 8 at bit 17, M / 16 at bit 24
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) |
@@ -84,20 +92,76 @@ __device__ __forceinline__ float load_elem(const void* p, int bf16, long i) {
   return reinterpret_cast<const float*>(p)[i];
 }
 
-// 16 consecutive K values of one operand row into the hi / lo tiles
-// (8 bf16 = one 16-byte core-matrix row per store)
-__device__ __forceinline__ void stage_row(__nv_bfloat16* hi, __nv_bfloat16* lo, bool split,
-                                          int r, int kq, const float v[16]) {
+// An operand chunk of R rows x kTcK is R kTcK / 8 units of (one row, 8
+// consecutive k), one 16-byte core-matrix row each.  Eight consecutive
+// threads take the eight rows of a core matrix (conflict-free 16-byte
+// stores); where k runs contiguously in memory the next 24 threads take the
+// next three core matrices along k (128 contiguous bytes per row), where
+// rows do, along the rows.
+template <int R>
+__device__ __forceinline__ void unit_of(int u, bool k_fast, int& row, int& k) {
+  const int g = u >> 3;
+  if (k_fast) {
+    row = (g / (kTcK / 8)) * 8 + (u & 7);
+    k = (g % (kTcK / 8)) * 8;
+  } else {
+    row = (g % (R / 8)) * 8 + (u & 7);
+    k = (g / (R / 8)) * 8;
+  }
+}
+
+// `vec`: k runs contiguously and every unit starts on a 16-byte boundary, so
+// a whole unit is two (FP32) or one (BF16) 16-byte loads
+__device__ __forceinline__ bool vector_units(const void* p, int bf16, long ld_r, long ld_k) {
+  return ld_k == 1 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0 && ld_r % (bf16 ? 8 : 4) == 0;
+}
+
+template <int R>
+__device__ __forceinline__ void load_units(float v[][8], const void* p, int bf16, bool vec,
+                                           long ld_r, long ld_k, int r0, int rows, int k0, int K) {
 #pragma unroll
-  for (int half = 0; half < 2; half++) {
-    const int k = kq * 16 + half * 8;
-    const uint32_t off = (uint32_t)(((r >> 3) * (kTcK / 8) + (k >> 3)) * 64 + (r & 7) * 8);
+  for (int q = 0; q < R * kTcK / 8 / kThreads; q++) {
+    int row, k;
+    unit_of<R>(threadIdx.x + q * kThreads, ld_k == 1, row, k);
+    const long base = (long)(r0 + row) * ld_r + (long)(k0 + k) * ld_k;
+    if (vec && r0 + row < rows && k0 + k + 8 <= K) {
+      if (bf16) {
+        const uint4 w = *reinterpret_cast<const uint4*>(
+            reinterpret_cast<const __nv_bfloat16*>(p) + base);
+        const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          v[q][2 * e] = __uint_as_float(u[e] << 16);
+          v[q][2 * e + 1] = __uint_as_float(u[e] & 0xFFFF0000u);
+        }
+      } else {
+        const float4 x = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + base);
+        const float4 y =
+            *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + base + 4);
+        v[q][0] = x.x, v[q][1] = x.y, v[q][2] = x.z, v[q][3] = x.w;
+        v[q][4] = y.x, v[q][5] = y.y, v[q][6] = y.z, v[q][7] = y.w;
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; e++)
+        v[q][e] = (r0 + row < rows && k0 + k + e < K) ? load_elem(p, bf16, base + e * ld_k) : 0.f;
+    }
+  }
+}
+
+template <int R>
+__device__ __forceinline__ void stage_units(__nv_bfloat16* hi, __nv_bfloat16* lo, bool split,
+                                            bool k_fast, const float v[][8]) {
+#pragma unroll
+  for (int q = 0; q < R * kTcK / 8 / kThreads; q++) {
+    int row, k;
+    unit_of<R>(threadIdx.x + q * kThreads, k_fast, row, k);
+    const uint32_t off = (uint32_t)(((row >> 3) * (kTcK / 8) + (k >> 3)) * 64 + (row & 7) * 8);
     __align__(16) __nv_bfloat16 h[8], l[8];
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-      const float x = v[half * 8 + q];
-      h[q] = __float2bfloat16_rn(x);
-      l[q] = __float2bfloat16_rn(x - __bfloat162float(h[q]));
+    for (int e = 0; e < 8; e++) {
+      h[e] = __float2bfloat16_rn(v[q][e]);
+      l[e] = __float2bfloat16_rn(v[q][e] - __bfloat162float(h[e]));
     }
     *reinterpret_cast<uint4*>(hi + off) = *reinterpret_cast<const uint4*>(h);
     if (split) *reinterpret_cast<uint4*>(lo + off) = *reinterpret_cast<const uint4*>(l);
@@ -107,17 +171,17 @@ __device__ __forceinline__ void stage_row(__nv_bfloat16* hi, __nv_bfloat16* lo, 
 __global__ void __launch_bounds__(kThreads)
     tc_gemm_kernel(int M, int N, int K, const void* __restrict__ A, int a_bf16, long lda_m,
                    long lda_k, const void* __restrict__ B, int b_bf16, long ldb_k, long ldb_n,
-                   float* __restrict__ C, long ldc, const float* __restrict__ bias, int act) {
+                   float* __restrict__ C, long ldc, const float* __restrict__ bias, int act,
+                   const float* __restrict__ Y, float* __restrict__ a_sum) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __nv_bfloat16* Ahi = reinterpret_cast<__nv_bfloat16*>(smem);
-  __nv_bfloat16* Alo = Ahi + kTileElems;
-  __nv_bfloat16* Bhi = Alo + kTileElems;
-  __nv_bfloat16* Blo = Bhi + kTileElems;
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(Blo + kTileElems);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar + 1);
+  __nv_bfloat16* stage = reinterpret_cast<__nv_bfloat16*>(smem);
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(stage + 2 * kStageElems);   // one per stage
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar + 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * kTcM, n0 = blockIdx.x * kTcN;
   const bool a_split = !a_bf16, b_split = !b_bf16;
+  const bool a_vec = vector_units(A, a_bf16, lda_m, lda_k);
+  const bool b_vec = vector_units(B, b_bf16, ldb_n, ldb_k);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_addr(tmem_slot)),
@@ -126,40 +190,48 @@ __global__ void __launch_bounds__(kThreads)
   }
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(mbar)), "r"(1));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(mbar + 1)), "r"(1));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  const int r = threadIdx.x % kTcM, kq = threadIdx.x / kTcM;  // operand row, which 16 of 32
-  const int ma = m0 + r, nb = n0 + r;
   const uint32_t lbo = 128, sbo = (kTcK / 8) * 128;
   const int n_chunks = (K + kTcK - 1) / kTcK;
   bool ok = true;
+  float row_sum = 0.f;
   for (int c = 0; c < n_chunks && ok; c++) {
-    if (c > 0) ok = mbar_wait(smem_addr(mbar), (uint32_t)(c - 1) & 1u);  // buffers released
-    if (ok) {
-      float av[16], bv[16];
+    float av[kATile / 8 / kThreads][8], bv[kBTile / 8 / kThreads][8];
+    load_units<kTcM>(av, A, a_bf16, a_vec, lda_m, lda_k, m0, M, c * kTcK, K);
+    load_units<kTcN>(bv, B, b_bf16, b_vec, ldb_n, ldb_k, n0, N, c * kTcK, K);
+    if (a_sum) {
+      // rows contiguous in memory: every unit of a thread has the same row
+      // (threads t + 128 j share one), so its values add up here
 #pragma unroll
-      for (int q = 0; q < 16; q++) {
-        const int k = c * kTcK + kq * 16 + q;
-        av[q] = (ma < M && k < K) ? load_elem(A, a_bf16, (long)ma * lda_m + (long)k * lda_k) : 0.f;
-        bv[q] = (nb < N && k < K) ? load_elem(B, b_bf16, (long)k * ldb_k + (long)nb * ldb_n) : 0.f;
-      }
-      stage_row(Ahi, Alo, a_split, r, kq, av);
-      stage_row(Bhi, Blo, b_split, r, kq, bv);
+      for (int u = 0; u < kATile / 8 / kThreads; u++)
+        row_sum += ((av[u][0] + av[u][1]) + (av[u][2] + av[u][3])) +
+                   ((av[u][4] + av[u][5]) + (av[u][6] + av[u][7]));
+    }
+    const int q = c & 1;
+    if (c > 1) ok = mbar_wait(smem_addr(mbar + q), (uint32_t)(c / 2 - 1) & 1u);   // stage released
+    __nv_bfloat16* Ahi = stage + q * kStageElems;
+    __nv_bfloat16* Alo = Ahi + kATile;
+    __nv_bfloat16* Bhi = Alo + kATile;
+    __nv_bfloat16* Blo = Bhi + kBTile;
+    if (ok) {
+      stage_units<kTcM>(Ahi, Alo, a_split, lda_k == 1, av);
+      stage_units<kTcN>(Bhi, Blo, b_split, ldb_k == 1, bv);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     ok = __syncthreads_and(ok ? 1 : 0) != 0;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok && threadIdx.x == 0) {
       const uint32_t ahi = smem_addr(Ahi), alo = smem_addr(Alo);
       const uint32_t bhi = smem_addr(Bhi), blo = smem_addr(Blo);
-#pragma unroll
-      for (int st = 0; st < kTcK / 16; st++) {
+      const int steps = (min(K - c * kTcK, kTcK) + 15) / 16;   // the rest of a chunk is zeros
+      for (int st = 0; st < steps; st++) {
         const uint32_t koff = st * 256;   // 16 K values = two core matrices
         const uint64_t dah = mat_desc(ahi + koff, lbo, sbo), dbh = mat_desc(bhi + koff, lbo, sbo);
         mma_bf16(tmem, dah, dbh, (c > 0 || st > 0) ? 1u : 0u);
@@ -168,50 +240,67 @@ __global__ void __launch_bounds__(kThreads)
       }
       asm volatile(
           "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-              smem_addr(mbar))
+              smem_addr(mbar + q))
           : "memory");
     }
   }
-  if (ok && n_chunks > 0) ok = mbar_wait(smem_addr(mbar), (uint32_t)(n_chunks - 1) & 1u);
+  // the last chunk's commit covers every MMA issued (they complete in order)
+  if (ok && n_chunks > 0)
+    ok = mbar_wait(smem_addr(mbar + ((n_chunks - 1) & 1)), (uint32_t)((n_chunks - 1) / 2) & 1u);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   ok = __syncthreads_and(ok ? 1 : 0) != 0;
+  if (a_sum && blockIdx.x == 0) {
+    // (the stages are free: every MMA has completed)
+    float* part = reinterpret_cast<float*>(smem);
+    int r, k;
+    unit_of<kTcM>(threadIdx.x, false, r, k);
+    part[(threadIdx.x / kTcM) * kTcM + r] = row_sum;
+    __syncthreads();
+    if (threadIdx.x < kTcM && m0 + threadIdx.x < M)
+      a_sum[m0 + threadIdx.x] = (part[threadIdx.x] + part[kTcM + threadIdx.x]) +
+                                (part[2 * kTcM + threadIdx.x] + part[3 * kTcM + threadIdx.x]);
+  }
   const int row = (warp & 3) * 32 + lane;
   const int m = m0 + row;
-  for (int c0 = (warp >> 2) * 64; c0 < (warp >> 2) * 64 + 64; c0 += 16) {
-    uint32_t v[16];
-    if (ok && n_chunks > 0) {
-      const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
-          "%11, %12, %13, %14, %15}, [%16];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-            "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
-            "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(taddr));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    } else {
+  const int c0 = (warp >> 2) * 8;
+  uint32_t v[8];
+  if (ok && n_chunks > 0) {
+    const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+          "=r"(v[7])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  } else {
 #pragma unroll
-      for (int q = 0; q < 16; q++) v[q] = ok ? 0u : 0x7FC00000u;   // K = 0: zero; timeout: NaN
-    }
-    if (m < M)
-#pragma unroll
-      for (int q = 0; q < 16; q++) {
-        const int n = n0 + c0 + q;
-        if (n < N) {
-          float y = __uint_as_float(v[q]) + (bias ? bias[n] : 0.f);
-          if (act == 1) y = tanhf(y);
-          C[(long)m * ldc + n] = y;
-        }
-      }
+    for (int q = 0; q < 8; q++) v[q] = ok ? 0u : 0x7FC00000u;   // K = 0: zero; timeout: NaN
   }
+  if (m < M)
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int n = n0 + c0 + q;
+      if (n < N) {
+        float y = __uint_as_float(v[q]) + (bias ? bias[n] : 0.f);
+        if (act == 1) y = tanhf(y);
+        if (Y) {
+          const float t = Y[(long)m * ldc + n];
+          y *= 1.0f - t * t;
+        }
+        C[(long)m * ldc + n] = y;
+      }
+    }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
     if (!ok) {
-      // after a timeout the MMAs may still run: one more bounded wait on each phase
+      // after a timeout the MMAs may still run: one more bounded wait on each
+      // stage and phase
       if (lane == 0) atomicAdd(&g_mlp_timeouts, 1u);
-      mbar_wait(smem_addr(mbar), 0);
-      mbar_wait(smem_addr(mbar), 1);
+      for (int q = 0; q < 2; q++) {
+        mbar_wait(smem_addr(mbar + q), 0);
+        mbar_wait(smem_addr(mbar + q), 1);
+      }
     }
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcN));
   }
@@ -239,11 +328,23 @@ __global__ void column_sum_kernel(const float* X, long rows, long cols, float* o
   }
 }
 
-__global__ void adam_kernel(float* w, const float* g, float* m, float* v, long n, float lr,
-                            float b1, float b2, float eps, float c1, float c2,
-                            __nv_bfloat16* w_bf16) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// every tensor of the network in one launch: one launch of 4.3 us where ten of
+// 3.3 us each were almost all launch latency
+constexpr int kAdamTensors = 16;
+struct AdamTensors {
+  int count;
+  unsigned first[kAdamTensors + 1];   // first block of each tensor
+  long n[kAdamTensors];
+  float* w[kAdamTensors];
+  const float* g[kAdamTensors];
+  float* m[kAdamTensors];
+  float* v[kAdamTensors];
+  __nv_bfloat16* wb[kAdamTensors];
+};
+
+__device__ __forceinline__ void adam_update(float* w, const float* g, float* m, float* v, long i,
+                                            float lr, float b1, float b2, float eps, float c1,
+                                            float c2, __nv_bfloat16* w_bf16) {
   const float gi = g[i];
   const float mi = b1 * m[i] + (1.f - b1) * gi;
   const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
@@ -252,6 +353,22 @@ __global__ void adam_kernel(float* w, const float* g, float* m, float* v, long n
   const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
   w[i] = wi;
   if (w_bf16) w_bf16[i] = __float2bfloat16_rn(wi);
+}
+
+__global__ void adam_multi_kernel(const __grid_constant__ AdamTensors a, float lr, float b1,
+                                  float b2, float eps, float c1, float c2) {
+  int t = 0;
+  while (t + 1 < a.count && blockIdx.x >= a.first[t + 1]) t++;
+  const long i = (long)(blockIdx.x - a.first[t]) * blockDim.x + threadIdx.x;
+  if (i < a.n[t])
+    adam_update(a.w[t], a.g[t], a.m[t], a.v[t], i, lr, b1, b2, eps, c1, c2, a.wb[t]);
+}
+
+__global__ void adam_kernel(float* w, const float* g, float* m, float* v, long n, float lr,
+                            float b1, float b2, float eps, float c1, float c2,
+                            __nv_bfloat16* w_bf16) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) adam_update(w, g, m, v, i, lr, b1, b2, eps, c1, c2, w_bf16);
 }
 
 __global__ void mse_grad_kernel(const float* Y, const float* T, float* dY, long n, float scale) {
@@ -266,6 +383,21 @@ __global__ void to_bf16_kernel(const float* x, __nv_bfloat16* y, long n) {
 
 int status(cudaError_t e) { return e == cudaSuccess ? NLA3D_OK : NLA3D_ERR_CUDA; }
 
+int launch_gemm(int M, int N, int K, const void* A, int a_bf16, int64_t lda_m, int64_t lda_k,
+                const void* B, int b_bf16, int64_t ldb_k, int64_t ldb_n, float* C, int64_t ldc,
+                const float* bias, int act, const float* Y, float* a_sum, cudaStream_t stream) {
+  if (M == 0 || N == 0) return NLA3D_OK;
+  // 160 KB of shared memory: above the default limit (an attribute of the
+  // function on the current device, not of a stream)
+  const cudaError_t e = cudaFuncSetAttribute(
+      tc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
+  if (e != cudaSuccess) return status(e);
+  const dim3 grid((N + kTcN - 1) / kTcN, (M + kTcM - 1) / kTcM);
+  tc_gemm_kernel<<<grid, kThreads, kTcSmem, stream>>>(M, N, K, A, a_bf16, lda_m, lda_k, B, b_bf16,
+                                                      ldb_k, ldb_n, C, ldc, bias, act, Y, a_sum);
+  return status(cudaGetLastError());
+}
+
 }  // namespace
 
 extern "C" {
@@ -275,11 +407,28 @@ int nla3d_mlp_gemm(int M, int N, int K, const void* A, int a_bf16, int64_t lda_m
                    const float* bias, int act, void* stream) {
   if (M < 0 || N < 0 || K < 0 || (K > 0 && (!A || !B)) || !C || (act != 0 && act != 1))
     return NLA3D_ERR_ARG;
-  if (M == 0 || N == 0) return NLA3D_OK;
-  const dim3 grid((N + kTcN - 1) / kTcN, (M + kTcM - 1) / kTcM);
-  tc_gemm_kernel<<<grid, kThreads, kTcSmem, (cudaStream_t)stream>>>(
-      M, N, K, A, a_bf16, lda_m, lda_k, B, b_bf16, ldb_k, ldb_n, C, ldc, bias, act);
-  return status(cudaGetLastError());
+  return launch_gemm(M, N, K, A, a_bf16, lda_m, lda_k, B, b_bf16, ldb_k, ldb_n, C, ldc, bias, act,
+                     nullptr, nullptr, (cudaStream_t)stream);
+}
+
+int nla3d_mlp_layer_grads(int batch, int n_out, int n_in, const float* dY, const float* X,
+                          float* dW, float* db, void* stream) {
+  if (batch < 0 || n_out < 0 || n_in < 0 || !dW || !db || (batch > 0 && (!dY || !X)))
+    return NLA3D_ERR_ARG;
+  // dW[o,i] = sum_b dY[b,o] X[b,i], db[o] = sum_b dY[b,o]: A = dY^T (rows
+  // contiguous), whose row sums the first column of tiles forms on the way
+  if (n_in == 0) return nla3d_mlp_column_sum(dY ? dY : db, batch, n_out, db, stream);
+  return launch_gemm(n_out, n_in, batch, dY, 0, 1, n_out, X, 0, n_in, 1, dW, n_in, nullptr, 0,
+                     nullptr, db, (cudaStream_t)stream);
+}
+
+int nla3d_mlp_input_grad(int batch, int n_out, int n_in, const float* dY, const uint16_t* W_bf16,
+                         const float* Y, float* dX, void* stream) {
+  if (batch < 0 || n_out < 0 || n_in < 0 || !dX || (batch > 0 && n_out > 0 && (!dY || !W_bf16)))
+    return NLA3D_ERR_ARG;
+  // dX[b,i] = (sum_o dY[b,o] W[o,i]) (1 - Y[b,i]^2), Y the layer's tanh input
+  return launch_gemm(batch, n_in, n_out, dY, 0, n_out, 1, W_bf16, 1, n_in, 1, dX, n_in, nullptr, 0,
+                     Y, nullptr, (cudaStream_t)stream);
 }
 
 int nla3d_mlp_status(uint32_t* timeouts) {
@@ -314,6 +463,36 @@ int nla3d_mlp_adam(float* w, const float* g, float* m, float* v, int64_t n, floa
   adam_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
       w, g, m, v, n, lr, beta1, beta2, eps, c1, c2, reinterpret_cast<__nv_bfloat16*>(w_bf16));
   return status(cudaGetLastError());
+}
+
+int nla3d_mlp_adam_multi(int count, float* const* w, const float* const* g, float* const* m,
+                         float* const* v, const int64_t* n, uint16_t* const* w_bf16, float lr,
+                         float beta1, float beta2, float eps, int step, void* stream) {
+  if (count < 0 || step < 1 || (count > 0 && (!w || !g || !m || !v || !n || !w_bf16)))
+    return NLA3D_ERR_ARG;
+  for (int t = 0; t < count; t++)
+    if (!w[t] || !g[t] || !m[t] || !v[t] || n[t] < 0 || (n[t] + 255) / 256 > 0x7FFFFFFF / kAdamTensors)
+      return NLA3D_ERR_ARG;
+  const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
+  for (int t0 = 0; t0 < count; t0 += kAdamTensors) {
+    AdamTensors a{};
+    a.count = count - t0 < kAdamTensors ? count - t0 : kAdamTensors;
+    for (int t = 0; t < a.count; t++) {
+      a.n[t] = (long)n[t0 + t];
+      a.w[t] = w[t0 + t];
+      a.g[t] = g[t0 + t];
+      a.m[t] = m[t0 + t];
+      a.v[t] = v[t0 + t];
+      a.wb[t] = reinterpret_cast<__nv_bfloat16*>(w_bf16[t0 + t]);
+      a.first[t + 1] = a.first[t] + (unsigned)((n[t0 + t] + 255) / 256);
+    }
+    if (!a.first[a.count]) continue;
+    adam_multi_kernel<<<a.first[a.count], 256, 0, (cudaStream_t)stream>>>(a, lr, beta1, beta2, eps,
+                                                                          c1, c2);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return status(e);
+  }
+  return NLA3D_OK;
 }
 
 int nla3d_mlp_mse_grad(const float* Y, const float* T, float* dY, int64_t n, float scale,

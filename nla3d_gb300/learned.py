@@ -146,6 +146,7 @@ class MLP:
         """X: float32 cuda tensor (B, in).  Returns activations [X, h1, ..., out]."""
         acts = [X]
         L = len(self.W)
+        stream = self.stream
         for l in range(L):
             out_dim, in_dim = self.W[l].shape
             Y = self.torch.empty((X.shape[0], out_dim), dtype=self.torch.float32, device=self.dev)
@@ -153,7 +154,7 @@ class MLP:
             self._ck(self.lib.nla3d_mlp_gemm(X.shape[0], out_dim, in_dim, acts[-1].data_ptr(), 0,
                                              in_dim, 1, self.Wb[l].data_ptr(), 1, 1, in_dim,
                                              Y.data_ptr(), out_dim, self.b[l].data_ptr(),
-                                             1 if l < L - 1 else 0, self.stream))
+                                             1 if l < L - 1 else 0, stream))
             acts.append(Y)
         return acts
 
@@ -162,28 +163,24 @@ class MLP:
         torch = self.torch
         L = len(self.W)
         B = dOut.shape[0]
+        stream = self.stream
         gW, gb = [None] * L, [None] * L
         d = dOut
         for l in range(L - 1, -1, -1):
             out_dim, in_dim = self.W[l].shape
-            if l < L - 1:
-                self._ck(self.lib.nla3d_mlp_tanh_backward(acts[l + 1].data_ptr(), d.data_ptr(),
-                                                          d.numel(), self.stream))
             dW = torch.empty((out_dim, in_dim), dtype=torch.float32, device=self.dev)
-            # dW[o,i] = sum_b d[b,o] X[b,i]: A = d^T (A[o,b] at b*out + o), B = X (B[b,i] at b*in + i)
-            self._ck(self.lib.nla3d_mlp_gemm(out_dim, in_dim, B, d.data_ptr(), 0, 1, out_dim,
-                                             acts[l].data_ptr(), 0, in_dim, 1, dW.data_ptr(), in_dim,
-                                             None, 0, self.stream))
             db = torch.empty(out_dim, dtype=torch.float32, device=self.dev)
-            self._ck(self.lib.nla3d_mlp_column_sum(d.data_ptr(), B, out_dim, db.data_ptr(),
-                                                   self.stream))
+            # dW[o,i] = sum_b d[b,o] X[b,i], db[o] = sum_b d[b,o]
+            self._ck(self.lib.nla3d_mlp_layer_grads(B, out_dim, in_dim, d.data_ptr(),
+                                                    acts[l].data_ptr(), dW.data_ptr(),
+                                                    db.data_ptr(), stream))
             gW[l], gb[l] = dW, db
             if l > 0:
                 dX = torch.empty((B, in_dim), dtype=torch.float32, device=self.dev)
-                # dX[b,i] = sum_o d[b,o] W[o,i]: A = d (A[b,o] at b*out + o), B = W (B[o,i] at o*in + i)
-                self._ck(self.lib.nla3d_mlp_gemm(B, in_dim, out_dim, d.data_ptr(), 0, out_dim, 1,
-                                                 self.Wb[l].data_ptr(), 1, in_dim, 1, dX.data_ptr(),
-                                                 in_dim, None, 0, self.stream))
+                # dX[b,i] = sum_o d[b,o] W[o,i], through the tanh that made acts[l]
+                self._ck(self.lib.nla3d_mlp_input_grad(B, out_dim, in_dim, d.data_ptr(),
+                                                       self.Wb[l].data_ptr(), acts[l].data_ptr(),
+                                                       dX.data_ptr(), stream))
                 d = dX
         return gW, gb
 
@@ -196,14 +193,20 @@ class MLP:
 
     def adam(self, gW, gb, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.step_count += 1
-        for l in range(len(self.W)):
-            mW, vW, mb, vb = self.state[l]
-            self._ck(self.lib.nla3d_mlp_adam(self.W[l].data_ptr(), gW[l].data_ptr(), mW.data_ptr(),
-                                             vW.data_ptr(), self.W[l].numel(), lr, b1, b2, eps,
-                                             self.step_count, self.Wb[l].data_ptr(), self.stream))
-            self._ck(self.lib.nla3d_mlp_adam(self.b[l].data_ptr(), gb[l].data_ptr(), mb.data_ptr(),
-                                             vb.data_ptr(), self.b[l].numel(), lr, b1, b2, eps,
-                                             self.step_count, None, self.stream))
+        w = self.W + self.b
+        g = list(gW) + list(gb)
+        m = [t[0] for t in self.state] + [t[2] for t in self.state]
+        v = [t[1] for t in self.state] + [t[3] for t in self.state]
+        n = len(w)
+
+        def pointers(ts):
+            return (ctypes.c_void_p * n)(*[t.data_ptr() for t in ts])
+
+        wb = (ctypes.c_void_p * n)(*[t.data_ptr() for t in self.Wb])
+        sizes = (ctypes.c_int64 * n)(*[t.numel() for t in w])
+        self._ck(self.lib.nla3d_mlp_adam_multi(n, pointers(w), pointers(g), pointers(m),
+                                               pointers(v), sizes, wb, lr, b1, b2, eps,
+                                               self.step_count, self.stream))
 
     # ---- training on numpy data ----
     def fit(self, X, Y, epochs=200, batch=256, lr=1e-3, seed=0, log=None):
