@@ -33,27 +33,25 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-# FP64 flop per SOLID81 element of the algorithm the kernel runs (8 Gauss
-# points x 3628: kinematics 189, material + S + wDd 436, -wFS / w cof F 96,
-# tangent tensor A 513, h_a = A^T G_a for the 6 blocks i <= k 720, F_u + K_up
-# 288, the 231 accumulated K_uu entries 1386; plus 96, and 483 for the 69
-# entries of node 7's column and block derived from sum_b G_b = 0).  The
-# executed FP64 instruction counters of one ncu capture give 29,467 per
-# element (2 DFMA + DMUL + DADD); that figure is used.  The Bh^T D Bh formulation costs 69,072
-# (8 x 8634) for the same element.
-FLOP_PER_ELEM = 29467
+# FP64 flop per SOLID81 element the FP64 kernel executes (Mooney-Rivlin;
+# 4,688 DFMA + 3,044 DADD + 1,464 DMUL thread instructions per element in one
+# ncu capture; 2 DFMA + DADD + DMUL).  The kernel works in the element's
+# reference coordinates and sums over the Gauss points by Walsh-Hadamard
+# transforms; the Bh^T D Bh formulation costs 69,072 (8 x 8634) for the same
+# element.
+FLOP_PER_ELEM = 13884
 FLOP_PER_ELEM_BTDB = 69072
-# FP64 instructions per element in the same capture (12,744 DFMA + 3,096
-# DMUL + 883 DADD): a DMUL or DADD takes the pipe as long as a DFMA for half
-# the flops, so the pipe's instruction rate is the tighter ceiling.
-FP64_INSTR_PER_ELEM = 16723
-# DRAM bytes per element of solid81_kernel<double> and of the K gather in one
+# FP64 instructions per element in the same capture: a DMUL or DADD takes the
+# pipe as long as a DFMA for half the flops, so the pipe's instruction rate is
+# the tighter ceiling.
+FP64_INSTR_PER_ELEM = 9196
+# DRAM bytes per element of solid81_fp64_kernel and of the K gather in one
 # ncu capture of a 40^3 block (64,000 elements, 9,675,406 K slots), used to
 # scale the traffic to the measured launch; the element kernel's writes are a
 # lower bound there (L2 still held part of them when the kernel ended).
-DRAM_BYTES_PER_ELEM_SOLID81 = (108.598016e6 + 122.938624e6) / 64000
+DRAM_BYTES_PER_ELEM_SOLID81 = (51.446784e6 + 118.781952e6) / 64000
 DRAM_BYTES_PER_ELEM_GATHER_K = (301.560064e6 + 62.591488e6) / 64000
-# Executed arithmetic per element of solid81_kernel<float> (mixed), from the
+# Executed arithmetic per element of solid81_mixed_kernel, from the
 # instruction counters of one ncu capture of a 40^3 block (64,000 elements):
 # FP32 2 FFMA + FADD + FMUL and FP64 2 DFMA + DADD + DMUL per element.
 MIXED_FP32_FLOP_PER_ELEM = 67044
@@ -654,7 +652,7 @@ def run_ours(args):
         issue_peak = sms * 4 * clk_mhz * 1e6
         ai = MIXED_WARP_INSTR_PER_ELEM * mesh.n_elems / mel
         mixed["roofline"] = {
-            "bound": "issue", "kernel": "solid81_kernel<float>",
+            "bound": "issue", "kernel": "solid81_mixed_kernel",
             "achieved": ai / 1e9, "peak": issue_peak / 1e9, "unit": "G warp-instr/s",
             "frac": ai / issue_peak,
             "fp32": {"achieved": a32 / 1e12, "peak": fp32_peak / 1e12, "unit": "TFLOP/s",
@@ -700,7 +698,7 @@ def run_ours(args):
                      "traffic": DRAM_BYTES_PER_ELEM_SOLID81 * mesh.n_elems,
                      "traffic_source": "ncu dram bytes of a 64,000-element launch, "
                                        "scaled by elements",
-                     "kernel": "solid81_kernel<double>",
+                     "kernel": "solid81_fp64_kernel",
                      "algorithmic": f"{FLOP_PER_ELEM} FP64 flop/element x {mesh.n_elems}",
                      "btdb_equivalent_tflops": FLOP_PER_ELEM_BTDB * mesh.n_elems
                      / (elem_ms * 1e-3) / 1e12,

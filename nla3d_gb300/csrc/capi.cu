@@ -6,7 +6,8 @@
 // pattern, K and F (each is one reference FEStorage); on the device they are
 // concatenated so that one launch of each kernel assembles all of them:
 //
-//   Gt      24 x 8E  double  dN/dX per Gauss point, structure of arrays
+//   geo     10 x 8E  double  element geometry, structure of arrays (FP64; mixed
+//                            contexts hold Gdf, dN/dX as 24 x 8E float pairs)
 //   wdet    8E       double  Gauss weight * det J
 //   conn    8E       uint32  node ids, global (mesh node offset added)
 //   node_eq 4N       uint32  equations of UX, UY, UZ (+ pad), global 1-based
@@ -64,7 +65,7 @@ struct nla3d_ctx {
   uint32_t* d_node_eq3 = nullptr;
   uint32_t* d_p_eq = nullptr;
   double* d_eparams = nullptr;
-  double* d_Gt = nullptr;
+  double* d_geo = nullptr;
   double* d_wdet = nullptr;
   double* d_U = nullptr;
   double* d_Ustate = nullptr;
@@ -319,7 +320,7 @@ cudaError_t enqueue_elements(nla3d_ctx* c, uint32_t e0, uint32_t e1) {
     a.e_begin = e0;
     a.n_elems = e1;
     a.n_total = (uint32_t)c->E();
-    a.Gt = c->d_Gt;
+    a.geo = c->d_geo;
     a.wdet = c->d_wdet;
     a.conn = c->d_conn;
     a.node_eq3 = c->d_node_eq3;
@@ -330,6 +331,7 @@ cudaError_t enqueue_elements(nla3d_ctx* c, uint32_t e0, uint32_t e1) {
     a.mat_id = m0.mat_id;
     for (int i = 0; i < 5; i++) a.mc[i] = m0.mat_c[i];
     a.kbulk = bulk_of(m0);
+    a.inv_kb = 1.0 / a.kbulk;
     a.elem_mesh = c->uniform_material ? nullptr : c->d_elem_mesh;
     a.mesh_mat = c->uniform_material ? nullptr : c->d_mesh_mat;
     a.kpos = c->layout ? c->d_kpos : nullptr;
@@ -342,7 +344,6 @@ cudaError_t enqueue_elements(nla3d_ctx* c, uint32_t e0, uint32_t e1) {
       a.wdf = c->d_wdf;
       for (int i = 0; i < 5; i++) a.mcd[i] = split_pair(m0.mat_c[i]);
       a.inv_kbd = split_pair(1.0 / a.kbulk);
-      a.inv_kb = 1.0 / a.kbulk;
       a.mesh_mat_df = c->uniform_material ? nullptr : c->d_mesh_mat_df;
     }
     e = launch_solid81_shaped(a, c->precision == NLA3D_PREC_MIXED, c->shape, c->stream);
@@ -969,15 +970,15 @@ int nla3d_init_solution_data(nla3d_ctx* c) {
   CK(cudaMemsetAsync(c->d_status, 0, sizeof(ElementStatus), c->stream));
   CK(cudaMemsetAsync(&c->d_status->first, 0xFF, sizeof(uint32_t), c->stream));
   if (c->hm[0].etype == NLA3D_SOLID81) {
-    // FP64 contexts keep dN/dX as doubles, mixed ones as float pairs only
+    // FP64 contexts keep the geometry of their kernel, mixed ones dN/dX as float pairs
     if (mixed_solid) {
       CK(dalloc(c, &c->d_Gdf, 24 * 8 * E));
       CK(dalloc(c, &c->d_wdf, 8 * E));
     } else {
-      CK(dalloc(c, &c->d_Gt, 24 * 8 * E));
+      CK(dalloc(c, &c->d_geo, kSolidGeo * 8 * E));
     }
     CK(dalloc(c, &c->d_wdet, 8 * E));
-    JacobianArgs ja{(uint32_t)E, c->d_xyz, c->d_conn, c->d_Gt, c->d_wdet, c->d_status,
+    JacobianArgs ja{(uint32_t)E, c->d_xyz, c->d_conn, c->d_geo, c->d_wdet, c->d_status,
                     c->d_Gdf, c->d_wdf};
     CK(launch_solid81_jacobian(ja, c->stream));
     c->launches++;

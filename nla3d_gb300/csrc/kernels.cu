@@ -13,18 +13,16 @@
 //   Kup_a  +=  w * (cof(F) G_a)           ( = w/2 B^T J C^-1, since J F C^-1 = cof F )
 //   Fp     += -(J - 1 - p/k) w ;  Kpp += -w / k
 // Writing Bh out, both Kuu terms are one contraction with a symmetric 9x9
-// tensor per Gauss point:
+// tensor per Gauss point,
 //   Kuu(a,i; b,k) += sum_{L,N} G_aL A[iL][kN] G_bN,
-//   A[iL][kN] = sum_{J,M} F_iJ wDd'[(JL)][(MN)] F_kM + delta_ik w S_LN,
-// so one Gauss point costs 45 entries of A (about 300 FMA), h_a[ik] = A^T G_a
-// per node and 3 FMA per Kuu entry, instead of 6 + the geometric term per
-// entry and D Bh per node.  Since A is symmetric, K(a,i; b,k) = h_b[ki] . G_a
-// as well, so h is formed only for i <= k (6 of the 9 blocks, 54 FMA per
-// node) and the entries with i > k (off-diagonal node blocks only) read
-// h_b[ki] and G_a.  These are the reference's products with the
-// structural zeros of B, B_NL and Omega removed and the sums regrouped; they
-// agree with the reference to rounding (the tests bound the difference at
-// 1e-12 relative).
+//   A[iL][kN] = sum_{J,M} F_iJ wDd'[(JL)][(MN)] F_kM + delta_ik w S_LN.
+// The mixed kernel forms A and h_a[ik] = A^T G_a per node (i <= k: A is
+// symmetric) and 3 FMA per Kuu entry and Gauss point.  The FP64 kernel writes
+// the same contraction in the element's reference coordinates and sums over
+// the Gauss points first (see solid81_fp64_kernel).  These are the
+// reference's products with the structural zeros of B, B_NL and Omega removed
+// and the sums regrouped; they agree with the reference to rounding (the
+// tests bound the difference at 1e-12 relative).
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -43,67 +41,18 @@ constexpr int kKuuPerElem = 300;
 constexpr int kOwned = (kEPW * kKuuPerElem + 31) / 32;  // Kuu entries per lane (38)
 constexpr double kGaussA = 0.5773502691896258;        // isoparametric.h:127
 
-// Kuu entry t (assemble3 order, SOLID81.h:62-74) -> (a, i, b, k) packed.
-__constant__ uchar4 c_kuu_entry[kKuuPerElem];
-
-// FP64 kernel: the shape gradients of an element sum to zero at every Gauss
-// point (sum_b G_b = J^-1 sum_b dN_b/dxi = 0), so K(a,i; 7,k) = sum_g h_a . G_7
-// = -sum_{b<7} K(a,i; b,k), and likewise h_7 = -sum_{a<7} h_a.  The 63
-// entries of node 7's column (a < 7, all nine (i,k)) are formed from the
-// accumulated ones after the Gauss-point loop (7 adds each, in a fixed
-// order), and then the 6 of node 7's own block, K(7,i; 7,k) = -sum_{a<7}
-// K(a,i; 7,k), from those: 231 of the 300 entries take 24 FMAs each inside
-// the loop, the minimum for blocks whose rows and columns sum to zero.  The
-// formed entries differ from the direct sums by rounding only
-// (|sum_b G_b| ~ eps |G|).
-constexpr int kKuuColumn = 63;                                       // first pass
-constexpr int kKuuCorner = 6;                                        // second pass
-constexpr int kKuuDerived = kKuuColumn + kKuuCorner;                 // 69
-constexpr int kKuuOwned = kKuuPerElem - kKuuDerived;                 // 231
-constexpr int kOwned64 = (kEPW * kKuuOwned + 31) / 32;               // per lane (29)
-// FP64 kernel block header: ownership words, stage positions, derived table
-constexpr size_t kHead64Bytes =
-    (sizeof(uint32_t) * kOwned64 * 32 + sizeof(uint16_t) * kOwned64 * 32 +
-     sizeof(uint16_t) * kKuuDerived * 8 + 15) / 16 * 16;
-__constant__ uint16_t c_kuu_owned[kKuuOwned];            // owned m -> assemble3 t
-__constant__ uint16_t c_kuu_derived[kKuuDerived * 8];    // target t, then its 7 sources
-
-// Mixed kernel: position in assemble3 order of the Kuu entry that
-// D[(i,k), a, b] = sum h_a[ik] . G_b (i <= k) stands for, at [(a * 6 +
+// Position in assemble3 order (SOLID81.h:62-74) of the Kuu entry that
+// D[(i,k), a, b] = K(a,i; b,k) (i <= k) stands for, at [(a * 6 +
 // hblock(i,k)) * 8 + b]: K(a,i; b,k) when a <= b, K(b,k; a,i) when a > b;
 // 0xFFFF where a > b and i == k (the same entry as D[(i,i), b, a]).
 constexpr int kDpos = 8 * 6 * 8;
 constexpr size_t kDposBytes = kDpos * sizeof(uint16_t);
 __constant__ uint16_t c_dpos[kDpos];
 
-// -w F S: FP64, or a float pair (hi, lo) in the mixed kernel
-template <typename TT>
-struct ResidualType {
-  using type = double;
-};
-template <>
-struct ResidualType<float> {
-  using type = float2;
-};
-
-// FP64 kernel: stride of one (i, k) block of h (3 N x 32 slots) in the warp
-// scratch.
-constexpr int kHStride = 96;
-
 // the (i, k) blocks of h that are formed: i <= k, packed (6 blocks)
 __host__ __device__ constexpr int hblock(int i, int k) {  // i <= k
   return 3 * i - (i * (i - 1)) / 2 + (k - i);
 }
-
-template <typename TT>
-struct WarpSmem {
-  typename ResidualType<TT>::type wP[9][32];  // per (element q, Gauss point g): -w F S
-  TT wCof[9][32];      //  w cof(F)
-  TT A[45][32];        //  symmetric 9x9 tangent tensor A[iL][kN], packed upper
-  TT H[6 * kHStride];  // per (element q, node a) at the current Gauss point:
-                       //  h_a[ik][N], i <= k, at hblock(i,k) * kHStride + 32 N + slot
-  TT G[3][32];         //  G_a
-};
 
 // Mixed kernel: -w F S (float pairs) and w cof F (FP64: the pressure
 // coupling K_up keeps FP64) are only needed between phase 1 and the residual
@@ -112,8 +61,7 @@ struct WarpSmem {
 // (element q, Gauss point g) they sit at slot g * 4 + q, so the pass's
 // broadcast reads of one Gauss point hit four consecutive words.  h stays in
 // registers (each lane keeps its own node's).
-template <>
-struct WarpSmem<float> {
+struct MixedSmem {
   float A[45][32];
   union {
     float stage[4 * 300];   // the quad's Kuu entries in assemble3 order, for the write
@@ -532,53 +480,616 @@ __device__ __forceinline__ void material_mixed(int mat_id, const float2* mcd, co
                                    sI, wD);
 }
 
-template <typename TT, int WPB>
+// ---------------------------------------------------------------------------
+// FP64 kernel.  The FP64 pipe is what bounds it (1/64 of the FP32 rate: about
+// 59 clocks per warp instruction and scheduler), so the algebra is arranged
+// for the fewest FP64 instructions:
+//
+//  - Everything is written in the element's reference coordinates xi_p, where
+//    the shape gradients at the 2 x 2 x 2 Gauss points are constants: with
+//    sigma_d = +-1 the sign of coordinate d at a node b or a Gauss point g and
+//    s = 1/sqrt(3),
+//      dN_b/dxi_p (g) = 1/8 sum_{P not containing p} s^|P| phi_{P+p}(b) chi_P(g),
+//    phi_S(b), chi_S(g) = prod_{d in S} sigma_d (P, S subsets of the three
+//    coordinates).  The material works on covariant components: with F_ip =
+//    dx_i/dxi_p, the metric g^{pq} = (dxi_p/dX . dxi_q/dX) in the place of I,
+//    V = F^-T, FI = F g, b = FI F^T:
+//      I1 = FI : F,  C^-1 -> V^T V,  J = det F / det(dX/dxi),
+//      F A = FI - I1/3 V,  F B = I1 FI - b FI - 2 I2/3 V,
+//      w F S = ko1 F A + ko2 F B + p J V,  w cof(F) dN/dX -> cof(F) dN/dxi,
+//    and the tangent tensor is a sum of products of those 3 x 3 matrices
+//      A[ip][kq] = V_ip X_kq + X_ip V_kq - sIIt/2 V_iq V_kp + k11 FA_ip FA_kq
+//                  + sI (FI_ip FI_kq - FI_iq FI_kp / 2 - b_ik g^{pq} / 2)
+//                  + delta_ik (S^{pq} - sIIt/2 C^-1^{pq})       (times w),
+//    X = -k1 FA - k2 FB + c0/2 V: 2 or 3 FMA per entry instead of 6 and the
+//    21 Voigt entries of D.
+//  - Sum over the Gauss points: the products chi_P chi_Q make it a
+//    Walsh-Hadamard transform of each tensor entry over the 8 points (24 adds
+//    each for 45 entries of A, 9 of w F S, 9 of cof F), instead of h_a and 3
+//    FMA per Kuu entry and Gauss point.
+//  - Kuu(a,i; b,k) is then a sum of those over the (P, p), (Q, q) of both
+//    sides: for each of the 7 modes P+p, seven sums over the modes Q+q and
+//    their butterfly to the 8 nodes b (22 adds / FMA), then for each b the
+//    butterfly over the modes to the 8 nodes a.
+//  9,196 FP64 instructions per element (Mooney-Rivlin, counted by ncu) where
+//  the form with h_a and 231 accumulated entries took 16,723.  Element launch
+//  at 1e6 elements, Mooney-Rivlin: 28.0 -> 17.3 ms; at 216,000: 3.96 ms, and
+//  3.05 ms Neo-Hookean.  The FP64 pipe is 87% busy; what is left is the two
+//  warps per scheduler that shared memory allows waiting at the exchanges
+//  (short scoreboard).
+//
+// One warp per four elements.  Lane = (element, node) for the displacements'
+// butterfly to modes (exact differences to node 0 first), (element, Gauss
+// point) for the material, (tensor entry, element) for the transforms, then
+// (block (i, k), element) and (element, node b).  All exchange is through the
+// warp's shared memory (25 KB: eight warps per SM).
+
+// warp scratch, in doubles: 63 tensor rows of 4 elements x (8 points + pad);
+// the mode-to-node sums T reuse the rows of w F S and cof F, the finished
+// entries' stage the rows of A
+constexpr int kFRow = 36, kFElem = 9;
+constexpr int kFRowsA = 45;                      // A by (i, k) block: 6 or 9 entries
+constexpr int kFRowP = kFRowsA, kFRowCof = kFRowsA + 9, kFRows = kFRowsA + 18;
+// T: for each mode of the a side, 24 (block, element) x 8 nodes (+ pad).  The
+// one-coordinate modes come last: they are written while w F S and cof F,
+// which the four other blocks overwrite, are still read
+constexpr int kFTMode = 24 * 9;
+constexpr int kFT = kFRowsA * kFRow;
+__host__ __device__ constexpr int f64_T(int mode) {
+  return kFT + kFTMode * (mode == 3 ? 0 : mode == 5 ? 1 : mode == 6 ? 2 : mode == 7 ? 3
+                          : mode == 1 ? 4 : mode == 2 ? 5 : 6);
+}
+constexpr int kFModes = kFRows * kFRow;          // modal positions: 3 x 32, before T exists
+constexpr int kFWarp = kFT + 7 * kFTMode;
+constexpr size_t kHead64Bytes = (kDposBytes + sizeof(uint16_t) * kFRows + 15) / 16 * 16;
+static_assert(kFModes + 96 <= kFWarp && 4 * kKuuPerElem <= kFT, "scratch layout");
+static_assert(kFT + 4 * kFTMode >= kFRows * kFRow, "one-coordinate modes beyond the F rows");
+
+// first A row of block (i, k), i <= k (hblock order), and the entry within it
+__device__ __forceinline__ constexpr int f64_block_row(int ik) {
+  return ik == 0 ? 0 : ik == 1 ? 6 : ik == 2 ? 15 : ik == 3 ? 24 : ik == 4 ? 30 : 39;
+}
+__host__ __device__ constexpr int sym3(int p, int q) {
+  return p <= q ? 3 * p - p * (p - 1) / 2 + (q - p) : 3 * q - q * (q - 1) / 2 + (p - q);
+}
+// node with the sign bits `mask` (bit d set: +1 in coordinate d), and back
+__host__ __device__ constexpr int hex_corner(int mask) {
+  return (mask & 2) ? (mask ^ 1) : mask;
+}
+
+// The butterfly of an element's eight lanes from corner values to shape modes
+// (lane sub holds corner hex_corner(sub), then mode sub; not divided by 8),
+// and dx_i/dxi_p at the lane's Gauss point from the seven modes m (stride ld).
+// The geometry set-up and the element kernel share them, with every rounding
+// spelled out, so that an element at rest finds det F = w bit for bit and
+// det F - w loses nothing to a small strain.
+__device__ __forceinline__ double corners_to_mode(double v, int sub) {
+  v -= __shfl_sync(0xFFFFFFFFu, v, threadIdx.x & 24);
+#pragma unroll
+  for (int d = 1; d < 8; d <<= 1) {
+    const double o = __shfl_xor_sync(0xFFFFFFFFu, v, d);
+    v = (sub & d) ? __dsub_rn(v, o) : __dadd_rn(v, o);
+  }
+  return v;
+}
+
+struct GaussSigns {
+  double x, y, z, xy, xz, yz;   // sigma_d / sqrt(3), and their products
+};
+
+__device__ __forceinline__ GaussSigns gauss_signs(int g) {
+  GaussSigns s;
+  s.x = (g & 1) ? kGaussA : -kGaussA;
+  s.y = (g & 2) ? kGaussA : -kGaussA;
+  s.z = (g & 4) ? kGaussA : -kGaussA;
+  s.xy = __dmul_rn(s.x, s.y);
+  s.xz = __dmul_rn(s.x, s.z);
+  s.yz = __dmul_rn(s.y, s.z);
+  return s;
+}
+
+__device__ __forceinline__ void mode_gradient(const double m[8], const GaussSigns& s, double F[3]) {
+  F[0] = fma(s.yz, m[7], fma(s.z, m[5], fma(s.y, m[3], m[1])));
+  F[1] = fma(s.xz, m[7], fma(s.z, m[6], fma(s.x, m[3], m[2])));
+  F[2] = fma(s.xy, m[7], fma(s.y, m[6], fma(s.x, m[5], m[4])));
+}
+
+__device__ __forceinline__ double minor2(double a, double b, double c, double d) {
+  return fma(a, b, -__dmul_rn(c, d));   // a b - c d
+}
+
+// cof F (F^-T det F) and det F
+__device__ __forceinline__ double cofactors(const double F[9], double cof[9]) {
+  cof[0] = minor2(F[4], F[8], F[5], F[7]);
+  cof[1] = minor2(F[5], F[6], F[3], F[8]);
+  cof[2] = minor2(F[3], F[7], F[4], F[6]);
+  cof[3] = minor2(F[2], F[7], F[1], F[8]);
+  cof[4] = minor2(F[0], F[8], F[2], F[6]);
+  cof[5] = minor2(F[1], F[6], F[0], F[7]);
+  cof[6] = minor2(F[1], F[5], F[2], F[4]);
+  cof[7] = minor2(F[2], F[3], F[0], F[5]);
+  cof[8] = minor2(F[0], F[4], F[1], F[3]);
+  return fma(F[2], cof[2], fma(F[1], cof[1], __dmul_rn(F[0], cof[0])));
+}
+
+// v / 8, by the exponent (an integer subtraction, not an FP64 multiply)
+__device__ __forceinline__ double eighth(double v) {
+  const int hi = __double2hiint(v);
+  if ((hi & 0x7FF00000) <= (3 << 20) || (hi & 0x7FF00000) == 0x7FF00000) return 0.125 * v;
+  return __hiloint2double(hi - (3 << 20), __double2loint(v));
+}
+
+// J^(-1/3): the float estimate x0 improved by one third-order Householder step
+// for x^-3 = J: with e = 1 - J x0^3, J^(-1/3) = x0 (1 - e)^(-1/3)
+// = x0 (1 + e/3 + 2 e^2/9 + O(e^3)), |e| < 2^-20; rcbrt() outside the floats'
+// comfortable range
+__device__ __forceinline__ double inv_cbrt(double J) {
+  if (!(J > 1e-30 && J < 1e30)) return rcbrt(J);
+  const double x0 = (double)rcbrtf((float)J);
+  const double e = fma(-J, x0 * x0 * x0, 1.0);
+  return fma(x0 * e, fma(2.0 / 9.0, e, 1.0 / 3.0), x0);
+}
+
+// o[mask of b] = sum over the modes of c_mode phi_mode(b) M_mode, c = 1, s, s^2
+// for one, two, three coordinates
+__device__ __forceinline__ void modes_to_nodes(const double M[8], double o[8]) {
+  constexpr double s = kGaussA;
+#pragma unroll
+  for (int x = 0; x < 2; x++) {
+    const double sx = x ? s : -s;
+    const double p2 = fma(sx, M[3], M[2]), p4 = fma(sx, M[5], M[4]), p6 = fma(sx, M[7], M[6]);
+    const double m1 = x ? M[1] : -M[1];
+    const double xy[2] = {m1 - p2, m1 + p2};
+    const double z[2] = {fma(-s, p6, p4), fma(s, p6, p4)};
+#pragma unroll
+    for (int y = 0; y < 2; y++) {
+      o[x + 2 * y] = xy[y] - z[y];
+      o[x + 2 * y + 4] = xy[y] + z[y];
+    }
+  }
+}
+
+template <int WPB>
 __global__ void __launch_bounds__(WPB * 32)
-    solid81_kernel(const Solid81Args a) {
+    solid81_fp64_kernel(const Solid81Args a) {
   if (a.skip && *a.skip) return;
-  constexpr bool kMixed = std::is_same<TT, float>::value;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  // block header: the FP64 kernel's Kuu ownership words, the mixed kernel's
-  // D -> assemble3 position table
-  uint32_t* dec = reinterpret_cast<uint32_t*>(smem_raw);  // [kOwned64][32]
-  // FP64 kernel: each owned entry's stage position, and the derived entries'
-  // table (per-lane indices: shared memory, not the constant cache)
-  uint16_t* opos = reinterpret_cast<uint16_t*>(dec + kOwned64 * 32);   // [kOwned64][32]
-  uint16_t* dtab = opos + kOwned64 * 32;                               // [kKuuDerived][8]
   uint16_t* dpos = reinterpret_cast<uint16_t*>(smem_raw);  // [kDpos]
-  constexpr size_t kHead = kMixed ? kDposBytes : kHead64Bytes;
-  WarpSmem<TT>* sm = reinterpret_cast<WarpSmem<TT>*>(smem_raw + kHead) + (threadIdx.x >> 5);
+  // first double of the tensor rows: the 27 entries with p != q, then the 36
+  // that need four characters, p = 0, 1, 2 in turn
+  uint16_t* rows = dpos + kDpos;
+  double* sm = reinterpret_cast<double*>(smem_raw + kHead64Bytes) + kFWarp * (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  for (int v = threadIdx.x; v < kDpos; v += blockDim.x) dpos[v] = c_dpos[v];
+  if (threadIdx.x < 6) {
+    const int ik = threadIdx.x;
+    const bool diag = ik == 0 || ik == 3 || ik == 5;
+    // entries p != q before this block: 3 per i = k block, 6 per i < k block
+    int n = ik == 0 ? 0 : ik == 1 ? 3 : ik == 2 ? 9 : ik == 3 ? 15 : ik == 4 ? 18 : 24;
+    for (int p = 0; p < 3; p++)
+      for (int r = diag ? p : 0; r < 3; r++) {
+        const int row = kFRow * (f64_block_row(ik) + (diag ? sym3(p, r) : 3 * p + r));
+        if (p == r) rows[27 + 3 * ik + p] = (uint16_t)row;
+        else rows[n++] = (uint16_t)row;
+      }
+  } else if (threadIdx.x < 24) {
+    const int c = threadIdx.x - 6;   // the 18 rows of w F S and cof F
+    rows[27 + 18 + c] = (uint16_t)(kFRow * (kFRowP + c));
+  }
+  __syncthreads();
+
+  const uint32_t E = a.n_elems;  // end of this launch's element range
+  const uint64_t E8 = (uint64_t)(a.n_total ? a.n_total : E) * 8;
+  const uint64_t n_quads = (E + kEPW - 1) / kEPW;
+  const uint64_t warp_global = (uint64_t)blockIdx.x * WPB + (threadIdx.x >> 5);
+  const uint64_t warp_stride = (uint64_t)gridDim.x * WPB;
+  const int q = lane >> 3, sub = lane & 7;
+  const GaussSigns sg = gauss_signs(sub);
+
+  for (uint64_t quad = a.e_begin / kEPW + warp_global; quad < n_quads; quad += warp_stride) {
+    const uint32_t e0 = (uint32_t)(quad * kEPW);
+    const uint32_t e = e0 + q;
+    const bool valid = e < E;
+    const uint32_t ec = valid ? e : E - 1;
+    const uint64_t tg = (uint64_t)ec * 8 + sub;
+
+    // ---- modal positions, lane = (element, node), then mode ----
+    double xm[3];
+    bool moved = false;   // this mode's displacement is not exactly zero
+#pragma unroll
+    for (int i = 0; i < 3; i++) xm[i] = __ldg(a.geo + (7 + i) * E8 + tg);
+    if (a.have_state) {
+      const uint32_t nid = __ldg(a.conn + (uint64_t)ec * 8 + hex_corner(sub));
+      const uint4 eq = __ldg(reinterpret_cast<const uint4*>(a.node_eq3) + (nid - 1));
+      const double u[3] = {a.U_state[eq.x - 1], a.U_state[eq.y - 1], a.U_state[eq.z - 1]};
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const double um = corners_to_mode(u[i], sub);
+        moved |= um != 0.0;
+        xm[i] = fma(0.125, um, xm[i]);   // mode 0 (the translation) is not read
+      }
+    }
+    // an element at rest (or translated): F = I, so F A = F B = 0 and I1 = 3
+    // hold exactly, as the reference finds them (and J = 1, from det F = w);
+    // rounding would leave ~eps in their place and a residual that should
+    // vanish would not
+    const bool rest = ((__ballot_sync(0xFFFFFFFFu, moved) >> (8 * q)) & 0xFFu) == 0;
+#pragma unroll
+    for (int i = 0; i < 3; i++) sm[kFModes + 32 * i + lane] = xm[i];
+    const double w = __ldg(a.wdet + tg), rw = __ldg(a.geo + 6 * E8 + tg);
+    double g[6];
+#pragma unroll
+    for (int c = 0; c < 6; c++) g[c] = __ldg(a.geo + c * E8 + tg);
+    const double pc = a.U_cur[a.p_eq[ec] - 1];
+    const double ps = a.have_state ? a.U_state[a.p_eq[ec] - 1] : 0.0;
+    int mat_id = a.mat_id;
+    const double* mc = a.mc;
+    double inv_kb = a.inv_kb;
+    if (a.elem_mesh) {
+      const double* mm = a.mesh_mat + 8 * (uint64_t)__ldg(a.elem_mesh + ec);
+      mat_id = (int)mm[0];
+      mc = mm + 1;
+      inv_kb = mm[7];
+    }
+    __syncwarp();
+
+    // ---- material, lane = (element, Gauss point) ----
+    double Fp_part, Kpp_part;
+    {
+      double F[9], cof[9];
+#pragma unroll
+      for (int i = 0; i < 3; i++) mode_gradient(sm + kFModes + 32 * i + 8 * q, sg, F + 3 * i);
+      const double detF = cofactors(F, cof);
+#pragma unroll
+      for (int c = 0; c < 9; c++) sm[(kFRowCof + c) * kFRow + kFElem * q + sub] = cof[c];
+      // J = det F / w > 0 as sqrt(det C) gives it; an inverted element (det F
+      // <= 0) is flagged
+      const double dw = fabs(detF) - w;   // (J - 1) w
+      const double J = fma(dw, rw, 1.0);
+      const bool bad = valid && !(J > 0.0 && isfinite(J) && detF > 0.0 && w > 0.0);
+      const unsigned ballot = __ballot_sync(0xFFFFFFFFu, bad);
+      if (sub == 0 && ((ballot >> (q * 8)) & 0xFFu)) flag_element(a.status, e + 1);
+      Kpp_part = -inv_kb * w;
+      Fp_part = fma(-pc, Kpp_part, -dw);   // -(J - 1 - p / K) w
+      const double rc = inv_cbrt(J);
+      const double pp = rc * rc;       // J^(-2/3)
+      const double id = copysign(rw * (pp * rc), detF);   // 1 / det F = 1 / (J det dX/dxi)
+      double V[9], FI[9];
+#pragma unroll
+      for (int c = 0; c < 9; c++) V[c] = cof[c] * id;
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int p = 0; p < 3; p++)
+          FI[3 * i + p] = F[3 * i] * g[sym3(0, p)] + F[3 * i + 1] * g[sym3(1, p)] +
+                          F[3 * i + 2] * g[sym3(2, p)];
+      double I1 = FI[0] * F[0];
+#pragma unroll
+      for (int c = 1; c < 9; c++) I1 = fma(FI[c], F[c], I1);
+      if (rest) I1 = 3.0;
+      const double t13 = (1.0 / 3.0) * I1;
+      const double pj = pc * J, pJs = ps * J;
+      const double w64 = w * 0.015625;   // the two factors 1/8 of dN/dxi
+      double FA[9];
+#pragma unroll
+      for (int c = 0; c < 9; c++) FA[c] = rest ? 0.0 : fma(-t13, V[c], FI[c]);
+      double CI[6];
+#pragma unroll
+      for (int p = 0; p < 3; p++)
+#pragma unroll
+        for (int r = p; r < 3; r++)
+          CI[sym3(p, r)] = V[p] * V[r] + V[3 + p] * V[3 + r] + V[6 + p] * V[6 + r];
+      auto store_A = [&](int i, int k, int p, int r, double v) {
+        const int row = f64_block_row(hblock(i, k)) + (i == k ? sym3(p, r) : 3 * p + r);
+        sm[row * kFRow + kFElem * q + sub] = v;
+      };
+      // (warp-uniform: the general form serves every lane of a mixed warp)
+      const bool general = __any_sync(0xFFFFFFFFu, mat_id != 1);
+      double X[9], hV[9];
+      if (!general) {
+        const double a1 = 0.5 * mc[0];
+        const double ko1 = a.have_state ? 2 * a1 * pp : 0.0;
+        const double k1 = (4.0 / 3.0) * a1 * pp;
+        const double c0 = pj - k1 * t13;
+        const double h = -0.5 * w64 * (2.0 * pj - k1 * I1);
+        const double pk = -w * ko1, pv = -w * pJs;
+#pragma unroll
+        for (int c = 0; c < 9; c++)
+          sm[(kFRowP + c) * kFRow + kFElem * q + sub] = fma(pk, FA[c], pv * V[c]);
+        const double xk = -w64 * k1, xv = 0.5 * w64 * c0;
+        const double eg = w64 * ko1, ec2 = w64 * (pJs - ko1 * t13) + h;
+        double Ed[6];
+#pragma unroll
+        for (int c = 0; c < 6; c++) Ed[c] = fma(ec2, CI[c], eg * g[c]);
+#pragma unroll
+        for (int c = 0; c < 9; c++) {
+          X[c] = fma(xk, FA[c], xv * V[c]);
+          hV[c] = h * V[c];
+        }
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          // i = k: the two V V terms join in Y = X + h V
+          double Y[3];
+#pragma unroll
+          for (int p = 0; p < 3; p++) Y[p] = X[3 * i + p] + hV[3 * i + p];
+#pragma unroll
+          for (int p = 0; p < 3; p++)
+#pragma unroll
+            for (int r = p; r < 3; r++)
+              store_A(i, i, p, r,
+                      fma(V[3 * i + p], Y[r], fma(X[3 * i + p], V[3 * i + r], Ed[sym3(p, r)])));
+#pragma unroll
+          for (int k = i + 1; k < 3; k++)
+#pragma unroll
+            for (int p = 0; p < 3; p++)
+#pragma unroll
+              for (int r = 0; r < 3; r++)
+                store_A(i, k, p, r,
+                        fma(V[3 * i + p], X[3 * k + r],
+                            fma(X[3 * i + p], V[3 * k + r], hV[3 * i + r] * V[3 * k + p])));
+        }
+      } else {
+        const double pppp = pp * pp;     // J^(-4/3)
+        double b[6];
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+          for (int k = i; k < 3; k++)
+            b[sym3(i, k)] = FI[3 * i] * F[3 * k] + FI[3 * i + 1] * F[3 * k + 1] +
+                            FI[3 * i + 2] * F[3 * k + 2];
+        const double I2 = b[0] * b[3] + b[3] * b[5] + b[0] * b[5] - b[1] * b[1] - b[4] * b[4] -
+                          b[2] * b[2];
+        const double t23 = (2.0 / 3.0) * I2;
+        // W derivatives at (I1 J^-2/3, I2 J^-4/3) (materials_hyperelastic.cpp:135-204)
+        double a1, a2 = 0.0, a11 = 0.0;
+        if (mat_id == 1) {
+          a1 = 0.5 * mc[0];
+        } else if (mat_id == 2) {
+          const double d = I1 * pp - 3.0;
+          a1 = mc[0] + 2 * mc[1] * d + 3 * mc[2] * d * d;
+          a2 = mc[3];
+          a11 = 2 * mc[1] + 6 * mc[2] * d;
+        } else {
+          a1 = mc[0];
+          a2 = mc[1];
+        }
+        const double st = a.have_state ? 1.0 : 0.0;
+        const double ko1 = st * (2 * a1 * pp), ko2 = st * (2 * a2 * pppp);
+        const double k11 = 4.0 * a11 * pppp, k1 = (4.0 / 3.0) * a1 * pp, k2 = (8.0 / 3.0) * a2 * pppp;
+        const double c0 = pj - k1 * t13 - k2 * t23;
+        const double h = -0.5 * w64 * (2.0 * pj - k1 * I1 - k2 * I2);
+        const double sI = 1.5 * w64 * k2;
+        const double pk = -w * ko1, pb = -w * ko2, pv = -w * pJs;
+        const double xk = -w64 * k1, xb = -w64 * k2, xv = 0.5 * w64 * c0;
+        const double w11 = w64 * k11;
+        const bool biderman = __any_sync(0xFFFFFFFFu, a11 != 0.0);
+#pragma unroll
+        for (int c = 0; c < 9; c++) {
+          const int i = c / 3, p = c % 3;
+          const double fc = b[sym3(i, 0)] * FI[p] + b[sym3(i, 1)] * FI[3 + p] +
+                            b[sym3(i, 2)] * FI[6 + p];
+          const double FB = rest ? 0.0 : fma(-t23, V[c], fma(I1, FI[c], -fc));
+          sm[(kFRowP + c) * kFRow + kFElem * q + sub] = fma(pk, FA[c], fma(pb, FB, pv * V[c]));
+          X[c] = fma(xk, FA[c], fma(xb, FB, xv * V[c]));
+          hV[c] = h * V[c];
+        }
+        // S^{pq} = (ko1 + ko2 I1) g - ko2 C^{pq} + (p J - ko1 I1/3 - ko2 2 I2/3) C^-1
+        const double eg = w64 * (ko1 + ko2 * I1), ecc = -w64 * ko2;
+        const double ec2 = w64 * (pJs - ko1 * t13 - ko2 * t23) + h;
+        const double hI = 0.5 * sI;
+        double Ed[6];
+#pragma unroll
+        for (int p = 0; p < 3; p++)
+#pragma unroll
+          for (int r = p; r < 3; r++) {
+            const int c = sym3(p, r);
+            const double C = FI[p] * FI[r] + FI[3 + p] * FI[3 + r] + FI[6 + p] * FI[6 + r];
+            Ed[c] = fma(ecc, C, fma(ec2, CI[c], eg * g[c]));
+          }
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          double Y[3], Z[3], Z2[3], W3[3];
+          const double bi = -hI * b[sym3(i, i)];
+#pragma unroll
+          for (int p = 0; p < 3; p++) {
+            Y[p] = X[3 * i + p] + hV[3 * i + p];
+            Z[p] = hI * FI[3 * i + p];
+            if (i < 2) Z2[p] = sI * FI[3 * i + p];
+            if (biderman) W3[p] = w11 * FA[3 * i + p];
+          }
+#pragma unroll
+          for (int p = 0; p < 3; p++)
+#pragma unroll
+            for (int r = p; r < 3; r++) {
+              double v = fma(bi, g[sym3(p, r)], Ed[sym3(p, r)]);
+              v = fma(Z[p], FI[3 * i + r], v);
+              v = fma(V[3 * i + p], Y[r], fma(X[3 * i + p], V[3 * i + r], v));
+              if (biderman) v = fma(W3[p], FA[3 * i + r], v);
+              store_A(i, i, p, r, v);
+            }
+#pragma unroll
+          for (int k = i + 1; k < 3; k++) {
+            const double bk = -hI * b[sym3(i, k)];
+            double bg[6];
+#pragma unroll
+            for (int c = 0; c < 6; c++) bg[c] = bk * g[c];
+#pragma unroll
+            for (int p = 0; p < 3; p++)
+#pragma unroll
+              for (int r = 0; r < 3; r++) {
+                double v = fma(-Z[r], FI[3 * k + p], bg[sym3(p, r)]);
+                v = fma(Z2[p], FI[3 * k + r], v);
+                v = fma(hV[3 * i + r], V[3 * k + p], v);
+                v = fma(V[3 * i + p], X[3 * k + r], fma(X[3 * i + p], V[3 * k + r], v));
+                if (biderman) v = fma(W3[p], FA[3 * k + r], v);
+                store_A(i, k, p, r, v);
+              }
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) {
+      Fp_part += __shfl_xor_sync(0xFFFFFFFFu, Fp_part, off);
+      Kpp_part += __shfl_xor_sync(0xFFFFFFFFu, Kpp_part, off);
+    }
+    __syncwarp();
+
+    // ---- sums over the Gauss points: the rows' transforms, in place ----
+    // An entry (p, q) with p = q, and every entry (i, p) of w F S and cof F,
+    // is read only at the characters without coordinate p: its two halves in
+    // p are added and four points transformed (12 adds instead of 24).
+#pragma unroll 2
+    for (int r = 0; r < 4; r++) {
+      const int t = lane + 32 * r;   // 27 entries p != q x 4 elements
+      if (t >= 27 * kEPW) break;
+      double* W = sm + rows[t >> 2] + kFElem * (t & 3);
+      double v[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) v[j] = W[j];
+#pragma unroll
+      for (int d = 1; d < 8; d <<= 1)
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+          if (!(j & d)) {
+            const double lo = v[j], hi = v[j | d];
+            v[j] = lo + hi;
+            v[j | d] = hi - lo;
+          }
+#pragma unroll
+      for (int j = 0; j < 8; j++) W[j] = v[j];
+    }
+#pragma unroll 2
+    for (int r = 0; r < 5; r++) {
+      const int t = lane + 32 * r;   // 36 entries x 4 elements
+      if (t >= 36 * kEPW) break;
+      const int n = t >> 2;
+      const int p = n % 3;
+      double* W = sm + rows[27 + n] + kFElem * (t & 3);
+      const int mp = 1 << p, ma = p == 0 ? 2 : 1, mb = p == 2 ? 2 : 4;
+      const double v0 = W[0] + W[mp], va = W[ma] + W[ma + mp], vb = W[mb] + W[mb + mp],
+                   vab = W[ma + mb] + W[7];
+      const double s0 = v0 + va, d0 = va - v0, s1 = vb + vab, d1 = vab - vb;
+      W[0] = s0 + s1;
+      W[ma] = d0 + d1;
+      W[mb] = s1 - s0;
+      W[ma + mb] = d1 - d0;
+    }
+    __syncwarp();
+
+    // destination of contribution idx: slot-ordered (kpos) or element-ordered
+    auto kdst = [&](uint64_t idx) -> uint64_t { return a.kpos ? (uint64_t)__ldg(a.kpos + idx) : idx; };
+    auto fdst = [&](uint64_t idx) -> uint64_t { return a.fpos ? (uint64_t)__ldg(a.fpos + idx) : idx; };
+
+    // ---- modes of both sides, the b side to nodes ----
+    // lanes 0 .. 23 = (block (i, k), element), one mode of the a side per
+    // round; F_u and K_up (six components x four elements) have the form of a
+    // one-coordinate mode and take the eight lanes left in those three rounds
+    {
+      const bool spare = lane >= 24;
+      const int ik = spare ? 0 : lane >> 2, el = lane & 3;
+      const bool diag = ik == 0 || ik == 3 || ik == 5;
+      const double* W = sm + (spare ? kFRowP : f64_block_row(ik)) * kFRow + kFElem * el;
+      int off[3][3];
+#pragma unroll
+      for (int p = 0; p < 3; p++)
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+          off[p][r] = kFRow * (spare ? 3 * (2 * p + ((lane >> 2) & 1)) + r
+                                     : diag ? sym3(p, r) : 3 * p + r);
+#pragma unroll
+      for (int round = 0; round < 7; round++) {
+        const int al = round == 0 ? 1 : round == 1 ? 2 : round == 2 ? 4 : round == 3 ? 3
+                     : round == 4 ? 5 : round == 5 ? 6 : 7;
+        if (round == 3) {
+          __syncwarp();
+          if (spare) break;
+        }
+        double M[8], o[8];
+#pragma unroll
+        for (int be = 1; be < 8; be++) {
+          double v = 0.0;
+          bool first = true;
+#pragma unroll
+          for (int p = 0; p < 3; p++) {
+            if (!(al >> p & 1)) continue;
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+              if (!(be >> r & 1)) continue;
+              const double x = W[off[p][r] + ((al ^ (1 << p)) ^ (be ^ (1 << r)))];
+              v = first ? x : v + x;
+              first = false;
+            }
+          }
+          M[be] = v;
+        }
+        modes_to_nodes(M, o);
+        if (!spare) {
+          double* T = sm + f64_T(al) + 9 * lane;
+#pragma unroll
+          for (int b = 0; b < 8; b++) T[b] = o[b];
+        } else {
+          const int c = 2 * round + ((lane >> 2) & 1);   // c < 3: F_u, else K_up
+          const uint32_t ee = e0 + el;
+          if (ee < E) {
+#pragma unroll
+            for (int b = 0; b < 8; b++) {
+              const int n = hex_corner(b);
+              const double v = eighth(o[b]);
+              if (c < 3) a.contribF[fdst((uint64_t)ee * kSolidFc + 3 * n + c)] = v;
+              else a.contribK[kdst((uint64_t)ee * kSolidKc + 300 + 3 * n + c - 3)] = v;
+            }
+          }
+        }
+      }
+    }
+    __syncwarp();
+
+    // ---- the a side to nodes: lane = (element, node b), block by block ----
+    {
+      const int nb = hex_corner(sub);
+#pragma unroll
+      for (int ik = 0; ik < 6; ik++) {
+        double M[8], o[8];
+#pragma unroll
+        for (int al = 1; al < 8; al++) M[al] = sm[f64_T(al) + 9 * (ik * 4 + q) + sub];
+        modes_to_nodes(M, o);
+#pragma unroll
+        for (int m = 0; m < 8; m++) {
+          const uint32_t pos = dpos[(hex_corner(m) * 6 + ik) * 8 + nb];
+          if (pos != 0xFFFFu) sm[q * kKuuPerElem + pos] = o[m];
+        }
+      }
+    }
+    __syncwarp();
+#pragma unroll 4
+    for (int m = 0; m < kOwned; m++) {
+      const int x = lane + 32 * m;
+      if (x < kEPW * kKuuPerElem) {
+        const int qq = x / kKuuPerElem, t = x - qq * kKuuPerElem;
+        const uint32_t ee = e0 + qq;
+        if (ee < E) a.contribK[kdst((uint64_t)ee * kSolidKc + t)] = sm[x];
+      }
+    }
+    if (valid && sub == 0) {
+      a.contribK[kdst((uint64_t)e * kSolidKc + 324)] = Kpp_part;
+      a.contribF[fdst((uint64_t)e * kSolidFc + 24)] = Fp_part;
+    }
+    __syncwarp();
+  }
+}
+
+template <int WPB>
+__global__ void __launch_bounds__(WPB * 32)
+    solid81_mixed_kernel(const Solid81Args a) {
+  if (a.skip && *a.skip) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  // block header: the D -> assemble3 position table
+  uint16_t* dpos = reinterpret_cast<uint16_t*>(smem_raw);  // [kDpos]
+  MixedSmem* sm = reinterpret_cast<MixedSmem*>(smem_raw + kDposBytes) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
-  if constexpr (kMixed) {
-    for (int v = threadIdx.x; v < kDpos; v += blockDim.x) dpos[v] = c_dpos[v];
-  } else
-  // Ownership of Kuu entries: lane owns x = lane + 32 m of the 4*231 owned
-  // entries of its warp's element quad.  Decode once: smem offsets of
-  // H[ik][.][slot a] and G[.][slot b].
-  for (int v = threadIdx.x; v < kOwned64 * 32; v += blockDim.x) {
-    const int m = v / 32, l = v % 32;
-    const int x = l + 32 * m;
-    // entries past the quad's 924 read slot 0 (in bounds) and are never written
-    uint32_t word = 0u;
-    uint16_t where = 0xFFFFu;
-    if (x < kEPW * kKuuOwned) {
-      const int q = x / kKuuOwned;
-      const int t = c_kuu_owned[x - q * kKuuOwned];
-      where = (uint16_t)(q * kKuuPerElem + t);
-      const uchar4 en = c_kuu_entry[t];  // (a, i, b, k)
-      // i <= k: h_a[ik] . G_b;  i > k: h_b[ki] . G_a (A symmetric)
-      const bool up = en.y <= en.w;
-      const uint32_t hb = up ? hblock(en.y, en.w) : hblock(en.w, en.y);
-      const uint32_t ho = hb * kHStride + q * 8 + (up ? en.x : en.z);
-      const uint32_t go = q * 8 + (up ? en.z : en.x);
-      word = ho | (go << 16);
-    }
-    dec[m * 32 + l] = word;
-    opos[m * 32 + l] = where;
-  }
-  if constexpr (!kMixed)
-    for (int v = threadIdx.x; v < kKuuDerived * 8; v += blockDim.x) dtab[v] = c_kuu_derived[v];
+  for (int v = threadIdx.x; v < kDpos; v += blockDim.x) dpos[v] = c_dpos[v];
   __syncthreads();
 
   const uint32_t E = a.n_elems;  // end of this launch's element range
@@ -596,13 +1107,13 @@ __global__ void __launch_bounds__(WPB * 32)
     const uint32_t ec = valid ? e : E - 1;
 
     // ---------------- phase 1: lane = (element q, Gauss point g) ----------------
-    double Fp_part = 0.0, Kpp_part = 0.0;  // FP64 in both kernels
+    double Fp_part = 0.0, Kpp_part = 0.0;  // FP64
     {
       const int g = sub;
       const uint64_t tg = (uint64_t)ec * 8 + g;
-      TT Fm[9], wS[6], wD[21];
+      float Fm[9], wS[6], wD[21];
       bool bad;
-      if constexpr (kMixed) {
+      {
         // the residual chain in float pairs, the tangent inputs rounded to float
         const dw w = dw_of(__ldg(a.wdf + tg));
         const dw pc = dw_from_double(a.U_cur[a.p_eq[ec] - 1]);
@@ -733,90 +1244,6 @@ __global__ void __launch_bounds__(WPB * 32)
         Fp_part = -(Jd - 1 - pcd * inv_kbd) * wd;
         Kpp_part = -inv_kbd * wd;
         bad = valid && !(Jd > 0.0 && isfinite(Jd) && J.h > 0.0f && isfinite(J.h) && wd > 0.0);
-      } else {
-        const double w = a.wdet[tg];
-        const double pc = a.U_cur[a.p_eq[ec] - 1];
-        double O[9];
-        double C[6];
-        double ps = 0.0;
-        if (a.have_state) {
-          double G[24];
-#pragma unroll
-          for (int c = 0; c < 24; c++) G[c] = __ldg(a.Gt + c * E8 + tg);
-#pragma unroll
-          for (int c = 0; c < 9; c++) O[c] = 0.0;
-#pragma unroll
-          for (int n = 0; n < 8; n++) {
-            const uint32_t nid = __ldg(a.conn + (uint64_t)ec * 8 + n);
-            const uint4 eq = __ldg(reinterpret_cast<const uint4*>(a.node_eq3) + (nid - 1));
-            const double ux = a.U_state[eq.x - 1], uy = a.U_state[eq.y - 1],
-                         uz = a.U_state[eq.z - 1];
-#pragma unroll
-            for (int j = 0; j < 3; j++) {
-              O[0 + j] = fma(ux, G[3 * n + j], O[0 + j]);
-              O[3 + j] = fma(uy, G[3 * n + j], O[3 + j]);
-              O[6 + j] = fma(uz, G[3 * n + j], O[6 + j]);
-            }
-          }
-          ps = a.U_state[a.p_eq[ec] - 1];
-          // C = F^T F from O (SOLID81.cpp:105-110)
-          C[0] = 1.0 + 2 * O[0] + O[0] * O[0] + O[3] * O[3] + O[6] * O[6];
-          C[3] = 1.0 + 2 * O[4] + O[1] * O[1] + O[4] * O[4] + O[7] * O[7];
-          C[5] = 1.0 + 2 * O[8] + O[2] * O[2] + O[5] * O[5] + O[8] * O[8];
-          C[1] = O[1] + O[3] + O[0] * O[1] + O[3] * O[4] + O[6] * O[7];
-          C[4] = O[5] + O[7] + O[1] * O[2] + O[4] * O[5] + O[7] * O[8];
-          C[2] = O[2] + O[6] + O[0] * O[2] + O[3] * O[5] + O[6] * O[8];
-        } else {
-          // state right after Element::pre(): C = I, S = 0, O = 0 (SOLID81.cpp:17-19)
-#pragma unroll
-          for (int c = 0; c < 9; c++) O[c] = 0.0;
-          C[0] = C[3] = C[5] = 1.0;
-          C[1] = C[2] = C[4] = 0.0;
-        }
-        int mat_id = a.mat_id;
-        const double* mc = a.mc;
-        double kbulk = a.kbulk;
-        if (a.elem_mesh) {
-          const double* mm = a.mesh_mat + 8 * (uint64_t)__ldg(a.elem_mesh + ec);
-          mat_id = (int)mm[0];
-          mc = mm + 1;
-          kbulk = mm[6];
-        }
-        const double inv_kb = 1.0 / kbulk;
-        MatOut<TT> mo;
-        material<TT>(mat_id, mc, C, ps, pc, w, mo, wD);
-        if (!a.have_state) {
-#pragma unroll
-          for (int i = 0; i < 6; i++) mo.S[i] = 0.0;
-        }
-        const double J = mo.J;
-        const double F[9] = {1.0 + O[0], O[1], O[2], O[3], 1.0 + O[4], O[5], O[6], O[7], 1.0 + O[8]};
-        const double S3[9] = {mo.S[0], mo.S[1], mo.S[2], mo.S[1], mo.S[3], mo.S[4],
-                              mo.S[2], mo.S[4], mo.S[5]};
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-          for (int k = 0; k < 3; k++) {
-            const double fs = F[3 * i + 0] * S3[0 + k] + F[3 * i + 1] * S3[3 + k] +
-                              F[3 * i + 2] * S3[6 + k];
-            sm->wP[3 * i + k][lane] = -w * fs;
-          }
-        const double cof[9] = {F[4] * F[8] - F[5] * F[7], F[5] * F[6] - F[3] * F[8],
-                               F[3] * F[7] - F[4] * F[6], F[2] * F[7] - F[1] * F[8],
-                               F[0] * F[8] - F[2] * F[6], F[1] * F[6] - F[0] * F[7],
-                               F[1] * F[5] - F[2] * F[4], F[2] * F[3] - F[0] * F[5],
-                               F[0] * F[4] - F[1] * F[3]};
-#pragma unroll
-        for (int c = 0; c < 9; c++) sm->wCof[c][lane] = w * cof[c];
-#pragma unroll
-        for (int c = 0; c < 9; c++) Fm[c] = (TT)F[c];
-#pragma unroll
-        for (int c = 0; c < 6; c++) wS[c] = (TT)(w * mo.S[c]);
-        Fp_part = -(J - 1 - pc * inv_kb) * w;
-        Kpp_part = -inv_kb * w;
-        // J = sqrt(det C) cannot see an inverted element; det F can
-        const double detF = F[0] * cof[0] + F[1] * cof[1] + F[2] * cof[2];
-        bad = valid && !(J > 0.0 && isfinite(J) && detF > 0.0 && w > 0.0);
       }
       // A[iL][kN] = sum_J F_iJ (sum_M wD[(JL)][(MN)] F_kM) + delta_ik w S_LN,
       // one row (i, L) at a time
@@ -824,7 +1251,7 @@ __global__ void __launch_bounds__(WPB * 32)
       for (int i = 0; i < 3; i++)
 #pragma unroll
         for (int L = 0; L < 3; L++) {
-          TT T6[6];
+          float T6[6];
 #pragma unroll
           for (int t = 0; t < 6; t++)
             T6[t] = Fm[3 * i + 0] * wD[sym6u(voigt(0, L), t)] +
@@ -835,7 +1262,7 @@ __global__ void __launch_bounds__(WPB * 32)
 #pragma unroll
             for (int N = 0; N < 3; N++) {
               if (3 * k + N < 3 * i + L) continue;
-              TT v = T6[voigt(0, N)] * Fm[3 * k + 0] + T6[voigt(1, N)] * Fm[3 * k + 1] +
+              float v = T6[voigt(0, N)] * Fm[3 * k + 0] + T6[voigt(1, N)] * Fm[3 * k + 1] +
                      T6[voigt(2, N)] * Fm[3 * k + 2];
               if (i == k) v += wS[voigt(L, N)];
               sm->A[sym9(3 * i + L, 3 * k + N)][lane] = v;
@@ -855,7 +1282,7 @@ __global__ void __launch_bounds__(WPB * 32)
     auto kdst = [&](uint64_t idx) -> uint64_t { return a.kpos ? (uint64_t)__ldg(a.kpos + idx) : idx; };
     auto fdst = [&](uint64_t idx) -> uint64_t { return a.fpos ? (uint64_t)__ldg(a.fpos + idx) : idx; };
 
-    if constexpr (kMixed) {
+    {
       // Residual and pressure coupling, lane = (element q, node a), before the
       // Gauss point loop reuses the scratch that holds -w F S and w cof F:
       //   F_u(a, i) = sum_g sum_L (-w F S)_g[iL] G_g[aL]   (float pairs),
@@ -907,7 +1334,7 @@ __global__ void __launch_bounds__(WPB * 32)
     }
 
     // ---------------- phases 2 + 3 per Gauss point ----------------
-    if constexpr (kMixed) {
+    {
       // Lane (q, a) keeps h_a[ik] (i <= k, its own node) in registers and
       // accumulates D[(ik), a, b] = sum_g h_a[ik] . G_b for all 8 nodes b:
       // 48 sums of 3 FMA per Gauss point from 3 shared loads per node b.
@@ -975,130 +1402,44 @@ __global__ void __launch_bounds__(WPB * 32)
         }
       }
       __syncwarp();
-    } else {
-    TT acc[kOwned64];
-#pragma unroll
-    for (int m = 0; m < kOwned64; m++) acc[m] = (TT)0;
-    double Fu[3] = {0.0, 0.0, 0.0};   // FP64 kernel (the mixed one wrote F_u and
-    double Kup[3] = {0.0, 0.0, 0.0};  // K_up above)
-    const int node = sub;
-    for (int g = 0; g < 8; g++) {
-      const int s1 = q * 8 + g;
-      {
-        // phase 2: lane = (element q, node a)
-        const uint64_t tg = (uint64_t)ec * 8 + g;
-        TT gg[3];
-        if constexpr (kMixed) {
-          // the tangent uses the high parts
-          gg[0] = __ldg(a.Gdf + (3 * node + 0) * E8 + tg).x;
-          gg[1] = __ldg(a.Gdf + (3 * node + 1) * E8 + tg).x;
-          gg[2] = __ldg(a.Gdf + (3 * node + 2) * E8 + tg).x;
-        } else {
-          const double G0 = __ldg(a.Gt + (3 * node + 0) * E8 + tg);
-          const double G1 = __ldg(a.Gt + (3 * node + 1) * E8 + tg);
-          const double G2 = __ldg(a.Gt + (3 * node + 2) * E8 + tg);
-          // residual and pressure coupling in FP64, one FMA chain per entry
-          // (three FMAs per Gauss point instead of a product, two FMAs and an add)
-#pragma unroll
-          for (int i = 0; i < 3; i++) {
-            Fu[i] = fma(sm->wP[3 * i + 0][s1], G0, Fu[i]);
-            Fu[i] = fma(sm->wP[3 * i + 1][s1], G1, Fu[i]);
-            Fu[i] = fma(sm->wP[3 * i + 2][s1], G2, Fu[i]);
-            Kup[i] = fma(sm->wCof[3 * i + 0][s1], G0, Kup[i]);
-            Kup[i] = fma(sm->wCof[3 * i + 1][s1], G1, Kup[i]);
-            Kup[i] = fma(sm->wCof[3 * i + 2][s1], G2, Kup[i]);
-          }
-          gg[0] = (TT)G0;
-          gg[1] = (TT)G1;
-          gg[2] = (TT)G2;
-        }
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-          for (int k = i; k < 3; k++)
-#pragma unroll
-            for (int N = 0; N < 3; N++)
-              sm->H[hblock(i, k) * kHStride + 32 * N + lane] =
-                  gg[0] * sm->A[sym9(3 * i + 0, 3 * k + N)][s1] +
-                  gg[1] * sm->A[sym9(3 * i + 1, 3 * k + N)][s1] +
-                  gg[2] * sm->A[sym9(3 * i + 2, 3 * k + N)][s1];
-#pragma unroll
-        for (int c = 0; c < 3; c++) sm->G[c][lane] = gg[c];
-      }
-      __syncwarp();
-      {
-        // phase 3: owned Kuu entries, K(a,i; b,k) += h_a[ik] . G_b
-        const TT* Hf = sm->H;
-        const TT* Gf = &sm->G[0][0];
-#pragma unroll
-        for (int m = 0; m < kOwned64; m++) {
-          const uint32_t word = dec[m * 32 + lane];
-          const uint32_t ho = word & 0xFFFFu, go = word >> 16;
-          TT v = acc[m];
-          v += Hf[ho] * Gf[go];
-          v += Hf[ho + 32] * Gf[go + 32];
-          v += Hf[ho + 64] * Gf[go + 64];
-          acc[m] = v;
-        }
-      }
-      __syncwarp();
     }
-
-    // ---------------- write the element contributions ----------------
-    // the owned entries into the quad's stage (assemble3 order; A's scratch,
-    // dead after the Gauss-point loop), node 7's column from them, node 7's
-    // block from that column, then all 4 x 300 written coalesced
-    TT* stage = &sm->A[0][0];
-#pragma unroll
-    for (int m = 0; m < kOwned64; m++) {
-      const uint16_t where = opos[m * 32 + lane];
-      if (where != 0xFFFFu) stage[where] = acc[m];
-    }
-    __syncwarp();
-    for (int dx = lane; dx < kEPW * kKuuColumn; dx += 32) {
-      const int qq = dx / kKuuColumn, j = dx - qq * kKuuColumn;
-      const TT* st = stage + qq * kKuuPerElem;
-      const uint16_t* dj = dtab + j * 8;
-      TT v = st[dj[1]];
-#pragma unroll
-      for (int c = 2; c < 8; c++) v += st[dj[c]];
-      stage[qq * kKuuPerElem + dj[0]] = -v;
-    }
-    __syncwarp();
-    if (lane < kEPW * kKuuCorner) {
-      const int qq = lane / kKuuCorner, j = kKuuColumn + lane - qq * kKuuCorner;
-      const TT* st = stage + qq * kKuuPerElem;
-      const uint16_t* dj = dtab + j * 8;
-      TT v = st[dj[1]];
-#pragma unroll
-      for (int c = 2; c < 8; c++) v += st[dj[c]];
-      stage[qq * kKuuPerElem + dj[0]] = -v;
-    }
-    __syncwarp();
-#pragma unroll 4
-    for (int m = 0; m < kOwned; m++) {
-      const int x = lane + 32 * m;
-      if (x < kEPW * kKuuPerElem) {
-        const int qq = x / kKuuPerElem, t = x - qq * kKuuPerElem;
-        const uint32_t ee = e0 + qq;
-        if (ee < E) a.contribK[kdst((uint64_t)ee * kSolidKc + t)] = stage[x];
-      }
-    }
-    if (valid) {
-      const uint64_t kb = (uint64_t)e * kSolidKc, fb = (uint64_t)e * kSolidFc;
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        a.contribK[kdst(kb + 300 + 3 * node + i)] = Kup[i];
-        a.contribF[fdst(fb + 3 * node + i)] = Fu[i];
-      }
-      if (node == 0) {
-        a.contribK[kdst(kb + 324)] = Kpp_part;
-        a.contribF[fdst(fb + 24)] = Fp_part;
-      }
-    }
-    __syncwarp();
-    }  // FP64 kernel
   }
+}
+
+// The FP64 kernel's element geometry, lane = (element, corner / mode / Gauss
+// point): shape modes of the positions (relative to node 0: no digits lost to
+// the element's distance from the origin), and at the Gauss point w = det
+// dX/dxi, 1 / w and the metric dxi_p/dX . dxi_q/dX.
+__global__ void __launch_bounds__(256) solid81_geometry_kernel(const JacobianArgs a) {
+  if (a.skip && *a.skip) return;
+  __shared__ double modes[3][256];
+  const uint64_t E8 = (uint64_t)a.n_elems * 8;
+  const uint64_t t0 = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+  const bool valid = t0 < E8;
+  const uint64_t t = valid ? t0 : E8 - 8 + (t0 & 7);   // whole elements per eight lanes
+  const int sub = threadIdx.x & 7;
+  const uint32_t nid = a.conn[(t & ~7ull) + hex_corner(sub)];
+  for (int i = 0; i < 3; i++)
+    modes[i][threadIdx.x] = 0.125 * corners_to_mode(a.xyz[(uint64_t)(nid - 1) * 3 + i], sub);
+  __syncwarp();
+  const GaussSigns sg = gauss_signs(sub);
+  double F[9], cof[9];
+  for (int i = 0; i < 3; i++) mode_gradient(&modes[i][threadIdx.x & ~7], sg, F + 3 * i);
+  const double det = cofactors(F, cof);
+  if (!valid) return;
+  const double r = 1.0 / det;
+  for (int p = 0; p < 3; p++)
+    for (int s = p; s < 3; s++) {
+      // dxi_p/dX_i = cof_ip / det
+      double v = 0.0;
+      for (int i = 0; i < 3; i++) v += (cof[3 * i + p] * r) * (cof[3 * i + s] * r);
+      a.geo[sym3(p, s) * E8 + t] = v;
+    }
+  a.geo[6 * E8 + t] = r;
+  for (int i = 0; i < 3; i++) a.geo[(7 + i) * E8 + t] = sub ? modes[i][threadIdx.x] : 0.0;
+  a.wdet[t] = det;
+  // isoparametric.cpp:177 logs det < 1e-20; here it is an element status
+  if (!(det >= 1.0e-20) && sub == 0) flag_element(a.status, (uint32_t)(t >> 3) + 1);
 }
 
 __global__ void solid81_jacobian_kernel(const JacobianArgs a) {
@@ -1142,17 +1483,12 @@ __global__ void solid81_jacobian_kernel(const JacobianArgs a) {
     for (int i = 0; i < 3; i++) {
       double v = 0.0;
       for (int j = 0; j < 3; j++) v += Ji[3 * i + j] * dN[3 * n + j];
-      if (a.Gt) a.Gt[(uint64_t)(3 * n + i) * E8 + t] = v;
-      if (a.Gdf) {
-        const dw p = dw_from_double(v);
-        a.Gdf[(uint64_t)(3 * n + i) * E8 + t] = make_float2(p.h, p.l);
-      }
+      const dw p = dw_from_double(v);
+      a.Gdf[(uint64_t)(3 * n + i) * E8 + t] = make_float2(p.h, p.l);
     }
   a.wdet[t] = 1.0 * det;
-  if (a.wdf) {
-    const dw p = dw_from_double(1.0 * det);
-    a.wdf[t] = make_float2(p.h, p.l);
-  }
+  const dw pw = dw_from_double(1.0 * det);
+  a.wdf[t] = make_float2(pw.h, pw.l);
   // isoparametric.cpp:177 logs det < 1e-20; here it is an element status
   if (!(det >= 1.0e-20) && g == 0) flag_element(a.status, e + 1);
 }
@@ -1566,21 +1902,17 @@ cudaError_t ensure_tables() {
   if (g_tables_ready[dev].load(std::memory_order_acquire)) return cudaSuccess;
   std::lock_guard<std::mutex> lock(g_tables_mutex);
   if (g_tables_ready[dev].load(std::memory_order_relaxed)) return cudaSuccess;
-  uchar4 h[kKuuPerElem];
+  // assemble3's order of the entries (a, i, b, k) (SOLID81.h:62-74)
+  int tpos[8][3][8][3];
   int t = 0;
   for (int i = 0; i < 8; i++)
     for (int di = 0; di < 3; di++)
       for (int j = i; j < 8; j++)
         for (int dj = 0; dj < 3; dj++) {
           if (i == j && dj < di) continue;
-          h[t++] = make_uchar4((unsigned char)i, (unsigned char)di, (unsigned char)j,
-                               (unsigned char)dj);
+          tpos[i][di][j][dj] = t++;
         }
-  err = cudaMemcpyToSymbol(c_kuu_entry, h, sizeof(h));
-  if (err != cudaSuccess) return err;
   // D[(i,k), a, b] -> assemble3 position (see c_dpos)
-  int tpos[8][3][8][3];
-  for (int u = 0; u < kKuuPerElem; u++) tpos[h[u].x][h[u].y][h[u].z][h[u].w] = u;
   uint16_t dp[kDpos];
   for (int a = 0; a < 8; a++)
     for (int i = 0; i < 3; i++)
@@ -1591,33 +1923,6 @@ cudaError_t ensure_tables() {
           else dp[at] = i == k ? (uint16_t)0xFFFF : (uint16_t)tpos[b][k][a][i];
         }
   err = cudaMemcpyToSymbol(c_dpos, dp, sizeof(dp));
-  if (err != cudaSuccess) return err;
-  // FP64 kernel: node 7's column and block (derived) and the other entries
-  // (owned); the column's 63 rows come first, the block's 6 after them
-  uint16_t own[kKuuOwned], der[kKuuDerived * 8];
-  int no = 0, nd = 0, nc = kKuuColumn;
-  for (int u = 0; u < kKuuPerElem; u++) {
-    const int a = h[u].x, i = h[u].y, b = h[u].z, k = h[u].w;
-    if (b == 7 && a < 7) {
-      uint16_t* row = der + 8 * nd++;
-      row[0] = (uint16_t)u;
-      for (int bb = 0; bb < 7; bb++)   // K(a,i; bb,k) by its assemble3 position
-        row[1 + bb] = (uint16_t)(a < bb ? tpos[a][i][bb][k]
-                                 : a > bb ? tpos[bb][k][a][i]
-                                 : (i <= k ? tpos[a][i][a][k] : tpos[a][k][a][i]));
-    } else if (b == 7 && a == 7) {
-      if (nc >= kKuuDerived) return cudaErrorInvalidValue;
-      uint16_t* row = der + 8 * nc++;
-      row[0] = (uint16_t)u;
-      for (int aa = 0; aa < 7; aa++)   // K(aa,i; 7,k): node 7's column, formed first
-        row[1 + aa] = (uint16_t)tpos[aa][i][7][k];
-    } else {
-      own[no++] = (uint16_t)u;
-    }
-  }
-  if (no != kKuuOwned || nd != kKuuColumn || nc != kKuuDerived) return cudaErrorInvalidValue;
-  err = cudaMemcpyToSymbol(c_kuu_owned, own, sizeof(own));
-  if (err == cudaSuccess) err = cudaMemcpyToSymbol(c_kuu_derived, der, sizeof(der));
   if (err == cudaSuccess) g_tables_ready[dev].store(true, std::memory_order_release);
   return err;
 }
@@ -1625,25 +1930,25 @@ cudaError_t ensure_tables() {
 }  // namespace
 
 size_t solid81_smem_bytes_wpb(bool mixed, int wpb) {
-  const size_t head = mixed ? kDposBytes : kHead64Bytes;
-  return head + wpb * (mixed ? sizeof(WarpSmem<float>) : sizeof(WarpSmem<double>));
+  return mixed ? kDposBytes + wpb * sizeof(MixedSmem) : kHead64Bytes + wpb * kFWarp * sizeof(double);
 }
 
 size_t solid81_smem_bytes(bool mixed) { return solid81_smem_bytes_wpb(mixed, kWarpsPerBlock); }
 
-template <typename TT>
-void* solid81_fn(int wpb) {
+using Solid81Kernel = void (*)(Solid81Args);
+
+Solid81Kernel solid81_fn(bool mixed, int wpb) {
   switch (wpb) {
-    case 2: return (void*)solid81_kernel<TT, 2>;
-    case 8: return (void*)solid81_kernel<TT, 8>;
-    default: return (void*)solid81_kernel<TT, 4>;
+    case 2: return mixed ? solid81_mixed_kernel<2> : solid81_fp64_kernel<2>;
+    case 8: return mixed ? solid81_mixed_kernel<8> : solid81_fp64_kernel<8>;
+    default: return mixed ? solid81_mixed_kernel<4> : solid81_fp64_kernel<4>;
   }
 }
 
 cudaError_t prepare_device_tables() { return ensure_tables(); }
 
 int solid81_max_blocks_per_sm(bool mixed, int wpb) {
-  void* fn = mixed ? solid81_fn<float>(wpb) : solid81_fn<double>(wpb);
+  const void* fn = reinterpret_cast<const void*>(solid81_fn(mixed, wpb));
   const size_t smem = solid81_smem_bytes_wpb(mixed, wpb);
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
@@ -1674,15 +1979,7 @@ cudaError_t launch_solid81_shaped(const Solid81Args& a, bool mixed, Solid81Shape
   const uint64_t need = (quads + wpb - 1) / wpb;
   if (blocks > need) blocks = need;
   const dim3 grid((unsigned)blocks), block(wpb * 32);
-  if (mixed) {
-    if (wpb == 2) solid81_kernel<float, 2><<<grid, block, smem, s>>>(a);
-    else if (wpb == 8) solid81_kernel<float, 8><<<grid, block, smem, s>>>(a);
-    else solid81_kernel<float, 4><<<grid, block, smem, s>>>(a);
-  } else {
-    if (wpb == 2) solid81_kernel<double, 2><<<grid, block, smem, s>>>(a);
-    else if (wpb == 8) solid81_kernel<double, 8><<<grid, block, smem, s>>>(a);
-    else solid81_kernel<double, 4><<<grid, block, smem, s>>>(a);
-  }
+  solid81_fn(mixed, wpb)<<<grid, block, smem, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -1690,7 +1987,9 @@ cudaError_t launch_solid81_jacobian(const JacobianArgs& a, cudaStream_t s) {
   const uint64_t n = (uint64_t)a.n_elems * 8;
   if (n == 0) return cudaSuccess;
   const int bs = 256;
-  solid81_jacobian_kernel<<<(unsigned)((n + bs - 1) / bs), bs, 0, s>>>(a);
+  const unsigned blocks = (unsigned)((n + bs - 1) / bs);
+  if (a.geo) solid81_geometry_kernel<<<blocks, bs, 0, s>>>(a);
+  else solid81_jacobian_kernel<<<blocks, bs, 0, s>>>(a);
   return cudaGetLastError();
 }
 

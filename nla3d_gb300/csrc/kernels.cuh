@@ -7,6 +7,7 @@
 namespace nla3d_gpu {
 
 constexpr int kSolidKc = 325;  // SOLID81 K contributions per element (300 Kuu + 24 Kup + 1 Kpp)
+constexpr int kSolidGeo = 10;  // FP64 geometry values per Gauss point
 constexpr int kSolidFc = 25;   // SOLID81 F contributions per element (24 Fu + 1 Fp)
 
 struct ElementStatus {
@@ -16,7 +17,10 @@ struct ElementStatus {
 
 struct Solid81Args {
   uint32_t n_elems;
-  const double* Gt;         // dN/dX, structure of arrays: Gt[c * E8 + e*8 + g], c = 3*node + dim
+  // FP64: element geometry, structure of arrays geo[c * E8 + e*8 + g]: c = 0..5
+  // the metric dxi_p/dX . dxi_q/dX (11 12 13 22 23 33) and 6 the inverse det
+  // dX/dxi at Gauss point g, 7..9 the x, y, z coefficient of shape mode g
+  const double* geo;
   const double* wdet;       // Gauss weight * det J, [e*8 + g]
   const uint32_t* conn;     // 8 node ids per element, 1-based
   const uint32_t* node_eq3; // per node: equation numbers of UX, UY, UZ (1-based), 4 per node
@@ -40,18 +44,18 @@ struct Solid81Args {
   double* contribF;         // [E * 25]
   ElementStatus* status;
   // element range [e_begin, n_elems) of a mesh of n_total elements (the
-  // structure-of-arrays stride of Gt); e_begin a multiple of 4; n_total 0
+  // structure-of-arrays stride of geo / Gdf); e_begin a multiple of 4; n_total 0
   // means n_elems
   uint32_t e_begin;
   uint32_t n_total;
   // mixed precision only: inputs of the residual as float pairs (hi, lo)
-  // with hi + lo = the double to 2^-48 (Gdf replaces Gt, same layout); the
-  // residual is computed in float-pair arithmetic
+  // with hi + lo = the double to 2^-48; the residual is computed in
+  // float-pair arithmetic.  Gdf: dN/dX, Gdf[c * E8 + e*8 + g], c = 3*node + dim
   const float2* Gdf;
   const float2* wdf;        // w det J
   float2 mcd[5];            // material constants
   float2 inv_kbd;           // 1 / K
-  double inv_kb;            // 1 / K in FP64 (the mixed kernel's volumetric terms)
+  double inv_kb;            // 1 / K in FP64
   const float2* mesh_mat_df;  // per mesh: 8 pairs (-, c0..c4, K, 1/K) when elem_mesh != nullptr
   // optional: a device word; when non-null and non-zero the launch does
   // nothing (set by a kernel that found invalid indices in the inputs)
@@ -62,10 +66,10 @@ struct JacobianArgs {
   uint32_t n_elems;
   const double* xyz;
   const uint32_t* conn;
-  double* Gt;               // FP64 dN/dX, or nullptr
+  double* geo;              // FP64: the geometry of Solid81Args, or nullptr
   double* wdet;
   ElementStatus* status;
-  float2* Gdf;              // the same as float pairs (mixed precision), or nullptr
+  float2* Gdf;              // mixed precision: dN/dX as float pairs, or nullptr
   float2* wdf;
   // optional: a device word; when non-null and non-zero the launch does
   // nothing (set by a kernel that found invalid indices in the inputs)

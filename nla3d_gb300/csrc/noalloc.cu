@@ -6,8 +6,8 @@
 // where cudaMalloc's implicit device synchronisation and unpredictable cost
 // are not acceptable.  For them nla3d_assemble_solid81_noalloc() takes every
 // input and output as a device pointer owned by the caller and keeps its
-// intermediate data (per-Gauss-point shape-function gradients and the element
-// contributions) in a fixed array compiled into this library.
+// intermediate data (per-Gauss-point geometry and the element contributions)
+// in a fixed array compiled into this library.
 //
 // The array, g_noalloc_scratch, is NLA3D_NOALLOC_SCRATCH_BYTES (64 MiB) of
 // device memory that every GPU which loads the library holds until the
@@ -46,8 +46,8 @@ using namespace nla3d_gpu;
 namespace {
 
 constexpr uint64_t kScratchDoubles = NLA3D_NOALLOC_SCRATCH_BYTES / sizeof(double);
-// per element: Gt (24 x 8) + w det J (8) + K contributions (325) + F contributions (25)
-constexpr uint64_t kDoublesPerElem = 24 * 8 + 8 + kSolidKc + kSolidFc;
+// per element: geometry (10 x 8) + w det J (8) + K contributions (325) + F contributions (25)
+constexpr uint64_t kDoublesPerElem = kSolidGeo * 8 + 8 + kSolidKc + kSolidFc;
 static_assert(NLA3D_NOALLOC_MAX_ELEMS * kDoublesPerElem <= kScratchDoubles,
               "NLA3D_NOALLOC_MAX_ELEMS does not fit the scratch array");
 
@@ -141,8 +141,8 @@ extern "C" int nla3d_assemble_solid81_noalloc(const nla3d_solid81_noalloc_args* 
   if (rc != NLA3D_OK) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const uint64_t E = a->n_elems;
-  double* Gt = d->scratch;
-  double* wdet = Gt + 24 * 8 * E;
+  double* geo = d->scratch;
+  double* wdet = geo + kSolidGeo * 8 * E;
   double* contribK = wdet + 8 * E;
   double* contribF = contribK + kSolidKc * E;
 
@@ -156,13 +156,13 @@ extern "C" int nla3d_assemble_solid81_noalloc(const nla3d_solid81_noalloc_args* 
   check_inputs_kernel<<<304, 256, 0, s>>>(*a, d->bad);
   if (cudaGetLastError() != cudaSuccess) return NLA3D_ERR_CUDA;
 
-  JacobianArgs ja{a->n_elems, a->xyz, a->conn, Gt, wdet, d->status};
+  JacobianArgs ja{a->n_elems, a->xyz, a->conn, geo, wdet, d->status};
   ja.skip = d->bad;
   if (launch_solid81_jacobian(ja, s) != cudaSuccess) return NLA3D_ERR_CUDA;
 
   Solid81Args ea{};
   ea.n_elems = a->n_elems;
-  ea.Gt = Gt;
+  ea.geo = geo;
   ea.wdet = wdet;
   ea.conn = a->conn;
   ea.node_eq3 = a->node_eq;
@@ -175,6 +175,7 @@ extern "C" int nla3d_assemble_solid81_noalloc(const nla3d_solid81_noalloc_args* 
   ea.kbulk = a->mat_id == NLA3D_MAT_NEO_HOOKEAN ? a->mat_c[1]
                                                 : (a->mat_id == NLA3D_MAT_BIDERMAN ? a->mat_c[4]
                                                                                    : a->mat_c[2]);
+  ea.inv_kb = 1.0 / ea.kbulk;
   ea.contribK = contribK;
   ea.contribF = contribF;
   ea.status = d->status;
