@@ -209,75 +209,144 @@ struct BigBatch {
 };
 
 // step 1: LDL^T of the pb x pb diagonal block, and the inverse of its unit
-// lower factor (64 x 64 column-major, kept per panel for step 2 and the solves)
+// lower factor (64 x 64 column-major, kept per panel for step 2 and the solves).
+//
+// One CTA per front: a chain of 64 pivots, bound by the latency of one step.
+// Thread (r, cg) keeps row r, columns 16 cg .. +15 in registers (the front's
+// columns are read and written coalesced along r); the group that owns column p
+// publishes it (unscaled) in shared memory, and one barrier later every thread
+// scales its own row's entry by the pivot and updates its columns.  FP64: the
+// pivot's thread inverts it for everyone, since 256 FP64 divisions a step keep
+// the pipe busy longer than the update; FP32: every thread divides, off the
+// chain of the pivot's thread.  The inverse is formed blockwise: four 16 x 16
+// blocks by substitution (a thread per column), then X10 = -X1 (L10 X0) for 16
+// and 32.  54 -> 19 us (FP32) and 136 -> 82 us (FP64) a launch (ncu, cold)
+// against the block in shared memory, where each step's update ran as a chain
+// of dependent shared-memory accesses and the inverse row by row as another.
+constexpr int kDiagLd = kPanel + 1;
+
+// X10 = -X1 (L10 X0) for every pair of H x H diagonal blocks: a thread owns
+// H / 8 consecutive columns of one row
+template <typename T, int H>
+__device__ __forceinline__ void join_inverses(const T* Lr, T* X) {
+  constexpr int kOut = H / 8;
+  const int pr = threadIdx.x / (8 * H), i = (threadIdx.x / 8) % H, j0 = (threadIdx.x % 8) * kOut;
+  const int o = 2 * H * pr;
+  T v[kOut] = {};
+#pragma unroll 4
+  for (int q = j0; q < H; q++) {   // X0 is lower triangular
+    const T l = Lr[(o + H + i) * kDiagLd + o + q];
+#pragma unroll
+    for (int u = 0; u < kOut; u++) v[u] += l * X[(o + q) * kDiagLd + o + j0 + u];
+  }
+  T* out = X + (o + H + i) * kDiagLd + o + j0;
+#pragma unroll
+  for (int u = 0; u < kOut; u++) out[u] = v[u];   // L10 X0 in X10's place
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kOut; u++) v[u] = T(0);
+#pragma unroll 4
+  for (int q = 0; q <= i; q++) {   // X1 is lower triangular
+    const T x = X[(o + H + i) * kDiagLd + o + H + q];
+#pragma unroll
+    for (int u = 0; u < kOut; u++) v[u] -= x * X[(o + H + q) * kDiagLd + o + j0 + u];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kOut; u++) out[u] = v[u];
+  __syncthreads();
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
     batched_diag_kernel(BigBatch b, LdltDev d, T* __restrict__ front, int64_t p0,
                         T* __restrict__ Linv, const double* __restrict__ tau_p, double pivot_rel,
                         int* perturbed) {
-  extern __shared__ unsigned char diag_smem_raw[];
-  T(*B)[kPanel + 1] = reinterpret_cast<T(*)[kPanel + 1]>(diag_smem_raw);   // B[col][row]
-  unsigned char* diag_smem = diag_smem_raw + sizeof(T) * kPanel * (kPanel + 1);
+  static_assert(kThreads == 4 * kPanel, "four column groups of 16");
+  constexpr bool kShare = std::is_same<T, double>::value;
+  extern __shared__ __align__(16) unsigned char diag_smem_raw[];
+  T* Lr = reinterpret_cast<T*>(diag_smem_raw);   // Lr[r * kDiagLd + c]: unit lower factor
+  T* X = Lr + kPanel * kDiagLd;                  // X[r * kDiagLd + c]: its inverse
+  __shared__ __align__(16) T wcol[2][kPanel];
+  __shared__ T winv[2];
   const int s = b.list[blockIdx.x];
   const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
   const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
   if (p0 >= k) return;
   const int pb = (int)(k - p0 < kPanel ? k - p0 : kPanel);
-  T* F = front + d.front_off[s];
-  const int tc = threadIdx.x % kPanel, tr = threadIdx.x / kPanel;   // 64 columns x 4
-  for (int r = tr; r < pb; r += kThreads / kPanel)
-    if (tc < pb) B[tc][r] = r >= tc ? F[(p0 + r) + (p0 + tc) * m] : T(0);
-  __syncthreads();
+  T* F = front + d.front_off[s] + p0 + p0 * m;
+  const int r = threadIdx.x & (kPanel - 1), cg = threadIdx.x / kPanel;
+  T a[16];
+#pragma unroll
+  for (int j = 0; j < 16; j++) {
+    const int c = 16 * cg + j;
+    a[j] = r < pb && c <= r ? F[r + c * m] : (r == c ? T(1) : T(0));
+  }
   // the pivot bound in the front's precision (the guards compare in it)
   const T tau = (T)(pivot_rel * tau_p[0]);
-  // one barrier per pivot: every thread guards the pivot itself (only thread
-  // 0 counts); the columns right of p are updated with the unscaled column p
-  // (A_rc -= w_r w_c / d), which no later step writes, and every column is
-  // scaled by its pivot after the loop
-  for (int p = 0; p < pb; p++) {
-    const T raw = B[p][p];
-    const T dv = threadIdx.x == 0 ? guard_pivot(raw, tau, perturbed) : guard_value(raw, tau);
-    if (tc > p && tc < pb) {
-      const T lc = B[p][tc] / dv;
-      for (int r = tc + tr; r < pb; r += kThreads / kPanel) B[tc][r] -= B[p][r] * lc;
-    }
-    __syncthreads();
-  }
-  if (tc < pb) {
-    // column tc's diagonal is unchanged since its own step
-    const T dc = guard_value(B[tc][tc], tau);
-    for (int r = tc + 1 + tr; r < pb; r += kThreads / kPanel) B[tc][r] = B[tc][r] / dc;
-  }
-  __syncthreads();
-  if (threadIdx.x < pb) B[threadIdx.x][threadIdx.x] = guard_value(B[threadIdx.x][threadIdx.x], tau);
-  __syncthreads();
-  for (int r = tr; r < pb; r += kThreads / kPanel)
-    if (tc < pb && r >= tc) F[(p0 + r) + (p0 + tc) * m] = B[tc][r];
-  // inverse of the unit lower L11 in shared memory (X[col][row]): column c by
-  // the four consecutive lanes 4c .. 4c+3, row after row, each row's dot
-  // product split over the four lanes and summed by shuffles, so that only
-  // warp-level barriers separate the rows; then stored for step 2 and the solves
-  T(*X)[kPanel + 1] = reinterpret_cast<T(*)[kPanel + 1]>(diag_smem);
-  {
-    const int c = threadIdx.x >> 2, sub = threadIdx.x & 3;
-    if (c < pb)
-      for (int r = sub; r <= c; r += 4) X[c][r] = r == c ? T(1) : T(0);
-    __syncwarp();
-    for (int r = 1; r < pb; r++) {
-      T part = T(0);
-      if (c < r)
-        for (int q = c + sub; q < r; q += 4) part += B[q][r] * X[c][q];
-      part += __shfl_xor_sync(0xffffffffu, part, 1);
-      part += __shfl_xor_sync(0xffffffffu, part, 2);
-      if (sub == 0 && c < r) X[c][r] = -part;
-      __syncwarp();
+  for (int blk = 0; blk < 4; blk++) {
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+      const int p = 16 * blk + j;
+      if (p >= pb) break;
+      T* w = wcol[p & 1];
+      const bool own = cg == blk && r == p;
+      if (cg == blk) w[r] = a[j];
+      if (kShare && own) {
+        a[j] = guard_pivot(a[j], tau, perturbed);
+        winv[p & 1] = T(1) / a[j];
+      }
+      __syncthreads();
+      // (rows up to p are final; a warp holds 32 rows of one column group)
+      if (cg < blk || (r | 31) < p) continue;
+      T l;
+      if (kShare) {
+        l = w[r] * winv[p & 1];
+      } else {
+        // every thread guards the pivot itself; its owner counts and keeps it
+        const T dv = own ? guard_pivot(w[p], tau, perturbed) : guard_value(w[p], tau);
+        if (own) a[j] = dv;
+        l = w[r] / dv;
+      }
+      if (cg == blk) {
+#pragma unroll
+        for (int c = j + 1; c < 16; c++) a[c] -= l * w[16 * blk + c];
+        if (r > p) a[j] = l;
+      } else {
+#pragma unroll
+        for (int c = 0; c < 16; c++) a[c] -= l * w[16 * cg + c];
+      }
     }
   }
+#pragma unroll
+  for (int j = 0; j < 16; j++) {
+    const int c = 16 * cg + j;
+    if (r < pb && c <= r) F[r + c * m] = a[j];
+    Lr[r * kDiagLd + c] = r > c && r < pb ? a[j] : T(0);
+    X[r * kDiagLd + c] = r == c ? T(1) : T(0);
+  }
   __syncthreads();
+  if (threadIdx.x < kPanel) {
+    // columns of the four 16 x 16 diagonal blocks' inverses
+    const int o = threadIdx.x & ~15, c = threadIdx.x & 15;
+    T x[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      T v = T(0);
+#pragma unroll
+      for (int q = 0; q < i; q++) v += Lr[(o + i) * kDiagLd + o + q] * x[q];
+      x[i] = i < c ? T(0) : (i == c ? T(1) : -v);
+      if (i > c) X[(o + i) * kDiagLd + o + c] = x[i];
+    }
+  }
+  __syncthreads();
+  join_inverses<T, 16>(Lr, X);
+  join_inverses<T, 32>(Lr, X);
   T* Li = Linv + b.li_off[blockIdx.x] + (uint64_t)(p0 / kPanel) * kPanel * kPanel;
-  for (int t = threadIdx.x; t < pb * kPanel; t += blockDim.x) {
-    const int r = t % kPanel, c = t / kPanel;
-    if (r < pb) Li[r + c * kPanel] = X[c][r];
+#pragma unroll
+  for (int j = 0; j < 16; j++) {
+    const int c = 16 * cg + j;
+    if (r < pb && c < pb) Li[r + c * kPanel] = X[r * kDiagLd + c];
   }
 }
 
@@ -1845,7 +1914,7 @@ cudaError_t enqueue_factor(nla3d_ldlt* h, const double* values) {
       for (int64_t o0 = 0; o0 < L.large_max_k; o0 += kOuter) {
         const int64_t o_end = std::min<int64_t>(o0 + kOuter, L.large_max_k);
         for (int64_t p0 = o0; p0 < o_end; p0 += kPanel) {
-          batched_diag_kernel<T><<<nf, kThreads, 2 * sizeof(T) * kPanel * (kPanel + 1), st>>>(
+          batched_diag_kernel<T><<<nf, kThreads, 2 * sizeof(T) * kPanel * kDiagLd, st>>>(
               bb, h->dev, front, p0, Li, h->d_maxabs, h->pivot_rel, h->d_perturbed);
           const int64_t rest = L.large_max_m - p0 - 1;   // rows past the smallest panel
           if (rest <= 0) continue;
