@@ -38,6 +38,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <type_traits>
 #include <string>
 #include <vector>
@@ -51,7 +52,6 @@ constexpr int kThreads = 256;
 constexpr int kSmallFront = 128;   // fronts up to this many rows: one block each, in smem
 constexpr int kPanel = 64;         // panel width of the blocked path
 constexpr int kOuter = 256;        // outer block of the blocked path (4 panels)
-constexpr int kTile = 64;          // panel-row tile of the blocked path
 
 struct LdltDev {
   const uint64_t* front_off;
@@ -350,67 +350,6 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// step 2: the panel rows i >= q0 = p0+pb: W = F21 Linv^T (W = L21 D), F21 <- W D^-1;
-// 64-row tiles, 4 rows x 4 columns per thread
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-    batched_panel_kernel(BigBatch b, LdltDev d, T* __restrict__ front, int64_t p0,
-                         const T* __restrict__ Linv, T* __restrict__ Wbuf) {
-  __shared__ T As[16][kTile + 1];
-  __shared__ T Bs[16][kPanel + 1];
-  __shared__ T Dv[kPanel];
-  const int s = b.list[blockIdx.y];
-  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
-  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
-  if (p0 >= k) return;
-  const int pb = (int)(k - p0 < kPanel ? k - p0 : kPanel);
-  const int64_t q0 = p0 + pb;
-  const int64_t i0 = q0 + (int64_t)blockIdx.x * kTile;
-  if (i0 >= m) return;
-  T* F = front + d.front_off[s];
-  T* W = Wbuf + b.w_off[blockIdx.y];
-  const T* Li = Linv + b.li_off[blockIdx.y] + (uint64_t)(p0 / kPanel) * kPanel * kPanel;
-  for (int t = threadIdx.x; t < pb; t += blockDim.x) Dv[t] = F[(p0 + t) + (p0 + t) * m];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  T acc[4][4] = {};
-  for (int c0 = 0; c0 < pb; c0 += 16) {
-    for (int t = threadIdx.x; t < 16 * kTile; t += blockDim.x) {
-      const int cc = t / kTile, rr = t % kTile;
-      const int c2 = c0 + cc;
-      const int64_t i = i0 + rr;
-      As[cc][rr] = (c2 < pb && i < m) ? F[i + (p0 + c2) * m] : T(0);
-      // Bs[c2][c] = Linv[c][c2]
-      Bs[cc][rr] = (c2 < pb && rr < pb) ? Li[rr + c2 * kPanel] : T(0);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int cc = 0; cc < 16; cc++) {
-      T a[4], bb[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) a[u] = As[cc][ty * 4 + u];
-#pragma unroll
-      for (int v = 0; v < 4; v++) bb[v] = Bs[cc][tx * 4 + v];
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-#pragma unroll
-        for (int v = 0; v < 4; v++) acc[u][v] += a[u] * bb[v];
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int u = 0; u < 4; u++) {
-    const int64_t i = i0 + ty * 4 + u;
-    if (i >= m) continue;
-#pragma unroll
-    for (int v = 0; v < 4; v++) {
-      const int c = tx * 4 + v;
-      if (c >= pb) continue;
-      W[i + (int64_t)(p0 % kOuter + c) * m] = acc[u][v];
-      F[i + (p0 + c) * m] = acc[u][v] / Dv[c];
-    }
-  }
-}
-
 // step 3: update of the lower triangle, F[i][j] -= sum_c L[i][lc0 + c] W[j][wc0 + c]
 // for jb <= j < je, i >= j:
 //   inner (outer == 0, after panel p0): the panel's kw = pb columns into the
@@ -445,8 +384,9 @@ __device__ __forceinline__ bool update_range(int64_t p0, int outer, int64_t k, i
 }
 
 // BT x BT tiles (blockIdx.x rows, .y columns, both from jb), front
-// blockIdx.z, RT x RT outputs per thread (64 / 4 for FP64, whose FMA pipe
-// bounds it anyway; 128 / 8 for FP32).  A thread owns rows tx + 16u and
+// blockIdx.z, RT x RT outputs per thread (32 / 2 for FP64: its pipe bounds the
+// kernel, one SM takes 64 us for a 64 x 64 tile of a rank-64 update, and
+// smaller tiles reach more SMs; 128 / 8 for FP32).  A thread owns rows tx + 16u and
 // columns ty + 16v: shared-memory reads are conflict-free or broadcast and
 // the stores run down the columns.  The next 16-wide slice of the operands
 // is loaded into registers while the current one is multiplied.
@@ -523,7 +463,7 @@ __global__ void __launch_bounds__(kThreads)
 
 template <typename T>
 struct TrailingShape {
-  static constexpr int BT = 64, RT = 4;
+  static constexpr int BT = 32, RT = 2;
 };
 template <>
 struct TrailingShape<float> {
@@ -539,7 +479,6 @@ struct TrailingShape<float> {
 // operands taken in chunks of 32 columns, each chunk 4 k-steps x 3 MMAs
 // (hi.hi + hi.lo + lo.hi, FP32 accumulation in TMEM).
 constexpr int kTcM = 128, kTcN = 128, kTcKH = 32;   // tile rows, columns, K per chunk
-constexpr int kTcThreads = 256;                      // the packing kernel's block
 constexpr uint32_t kTcTileFloats = kTcM * kTcKH;     // one 128 x 32 operand chunk
 // instruction descriptor: D F32 (bit 4), A and B TF32 (bits 7, 10), both
 // K-major, N / 8 at bit 17, M / 16 at bit 24
@@ -594,11 +533,14 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t a, uint64_t b, ui
 //
 // An update (update_range: the rank-256 one after an outer block, or a
 // panel's rank-64 one inside its block) reads the same operands from every
-// tile of a row or column: L[jb + 128 r .. +127][lc0 .. lc0 + kw) and
-// W[jb + 128 r .. +127][wc0 .. wc0 + kw).  pack_update_kernel splits them
-// into TF32 high and low parts once per update and stores them, per 128-row
-// block r and 32-column chunk c, as four 16 KB tiles (A hi, A lo, B hi, B lo)
-// in the MMA's shared-memory layout (tc_off).  tc_packed_kernel is persistent
+// tile of a row or column: L and W = L D of its columns.  batched_panel_kernel
+// writes them once, split into TF32 high and low parts: per 128-row block
+// (counted from the outer block's first row o0) and 32-column chunk, four 16
+// KB tiles (A = L hi, lo, B = W hi, lo) in the MMA's shared-memory layout
+// (tc_off), so a panel's chunks serve its own update and the outer block's.
+// Tiles are aligned to o0; rows and columns of a tile outside the update's
+// range are computed from whatever their slots hold and not stored.
+// tc_packed_kernel is persistent
 // (one CTA per SM walking a host-built list of the level's tiles) and
 // warp-specialised:
 //   warp 0 (one lane): copies each chunk's four tiles into a ring of
@@ -624,46 +566,109 @@ constexpr int kPkStages = 3;
 constexpr size_t kPkSmem = (size_t)kPkStages * 4 * kPkTile * sizeof(float) + 256;
 constexpr int kOuterThreads = 320;   // tc_packed_kernel: producer, MMA, 8 epilogue warps
 
-__global__ void __launch_bounds__(kTcThreads)
-    pack_update_kernel(BigBatch b, LdltDev d, const float* __restrict__ front, int64_t p0,
-                       int outer, const float* __restrict__ Wbuf, float* __restrict__ packed) {
-  const int s = b.list[blockIdx.z];
+// step 2: the panel rows i >= q0 = p0+pb: W = F21 Linv^T (W = L21 D), F21 <- W
+// D^-1; PanelRows<T> rows per CTA, all 64 columns of both operands loaded at
+// once.  Thread (tx, ty) owns columns 4 tx .. +3 of rows ty + 16 u; a warp
+// holds two neighbouring tx, so it stops its sum where its columns of Linv^T
+// (upper triangular) end.  FP64: 16 rows per CTA, since one SM's FP64 pipe
+// would take 64 us for 64 rows and most launches have fewer tiles than SMs.
+// Tensor-core fronts (kPack): instead of W, both operands of the updates that
+// follow are written here, split and in the MMA's layout (see tc_packed_kernel).
+template <typename T>
+struct PanelRows {
+  static constexpr int value = 64;
+};
+template <>
+struct PanelRows<double> {
+  static constexpr int value = 16;
+};
+
+template <typename T, bool kPack>
+__global__ void __launch_bounds__(kThreads)
+    batched_panel_kernel(BigBatch b, LdltDev d, T* __restrict__ front, int64_t p0,
+                         const T* __restrict__ Linv, T* __restrict__ Wbuf,
+                         float* __restrict__ packed) {
+  constexpr int R = PanelRows<T>::value, RU = R / 16;
+  __shared__ T As[kPanel][R];
+  __shared__ __align__(16) T Bs[kPanel][kPanel];
+  __shared__ T Dv[kPanel];
+  const int s = b.list[blockIdx.y];
   const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
   const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
-  UpdateRange ur;
-  if (!update_range(p0, outer, k, m, ur)) return;
-  const int rb = blockIdx.x, ch = blockIdx.y;
-  const int64_t r0 = ur.jb + (int64_t)rb * kTcM;
-  if (r0 >= m || ch * kTcKH >= ur.kw) return;
-  const float* F = front + d.front_off[s];
-  const float* W = Wbuf + b.w_off[blockIdx.z];
-  float* P = packed + b.pk_off[blockIdx.z] + (uint64_t)(rb * kPkChunks + ch) * 4 * kPkTile;
-  // thread: row r, four groups of 4 consecutive columns (16-byte stores)
-  const int r = threadIdx.x % kTcM, g0 = (threadIdx.x / kTcM) * 4;
-  const int64_t i = r0 + r;
+  if (p0 >= k) return;
+  const int pb = (int)(k - p0 < kPanel ? k - p0 : kPanel);
+  const int64_t q0 = p0 + pb;
+  const int64_t i0 = q0 + (int64_t)blockIdx.x * R;
+  if (i0 >= m) return;
+  T* F = front + d.front_off[s];
+  const T* Li = Linv + b.li_off[blockIdx.y] + (uint64_t)(p0 / kPanel) * kPanel * kPanel;
+  if (threadIdx.x < kPanel)
+    Dv[threadIdx.x] = threadIdx.x < pb ? F[(p0 + threadIdx.x) * (m + 1)] : T(1);
 #pragma unroll
-  for (int g = g0; g < g0 + 4; g++) {
-    float4 ah, al, wh, wl;
-    float* ahp = &ah.x;
-    float* alp = &al.x;
-    float* whp = &wh.x;
-    float* wlp = &wl.x;
+  for (int q = 0; q < kPanel * R / kThreads; q++) {
+    const int t = threadIdx.x + q * kThreads;
+    const int rr = t % R, c2 = t / R;
+    As[c2][rr] = (c2 < pb && i0 + rr < m) ? F[i0 + rr + (p0 + c2) * m] : T(0);
+  }
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const int c = ch * kTcKH + g * 4 + e;
-      const bool in = c < ur.kw && i < m;
-      const float av = in ? F[i + (ur.lc0 + c) * m] : 0.0f;
-      const float wv = in && i < ur.je ? W[i + (ur.wc0 + c) * m] : 0.0f;   // B: columns < je
-      ahp[e] = tf32_hi(av);
-      alp[e] = av - ahp[e];
-      whp[e] = tf32_hi(wv);
-      wlp[e] = wv - whp[e];
+  for (int q = 0; q < kPanel * kPanel / kThreads; q++) {
+    const int t = threadIdx.x + q * kThreads;
+    const int c = t % kPanel, c2 = t / kPanel;
+    Bs[c2][c] = (c2 < pb && c < pb) ? Li[c + c2 * kPanel] : T(0);   // Linv[c][c2]
+  }
+  __syncthreads();
+  const int tx = threadIdx.x / 16, ty = threadIdx.x % 16;
+  const int end = min(pb, 8 * (int)(threadIdx.x / 32) + 8);
+  T acc[RU][4] = {};
+#pragma unroll 4
+  for (int c2 = 0; c2 < end; c2++) {
+    T bb[4];
+#pragma unroll
+    for (int v = 0; v < 4; v++) bb[v] = Bs[c2][tx * 4 + v];
+#pragma unroll
+    for (int u = 0; u < RU; u++) {
+      const T av = As[c2][ty + 16 * u];
+#pragma unroll
+      for (int v = 0; v < 4; v++) acc[u][v] += av * bb[v];
     }
-    const uint32_t o = tc_off(r, g * 4);
-    *reinterpret_cast<float4*>(P + o) = ah;
-    *reinterpret_cast<float4*>(P + kPkTile + o) = al;
-    *reinterpret_cast<float4*>(P + 2 * kPkTile + o) = wh;
-    *reinterpret_cast<float4*>(P + 3 * kPkTile + o) = wl;
+  }
+#pragma unroll
+  for (int u = 0; u < RU; u++) {
+    const int64_t i = i0 + ty + 16 * u;
+    if (i >= m) continue;
+    T l[4];
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+      const int c = tx * 4 + v;
+      l[v] = acc[u][v] / Dv[c];
+      if (c >= pb) continue;
+      F[i + (p0 + c) * m] = l[v];
+      if constexpr (!kPack)
+        Wbuf[b.w_off[blockIdx.y] + i + (int64_t)(p0 % kOuter + c) * m] = acc[u][v];
+    }
+    if constexpr (kPack) {
+      // columns past pb are zeros: they end the update's last chunk
+      const int64_t rel = i - (p0 - p0 % kOuter);
+      const int c = (int)(p0 % kOuter) + tx * 4;
+      float* P = packed + b.pk_off[blockIdx.y] +
+                 ((uint64_t)(rel / kTcM) * kPkChunks + c / kTcKH) * 4 * kPkTile +
+                 tc_off((int)(rel % kTcM), c % kTcKH);
+      float h[4], e[4];
+#pragma unroll
+      for (int v = 0; v < 4; v++) {
+        h[v] = tf32_hi(l[v]);
+        e[v] = l[v] - h[v];
+      }
+      *reinterpret_cast<float4*>(P) = make_float4(h[0], h[1], h[2], h[3]);
+      *reinterpret_cast<float4*>(P + kPkTile) = make_float4(e[0], e[1], e[2], e[3]);
+#pragma unroll
+      for (int v = 0; v < 4; v++) {
+        h[v] = tf32_hi(acc[u][v]);
+        e[v] = acc[u][v] - h[v];
+      }
+      *reinterpret_cast<float4*>(P + 2 * kPkTile) = make_float4(h[0], h[1], h[2], h[3]);
+      *reinterpret_cast<float4*>(P + 3 * kPkTile) = make_float4(e[0], e[1], e[2], e[3]);
+    }
   }
 }
 
@@ -680,8 +685,9 @@ __device__ __forceinline__ void expect_tx(uint32_t mbar, uint32_t bytes) {
                : "memory");
 }
 
-// one update tile of the level's outer-block list: large front z (index in
-// the level's list), tile row ti >= tile column tj
+// one update tile of a level's list: large front z (index in the level's
+// list), 128-row block ti and 128-column block tj <= ti from the outer block's
+// first row
 struct OuterTile {
   uint32_t z, tij;   // tij = ti << 16 | tj
 };
@@ -727,7 +733,7 @@ __global__ void __launch_bounds__(kOuterThreads, 1)
   };
   // the front of a tile: rows m, update range, chunks
   struct TileInfo {
-    int64_t m, je, i0, j0;
+    int64_t m, jb, je, i0, j0;
     int nch;
     const float* pa;
     const float* pb;
@@ -741,13 +747,16 @@ __global__ void __launch_bounds__(kOuterThreads, 1)
     UpdateRange ur;
     update_range(p0, outer, k, m, ur);   // the host listed only fronts whose range is not empty
     const uint32_t rI = ot.tij >> 16, rJ = ot.tij & 0xFFFFu;
+    const int64_t o0 = p0 - p0 % kOuter;
     ti.m = m;
+    ti.jb = ur.jb;
     ti.je = ur.je;
-    ti.i0 = ur.jb + (int64_t)rI * kTcM;
-    ti.j0 = ur.jb + (int64_t)rJ * kTcN;
+    ti.i0 = o0 + (int64_t)rI * kTcM;
+    ti.j0 = o0 + (int64_t)rJ * kTcN;
     ti.nch = (int)((ur.kw + kTcKH - 1) / kTcKH);
-    ti.pa = packed + b.pk_off[ot.z] + (uint64_t)rI * kPkBlock;
-    ti.pb = packed + b.pk_off[ot.z] + (uint64_t)rJ * kPkBlock;
+    const uint64_t chunk = (uint64_t)(ur.wc0 / kTcKH) * 4 * kPkTile;
+    ti.pa = packed + b.pk_off[ot.z] + (uint64_t)rI * kPkBlock + chunk;
+    ti.pb = packed + b.pk_off[ot.z] + (uint64_t)rJ * kPkBlock + chunk;
     ti.F = front + d.front_off[s];
   };
   bool ok = true;
@@ -844,7 +853,8 @@ __global__ void __launch_bounds__(kOuterThreads, 1)
       // the front's values of the first 32 columns first: their loads overlap
       // the tile's MMAs; the second 32 load while the first are stored
       float* fp = ti.F + i + (ti.j0 + cb) * ti.m;   // (i, j0 + cb); column stride m
-      const int64_t jlim = (row_in ? (i < ti.je - 1 ? i : ti.je - 1) : -1) - (ti.j0 + cb);
+      const int jlim = (int)((row_in ? (i < ti.je - 1 ? i : ti.je - 1) : -1) - (ti.j0 + cb));
+      const int jlo = (int)(ti.jb - (ti.j0 + cb));
       float cv[32];
 #pragma unroll
       for (int q = 0; q < 32; q++) cv[q] = q <= jlim ? fp[q * ti.m] : 0.0f;
@@ -881,11 +891,13 @@ __global__ void __launch_bounds__(kOuterThreads, 1)
         float nv[32];
         if (h == 0) {
 #pragma unroll
-          for (int q = 0; q < 32; q++) nv[q] = 32 + q <= jlim ? fp[(32 + q) * ti.m] : 0.0f;
+          for (int q = 0; q < 32; q++)
+            nv[q] = 32 + q <= jlim ? fp[(32 + q) * ti.m] : 0.0f;
         }
 #pragma unroll
         for (int q = 0; q < 32; q++)
-          if (h * 32 + q <= jlim) fp[(h * 32 + q) * ti.m] = cv[q] - __uint_as_float(v[q]);
+          if (h * 32 + q >= jlo && h * 32 + q <= jlim)
+            fp[(h * 32 + q) * ti.m] = cv[q] - __uint_as_float(v[q]);
         if (h == 0) {
 #pragma unroll
           for (int q = 0; q < 32; q++) cv[q] = nv[q];
@@ -1918,44 +1930,41 @@ cudaError_t enqueue_factor(nla3d_ldlt* h, const double* values) {
               bb, h->dev, front, p0, Li, h->d_maxabs, h->pivot_rel, h->d_perturbed);
           const int64_t rest = L.large_max_m - p0 - 1;   // rows past the smallest panel
           if (rest <= 0) continue;
-          const unsigned tiles = (unsigned)((rest + kTile - 1) / kTile);
-          batched_panel_kernel<T><<<dim3(tiles, nf), kThreads, 0, st>>>(bb, h->dev, front, p0,
-                                                                         Li, W);
-          // the panel's columns into the rest of its outer block (at most
-          // kOuter - kPanel columns)
-          if (p0 + kPanel < o_end) {
-            const int64_t pi = p0 / kPanel;
-            if (tc && L.itile_cnt[pi] > 0) {
-              const unsigned rb = (unsigned)((rest + kTcM - 1) / kTcM);
-              pack_update_kernel<<<dim3(rb, kPanel / kTcKH, nf), kTcThreads, 0, st>>>(
-                  bb, h->dev, reinterpret_cast<const float*>(front), p0, 0,
-                  reinterpret_cast<const float*>(W), h->d_pk);
+          constexpr int R = PanelRows<T>::value;
+          const dim3 panel_grid((unsigned)((rest + R - 1) / R), nf);
+          if constexpr (std::is_same<T, float>::value) {
+            if (tc) {
+              batched_panel_kernel<float, true><<<panel_grid, kThreads, 0, st>>>(
+                  bb, h->dev, front, p0, Li, nullptr, h->d_pk);
+              // the panel's columns into the rest of its outer block
+              const int64_t pi = p0 / kPanel;
               const int nt = (int)L.itile_cnt[pi];
-              tc_packed_kernel<<<(unsigned)std::min(nt, h->n_sm), kOuterThreads, kPkSmem, st>>>(
-                  bb, h->dev, reinterpret_cast<float*>(front), p0, 0, h->d_pk,
-                  h->d_tiles + L.itile_off[pi], nt, h->d_err);
-            } else if (!tc) {
-              update(p0, 0, rest, (unsigned)((kOuter - kPanel + BT - 1) / BT));
+              if (nt > 0)
+                tc_packed_kernel<<<(unsigned)std::min(nt, h->n_sm), kOuterThreads, kPkSmem, st>>>(
+                    bb, h->dev, front, p0, 0, h->d_pk, h->d_tiles + L.itile_off[pi], nt, h->d_err);
+              continue;
             }
           }
+          batched_panel_kernel<T, false><<<panel_grid, kThreads, 0, st>>>(bb, h->dev, front, p0, Li,
+                                                                         W, nullptr);
+          // (at most kOuter - kPanel columns)
+          if (p0 + kPanel < o_end)
+            update(p0, 0, rest, (unsigned)((kOuter - kPanel + BT - 1) / BT));
         }
-        // the outer block into every column after it (tensor-core fronts:
-        // its operands packed once, then the tiles with bulk copies)
+        // the outer block into every column after it
         const int64_t rest = L.large_max_m - o0 - 1;
-        if (rest > 0 && tc) {
-          const unsigned rb = (unsigned)((rest + kTcM - 1) / kTcM);
-          pack_update_kernel<<<dim3(rb, kPkChunks, nf), kTcThreads, 0, st>>>(
-              bb, h->dev, reinterpret_cast<const float*>(front), o0, 1,
-              reinterpret_cast<const float*>(W), h->d_pk);
-          const int64_t ob = o0 / kOuter;
-          const int nt = (int)L.tile_cnt[ob];
-          if (nt > 0)
-            tc_packed_kernel<<<(unsigned)std::min(nt, h->n_sm), kOuterThreads, kPkSmem, st>>>(
-                bb, h->dev, reinterpret_cast<float*>(front), o0, 1, h->d_pk,
-                h->d_tiles + L.tile_off[ob], nt, h->d_err);
-        } else if (rest > 0) {
-          update(o0, 1, rest, ~0u);
+        if (rest <= 0) continue;
+        if constexpr (std::is_same<T, float>::value) {
+          if (tc) {
+            const int64_t ob = o0 / kOuter;
+            const int nt = (int)L.tile_cnt[ob];
+            if (nt > 0)
+              tc_packed_kernel<<<(unsigned)std::min(nt, h->n_sm), kOuterThreads, kPkSmem, st>>>(
+                  bb, h->dev, front, o0, 1, h->d_pk, h->d_tiles + L.tile_off[ob], nt, h->d_err);
+            continue;
+          }
         }
+        update(o0, 1, rest, ~0u);
       }
     }
   }
@@ -2143,9 +2152,9 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
           if (o0 >= k) continue;
           const int64_t jb = std::min<int64_t>(o0 + kOuter, k);
           if (jb >= m) continue;
-          const int64_t rb = (m - jb + kTcM - 1) / kTcM;
-          for (int64_t ti = 0; ti < rb; ti++)
-            for (int64_t tj = 0; tj <= ti; tj++)
+          const int64_t b0 = (jb - o0) / kTcM, rb = (m - o0 + kTcM - 1) / kTcM;
+          for (int64_t ti = b0; ti < rb; ti++)
+            for (int64_t tj = b0; tj <= ti; tj++)
               tiles.push_back(OuterTile{(uint32_t)z, (uint32_t)(ti << 16 | tj)});
         }
         lv.tile_cnt.push_back((int64_t)tiles.size() - lv.tile_off.back());
@@ -2162,9 +2171,10 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
           const int64_t jb = p0 + std::min<int64_t>(kPanel, k - p0);
           const int64_t je = std::min<int64_t>(o0 + kOuter, k);
           if (jb >= je) continue;
-          const int64_t rb = (m - jb + kTcM - 1) / kTcM, cb = (je - jb + kTcN - 1) / kTcN;
-          for (int64_t ti = 0; ti < rb; ti++)
-            for (int64_t tj = 0; tj <= ti && tj < cb; tj++)
+          const int64_t b0 = (jb - o0) / kTcM, rb = (m - o0 + kTcM - 1) / kTcM;
+          const int64_t cb = (je - o0 + kTcN - 1) / kTcN;
+          for (int64_t ti = b0; ti < rb; ti++)
+            for (int64_t tj = b0; tj <= ti && tj < cb; tj++)
               tiles.push_back(OuterTile{(uint32_t)z, (uint32_t)(ti << 16 | tj)});
         }
         lv.itile_cnt.push_back((int64_t)tiles.size() - lv.itile_off.back());
@@ -2232,7 +2242,8 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
     LCK(dalloc(h, reinterpret_cast<double**>(&h->d_front), h->front_entries));
   const size_t nlinv = (size_t)std::max<uint64_t>(li_total, 1);
   if (precision) {
-    LCK(dalloc(h, reinterpret_cast<float**>(&h->d_W), (size_t)max_w));
+    // (tensor-core fronts keep the panels' operands packed instead)
+    LCK(dalloc(h, reinterpret_cast<float**>(&h->d_W), h->tc ? 1 : (size_t)max_w));
     LCK(dalloc(h, reinterpret_cast<float**>(&h->d_Linv), nlinv));
     LCK(cudaFuncSetAttribute(batched_diag_kernel<float>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2620,9 +2631,28 @@ int nla3d_ldlt_tc_check(int m, double* out) {
   float *F1 = nullptr, *F3 = nullptr, *dW = nullptr, *dP = nullptr;
   const size_t mp = (size_t)((m + kTcM - 1) / kTcM) * kPkBlock;
   std::vector<OuterTile> tl;   // the outer update's tiles, as the factorisation lists them
-  const int rbk = (m - kb + kTcM - 1) / kTcM;
-  for (int ti = 0; ti < rbk; ti++)
-    for (int tj = 0; tj <= ti; tj++) tl.push_back(OuterTile{0u, (uint32_t)(ti << 16 | tj)});
+  const int rbk = (m + kTcM - 1) / kTcM, b0 = kb / kTcM;
+  for (int ti = b0; ti < rbk; ti++)
+    for (int tj = b0; tj <= ti; tj++) tl.push_back(OuterTile{0u, (uint32_t)(ti << 16 | tj)});
+  // the operands as the panel kernel packs them (hi: to nearest, ties away)
+  std::vector<float> P(mp, 0.0f);
+  auto hi = [](float v) {
+    uint32_t u;
+    std::memcpy(&u, &v, 4);
+    u = (u + 0x1000u) & 0xFFFFE000u;
+    std::memcpy(&v, &u, 4);
+    return v;
+  };
+  for (int i = 0; i < m; i++)
+    for (int c = 0; c < kb; c++) {
+      float* t = P.data() + ((size_t)(i / kTcM) * kPkChunks + c / kTcKH) * 4 * kPkTile +
+                 (((i % kTcM) >> 3) * (kTcKH / 4) + ((c % kTcKH) >> 2)) * 32 + (i & 7) * 4 + (c & 3);
+      const float l = F0[(size_t)i + (size_t)c * m], w = W[(size_t)i + (size_t)c * m];
+      t[0] = hi(l);
+      t[kPkTile] = l - t[0];
+      t[2 * kPkTile] = hi(w);
+      t[3 * kPkTile] = w - t[2 * kPkTile];
+    }
   OuterTile* dT = nullptr;
   int n_sm = 1, dev = 0;
   int* err = nullptr;
@@ -2672,10 +2702,10 @@ int nla3d_ldlt_tc_check(int m, double* out) {
     const unsigned t128 = (unsigned)((rest + 127) / 128);
     batched_trailing_kernel<float, 128, 8><<<dim3(t128, t128, 1), kThreads>>>(bb, d, F1, 0, 1,
                                                                                dW);
-    pack_update_kernel<<<dim3(t128, kPkChunks, 1), kTcThreads>>>(bb, d, F3, 0, 1, dW, dP);
+    e = cudaMemcpy(dP, P.data(), mp * 4, cudaMemcpyHostToDevice);
     tc_packed_kernel<<<(unsigned)std::min<int>((int)tl.size(), n_sm), kOuterThreads, kPkSmem>>>(
         bb, d, F3, 0, 1, dP, dT, (int)tl.size(), err);
-    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e == cudaSuccess) e = cudaMemcpy(&tc_err, err, 4, cudaMemcpyDeviceToHost);
   }
