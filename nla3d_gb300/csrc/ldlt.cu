@@ -52,6 +52,9 @@ constexpr int kThreads = 256;
 constexpr int kSmallFront = 128;   // fronts up to this many rows: one block each, in smem
 constexpr int kPanel = 64;         // panel width of the blocked path
 constexpr int kOuter = 256;        // outer block of the blocked path (4 panels)
+constexpr int kInv = 512;          // pivots whose triangle is kept inverted for the solves
+constexpr int kNarrow = kPanel;    // fronts with up to this many pivots: one CTA per solve pass
+constexpr int kNarrowRows = 4096;  // ... and up to this many rows
 
 struct LdltDev {
   const uint64_t* front_off;
@@ -347,6 +350,119 @@ __global__ void __launch_bounds__(kThreads)
   for (int j = 0; j < 16; j++) {
     const int c = 16 * cg + j;
     if (r < pb && c < pb) Li[r + c * kPanel] = X[r * kDiagLd + c];
+    // and for the solves in the front's unused upper triangle, row c of the
+    // inverse down column c (here r runs over the row's entries)
+    if (r < c && c < pb) F[r + c * m] = X[c * kDiagLd + r];
+  }
+}
+
+// ---- inverses of the kInv x kInv diagonal blocks, for the solves ----
+//
+// A substitution through 64-pivot blocks is a chain of dependent launches as
+// long as the front's pivots; through the inverses X of larger blocks it is
+// two products per block.  Once a level is factored, its fronts' inverses are
+// joined in pairs on a second stream while the next levels are factored:
+// blocks of s = 64, 128, 256 pivots, X_CA = -X_C (L_CA X_A), two launches per
+// doubling over all pairs of the level.  X (unit lower triangular, diagonal
+// not stored) lies transposed in the front's upper triangle, X[i][j] at
+// row j of column i: it needs no memory, no kernel of the factorisation reads
+// there, and a row of X is contiguous.  kInv = 512: the joins of the
+// 139k-equation bar take 0.9 ms of kernels beside a 14 ms factorisation; a
+// doubling more costs four times the work of all before it.
+struct InvTask {
+  uint32_t z, j0;     // large front (index in the level's list), first pivot of the pair
+  uint32_t tile;      // row tile of C << 16 | column tile of A
+};
+
+template <typename T>
+struct InvTile {
+  static constexpr int BT = 64, RT = 4;
+};
+template <>
+struct InvTile<double> {
+  static constexpr int BT = 32, RT = 2;   // as the trailing updates
+};
+
+// pass 0: T = L_CA X_A;  pass 1: X_CA = -X_C T.  T: row c, kInv / 2 columns
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+    inv_join_kernel(const InvTask* __restrict__ tasks, BigBatch b, LdltDev d,
+                    T* __restrict__ front, const uint64_t* __restrict__ t_off,
+                    T* __restrict__ work, int s, int pass) {
+  constexpr int BT = InvTile<T>::BT, RT = InvTile<T>::RT, KS = 16;
+  constexpr int LPT = KS * BT / kThreads;
+  constexpr int kLdT = kInv / 2;
+  __shared__ T As[KS][BT + 1];
+  __shared__ T Bs[KS][BT + 1];
+  const InvTask t = tasks[blockIdx.x];
+  const int sn = b.list[t.z];
+  const int64_t m = d.row_ptr[sn + 1] - d.row_ptr[sn];
+  const int k = d.sn_first[sn + 1] - d.sn_first[sn];
+  T* F = front + d.front_off[sn];
+  T* W = work + t_off[t.z];
+  const int j0 = (int)t.j0, c0 = j0 + s + (int)(t.tile >> 16) * BT;
+  const int a0 = j0 + (int)(t.tile & 0xFFFFu) * BT;
+  const int cend = min(j0 + 2 * s, k);
+  const int qbeg = pass == 0 ? a0 : j0 + s;
+  const int qend = pass == 0 ? j0 + s : min(c0 + BT, cend);
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+  T acc[RT][RT] = {};
+  T ra[LPT], rb[LPT];
+  auto load = [&](int q0) {
+#pragma unroll
+    for (int e = 0; e < LPT; e++) {
+      const int i = threadIdx.x + e * kThreads;
+      const int rr = i % BT, q = q0 + i / BT;
+      if (pass == 0) {
+        const int c = c0 + rr, a = a0 + rr;
+        ra[e] = c < cend && q < qend ? F[c + (int64_t)q * m] : T(0);
+        rb[e] = q >= qend ? T(0) : q > a ? F[a + (int64_t)q * m] : q == a ? T(1) : T(0);
+      } else {
+        // X_C's rows run along q
+        const int q2 = q0 + i % KS, c = c0 + i / KS;
+        ra[e] = c >= cend || q2 >= qend ? T(0)
+                : c > q2                ? F[q2 + (int64_t)c * m]
+                : c == q2               ? T(1)
+                                        : T(0);
+        rb[e] = q < qend ? W[(uint64_t)q * kLdT + (a0 - j0) + rr] : T(0);
+      }
+    }
+  };
+  load(qbeg);
+  for (int q0 = qbeg; q0 < qend; q0 += KS) {
+#pragma unroll
+    for (int e = 0; e < LPT; e++) {
+      const int i = threadIdx.x + e * kThreads;
+      if (pass == 0) As[i / BT][i % BT] = ra[e];
+      else As[i % KS][i / KS] = ra[e];
+      Bs[i / BT][i % BT] = rb[e];
+    }
+    __syncthreads();
+    if (q0 + KS < qend) load(q0 + KS);
+#pragma unroll
+    for (int q = 0; q < KS; q++) {
+      T av[RT], bv[RT];
+#pragma unroll
+      for (int u = 0; u < RT; u++) av[u] = As[q][ty + 16 * u];
+#pragma unroll
+      for (int v = 0; v < RT; v++) bv[v] = Bs[q][tx + 16 * v];
+#pragma unroll
+      for (int u = 0; u < RT; u++)
+#pragma unroll
+        for (int v = 0; v < RT; v++) acc[u][v] += av[u] * bv[v];
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int u = 0; u < RT; u++) {
+    const int c = c0 + ty + 16 * u;
+    if (c >= cend) continue;
+#pragma unroll
+    for (int v = 0; v < RT; v++) {
+      const int a = a0 + tx + 16 * v;
+      if (pass == 0) W[(uint64_t)c * kLdT + a - j0] = acc[u][v];
+      else F[a + (int64_t)c * m] = -acc[u][v];
+    }
   }
 }
 
@@ -915,126 +1031,22 @@ __global__ void __launch_bounds__(kOuterThreads, 1)
 
 // ---- solve kernels ----
 
-__global__ void solve_init_kernel(int64_t n, const int32_t* __restrict__ perm,
-                                  const int32_t* __restrict__ col2sn, LdltDev d,
-                                  const double* __restrict__ b, double* __restrict__ vec) {
-  const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const int s = col2sn[j];
-  vec[d.vec_off[s] + (j - d.sn_first[s])] = b[perm[j]];
-}
-
-__global__ void vec_extend_add_kernel(const int32_t* __restrict__ children, LdltDev d,
-                                      double* __restrict__ vec) {
-  const int c = children[blockIdx.x];
-  const int p = d.sn_parent[c];
-  const int64_t mc = d.row_ptr[c + 1] - d.row_ptr[c];
-  const int64_t kc = d.sn_first[c + 1] - d.sn_first[c];
-  const double* src = vec + d.vec_off[c] + kc;
-  double* dst = vec + d.vec_off[p];
-  const uint32_t* rel = d.rel + d.rel_ptr[c];
-  for (int64_t i = threadIdx.x; i < mc - kc; i += blockDim.x) dst[rel[i]] += src[i];
-}
-
-// forward: v[0:k] <- D^-1 L11^-1 v[0:k], v[k:m] <- v[k:m] - L21 (L11^-1 v[0:k]);
-// blocks of 64 pivots: the block's unit triangle in shared memory, then one
-// pass over the rows below it
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-    forward_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
-                   double* __restrict__ vec) {
-  __shared__ double yb[kPanel];
-  const int s = list[blockIdx.x];
-  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
-  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
-  const T* F = front + d.front_off[s];
-  double* v = vec + d.vec_off[s];
-  for (int64_t c0 = 0; c0 < k; c0 += kPanel) {
-    const int cb = (int)(k - c0 < kPanel ? k - c0 : kPanel);
-    if (threadIdx.x < cb) yb[threadIdx.x] = v[c0 + threadIdx.x];
-    __syncthreads();
-    for (int c = 0; c < cb; c++) {
-      const int t = threadIdx.x;
-      if (t > c && t < cb) yb[t] -= (double)F[(c0 + t) + (c0 + c) * m] * yb[c];
-      __syncthreads();
-    }
-    if (threadIdx.x < cb) v[c0 + threadIdx.x] = yb[threadIdx.x];
-    for (int64_t i = c0 + cb + threadIdx.x; i < m; i += blockDim.x) {
-      double acc = 0.0;
-      for (int c = 0; c < cb; c++) acc += (double)F[i + (c0 + c) * m] * yb[c];
-      v[i] -= acc;
-    }
-    __syncthreads();
-  }
-  for (int64_t c = threadIdx.x; c < k; c += blockDim.x) v[c] /= (double)F[c + c * m];
-}
-
-// backward: x[0:k] = L11^-T (v[0:k] - L21^T x_rest), x_rest gathered from the
-// solved ancestors (factor order), written to xf; blocks of 64 pivots from the
-// last: the contributions of the solved pivots below the block (a warp per
-// column), then the block's triangle in shared memory
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-    backward_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
-                    double* __restrict__ vec, double* __restrict__ xf) {
-  __shared__ double xb[kPanel];
-  const int s = list[blockIdx.x];
-  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
-  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
-  const int32_t* rows = d.rows + d.row_ptr[s];
-  const T* F = front + d.front_off[s];
-  double* v = vec + d.vec_off[s];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nwarps = blockDim.x / 32;
-  for (int64_t c = warp; c < k; c += nwarps) {
-    double acc = 0.0, acc2 = 0.0;
-    int64_t i = k + lane;
-    for (; i + 32 < m; i += 64) {
-      acc += (double)F[i + c * m] * xf[rows[i]];
-      acc2 += (double)F[i + 32 + c * m] * xf[rows[i + 32]];
-    }
-    if (i < m) acc += (double)F[i + c * m] * xf[rows[i]];
-    acc += acc2;
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (lane == 0) v[c] -= acc;
-  }
-  __syncthreads();
-  for (int64_t c0 = ((k - 1) / kPanel) * kPanel; c0 >= 0; c0 -= kPanel) {
-    const int cb = (int)(k - c0 < kPanel ? k - c0 : kPanel);
-    for (int c = warp; c < cb; c += nwarps) {
-      double acc = 0.0;
-      for (int64_t i = c0 + cb + lane; i < k; i += 32) acc += (double)F[i + (c0 + c) * m] * v[i];
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-      if (lane == 0) xb[c] = v[c0 + c] - acc;
-    }
-    __syncthreads();
-    for (int c = cb - 1; c >= 0; c--) {
-      const int t = threadIdx.x;
-      if (t < c) xb[t] -= (double)F[(c0 + c) + (c0 + t) * m] * xb[c];
-      __syncthreads();
-    }
-    if (threadIdx.x < cb) v[c0 + threadIdx.x] = xb[threadIdx.x];
-    __syncthreads();
-  }
-  const int32_t f = d.sn_first[s];
-  for (int64_t c = threadIdx.x; c < k; c += blockDim.x) xf[f + c] = v[c];
-}
-
-// Solves of the large supernodes, batched per level like their factorisation
-// (blockIdx picks the supernode in the level's large list; each 64-pivot
-// diagonal block applied through its stored inverse).
-
-// after the forward panels: v[0:k] <- D^-1 v[0:k]
-template <typename T>
-__global__ void scale_pivots_kernel(BigBatch b, LdltDev d, const T* __restrict__ front,
-                                    double* __restrict__ vec) {
-  const int s = b.list[blockIdx.y];
-  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
-  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= k) return;
-  const T* F = front + d.front_off[s];
-  vec[d.vec_off[s] + c] /= (double)F[c + c * m];
+// The vectors of one level's fronts before its forward pass, one thread per
+// row: the right-hand side for a pivot row, plus the children's update rows in
+// child order (a list per row, built with the schedule).  The rows of a level
+// are contiguous, so this is one launch; adding one child ordinal per launch
+// took 100 launches a pass on the 139k-equation bar (0.6 of 4.4 ms).
+__global__ void gather_level_kernel(uint64_t p0, uint64_t p1, const int32_t* __restrict__ b_idx,
+                                    const uint32_t* __restrict__ ptr,
+                                    const uint32_t* __restrict__ src,
+                                    const double* __restrict__ b, double* __restrict__ vec) {
+  const uint64_t p = p0 + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (p >= p1) return;
+  const int32_t bi = b_idx[p];
+  double v = bi >= 0 ? b[bi] : 0.0;
+  const uint32_t e = ptr[p + 1];
+  for (uint32_t q = ptr[p]; q < e; q++) v += vec[src[q]];
+  vec[p] = v;
 }
 
 // Products of the large supernodes' solves.  With FP64 fronts they are FP64
@@ -1113,6 +1125,8 @@ __device__ __forceinline__ double widen(float f) {
   return __hiloint2double((int)hi, (int)lo);
 }
 
+__device__ __forceinline__ double widen(double f) { return f; }
+
 struct DotWide {
   using X = double;
   double s = 0.0;
@@ -1124,16 +1138,408 @@ struct DotWide {
   __device__ double value() const { return s; }
 };
 
-// backward, before the large supernodes' triangles: the solved ancestor
-// entries x[rows[i]], i >= k, gathered into v[k:m] (the update rows' slots,
-// free once the forward pass has added them into the parent), in the
-// products' operand form (a double, or its two-float split in its 8 bytes)
+// Solves of the small fronts: one CTA per front, FP64 products whatever the
+// fronts' type (FP32 entries widened by integer operations).
+// forward: v[0:k] <- D^-1 L11^-1 v[0:k], v[k:m] <- v[k:m] - L21 (L11^-1 v[0:k]);
+// blocks of 64 pivots: the block's unit triangle in shared memory, then one
+// pass over the rows below it
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+    forward_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
+                   double* __restrict__ vec) {
+  __shared__ double yb[kPanel];
+  const int s = list[blockIdx.x];
+  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
+  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
+  const T* F = front + d.front_off[s];
+  double* v = vec + d.vec_off[s];
+  for (int64_t c0 = 0; c0 < k; c0 += kPanel) {
+    const int cb = (int)(k - c0 < kPanel ? k - c0 : kPanel);
+    if (threadIdx.x < cb) yb[threadIdx.x] = v[c0 + threadIdx.x];
+    __syncthreads();
+    for (int c = 0; c < cb; c++) {
+      const int t = threadIdx.x;
+      if (t > c && t < cb) yb[t] -= widen(F[(c0 + t) + (c0 + c) * m]) * yb[c];
+      __syncthreads();
+    }
+    if (threadIdx.x < cb) v[c0 + threadIdx.x] = yb[threadIdx.x];
+    for (int64_t i = c0 + cb + threadIdx.x; i < m; i += blockDim.x) {
+      double acc = 0.0;
+      for (int c = 0; c < cb; c++) acc += widen(F[i + (c0 + c) * m]) * yb[c];
+      v[i] -= acc;
+    }
+    __syncthreads();
+  }
+  for (int64_t c = threadIdx.x; c < k; c += blockDim.x) v[c] /= widen(F[c + c * m]);
+}
+
+// backward: x[0:k] = L11^-T (v[0:k] - L21^T x_rest), x_rest gathered from the
+// solved ancestors (factor order), written to xf; blocks of 64 pivots from the
+// last: the contributions of the solved pivots below the block (a warp per
+// column), then the block's triangle in shared memory
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+    backward_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
+                    double* __restrict__ vec, double* __restrict__ xf) {
+  __shared__ double xb[kPanel];
+  const int s = list[blockIdx.x];
+  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
+  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
+  const int32_t* rows = d.rows + d.row_ptr[s];
+  const T* F = front + d.front_off[s];
+  double* v = vec + d.vec_off[s];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nwarps = blockDim.x / 32;
+  for (int64_t c = warp; c < k; c += nwarps) {
+    double acc = 0.0, acc2 = 0.0;
+    int64_t i = k + lane;
+    for (; i + 32 < m; i += 64) {
+      acc += widen(F[i + c * m]) * xf[rows[i]];
+      acc2 += widen(F[i + 32 + c * m]) * xf[rows[i + 32]];
+    }
+    if (i < m) acc += widen(F[i + c * m]) * xf[rows[i]];
+    acc += acc2;
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (lane == 0) v[c] -= acc;
+  }
+  __syncthreads();
+  for (int64_t c0 = ((k - 1) / kPanel) * kPanel; c0 >= 0; c0 -= kPanel) {
+    const int cb = (int)(k - c0 < kPanel ? k - c0 : kPanel);
+    for (int c = warp; c < cb; c += nwarps) {
+      double acc = 0.0;
+      for (int64_t i = c0 + cb + lane; i < k; i += 32) acc += widen(F[i + (c0 + c) * m]) * v[i];
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+      if (lane == 0) xb[c] = v[c0 + c] - acc;
+    }
+    __syncthreads();
+    for (int c = cb - 1; c >= 0; c--) {
+      const int t = threadIdx.x;
+      if (t < c) xb[t] -= widen(F[(c0 + c) + (c0 + t) * m]) * xb[c];
+      __syncthreads();
+    }
+    if (threadIdx.x < cb) v[c0 + threadIdx.x] = xb[threadIdx.x];
+    __syncthreads();
+  }
+  const int32_t f = d.sn_first[s];
+  for (int64_t c = threadIdx.x; c < k; c += blockDim.x) xf[f + c] = v[c];
+}
+
+// Small fronts of up to kTinyPivots pivots: a warp per front, lane = row
+// (kSmallFront / 32 rows each), the same FP64 products.  Forward: a column at
+// a time, v_i -= L[i][c] y_c; then D^-1.  Backward: from the last pivot, x_c =
+// v_c - sum_{i > c} L[i][c] x_i, the ancestors' entries gathered first.  Most
+// small fronts are leaves of one pivot and some 25 rows (10,293 in the
+// 139k-equation bar), for which a CTA each spent its time being launched;
+// with more pivots the warp's chain of columns is longer than the CTA's.
+constexpr int kTinyPivots = 8;
+constexpr int kSmallRows = kSmallFront / 32;
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+    fwd_tiny_kernel(const int32_t* __restrict__ list, int n, LdltDev d, const T* __restrict__ front,
+                   double* __restrict__ vec) {
+  const int q = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  if (q >= n) return;   // warp-uniform; no block barrier follows
+  const int s = list[q], lane = threadIdx.x & 31;
+  const int m = (int)(d.row_ptr[s + 1] - d.row_ptr[s]);
+  const int k = d.sn_first[s + 1] - d.sn_first[s];
+  const T* F = front + d.front_off[s];
+  double* v = vec + d.vec_off[s];
+  double x[kSmallRows];
+#pragma unroll
+  for (int u = 0; u < kSmallRows; u++) x[u] = lane + 32 * u < m ? v[lane + 32 * u] : 0.0;
+  const double piv = lane < k ? widen(F[lane + lane * m]) : 1.0;
+#pragma unroll 4
+  for (int c = 0; c < k; c++) {
+    const double yc = __shfl_sync(0xffffffffu, x[0], c);
+#pragma unroll
+    for (int u = 0; u < kSmallRows; u++) {
+      const int r = lane + 32 * u;
+      if (r > c && r < m) x[u] = fma(-widen(F[r + c * m]), yc, x[u]);
+    }
+  }
+  if (lane < k) x[0] = x[0] / piv;
+#pragma unroll
+  for (int u = 0; u < kSmallRows; u++)
+    if (lane + 32 * u < m) v[lane + 32 * u] = x[u];
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+    bwd_tiny_kernel(const int32_t* __restrict__ list, int n, LdltDev d, const T* __restrict__ front,
+                    const double* __restrict__ vec, double* __restrict__ xf) {
+  const int q = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  if (q >= n) return;   // warp-uniform; no block barrier follows
+  const int s = list[q], lane = threadIdx.x & 31;
+  const int m = (int)(d.row_ptr[s + 1] - d.row_ptr[s]);
+  const int k = d.sn_first[s + 1] - d.sn_first[s];
+  const int32_t* rows = d.rows + d.row_ptr[s];
+  const T* F = front + d.front_off[s];
+  const double* v = vec + d.vec_off[s];
+  double x[kSmallRows];
+#pragma unroll
+  for (int u = 0; u < kSmallRows; u++) {
+    const int r = lane + 32 * u;
+    x[u] = r < k ? v[r] : r < m ? xf[rows[r]] : 0.0;
+  }
+#pragma unroll 2
+  for (int c = k - 1; c >= 0; c--) {
+    double acc = 0.0;
+#pragma unroll
+    for (int u = 0; u < kSmallRows; u++) {
+      const int r = lane + 32 * u;
+      if (r > c && r < m) acc = fma(widen(F[r + c * m]), x[u], acc);
+    }
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == c) x[0] -= acc;
+  }
+  if (lane < k) xf[d.sn_first[s] + lane] = x[0];
+}
+
+// Solves of the large fronts, batched per level.  Fronts with up to kNarrow
+// pivots (and kNarrowRows rows) take one CTA each and pass; wider ones go by
+// blocks of kInv pivots, two launches per block and direction: the block
+// through its inverse X, then the rows below it (forward) or the pivots before
+// it (backward).  Every product chain is split so that its loads are issued
+// together, and partial sums are merged in a fixed order (run-to-run
+// identical).  The passes are bound by the latency of that chain of launches
+// near the root and by the fronts' bytes below it.  Blocks of 256 pivots with
+// 64 x 64 inverses took 59 block steps of 35 us a direction on the
+// 139k-equation bar, 4.4 ms a pass; these take 34 steps, 1.7 ms a pass.
+
+// forward, narrow fronts: y = X v, v[0:k] <- D^-1 y, v[k:m] -= L21 y
 template <typename T, typename D>
-__global__ void gather_rest_kernel(BigBatch b, LdltDev d, double* __restrict__ vec,
-                                   const double* __restrict__ xf) {
+__global__ void __launch_bounds__(kThreads)
+    fwd_narrow_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
+                      double* __restrict__ vec) {
+  using X = typename D::X;
+  static_assert(kThreads == 4 * kNarrow, "four threads per pivot row");
+  __shared__ X xs[kNarrow];
+  __shared__ X ys[kNarrow];
+  const int s = list[blockIdx.x];
+  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
+  const int k = d.sn_first[s + 1] - d.sn_first[s];
+  const T* F = front + d.front_off[s];
+  double* v = vec + d.vec_off[s];
+  const int t = threadIdx.x;
+  {
+    const int r = t >> 2, q = t & 3;
+    T f[kNarrow / 4];
+#pragma unroll
+    for (int u = 0; u < kNarrow / 4; u++) {
+      const int j = q + 4 * u;
+      f[u] = r < k && j < r ? F[j + r * m] : T(0);
+    }
+    if (t < k) xs[t] = D::split(v[t]);
+    __syncthreads();
+    D y;
+#pragma unroll
+    for (int u = 0; u < kNarrow / 4; u++)
+      if (r < k && q + 4 * u < r) y.add(f[u], xs[q + 4 * u]);
+    y.shfl_xor(1);
+    y.shfl_xor(2);
+    if (r < k && q == 0) {
+      const double yv = v[r] + y.value();
+      ys[r] = D::split(yv);
+      v[r] = yv / (double)F[r + r * m];
+    }
+  }
+  __syncthreads();
+  for (int64_t i = k + t; i < m; i += kThreads) {
+    const T* Fi = F + i;
+    D a0, a1;
+    for (int c = 0; c < k; c += 16) {
+      T f[16];
+#pragma unroll
+      for (int u = 0; u < 16; u++) f[u] = c + u < k ? Fi[(c + u) * m] : T(0);
+#pragma unroll
+      for (int u = 0; u < 16; u += 2) {
+        if (c + u < k) a0.add(f[u], ys[c + u]);
+        if (c + u + 1 < k) a1.add(f[u + 1], ys[c + u + 1]);
+      }
+    }
+    a0.merge(a1);
+    v[i] -= a0.value();
+  }
+}
+
+// backward, narrow fronts: t = v[0:k] - L21^T x_rest, x = X^T t; a warp takes
+// four columns of L21 at a time
+template <typename T, typename D>
+__global__ void __launch_bounds__(kThreads)
+    bwd_narrow_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
+                      const double* __restrict__ vec, double* __restrict__ xf) {
+  using X = typename D::X;
+  extern __shared__ __align__(16) unsigned char narrow_raw[];
+  X* xr = reinterpret_cast<X*>(narrow_raw);   // m - k
+  __shared__ X ts[kNarrow];
+  __shared__ double td[kNarrow];
+  const int s = list[blockIdx.x];
+  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
+  const int k = d.sn_first[s + 1] - d.sn_first[s];
+  const int u = (int)(m - k);
+  const int32_t* rows = d.rows + d.row_ptr[s] + k;
+  const T* F = front + d.front_off[s];
+  const double* v = vec + d.vec_off[s];
+  for (int i = threadIdx.x; i < u; i += kThreads) xr[i] = D::split(xf[rows[i]]);
+  const int j = threadIdx.x >> 2, q = threadIdx.x & 3;   // four threads per pivot
+  T fx[kNarrow / 4];
+#pragma unroll
+  for (int w = 0; w < kNarrow / 4; w++) {
+    const int i = q + 4 * w;
+    fx[w] = j < i && i < k ? F[j + i * m] : T(0);
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kCols = 4;
+  for (int c = warp * kCols; c < k; c += kThreads / 32 * kCols) {
+    const T* Fc = F + k + c * m;
+    D a[kCols];
+    const int nc = min(k - c, kCols);
+    for (int i = lane; i < u; i += 64) {
+      T f[2][kCols];
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int w = 0; w < kCols; w++)
+          f[h][w] = w < nc && i + 32 * h < u ? Fc[i + 32 * h + w * m] : T(0);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        if (i + 32 * h >= u) break;
+        const X x = xr[i + 32 * h];
+#pragma unroll
+        for (int w = 0; w < kCols; w++) a[w].add(f[h][w], x);
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int w = 0; w < kCols; w++) a[w].shfl_xor(o);
+#pragma unroll
+    for (int w = 0; w < kCols; w++)
+      if (lane == w && w < nc) {
+        const double tv = v[c + w] - a[w].value();
+        td[c + w] = tv;
+        ts[c + w] = D::split(tv);
+      }
+  }
+  __syncthreads();
+  D x;
+#pragma unroll
+  for (int w = 0; w < kNarrow / 4; w++)
+    if (j < q + 4 * w && q + 4 * w < k) x.add(fx[w], ts[q + 4 * w]);
+  x.shfl_xor(1);
+  x.shfl_xor(2);
+  if (j < k && q == 0) xf[d.sn_first[s] + j] = td[j] + x.value();
+}
+
+// forward, wide fronts, block o0: y = X v, a warp per row (a row of X is
+// contiguous; all its loads in flight)
+constexpr int kInvRows = kThreads / 32;
+template <typename T, typename D>
+__global__ void __launch_bounds__(kThreads)
+    fwd_inv_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
+                   int64_t o0, const double* __restrict__ vec, double* __restrict__ yv) {
+  using X = typename D::X;
+  __shared__ X xs[kInv];
+  const int s = list[blockIdx.y];
+  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
+  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
+  if (o0 >= k) return;
+  const int ob = (int)(k - o0 < kInv ? k - o0 : kInv);
+  const int r0 = blockIdx.x * kInvRows;
+  if (r0 >= ob) return;
+  const double* v = vec + d.vec_off[s] + o0;
+  const int lane = threadIdx.x & 31, i = r0 + (threadIdx.x >> 5);
+  T f[kInv / 32];
+  if (i < ob) {
+    const T* Fi = front + d.front_off[s] + o0 + (o0 + i) * m;
+#pragma unroll
+    for (int u = 0; u < kInv / 32; u++) f[u] = lane + 32 * u < i ? Fi[lane + 32 * u] : T(0);
+  }
+  for (int j = threadIdx.x; j < min(ob, r0 + kInvRows); j += kThreads) xs[j] = D::split(v[j]);
+  __syncthreads();
+  if (i >= ob) return;
+  D a[4];
+#pragma unroll
+  for (int u = 0; u < kInv / 32; u++)
+    if (lane + 32 * u < i) a[u & 3].add(f[u], xs[lane + 32 * u]);
+  a[0].merge(a[1]);
+  a[2].merge(a[3]);
+  a[0].merge(a[2]);
+  for (int o = 16; o > 0; o >>= 1) a[0].shfl_down(o);
+  if (lane == 0) yv[d.vec_off[s] + o0 + i] = v[i] + a[0].value();
+}
+
+// the warps' partial sums per lane, merged in a fixed order by warp 0
+template <int kWarps, typename D>
+__device__ __forceinline__ bool merge_warps(D& a, D (*part)[32]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  part[warp][lane] = a;
+  __syncthreads();
+  if (warp != 0) return false;
+#pragma unroll
+  for (int w = 1; w < kWarps; w++) a.merge(part[w][lane]);
+  return true;
+}
+
+// forward, wide fronts, block o0: v[i] -= sum_c L[i][o0+c] y_c for the rows
+// below the block: lane = row (each load one coalesced 32-row segment of a
+// column), a warp per 32 columns and 32 rows.  The block's column groups take
+// that many warps of the CTA; a block of few columns leaves warps for further
+// row groups (16 warps where a level has blocks above 256 pivots, else 8).
+template <typename T, typename D, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps)
+    fwd_rows_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
+                    int64_t o0, const double* __restrict__ yv, double* __restrict__ vec) {
+  using X = typename D::X;
+  __shared__ X yb[kInv];
+  __shared__ D part[kWarps][32];
+  const int s = list[blockIdx.y];
+  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
+  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
+  if (o0 >= k) return;
+  const int ob = (int)(k - o0 < kInv ? k - o0 : kInv);
+  const int groups = (ob + 31) / 32;   // <= kWarps: see the launch
+  const int row_groups = kWarps / groups;
+  const int64_t r0 = o0 + ob + (int64_t)blockIdx.x * 32 * row_groups;
+  if (r0 >= m) return;
+  double* v = vec + d.vec_off[s];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rg = warp / groups, cb = (warp - rg * groups) * 32;
+  const int64_t i = r0 + 32 * rg + lane;
+  const int nc = rg < row_groups && i < m ? min(ob - cb, 32) : 0;   // this warp's columns
+  T f[32];
+  const T* Fi = front + d.front_off[s] + i + (o0 + cb) * m;
+#pragma unroll
+  for (int u = 0; u < 32; u++) f[u] = u < nc ? Fi[(int64_t)u * m] : T(0);
+  for (int j = threadIdx.x; j < ob; j += 32 * kWarps)
+    yb[j] = D::split(yv[d.vec_off[s] + o0 + j]);
+  __syncthreads();
+  D a[4];
+#pragma unroll
+  for (int u = 0; u < 32; u++)
+    if (u < nc) a[u & 3].add(f[u], yb[cb + u]);
+  a[0].merge(a[1]);
+  a[2].merge(a[3]);
+  a[0].merge(a[2]);
+  part[warp][lane] = a[0];
+  __syncthreads();
+  if (cb == 0 && nc > 0) {
+    for (int w = 1; w < groups; w++) a[0].merge(part[warp + w][lane]);
+    v[i] -= a[0].value();
+  }
+}
+
+// backward, wide fronts: the solved ancestor entries x[rows[i]], i >= k,
+// gathered into v[k:m] (the update rows' slots, free once the forward pass has
+// added them into the parent), in the products' operand form (a double, or its
+// two-float split in its 8 bytes)
+template <typename T, typename D>
+__global__ void gather_rest_kernel(const int32_t* __restrict__ list, LdltDev d,
+                                   double* __restrict__ vec, const double* __restrict__ xf) {
   using X = typename D::X;
   static_assert(sizeof(X) == sizeof(double), "operand form fills a vector slot");
-  const int s = b.list[blockIdx.y];
+  const int s = list[blockIdx.y];
   const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
   const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
   const int64_t i = k + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1141,16 +1547,16 @@ __global__ void gather_rest_kernel(BigBatch b, LdltDev d, double* __restrict__ v
   reinterpret_cast<X*>(vec + d.vec_off[s])[i] = D::split(xf[d.rows[d.row_ptr[s] + i]]);
 }
 
-// backward: t_c = v_c - sum_{i >= k} L[i][c] xr_i (xr gathered into v[k:m]),
-// a warp per column: the column's contiguous segment and xr read by the
-// lanes, eight loads of each in flight, eight partial sums merged in a fixed
-// order
+// backward, wide fronts: t_c = y_c / d_c - sum_{i >= k} L[i][c] xr_i (xr
+// gathered into v[k:m]), a warp per column: the column's contiguous segment
+// and xr read by the lanes, eight loads of each in flight, eight partial sums
+// merged in a fixed order
 template <typename T, typename D>
 __global__ void __launch_bounds__(kThreads)
-    bwd_rest_kernel(BigBatch b, LdltDev d, const T* __restrict__ front,
-                    double* __restrict__ vec) {
+    bwd_rest_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
+                    const double* __restrict__ yv, double* __restrict__ vec) {
   using X = typename D::X;
-  const int s = b.list[blockIdx.y];
+  const int s = list[blockIdx.y];
   const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
   const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1176,509 +1582,80 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
   for (int u = 1; u < 8; u++) acc[0].merge(acc[u]);
   for (int o = 16; o > 0; o >>= 1) acc[0].shfl_down(o);
-  if (lane == 0) v[c] -= acc[0].value();
+  if (lane == 0) v[c] = yv[d.vec_off[s] + c] / (double)Fc[c] - acc[0].value();
 }
 
-// The forward and backward passes go by outer blocks of kOuter pivots (four
-// panels), two launches per outer block and level: the block's own triangle
-// by one CTA per supernode (panel by panel through the stored inverses, the
-// rows / columns inside the block updated in shared memory), then the rows
-// below it (forward) or the pivots before it (backward) with up to kOuter
-// products per entry.  Every product chain is split so that its loads are
-// issued together (the passes are bound by load latency, not bandwidth), and
-// the partial sums are merged in a fixed order (run-to-run identical).
+// backward, wide fronts, block o0: x = X^T t, lane = pivot j (row i of X gives
+// each lane its entry, coalesced), warp w takes the rows w, w + 32, ... from
+// the lanes' diagonal piece on; the solved pivots go to xf (factor order)
+constexpr int kColThreads = 1024;
+template <typename T, typename D>
+__global__ void __launch_bounds__(kColThreads)
+    bwd_inv_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
+                   int64_t o0, const double* __restrict__ vec, double* __restrict__ xf) {
+  using X = typename D::X;
+  __shared__ X ts[kInv];
+  __shared__ D part[kColThreads / 32][32];
+  const int s = list[blockIdx.y];
+  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
+  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
+  if (o0 >= k) return;
+  const int ob = (int)(k - o0 < kInv ? k - o0 : kInv);
+  const int j0 = blockIdx.x * 32;
+  if (j0 >= ob) return;
+  const double* v = vec + d.vec_off[s] + o0;
+  const int j = j0 + (threadIdx.x & 31), i0 = j0 + (threadIdx.x >> 5);
+  const T* Fj = front + d.front_off[s] + o0 + j + (o0 + i0) * m;   // X[i][j], i = i0 + 32 u
+  T f[kInv / 32];
+#pragma unroll
+  for (int u = 0; u < kInv / 32; u++)
+    f[u] = i0 + 32 * u < ob && i0 + 32 * u > j ? Fj[(int64_t)(32 * u) * m] : T(0);
+  for (int i = j0 + threadIdx.x; i < ob; i += kColThreads) ts[i] = D::split(v[i]);
+  __syncthreads();
+  D a[2];
+#pragma unroll
+  for (int u = 0; u < kInv / 32; u++)
+    if (i0 + 32 * u < ob && i0 + 32 * u > j) a[u & 1].add(f[u], ts[i0 + 32 * u]);
+  a[0].merge(a[1]);
+  if (merge_warps<kColThreads / 32>(a[0], part) && j < ob)
+    xf[d.sn_first[s] + o0 + j] = v[j] + a[0].value();
+}
 
-// forward, outer block o0: v_B <- L_BB^-1 v_B for the block's ob pivots.
-// Per panel: y = Linv v_p, then the rows below the panel inside the block,
-// both by four threads per row (16 products each, merged by shuffles).
+// backward, wide fronts, block o0: t[j] -= sum_c L[o0+c][j] x_c for the pivots
+// j < o0 (a warp per column j, lanes over the block's rows)
 template <typename T, typename D>
 __global__ void __launch_bounds__(kThreads)
-    fwd_block_kernel(BigBatch b, LdltDev d, const T* __restrict__ front,
-                     const T* __restrict__ Linv, int64_t o0, double* __restrict__ vec) {
+    bwd_cols_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
+                    int64_t o0, const double* __restrict__ xf, double* __restrict__ vec) {
   using X = typename D::X;
-  __shared__ double vb[kOuter];
-  __shared__ X xs[kPanel];
-  const int s = b.list[blockIdx.x];
+  __shared__ X xb[kInv];
+  const int s = list[blockIdx.y];
   const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
   const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
   if (o0 >= k) return;
-  const int ob = (int)(k - o0 < kOuter ? k - o0 : kOuter);
-  const T* F = front + d.front_off[s];
-  double* v = vec + d.vec_off[s];
-  const int t = threadIdx.x;
-  if (t < ob) vb[t] = v[o0 + t];
+  const int64_t j = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  if ((int64_t)blockIdx.x * (kThreads / 32) >= o0) return;
+  const int ob = (int)(k - o0 < kInv ? k - o0 : kInv);
+  for (int c = threadIdx.x; c < ob; c += kThreads) xb[c] = D::split(xf[d.sn_first[s] + o0 + c]);
   __syncthreads();
-  const int r = t >> 2, q = t & 3;   // kThreads = 4 x kPanel
-  for (int p = 0; p < ob; p += kPanel) {
-    const int cb = ob - p < kPanel ? ob - p : kPanel;
-    const T* Li = Linv + b.li_off[blockIdx.x] + (uint64_t)((o0 + p) / kPanel) * kPanel * kPanel;
-    // (entries past cb are zero: the row products below read all kPanel)
-    if (t < kPanel) xs[t] = D::split(t < cb ? vb[p + t] : 0.0);
-    __syncthreads();
-    // y_r = sum_c Linv[r][c] v_c (Linv's strict upper triangle holds zeros)
-    D y;
-    if (r < cb) {
-      D y1;
+  if (j >= o0) return;
+  const int lane = threadIdx.x & 31;
+  const T* Fj = front + d.front_off[s] + o0 + j * m;
+  D a[4];
+  int c = lane;
+  for (; c + 7 * 32 < ob; c += 8 * 32) {
+    T f[8];
 #pragma unroll
-      for (int j = 0; j < kPanel / 4; j += 2) {
-        const int c0 = q + 4 * j, c1 = c0 + 4;
-        if (c0 < cb) y.add(Li[r + c0 * kPanel], xs[c0]);
-        if (c1 < cb) y1.add(Li[r + c1 * kPanel], xs[c1]);
-      }
-      y.merge(y1);
-    }
-    y.shfl_xor(1);
-    y.shfl_xor(2);
-    __syncthreads();
-    if (r < cb && q == 0) {
-      const double yv = y.value();
-      vb[p + r] = yv;
-      xs[r] = D::split(yv);
-    }
-    __syncthreads();
-    // the rows below the panel inside the block: four threads per row, 16
-    // columns each
-    for (int i0 = p + cb; i0 < ob; i0 += kThreads / 4) {
-      const int i = i0 + r;
-      D a;
-      if (i < ob) {
-        const T* Fi = F + (o0 + i) + (o0 + p) * m;
-        const int c0 = q * (kPanel / 4);
-        T f[kPanel / 4];
+    for (int u = 0; u < 8; u++) f[u] = Fj[c + 32 * u];
 #pragma unroll
-        for (int u = 0; u < kPanel / 4; u++)
-          f[u] = c0 + u < cb ? Fi[(int64_t)(c0 + u) * m] : T(0);
-        D a1;
-#pragma unroll
-        for (int u = 0; u < kPanel / 4; u += 2) {
-          a.add(f[u], xs[c0 + u]);
-          a1.add(f[u + 1], xs[c0 + u + 1]);
-        }
-        a.merge(a1);
-      }
-      a.shfl_xor(1);
-      a.shfl_xor(2);
-      if (i < ob && q == 0) vb[i] -= a.value();
-    }
-    __syncthreads();
+    for (int u = 0; u < 8; u++) a[u & 3].add(f[u], xb[c + 32 * u]);
   }
-  if (t < ob) v[o0 + t] = vb[t];
-}
-
-// forward, outer block o0: v[i] -= sum_c L[i][o0+c] y_c for the rows below the
-// block, 32 rows per CTA: warp w takes the columns [32 w, 32 w + 32), lane =
-// row (each load one coalesced 32-row segment of a column, 32 in flight),
-// and the eight warps' partial sums are merged in a fixed order
-template <typename T, typename D>
-__global__ void __launch_bounds__(kThreads)
-    fwd_rows_block_kernel(BigBatch b, LdltDev d, const T* __restrict__ front, int64_t o0,
-                          double* __restrict__ vec) {
-  using X = typename D::X;
-  constexpr int kWarps = kThreads / 32;
-  static_assert(kWarps * 32 == kOuter, "one warp per 32 columns of the outer block");
-  __shared__ X yb[kOuter];
-  __shared__ D part[kWarps][32];
-  const int s = b.list[blockIdx.y];
-  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
-  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
-  if (o0 >= k) return;
-  const int ob = (int)(k - o0 < kOuter ? k - o0 : kOuter);
-  const int64_t r0 = o0 + ob + (int64_t)blockIdx.x * 32;
-  if (r0 >= m) return;
-  const T* F = front + d.front_off[s];
-  double* v = vec + d.vec_off[s];
-  if (threadIdx.x < ob) yb[threadIdx.x] = D::split(v[o0 + threadIdx.x]);
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t i = r0 + lane;
-  const int cbeg = warp * 32;
-  D a0, a1, a2, a3;
-  if (i < m && cbeg < ob) {
-    const T* Fi = F + i + (o0 + cbeg) * m;
-    if (ob - cbeg >= 32) {
-      T f[32];
-#pragma unroll
-      for (int u = 0; u < 32; u++) f[u] = Fi[(int64_t)u * m];
-#pragma unroll
-      for (int u = 0; u < 32; u += 4) {
-        a0.add(f[u], yb[cbeg + u]);
-        a1.add(f[u + 1], yb[cbeg + u + 1]);
-        a2.add(f[u + 2], yb[cbeg + u + 2]);
-        a3.add(f[u + 3], yb[cbeg + u + 3]);
-      }
-    } else {
-      for (int u = 0; u < ob - cbeg; u++) a0.add(Fi[(int64_t)u * m], yb[cbeg + u]);
-    }
-  }
-  a0.merge(a1);
-  a2.merge(a3);
-  a0.merge(a2);
-  part[warp][lane] = a0;
-  __syncthreads();
-  if (warp == 0 && i < m) {
-    D sum = part[0][lane];
-#pragma unroll
-    for (int w = 1; w < kWarps; w++) sum.merge(part[w][lane]);
-    v[i] -= sum.value();
-  }
-}
-
-// backward, outer block o0: x_B = L_BB^-T t_B for the block's pivots.  Per
-// panel (last first): the panel's inverse staged in shared memory (coalesced),
-// x = Linv^T t_p by four threads per pivot, then t_j -= sum_c L[p+c][j] x_c
-// for the block's pivots j before the panel by four threads per j (16
-// contiguous products each), the partial sums merged by shuffles
-template <typename T, typename D>
-__global__ void __launch_bounds__(kThreads)
-    bwd_block_kernel(BigBatch b, LdltDev d, const T* __restrict__ front,
-                     const T* __restrict__ Linv, int64_t o0, double* __restrict__ vec) {
-  using X = typename D::X;
-  __shared__ double tb[kOuter];
-  __shared__ X xs[kPanel];
-  __shared__ T Ls[kPanel][kPanel + 1];   // Ls[c][r] = Linv[r][c]
-  const int s = b.list[blockIdx.x];
-  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
-  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
-  if (o0 >= k) return;
-  const int ob = (int)(k - o0 < kOuter ? k - o0 : kOuter);
-  const T* F = front + d.front_off[s];
-  double* v = vec + d.vec_off[s];
-  const int t = threadIdx.x;
-  if (t < ob) tb[t] = v[o0 + t];
-  const int r = t >> 2, q = t & 3;   // kThreads = 4 x kPanel
-  for (int p = ((ob - 1) / kPanel) * kPanel; p >= 0; p -= kPanel) {
-    const int cb = ob - p < kPanel ? ob - p : kPanel;
-    const T* Li = Linv + b.li_off[blockIdx.x] + (uint64_t)((o0 + p) / kPanel) * kPanel * kPanel;
-#pragma unroll 4
-    for (int e = t; e < kPanel * kPanel; e += kThreads) {
-      const int er = e % kPanel, ec = e / kPanel;
-      Ls[ec][er] = er < cb && ec < cb ? Li[er + ec * kPanel] : T(0);
-    }
-    __syncthreads();
-    // (entries past cb are zero: the products below read all kPanel)
-    if (t < kPanel) xs[t] = D::split(t < cb ? tb[p + t] : 0.0);
-    __syncthreads();
-    // x_r = sum_{c >= r} Linv[c][r] t_c
-    D x;
-    if (r < cb) {
-      D x1;
-#pragma unroll
-      for (int j = 0; j < kPanel / 4; j += 2) {
-        const int c0 = q + 4 * j, c1 = c0 + 4;
-        if (c0 < cb) x.add(Ls[r][c0], xs[c0]);
-        if (c1 < cb) x1.add(Ls[r][c1], xs[c1]);
-      }
-      x.merge(x1);
-    }
-    x.shfl_xor(1);
-    x.shfl_xor(2);
-    __syncthreads();
-    if (r < cb && q == 0) {
-      const double xv = x.value();
-      tb[p + r] = xv;
-      xs[r] = D::split(xv);
-    }
-    __syncthreads();
-    // the pivots before the panel: column j's rows p .. p+cb, contiguous
-    for (int j0 = 0; j0 < p; j0 += kThreads / 4) {
-      const int j = j0 + r;
-      D a;
-      if (j < p) {
-        const T* Fj = F + (o0 + p) + (o0 + j) * m;
-        const int c0 = q * (kPanel / 4);
-        T f[kPanel / 4];
-#pragma unroll
-        for (int u = 0; u < kPanel / 4; u++) f[u] = c0 + u < cb ? Fj[c0 + u] : T(0);
-        D a1;
-#pragma unroll
-        for (int u = 0; u < kPanel / 4; u += 2) {
-          a.add(f[u], xs[c0 + u]);
-          a1.add(f[u + 1], xs[c0 + u + 1]);
-        }
-        a.merge(a1);
-      }
-      a.shfl_xor(1);
-      a.shfl_xor(2);
-      if (j < p && q == 0) tb[j] -= a.value();
-    }
-    __syncthreads();
-  }
-  if (t < ob) v[o0 + t] = tb[t];
-}
-
-// backward, outer block o0: t[j] -= sum_c L[o0+c][j] x_c for the pivots j < o0
-// (a warp per column j, lanes over the block's rows, eight loads in flight)
-template <typename T, typename D>
-__global__ void __launch_bounds__(kThreads)
-    bwd_cols_block_kernel(BigBatch b, LdltDev d, const T* __restrict__ front, int64_t o0,
-                          double* __restrict__ vec) {
-  using X = typename D::X;
-  __shared__ X xb[kOuter];
-  const int s = b.list[blockIdx.y];
-  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
-  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
-  if (o0 >= k) return;
-  const int64_t jbeg = (int64_t)blockIdx.x * 32;
-  if (jbeg >= o0) return;
-  const int ob = (int)(k - o0 < kOuter ? k - o0 : kOuter);
-  const T* F = front + d.front_off[s];
-  double* v = vec + d.vec_off[s];
-  if (threadIdx.x < ob) xb[threadIdx.x] = D::split(v[o0 + threadIdx.x]);
-  else if (threadIdx.x < kOuter) xb[threadIdx.x] = D::split(0.0);
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t jend = jbeg + 32 < o0 ? jbeg + 32 : o0;
-  for (int64_t j = jbeg + warp; j < jend; j += blockDim.x / 32) {
-    const T* Fj = F + o0 + j * m;
-    T f[kOuter / 32];
-#pragma unroll
-    for (int u = 0; u < kOuter / 32; u++) f[u] = lane + 32 * u < ob ? Fj[lane + 32 * u] : T(0);
-    D a0, a1;
-#pragma unroll
-    for (int u = 0; u < kOuter / 32; u += 2) {
-      a0.add(f[u], xb[lane + 32 * u]);
-      a1.add(f[u + 1], xb[lane + 32 * (u + 1)]);
-    }
-    a0.merge(a1);
-    for (int o = 16; o > 0; o >>= 1) a0.shfl_down(o);
-    if (lane == 0) v[j] -= a0.value();
-  }
-}
-
-// FP32 fronts: the block triangles with their operands staged in shared
-// memory by asynchronous copies issued when the CTA starts (the stored
-// inverses of the block's four panels and the block's strictly lower part,
-// 166 KB), in the order the panels use them, so that the pass waits for one
-// copy latency per block instead of a chain of them; everything after
-// reads shared memory.  Columns are padded to 65 floats (two-way bank
-// conflicts at most for the four-threads-per-row products).
-constexpr int kLd = kPanel + 1;
-constexpr int kStageLi = 4 * kPanel * kLd;    // the four inverses
-constexpr int kStageTri = 6 * kPanel * kLd;   // panel pi >= 1: its rows x the 64 pi columns before it
-constexpr size_t kStagedSmem = sizeof(float) * (kStageLi + kStageTri) + sizeof(double) * kOuter +
-                               sizeof(double) * kPanel;
-static_assert(kOuter == 4 * kPanel, "four panels per outer block");
-
-__device__ __forceinline__ int tri_off(int pi) { return kPanel * kLd * (pi * (pi - 1) / 2); }
-
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-// this thread's copies of all but the `pending` most recent groups have landed
-__device__ __forceinline__ void cp_async_wait(int pending) {
-  switch (pending) {
-    case 0: asm volatile("cp.async.wait_group 0;\n" ::: "memory"); break;
-    case 1: asm volatile("cp.async.wait_group 1;\n" ::: "memory"); break;
-    case 2: asm volatile("cp.async.wait_group 2;\n" ::: "memory"); break;
-    default: asm volatile("cp.async.wait_group 3;\n" ::: "memory"); break;
-  }
-}
-
-// forward, outer block o0, FP32 fronts (fwd_block_kernel's arithmetic): copy
-// group g holds panel g's inverse and the columns of panel g in the rows of
-// the later panels
-template <typename D>
-__global__ void __launch_bounds__(kThreads)
-    fwd_block_staged_kernel(BigBatch b, LdltDev d, const float* __restrict__ front,
-                            const float* __restrict__ Linv, int64_t o0,
-                            double* __restrict__ vec) {
-  using X = typename D::X;
-  static_assert(sizeof(X) == sizeof(double), "operand slots of 8 bytes");
-  extern __shared__ __align__(16) unsigned char staged_raw[];
-  float* Ls = reinterpret_cast<float*>(staged_raw);
-  float* Tb = Ls + kStageLi;
-  double* vb = reinterpret_cast<double*>(Tb + kStageTri);
-  X* xs = reinterpret_cast<X*>(vb + kOuter);
-  const int s = b.list[blockIdx.x];
-  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
-  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
-  if (o0 >= k) return;
-  const int ob = (int)(k - o0 < kOuter ? k - o0 : kOuter);
-  const int np = (ob + kPanel - 1) / kPanel;
-  const float* F = front + d.front_off[s];
-  const float* Li0 = Linv + b.li_off[blockIdx.x] + (uint64_t)(o0 / kPanel) * kPanel * kPanel;
-  double* v = vec + d.vec_off[s];
-  const int t = threadIdx.x;
-  for (int g = 0; g < np; g++) {
-    const int cbg = ob - g * kPanel < kPanel ? ob - g * kPanel : kPanel;
-    const float* Li = Li0 + (uint64_t)g * kPanel * kPanel;
-    for (int e = t; e < kPanel * kPanel; e += kThreads) {
-      const int er = e % kPanel, ec = e / kPanel;
-      if (er < cbg && ec < cbg) cp_async4(Ls + g * kPanel * kLd + ec * kLd + er, Li + e);
-    }
-    for (int pi = g + 1; pi < np; pi++) {
-      const int cbp = ob - pi * kPanel < kPanel ? ob - pi * kPanel : kPanel;
-      for (int e = t; e < kPanel * kPanel; e += kThreads) {
-        const int er = e % kPanel, ec = e / kPanel;
-        if (er < cbp)
-          cp_async4(Tb + tri_off(pi) + (g * kPanel + ec) * kLd + er,
-                    F + (o0 + pi * kPanel + er) + (o0 + g * kPanel + ec) * m);
-      }
-    }
-    cp_async_commit();
-  }
-  if (t < ob) vb[t] = v[o0 + t];
-  const int r = t >> 2, q = t & 3;   // kThreads = 4 x kPanel
-  for (int g = 0; g < np; g++) {
-    const int p = g * kPanel;
-    const int cb = ob - p < kPanel ? ob - p : kPanel;
-    cp_async_wait(np - 1 - g);
-    __syncthreads();
-    if (t < kPanel) xs[t] = D::split(t < cb ? vb[p + t] : 0.0);
-    __syncthreads();
-    // y_r = sum_c Linv[r][c] v_c
-    const float* L = Ls + g * kPanel * kLd;
-    D y;
-    if (r < cb) {
-      D y1;
-#pragma unroll
-      for (int j = 0; j < kPanel / 4; j += 2) {
-        const int c0 = q * (kPanel / 4) + j, c1 = c0 + 1;
-        if (c0 < cb) y.add(L[c0 * kLd + r], xs[c0]);
-        if (c1 < cb) y1.add(L[c1 * kLd + r], xs[c1]);
-      }
-      y.merge(y1);
-    }
-    y.shfl_xor(1);
-    y.shfl_xor(2);
-    __syncthreads();
-    if (r < cb && q == 0) {
-      const double yv = y.value();
-      vb[p + r] = yv;
-      xs[r] = D::split(yv);
-    }
-    __syncthreads();
-    // the rows of the later panels: four threads per row, 16 columns each
-    for (int i0 = p + cb; i0 < ob; i0 += kThreads / 4) {
-      const int i = i0 + r;
-      D a;
-      if (i < ob) {
-        const int pi = i / kPanel, rr = i - pi * kPanel;
-        const float* Tr = Tb + tri_off(pi) + p * kLd + rr;
-        D a1;
-#pragma unroll
-        for (int u = 0; u < kPanel / 4; u += 2) {
-          const int c0 = q * (kPanel / 4) + u, c1 = c0 + 1;
-          if (c0 < cb) a.add(Tr[c0 * kLd], xs[c0]);
-          if (c1 < cb) a1.add(Tr[c1 * kLd], xs[c1]);
-        }
-        a.merge(a1);
-      }
-      a.shfl_xor(1);
-      a.shfl_xor(2);
-      if (i < ob && q == 0) vb[i] -= a.value();
-    }
-    __syncthreads();
-  }
-  if (t < ob) v[o0 + t] = vb[t];
-}
-
-// backward, outer block o0, FP32 fronts (bwd_block_kernel's arithmetic):
-// copy groups in the backward order, group n = panel np-1-n's inverse and its
-// rows in the columns before it
-template <typename D>
-__global__ void __launch_bounds__(kThreads)
-    bwd_block_staged_kernel(BigBatch b, LdltDev d, const float* __restrict__ front,
-                            const float* __restrict__ Linv, int64_t o0,
-                            double* __restrict__ vec) {
-  using X = typename D::X;
-  static_assert(sizeof(X) == sizeof(double), "operand slots of 8 bytes");
-  extern __shared__ __align__(16) unsigned char staged_raw[];
-  float* Ls = reinterpret_cast<float*>(staged_raw);
-  float* Tb = Ls + kStageLi;
-  double* tb = reinterpret_cast<double*>(Tb + kStageTri);
-  X* xs = reinterpret_cast<X*>(tb + kOuter);
-  const int s = b.list[blockIdx.x];
-  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
-  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
-  if (o0 >= k) return;
-  const int ob = (int)(k - o0 < kOuter ? k - o0 : kOuter);
-  const int np = (ob + kPanel - 1) / kPanel;
-  const float* F = front + d.front_off[s];
-  const float* Li0 = Linv + b.li_off[blockIdx.x] + (uint64_t)(o0 / kPanel) * kPanel * kPanel;
-  double* v = vec + d.vec_off[s];
-  const int t = threadIdx.x;
-  for (int g = np - 1; g >= 0; g--) {
-    const int cbg = ob - g * kPanel < kPanel ? ob - g * kPanel : kPanel;
-    const float* Li = Li0 + (uint64_t)g * kPanel * kPanel;
-    for (int e = t; e < kPanel * kPanel; e += kThreads) {
-      const int er = e % kPanel, ec = e / kPanel;
-      if (er < cbg && ec < cbg) cp_async4(Ls + g * kPanel * kLd + ec * kLd + er, Li + e);
-    }
-    for (int e = t; e < kPanel * g * kPanel; e += kThreads) {
-      const int er = e % kPanel, ec = e / kPanel;   // row er of panel g, column ec < 64 g
-      if (er < cbg)
-        cp_async4(Tb + tri_off(g) + ec * kLd + er, F + (o0 + g * kPanel + er) + (o0 + ec) * m);
-    }
-    cp_async_commit();
-  }
-  if (t < ob) tb[t] = v[o0 + t];
-  const int r = t >> 2, q = t & 3;   // kThreads = 4 x kPanel
-  for (int g = np - 1; g >= 0; g--) {
-    const int p = g * kPanel;
-    const int cb = ob - p < kPanel ? ob - p : kPanel;
-    cp_async_wait(g);
-    __syncthreads();
-    if (t < kPanel) xs[t] = D::split(t < cb ? tb[p + t] : 0.0);
-    __syncthreads();
-    // x_r = sum_{c >= r} Linv[c][r] t_c (column r of the inverse)
-    const float* L = Ls + g * kPanel * kLd + r * kLd;
-    D x;
-    if (r < cb) {
-      D x1;
-#pragma unroll
-      for (int j = 0; j < kPanel / 4; j += 2) {
-        const int c0 = q * (kPanel / 4) + j, c1 = c0 + 1;
-        if (c0 < cb) x.add(L[c0], xs[c0]);
-        if (c1 < cb) x1.add(L[c1], xs[c1]);
-      }
-      x.merge(x1);
-    }
-    x.shfl_xor(1);
-    x.shfl_xor(2);
-    __syncthreads();
-    if (r < cb && q == 0) {
-      const double xv = x.value();
-      tb[p + r] = xv;
-      xs[r] = D::split(xv);
-    }
-    __syncthreads();
-    // the pivots before the panel: t_j -= sum_c L[p+c][j] x_c
-    for (int j0 = 0; j0 < p; j0 += kThreads / 4) {
-      const int j = j0 + r;
-      D a;
-      if (j < p) {
-        const float* Tj = Tb + tri_off(g) + j * kLd;
-        D a1;
-#pragma unroll
-        for (int u = 0; u < kPanel / 4; u += 2) {
-          const int c0 = q * (kPanel / 4) + u, c1 = c0 + 1;
-          if (c0 < cb) a.add(Tj[c0], xs[c0]);
-          if (c1 < cb) a1.add(Tj[c1], xs[c1]);
-        }
-        a.merge(a1);
-      }
-      a.shfl_xor(1);
-      a.shfl_xor(2);
-      if (j < p && q == 0) tb[j] -= a.value();
-    }
-    __syncthreads();
-  }
-  if (t < ob) v[o0 + t] = tb[t];
-}
-
-// the solved pivots of the large supernodes into xf (factor order)
-__global__ void store_pivots_kernel(BigBatch b, LdltDev d, const double* __restrict__ vec,
-                                    double* __restrict__ xf) {
-  const int s = b.list[blockIdx.y];
-  const int64_t k = d.sn_first[s + 1] - d.sn_first[s];
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= k) return;
-  xf[d.sn_first[s] + c] = vec[d.vec_off[s] + c];
+  for (; c < ob; c += 32) a[0].add(Fj[c], xb[c]);
+  a[0].merge(a[1]);
+  a[2].merge(a[3]);
+  a[0].merge(a[2]);
+  for (int o = 16; o > 0; o >>= 1) a[0].shfl_down(o);
+  if (lane == 0) vec[d.vec_off[s] + j] -= a[0].value();
 }
 
 __global__ void solve_finish_kernel(int64_t n, const int32_t* __restrict__ perm,
@@ -1793,6 +1770,7 @@ struct nla3d_ldlt {
   std::vector<void*> allocs;
   void* d_front = nullptr;
   double* d_vec = nullptr;
+  double* d_y = nullptr;        // wide fronts: L^-1 of their pivots' entries
   double* d_xf = nullptr;
   double* d_r = nullptr;
   double* d_dx = nullptr;
@@ -1819,9 +1797,16 @@ struct nla3d_ldlt {
   float* d_pk = nullptr;
   OuterTile* d_tiles = nullptr; // tensor-core fronts: every level's outer-block tile lists
   int n_sm = 0;
+  InvTask* d_inv = nullptr;     // the inverses' joins: every level's tasks
+  uint64_t* d_toff = nullptr;   // per large front: its part of the joins' workspace
+  void* d_work = nullptr;
+  cudaStream_t side = nullptr;  // the joins run beside the next levels
+  cudaEvent_t fork = nullptr, join = nullptr;
+  int32_t* d_bidx = nullptr;    // per front row (level order): its right-hand side entry or -1,
+  uint32_t* d_gptr = nullptr;   // and its children's update rows
+  uint32_t* d_gsrc = nullptr;
   uint64_t* d_adest = nullptr;
   int32_t* d_perm = nullptr;
-  int32_t* d_col2sn = nullptr;
   int32_t* d_lists = nullptr;   // level lists, small lists, extend-add child lists
   int64_t* d_fptr = nullptr;
   int32_t* d_fcol = nullptr;
@@ -1830,13 +1815,17 @@ struct nla3d_ldlt {
   // host schedule per level
   struct Level {
     int64_t all_off = 0, all_cnt = 0;     // every supernode of the level
-    int64_t small_off = 0, small_cnt = 0;
+    int64_t small_off = 0, small_cnt = 0, tiny_cnt = 0;   // the tiny ones come first
     int32_t small_max_m = 0;
     int64_t large_off = 0, large_cnt = 0; // fronts above kSmallFront rows
     int64_t wo_off = 0;                   // their W offsets in d_wo
     int64_t large_max_m = 0, large_max_k = 0;
     std::vector<int64_t> tile_off, tile_cnt;  // tensor-core fronts: per outer block, its tiles
     std::vector<int64_t> itile_off, itile_cnt;  // and per panel, its in-block update's tiles
+    int64_t inv_off[3] = {}, inv_cnt[3] = {};   // joins of 64-, 128-, 256-pivot blocks
+    uint64_t vec0 = 0, vec1 = 0;                // its fronts' rows in the solve vectors
+    int64_t narrow_off = 0, narrow_cnt = 0, narrow_max_u = 0;   // solves: large fronts by width
+    int64_t wide_off = 0, wide_cnt = 0, wide_max_m = 0, wide_max_k = 0;
     std::vector<int64_t> ea_off, ea_cnt;  // children of the level's parents, by ordinal
     std::vector<uint32_t> ea_gy;          // column blocks per child (its update's size)
   };
@@ -1885,6 +1874,7 @@ cudaError_t enqueue_factor(nla3d_ldlt* h, const double* values) {
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(h->d_perturbed, 0, 2 * sizeof(int), st);
   if (e != cudaSuccess) return e;
+  bool forked = false;
   {
     const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(
         kMaxBlocks, (S.nnz + kThreads - 1) / kThreads));
@@ -1966,74 +1956,86 @@ cudaError_t enqueue_factor(nla3d_ldlt* h, const double* values) {
         }
         update(o0, 1, rest, ~0u);
       }
+      // the solves' inverses on the side stream
+      if (L.inv_cnt[0]) {
+        if ((e = cudaEventRecord(h->fork, st)) != cudaSuccess) return e;
+        if ((e = cudaStreamWaitEvent(h->side, h->fork, 0)) != cudaSuccess) return e;
+        forked = true;
+        for (int q = 0; q < 3; q++)
+          for (int pass = 0; pass < 2 && L.inv_cnt[q]; pass++)
+            inv_join_kernel<T><<<(unsigned)L.inv_cnt[q], kThreads, 0, h->side>>>(
+                h->d_inv + L.inv_off[q], bb, h->dev, front, h->d_toff + L.wo_off,
+                static_cast<T*>(h->d_work), kPanel << q, pass);
+      }
     }
+  }
+  if (forked) {
+    if ((e = cudaEventRecord(h->join, h->side)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(st, h->join, 0)) != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }
 
 template <typename T, typename D>
 cudaError_t enqueue_solve_core(nla3d_ldlt* h, const double* b) {
-  const LdltSymbolic& S = h->S;
+  constexpr int kWarps = kThreads / 32;
   const T* front = static_cast<const T*>(h->d_front);
   cudaStream_t st = h->stream;
-  cudaError_t e = cudaMemsetAsync(h->d_vec, 0, sizeof(double) * S.vec_off.back(), st);
-  if (e != cudaSuccess) return e;
-  const unsigned nb = (unsigned)((S.n + kThreads - 1) / kThreads);
-  solve_init_kernel<<<nb, kThreads, 0, st>>>(S.n, h->d_perm, h->d_col2sn, h->dev, b, h->d_vec);
-  const T* Li = static_cast<const T*>(h->d_Linv);
   for (const auto& L : h->levels) {
-    for (size_t q = 0; q < L.ea_off.size(); q++)
-      if (L.ea_cnt[q])
-        vec_extend_add_kernel<<<(unsigned)L.ea_cnt[q], kThreads, 0, st>>>(h->d_lists + L.ea_off[q],
-                                                                           h->dev, h->d_vec);
-    if (L.small_cnt)
-      forward_kernel<T><<<(unsigned)L.small_cnt, kThreads, 0, st>>>(h->d_lists + L.small_off,
-                                                                    h->dev, front, h->d_vec);
-    if (L.large_cnt) {
-      const BigBatch bb{h->d_lists + L.large_off, h->d_wo + L.wo_off, h->d_lio + L.wo_off};
-      const unsigned nf = (unsigned)L.large_cnt;
-      for (int64_t o0 = 0; o0 < L.large_max_k; o0 += kOuter) {
-        if constexpr (std::is_same<T, float>::value)
-          fwd_block_staged_kernel<D><<<nf, kThreads, kStagedSmem, st>>>(bb, h->dev, front, Li, o0,
-                                                                        h->d_vec);
-        else
-          fwd_block_kernel<T, D><<<nf, kThreads, 0, st>>>(bb, h->dev, front, Li, o0, h->d_vec);
-        const int64_t rest = L.large_max_m - o0 - 1;
-        if (rest > 0)
-          fwd_rows_block_kernel<T, D><<<dim3((unsigned)((rest + 31) / 32), nf),
-                                     kThreads, 0, st>>>(bb, h->dev, front, o0, h->d_vec);
-      }
-      scale_pivots_kernel<T><<<dim3((unsigned)((L.large_max_k + kThreads - 1) / kThreads), nf),
-                               kThreads, 0, st>>>(bb, h->dev, front, h->d_vec);
+    gather_level_kernel<<<(unsigned)((L.vec1 - L.vec0 + kThreads - 1) / kThreads), kThreads, 0, st>>>(
+        L.vec0, L.vec1, h->d_bidx, h->d_gptr, h->d_gsrc, b, h->d_vec);
+    if (L.tiny_cnt)
+      fwd_tiny_kernel<T><<<(unsigned)((L.tiny_cnt + kWarps - 1) / kWarps), kThreads, 0, st>>>(
+          h->d_lists + L.small_off, (int)L.tiny_cnt, h->dev, front, h->d_vec);
+    if (L.small_cnt > L.tiny_cnt)
+      forward_kernel<T><<<(unsigned)(L.small_cnt - L.tiny_cnt), kThreads, 0, st>>>(
+          h->d_lists + L.small_off + L.tiny_cnt, h->dev, front, h->d_vec);
+    if (L.narrow_cnt)
+      fwd_narrow_kernel<T, D><<<(unsigned)L.narrow_cnt, kThreads, 0, st>>>(
+          h->d_lists + L.narrow_off, h->dev, front, h->d_vec);
+    const int32_t* wide = h->d_lists + L.wide_off;
+    const unsigned nf = (unsigned)L.wide_cnt;
+    for (int64_t o0 = 0; nf && o0 < L.wide_max_k; o0 += kInv) {
+      const int64_t ob = std::min<int64_t>(kInv, L.wide_max_k - o0);
+      fwd_inv_kernel<T, D><<<dim3((unsigned)((ob + kInvRows - 1) / kInvRows), nf), kThreads, 0, st>>>(
+          wide, h->dev, front, o0, h->d_vec, h->d_y);
+      const int64_t rest = L.wide_max_m - o0 - 1;
+      if (rest <= 0) continue;
+      const dim3 grid((unsigned)((rest + 31) / 32), nf);
+      if (ob > 256)
+        fwd_rows_kernel<T, D, 16><<<grid, 512, 0, st>>>(wide, h->dev, front, o0, h->d_y, h->d_vec);
+      else
+        fwd_rows_kernel<T, D, 8><<<grid, 256, 0, st>>>(wide, h->dev, front, o0, h->d_y, h->d_vec);
     }
   }
   for (auto it = h->levels.rbegin(); it != h->levels.rend(); ++it) {
     const auto& L = *it;
-    if (L.small_cnt)
-      backward_kernel<T><<<(unsigned)L.small_cnt, kThreads, 0, st>>>(h->d_lists + L.small_off,
-                                                                     h->dev, front, h->d_vec,
-                                                                     h->d_xf);
-    if (L.large_cnt) {
-      const BigBatch bb{h->d_lists + L.large_off, h->d_wo + L.wo_off, h->d_lio + L.wo_off};
-      const unsigned nf = (unsigned)L.large_cnt;
-      const int64_t rest = L.large_max_m - 1;
-      gather_rest_kernel<T, D><<<dim3((unsigned)((rest + kThreads - 1) / kThreads), nf), kThreads,
-                              0, st>>>(bb, h->dev, h->d_vec, h->d_xf);
-      bwd_rest_kernel<T, D><<<dim3((unsigned)((L.large_max_k + kThreads / 32 - 1) / (kThreads / 32)),
-                                nf),
-                           kThreads, 0, st>>>(bb, h->dev, front, h->d_vec);
-      for (int64_t o0 = ((L.large_max_k - 1) / kOuter) * kOuter; o0 >= 0; o0 -= kOuter) {
-        if constexpr (std::is_same<T, float>::value)
-          bwd_block_staged_kernel<D><<<nf, kThreads, kStagedSmem, st>>>(bb, h->dev, front, Li, o0,
-                                                                        h->d_vec);
-        else
-          bwd_block_kernel<T, D><<<nf, kThreads, 0, st>>>(bb, h->dev, front, Li, o0, h->d_vec);
-        if (o0 > 0)
-          bwd_cols_block_kernel<T, D><<<dim3((unsigned)((o0 + 31) / 32), nf), kThreads, 0, st>>>(
-              bb, h->dev, front, o0, h->d_vec);
-      }
-      store_pivots_kernel<<<dim3((unsigned)((L.large_max_k + kThreads - 1) / kThreads), nf),
-                            kThreads, 0, st>>>(bb, h->dev, h->d_vec, h->d_xf);
+    if (L.tiny_cnt)
+      bwd_tiny_kernel<T><<<(unsigned)((L.tiny_cnt + kWarps - 1) / kWarps), kThreads, 0, st>>>(
+          h->d_lists + L.small_off, (int)L.tiny_cnt, h->dev, front, h->d_vec, h->d_xf);
+    if (L.small_cnt > L.tiny_cnt)
+      backward_kernel<T><<<(unsigned)(L.small_cnt - L.tiny_cnt), kThreads, 0, st>>>(
+          h->d_lists + L.small_off + L.tiny_cnt, h->dev, front, h->d_vec, h->d_xf);
+    if (L.narrow_cnt)
+      bwd_narrow_kernel<T, D>
+          <<<(unsigned)L.narrow_cnt, kThreads, sizeof(double) * (size_t)L.narrow_max_u, st>>>(
+              h->d_lists + L.narrow_off, h->dev, front, h->d_vec, h->d_xf);
+    if (!L.wide_cnt) continue;
+    const int32_t* wide = h->d_lists + L.wide_off;
+    const unsigned nf = (unsigned)L.wide_cnt;
+    gather_rest_kernel<T, D>
+        <<<dim3((unsigned)((L.wide_max_m + kThreads - 1) / kThreads), nf), kThreads, 0, st>>>(
+            wide, h->dev, h->d_vec, h->d_xf);
+    bwd_rest_kernel<T, D>
+        <<<dim3((unsigned)((L.wide_max_k + kWarps - 1) / kWarps), nf), kThreads, 0, st>>>(
+            wide, h->dev, front, h->d_y, h->d_vec);
+    for (int64_t o0 = (L.wide_max_k - 1) / kInv * kInv; o0 >= 0; o0 -= kInv) {
+      const int64_t ob = std::min<int64_t>(kInv, L.wide_max_k - o0);
+      bwd_inv_kernel<T, D><<<dim3((unsigned)((ob + 31) / 32), nf), kColThreads, 0, st>>>(
+          wide, h->dev, front, o0, h->d_vec, h->d_xf);
+      if (o0 > 0)
+        bwd_cols_kernel<T, D><<<dim3((unsigned)((o0 + kWarps - 1) / kWarps), nf), kThreads, 0, st>>>(
+            wide, h->dev, front, o0, h->d_xf, h->d_vec);
     }
   }
   return cudaGetLastError();
@@ -2100,9 +2102,14 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   const int64_t ns = S.n_sn();
   const int nlev = (int)S.level_ptr.size() - 1;
   std::vector<int32_t> lists;
-  std::vector<int32_t> col2sn(S.n);
-  for (int64_t s = 0; s < ns; s++)
-    for (int32_t t = S.sn_first[s]; t < S.sn_first[s + 1]; t++) col2sn[t] = (int32_t)s;
+  LdltSolveLists solve_lists;
+  if (!ldlt_solve_lists(S, &solve_lists).empty()) {
+    delete h;
+    return NLA3D_ERR_RANGE;
+  }
+  std::vector<InvTask> inv_tasks;
+  std::vector<uint64_t> toff;
+  uint64_t max_work = 0;
   std::vector<uint64_t> wo, lio, pko;
   std::vector<OuterTile> tiles;
   int64_t max_w = 0, max_large_cnt = 0, max_pk = 0;
@@ -2114,14 +2121,16 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
     for (int32_t q = S.level_ptr[L]; q < S.level_ptr[L + 1]; q++) lists.push_back(S.level_list[q]);
     lv.all_cnt = (int64_t)lists.size() - lv.all_off;
     lv.small_off = (int64_t)lists.size();
-    for (int32_t q = S.level_ptr[L]; q < S.level_ptr[L + 1]; q++) {
-      const int32_t s = S.level_list[q];
-      if (S.m(s) <= kSmallFront) {
+    for (int tiny = 1; tiny >= 0; tiny--) {
+      for (int32_t q = S.level_ptr[L]; q < S.level_ptr[L + 1]; q++) {
+        const int32_t s = S.level_list[q];
+        if (S.m(s) > kSmallFront || (S.k(s) <= kTinyPivots) != (tiny != 0)) continue;
         lists.push_back(s);
         lv.small_max_m = std::max(lv.small_max_m, S.m(s));
       }
+      lv.small_cnt = (int64_t)lists.size() - lv.small_off;
+      if (tiny) lv.tiny_cnt = lv.small_cnt;
     }
-    lv.small_cnt = (int64_t)lists.size() - lv.small_off;
     lv.large_off = (int64_t)lists.size();
     lv.wo_off = (int64_t)wo.size();
     int64_t w = 0, pk = 0;
@@ -2141,6 +2150,49 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
       }
     }
     lv.large_cnt = (int64_t)lists.size() - lv.large_off;
+    // the solves: the large fronts by width, and the joins of the wide ones'
+    // inverses (narrow ones have no second 64-pivot block)
+    lv.vec0 = solve_lists.level_off[L];
+    lv.vec1 = solve_lists.level_off[L + 1];
+    for (int wide = 0; wide < 2; wide++) {
+      (wide ? lv.wide_off : lv.narrow_off) = (int64_t)lists.size();
+      for (int64_t z = 0; z < lv.large_cnt; z++) {
+        const int32_t s = lists[lv.large_off + z];
+        const int64_t m = S.m(s), k = S.k(s);
+        if ((k > kNarrow || m > kNarrowRows) != (wide != 0)) continue;
+        lists.push_back(s);
+        if (wide) {
+          lv.wide_max_m = std::max(lv.wide_max_m, m);
+          lv.wide_max_k = std::max(lv.wide_max_k, k);
+        } else {
+          lv.narrow_max_u = std::max(lv.narrow_max_u, m - k);
+        }
+      }
+    }
+    lv.narrow_cnt = lv.wide_off - lv.narrow_off;
+    lv.wide_cnt = (int64_t)lists.size() - lv.wide_off;
+    uint64_t work = 0;
+    for (int64_t z = 0; z < lv.large_cnt; z++) {
+      const int64_t k = S.k(lists[lv.large_off + z]);
+      toff.push_back(work);
+      if (k > kPanel) work += (uint64_t)k * (kInv / 2);
+    }
+    max_work = std::max(max_work, work);
+    const int bt = precision ? InvTile<float>::BT : InvTile<double>::BT;
+    for (int q = 0; q < 3; q++) {
+      const int64_t sz = (int64_t)kPanel << q;
+      lv.inv_off[q] = (int64_t)inv_tasks.size();
+      for (int64_t z = 0; z < lv.large_cnt; z++) {
+        const int64_t k = S.k(lists[lv.large_off + z]);
+        for (int64_t j0 = 0; j0 + sz < k; j0 += 2 * sz) {
+          const int64_t rows = std::min(sz, k - j0 - sz);
+          for (int64_t ct = 0; ct * bt < rows; ct++)
+            for (int64_t at = 0; at * bt < sz; at++)
+              inv_tasks.push_back(InvTask{(uint32_t)z, (uint32_t)j0, (uint32_t)(ct << 16 | at)});
+        }
+      }
+      lv.inv_cnt[q] = (int64_t)inv_tasks.size() - lv.inv_off[q];
+    }
     if (h->tc) {
       // every outer block's update tiles (the rule of update_range, outer):
       // per front with k > o0, rows and columns from jb = min(o0 + kOuter, k)
@@ -2223,7 +2275,8 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   e = cudaMemGetInfo(&free_b, &total_b);
   const size_t tsize = precision ? sizeof(float) : sizeof(double);
   const double need = (double)h->front_entries * tsize + (double)S.nnz * 8 + (double)S.n * 64 +
-                      (double)S.full_col.size() * 8 + (double)S.rows.size() * 8;
+                      (double)S.full_col.size() * 8 + (double)S.rows.size() * 24 +
+                      (double)max_work * tsize;
   int rc = NLA3D_OK;
   if (e != cudaSuccess)
     rc = cuda_fail(h, e, "cudaMemGetInfo");
@@ -2263,7 +2316,20 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   }
   LCK(upload(h, &h->d_wo, wo));
   LCK(upload(h, &h->d_lio, lio));
-  LCK(dalloc(h, &h->d_vec, S.vec_off.back()));
+  LCK(dalloc(h, &h->d_vec, S.rows.size()));
+  LCK(dalloc(h, &h->d_y, S.rows.size()));
+  LCK(upload(h, &h->d_bidx, solve_lists.b_idx));
+  LCK(upload(h, &h->d_gptr, solve_lists.ptr));
+  LCK(upload(h, &h->d_gsrc, solve_lists.src));
+  LCK(upload(h, &h->d_inv, inv_tasks));
+  LCK(upload(h, &h->d_toff, toff));
+  if (precision)
+    LCK(dalloc(h, reinterpret_cast<float**>(&h->d_work), (size_t)max_work));
+  else
+    LCK(dalloc(h, reinterpret_cast<double**>(&h->d_work), (size_t)max_work));
+  LCK(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
+  LCK(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
+  LCK(cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming));
   LCK(dalloc(h, &h->d_xf, S.n));
   LCK(dalloc(h, &h->d_rhs, S.n));
   LCK(dalloc(h, &h->d_r, S.n));
@@ -2287,7 +2353,6 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   }
   LCK(upload(h, &h->d_adest, S.a_dest));
   LCK(upload(h, &h->d_perm, S.perm));
-  LCK(upload(h, &h->d_col2sn, col2sn));
   LCK(upload(h, &h->d_lists, lists));
   LCK(upload(h, &h->d_fptr, S.full_ptr));
   LCK(upload(h, &h->d_fcol, S.full_col));
@@ -2297,7 +2362,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   int32_t *rw = nullptr, *sf = nullptr, *sp = nullptr;
   uint32_t* rl = nullptr;
   LCK(upload(h, &fo, S.front_off));
-  LCK(upload(h, &vo, S.vec_off));
+  LCK(upload(h, &vo, solve_lists.vec_off));
   LCK(upload(h, &rp, S.row_ptr));
   LCK(upload(h, &rw, S.rows));
   LCK(upload(h, &sf, S.sn_first));
@@ -2393,17 +2458,6 @@ cudaError_t enqueue_solve_any(nla3d_ldlt* h, const double* rhs, double* out, int
   const bool accurate = h->prec && h->solve_accurate;
   cudaGraphExec_t& exec = accurate ? h->solve_exec_acc : h->solve_exec;
   if (!exec) {
-    if (h->prec) {
-      // the staged block triangles take more than the default 48 KB
-      const void* kf[4] = {(const void*)fwd_block_staged_kernel<Dot<float>>,
-                           (const void*)bwd_block_staged_kernel<Dot<float>>,
-                           (const void*)fwd_block_staged_kernel<DotWide>,
-                           (const void*)bwd_block_staged_kernel<DotWide>};
-      for (const void* f : kf) {
-        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStagedSmem);
-        if (e != cudaSuccess) return e;
-      }
-    }
     cudaGraph_t g = nullptr;
     e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
@@ -2567,7 +2621,9 @@ int nla3d_ldlt_solve(nla3d_ldlt* h, const double* values, const double* b, doubl
     if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve");
     rel = rnorm / (bnorm > 0.0 ? bnorm : 1.0);
     if (!(rel > tol) || it >= max_refine) break;
-    if (it > 0 && !(rel < 0.1 * prev)) {
+    // (a step that cut less, but whose rate reaches tol with one more, is
+    // still cheaper than GMRES, which takes two applications at least)
+    if (it > 0 && !(rel < 0.1 * prev) && !(rel < prev && rel * (rel / prev) <= tol)) {
       h->solve_accurate = 1;
       e = gmres_refine(h, values, b, x, tol, max_refine, &it, &rel);
       if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve (GMRES)");
@@ -2735,6 +2791,9 @@ int nla3d_ldlt_destroy(nla3d_ldlt* h) {
   if (h->factor_exec) cudaGraphExecDestroy(h->factor_exec);
   if (h->solve_exec) cudaGraphExecDestroy(h->solve_exec);
   if (h->solve_exec_acc) cudaGraphExecDestroy(h->solve_exec_acc);
+  if (h->fork) cudaEventDestroy(h->fork);
+  if (h->join) cudaEventDestroy(h->join);
+  if (h->side) cudaStreamDestroy(h->side);
   for (void* p : h->allocs) cudaFree(p);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
   delete h;

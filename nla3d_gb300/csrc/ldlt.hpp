@@ -30,7 +30,6 @@ struct LdltSymbolic {
   std::vector<int64_t> rel_ptr;     // per supernode: its update rows' positions in the parent
   std::vector<uint32_t> rel;
   std::vector<uint64_t> front_off;  // m(s)^2 entries per front (column-major)
-  std::vector<uint64_t> vec_off;    // m(s) entries per front vector (solve)
   std::vector<uint64_t> a_dest;     // per input slot: index into the front buffer
   // full (both triangles) CSR of the input in input numbering, values by slot (SpMV)
   std::vector<int64_t> full_ptr;
@@ -56,3 +55,15 @@ std::string ldlt_nd_order(int64_t n, const uint32_t* iofeir, const uint32_t* col
                           const double* points, int64_t n_dofs, int32_t* order);
 std::string ldlt_analyze(int64_t n, const uint32_t* iofeir, const uint32_t* columns,
                          const int32_t* perm, LdltSymbolic* out);
+
+// The solve vectors' layout: front s's m(s) rows at vec_off[s], fronts in level
+// order (a level's rows are contiguous).  Row p starts from entry b_idx[p] of
+// the right-hand side (input numbering; -1: an update row, zero) and adds the
+// children's update rows src[ptr[p] .. ptr[p+1]), in child order.
+struct LdltSolveLists {
+  std::vector<uint64_t> vec_off;    // per supernode
+  std::vector<uint64_t> level_off;  // per level, + 1
+  std::vector<int32_t> b_idx;
+  std::vector<uint32_t> ptr, src;
+};
+std::string ldlt_solve_lists(const LdltSymbolic& S, LdltSolveLists* out);

@@ -429,13 +429,11 @@ std::string ldlt_analyze(int64_t n, const uint32_t* iofeir, const uint32_t* colu
   }
   // ---- offsets, statistics, levels ----
   S.front_off.assign(ns + 1, 0);
-  S.vec_off.assign(ns + 1, 0);
   S.level.assign(ns, 0);
   int32_t max_level = 0;
   for (int32_t s = 0; s < ns; s++) {
     const int64_t m = S.m(s), k = S.k(s);
     S.front_off[s + 1] = S.front_off[s] + (uint64_t)(m * m);
-    S.vec_off[s + 1] = S.vec_off[s] + (uint64_t)m;
     S.nnz_L += (uint64_t)(k * m - k * (k - 1) / 2);
     for (int64_t c = 0; c < k; c++) {
       const double r = (double)(m - c - 1);
@@ -558,5 +556,71 @@ std::string ldlt_analyze(int64_t n, const uint32_t* iofeir, const uint32_t* colu
   }
   S.perm.resize(n);
   for (int32_t t = 0; t < n; t++) S.perm[t] = p0[post[t]];
+  return "";
+}
+
+std::string ldlt_solve_lists(const LdltSymbolic& S, LdltSolveLists* out) {
+  const int64_t ns = S.n_sn();
+  const int nlev = (int)S.level_ptr.size() - 1;
+  const uint64_t total = S.rows.size();
+  if (total >= 0xFFFFFFFFull) return "solve vectors exceed 32-bit indices";
+  out->vec_off.assign(ns, 0);
+  out->level_off.assign(nlev + 1, 0);
+  // per front in level order: its rows' offset and its children's rows' offset
+  std::vector<uint64_t> src_off(ns, 0);
+  uint64_t v = 0, w = 0;
+  for (int L = 0; L < nlev; L++) {
+    out->level_off[L] = v;
+    for (int32_t q = S.level_ptr[L]; q < S.level_ptr[L + 1]; q++) {
+      const int32_t s = S.level_list[q];
+      out->vec_off[s] = v;
+      src_off[s] = w;
+      v += (uint64_t)S.m(s);
+      for (int32_t c = S.child_ptr[s]; c < S.child_ptr[s + 1]; c++)
+        w += (uint64_t)(S.rel_ptr[S.child_list[c] + 1] - S.rel_ptr[S.child_list[c]]);
+    }
+  }
+  out->level_off[nlev] = v;
+  out->b_idx.resize(total);
+  out->ptr.resize(total + 1);
+  out->src.resize(w);
+  out->ptr[total] = (uint32_t)w;
+  // every front fills its own rows and lists (fronts split over the threads)
+  auto fill = [&](int64_t q0, int64_t q1) {
+    std::vector<uint32_t> pos;
+    for (int64_t q = q0; q < q1; q++) {
+      const int32_t s = S.level_list[q];
+      const int64_t m = S.m(s), k = S.k(s);
+      const uint64_t o = out->vec_off[s];
+      for (int64_t i = 0; i < m; i++) out->b_idx[o + i] = i < k ? S.perm[S.sn_first[s] + i] : -1;
+      pos.assign(m + 1, 0);
+      for (int32_t c = S.child_ptr[s]; c < S.child_ptr[s + 1]; c++) {
+        const int32_t ch = S.child_list[c];
+        for (int64_t t = S.rel_ptr[ch]; t < S.rel_ptr[ch + 1]; t++) pos[S.rel[t] + 1]++;
+      }
+      for (int64_t i = 0; i < m; i++) pos[i + 1] += pos[i];
+      for (int64_t i = 0; i < m; i++) out->ptr[o + i] = (uint32_t)(src_off[s] + pos[i]);
+      for (int32_t c = S.child_ptr[s]; c < S.child_ptr[s + 1]; c++) {
+        const int32_t ch = S.child_list[c];
+        const uint64_t from = out->vec_off[ch] + (uint64_t)S.k(ch);
+        for (int64_t t = S.rel_ptr[ch]; t < S.rel_ptr[ch + 1]; t++)
+          out->src[src_off[s] + pos[S.rel[t]]++] = (uint32_t)(from + (uint64_t)(t - S.rel_ptr[ch]));
+      }
+    }
+  };
+  const int nt = (int)std::min<int64_t>(std::max(1u, std::thread::hardware_concurrency()),
+                                        std::max<int64_t>(1, ns / 256));
+  std::atomic<int64_t> next{0};
+  auto work = [&] {
+    for (;;) {
+      const int64_t q0 = next.fetch_add(64);
+      if (q0 >= ns) return;
+      fill(q0, std::min<int64_t>(ns, q0 + 64));
+    }
+  };
+  std::vector<std::thread> th;
+  for (int t = 1; t < nt; t++) th.emplace_back(work);
+  work();
+  for (auto& x : th) x.join();
   return "";
 }
