@@ -415,6 +415,16 @@ cudaError_t enqueue_gather_F(nla3d_ctx* c) {
   return e;
 }
 
+// K and F, all slots, in one launch
+cudaError_t enqueue_gather_both(nla3d_ctx* c) {
+  const bool slots = c->layout != 0;
+  const GatherArgs gk{c->Ktot(), c->d_kptr, slots ? nullptr : c->d_kids, c->d_contribK, c->d_K};
+  const GatherArgs gf{c->Utot(), c->d_fptr, slots ? nullptr : c->d_fids, c->d_contribF, c->d_F};
+  const cudaError_t e = launch_gather_pair(gk, gf, c->gather_bs, c->stream);
+  if (e == cudaSuccess) c->launches++;
+  return e;
+}
+
 // MPC rows after the element sums (FEStorage.cpp:41-61).
 cudaError_t enqueue_mpc(nla3d_ctx* c) {
   cudaError_t e = cudaSuccess;
@@ -460,9 +470,7 @@ cudaError_t enqueue_gather_C(nla3d_ctx* c) {
 }
 
 cudaError_t reset_status(nla3d_ctx* c) {
-  cudaError_t e = cudaMemsetAsync(c->d_status, 0, sizeof(ElementStatus), c->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(&c->d_status->first, 0xFF, sizeof(uint32_t), c->stream);
-  return e;
+  return cudaMemsetAsync(c->d_status, 0, sizeof(ElementStatus), c->stream);
 }
 
 cudaError_t enqueue_assembly(nla3d_ctx* c) {
@@ -475,10 +483,15 @@ cudaError_t enqueue_assembly(nla3d_ctx* c) {
   mark(0);
   if ((e = enqueue_elements(c, 0, (uint32_t)c->E())) != cudaSuccess) return e;
   mark(1);
-  if ((e = enqueue_gather_K(c, 0, c->Ktot())) != cudaSuccess) return e;
-  if ((e = enqueue_gather_C(c)) != cudaSuccess) return e;
-  mark(2);
-  if ((e = enqueue_gather_F(c)) != cudaSuccess) return e;
+  if (c->timing) {   // K and F apart, as kernel_times reports them
+    if ((e = enqueue_gather_K(c, 0, c->Ktot())) != cudaSuccess) return e;
+    if ((e = enqueue_gather_C(c)) != cudaSuccess) return e;
+    mark(2);
+    if ((e = enqueue_gather_F(c)) != cudaSuccess) return e;
+  } else {
+    if ((e = enqueue_gather_both(c)) != cudaSuccess) return e;
+    if ((e = enqueue_gather_C(c)) != cudaSuccess) return e;
+  }
   mark(3);
   if ((e = enqueue_mpc(c)) != cudaSuccess) return e;
   mark(4);
@@ -968,7 +981,6 @@ int nla3d_init_solution_data(nla3d_ctx* c) {
     }
   }
   CK(cudaMemsetAsync(c->d_status, 0, sizeof(ElementStatus), c->stream));
-  CK(cudaMemsetAsync(&c->d_status->first, 0xFF, sizeof(uint32_t), c->stream));
   if (c->hm[0].etype == NLA3D_SOLID81) {
     // FP64 contexts keep the geometry of their kernel, mixed ones dN/dX as float pairs
     if (mixed_solid) {
@@ -1353,7 +1365,7 @@ int nla3d_element_status(nla3d_ctx* c, uint32_t* count, uint32_t* first) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "element_status");
   if (count) *count = st.count;
-  if (first) *first = st.count ? st.first : 0;
+  if (first) *first = st.count ? st.first() : 0;
   return st.count ? NLA3D_ERR_ELEMENT : NLA3D_OK;
 }
 
@@ -1491,7 +1503,7 @@ int nla3d_graph_launch(nla3d_ctx* c) {
   if (!c || !c->graph_exec) return fail(c, NLA3D_ERR_ARG, "graph_launch without a captured graph");
   cudaError_t e = cudaGraphLaunch(c->graph_exec, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "graph_launch");
-  c->launches += 3 + (c->Mtot() ? 1 : 0) + (c->n_lmpc ? 1 : 0);
+  c->launches += 2 + (c->Mtot() ? 1 : 0) + (c->n_lmpc ? 1 : 0);
   return NLA3D_OK;
 }
 

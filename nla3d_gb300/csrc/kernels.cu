@@ -91,7 +91,7 @@ __device__ __forceinline__ int voigt(int J, int L) {
 
 __device__ __forceinline__ void flag_element(ElementStatus* st, uint32_t el1) {
   atomicAdd(&st->count, 1u);
-  atomicMin(&st->first, el1);
+  atomicMax(&st->first_inv, ~el1);
 }
 
 template <typename TT>
@@ -1518,12 +1518,12 @@ __device__ __forceinline__ double plus_zero_sum(double x) {
 }
 
 template <bool kIds>
-__global__ void __launch_bounds__(kMaxGatherBlock)
-    gather_sorted_kernel(const uint64_t s_begin, const uint64_t n_slots,
-                         const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ ids,
-                         const double* __restrict__ contrib, double* __restrict__ out,
-                         const uint32_t* __restrict__ skip) {
-  if (skip && *skip) return;  // the same word for every thread: a uniform exit
+__device__ __forceinline__ void gather_block(const uint64_t block, const uint64_t s_begin,
+                                             const uint64_t n_slots,
+                                             const uint32_t* __restrict__ ptr,
+                                             const uint32_t* __restrict__ ids,
+                                             const double* __restrict__ contrib,
+                                             double* __restrict__ out) {
   __shared__ uint32_t s_beg[kMaxGatherBlock];
   __shared__ uint32_t s_end[kMaxGatherBlock];
   __shared__ uint16_t s_slot[kMaxGatherBlock];
@@ -1531,7 +1531,7 @@ __global__ void __launch_bounds__(kMaxGatherBlock)
   __shared__ uint32_t s_total[kCountClasses];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n_warps = blockDim.x >> 5;
-  const uint64_t base = s_begin + (uint64_t)blockIdx.x * blockDim.x;
+  const uint64_t base = s_begin + block * blockDim.x;
   const uint64_t s = base + tid;
   uint32_t b = 0, e = 0;
   if (s < n_slots) {
@@ -1588,23 +1588,131 @@ __global__ void __launch_bounds__(kMaxGatherBlock)
   out[slot] = v;
 }
 
+template <bool kIds>
+__global__ void __launch_bounds__(kMaxGatherBlock)
+    gather_sorted_kernel(const uint64_t s_begin, const uint64_t n_slots,
+                         const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ ids,
+                         const double* __restrict__ contrib, double* __restrict__ out,
+                         const uint32_t* __restrict__ skip) {
+  if (skip && *skip) return;  // the same word for every thread: a uniform exit
+  gather_block<kIds>(blockIdx.x, s_begin, n_slots, ptr, ids, contrib, out);
+}
+
+// K and F in one launch, F's blocks after K's: a small model's assembly is as
+// long as its launches (1,000 elements: 28.7 -> 27.8 us a call with this,
+// one memset of the status instead of two, and the launch shape looked up once
+// per device)
+template <bool kIds>
+__global__ void __launch_bounds__(kMaxGatherBlock)
+    gather_pair_kernel(const GatherArgs k, const GatherArgs f, const uint32_t k_blocks) {
+  if (blockIdx.x < k_blocks)
+    gather_block<kIds>(blockIdx.x, k.s_begin, k.n_slots, k.ptr, k.ids, k.contrib, k.out);
+  else
+    gather_block<kIds>(blockIdx.x - k_blocks, f.s_begin, f.n_slots, f.ptr, f.ids, f.contrib, f.out);
+}
+
 // Sparse block products of the Newton iteration (FESolver.cpp:454-466):
 // one thread per output entry walks its precomputed list in the reference's
 // order; explicit _rn operations keep (K x) coef and the running sum from
 // being fused, so each entry is the reference's value bit for bit (structural
 // zeros, which the reference's symmetric product also visits, add +-0 there
-// and are not visited here).
-__global__ void block_mv_kernel(const BlockMvArgs a) {
+// and are not visited here).  The walk is a chain of two dependent loads per
+// entry: kMvBatch entries' indices, then their values and products, are in
+// flight before the ordered adds.  A row of more than kMvLong entries (a
+// rigid-body master couples to every slave) would still hold its warp for its
+// length: the warp forms such rows' products together, kMvChunk entries of up
+// to kMvRows rows at a time, and their own threads only add them (K(2) of a 9
+// x 11 x 43 bar, 20,103 rows, the longest 360 entries: 108 -> 49 us).  The skip
+// test and a coefficient of +-1 stay off the FP64 pipe; a skipped product is
+// -0, which changes no sum.
+constexpr int kMvBatch = 16;
+constexpr uint32_t kMvLong = 96;
+constexpr int kMvChunk = 64, kMvRows = 8, kMvThreads = 128;
+
+// |x| > 1e-20 (false for a NaN), on the bits
+__device__ __forceinline__ bool mv_counts(double x) {
+  const long long v = __double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll;
+  return v > __double_as_longlong(1e-20) && v <= 0x7FF0000000000000ll;
+}
+
+__global__ void __launch_bounds__(kMvThreads) block_mv_kernel(const BlockMvArgs a) {
+  __shared__ double prod[kMvThreads / 32][kMvRows][kMvChunk + 1];
   const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= a.n_out) return;
-  double acc = a.y[r];
-  const uint32_t e = __ldg(a.ptr + r + 1);
-  for (uint32_t k = __ldg(a.ptr + r); k < e; k++) {
-    const double xv = a.x[__ldg(a.xi + k)];
-    if (a.sym && !(fabs(xv) > 1e-20)) continue;
-    acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(__ldg(a.K + __ldg(a.slot + k)), xv), a.coef));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool in = r < a.n_out;
+  double acc = in ? a.y[r] : 0.0;
+  const uint32_t beg = in ? __ldg(a.ptr + r) : 0u, end = in ? __ldg(a.ptr + r + 1) : 0u;
+  const int unit = a.coef == 1.0 ? 1 : a.coef == -1.0 ? -1 : 0;
+  auto product = [&](double kv, double x) {
+    const double p = __dmul_rn(kv, x);
+    // (multiplying by +-1 rounds nothing; a NaN's sign is immaterial)
+    const double q = unit == 1 ? p : unit == -1 ? -p : __dmul_rn(p, a.coef);
+    return !a.sym || mv_counts(x) ? q : -0.0;
+  };
+  const bool is_long = end - beg > kMvLong;
+  for (uint32_t k = beg; k < end && !is_long; k += kMvBatch) {
+    uint32_t xi[kMvBatch], slot[kMvBatch];
+#pragma unroll
+    for (int u = 0; u < kMvBatch; u++) {
+      xi[u] = k + u < end ? __ldg(a.xi + k + u) : 0u;
+      slot[u] = k + u < end ? __ldg(a.slot + k + u) : 0u;
+    }
+    double x[kMvBatch], p[kMvBatch];
+#pragma unroll
+    for (int u = 0; u < kMvBatch; u++) {
+      x[u] = k + u < end ? a.x[xi[u]] : 0.0;
+      p[u] = k + u < end ? __ldg(a.K + slot[u]) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kMvBatch; u++) p[u] = product(p[u], x[u]);
+#pragma unroll
+    for (int u = 0; u < kMvBatch; u++)
+      if (k + u < end) acc = __dadd_rn(acc, p[u]);
   }
-  a.y[r] = acc;
+  __syncwarp();
+  for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, is_long); todo;) {
+    // the next kMvRows long rows of the warp
+    uint32_t rb[kMvRows], re[kMvRows];
+    int mine = -1;
+    uint32_t longest = 0;
+#pragma unroll
+    for (int i = 0; i < kMvRows; i++) {
+      const int l = todo ? __ffs(todo) - 1 : 0;
+      rb[i] = __shfl_sync(0xFFFFFFFFu, beg, l);
+      re[i] = __shfl_sync(0xFFFFFFFFu, end, l);
+      if (!todo) re[i] = rb[i];
+      else if (l == lane) mine = i;
+      longest = max(longest, re[i] - rb[i]);
+      todo &= todo - 1;
+    }
+    for (uint32_t o = 0; o < longest; o += kMvChunk) {
+#pragma unroll
+      for (int h = 0; h < kMvChunk / 32; h++) {
+        uint32_t xi[kMvRows], slot[kMvRows];
+        const uint32_t j = o + lane + 32 * h;
+#pragma unroll
+        for (int i = 0; i < kMvRows; i++) {
+          xi[i] = rb[i] + j < re[i] ? __ldg(a.xi + rb[i] + j) : 0u;
+          slot[i] = rb[i] + j < re[i] ? __ldg(a.slot + rb[i] + j) : 0u;
+        }
+        double x[kMvRows], p[kMvRows];
+#pragma unroll
+        for (int i = 0; i < kMvRows; i++) {
+          x[i] = rb[i] + j < re[i] ? a.x[xi[i]] : 0.0;
+          p[i] = rb[i] + j < re[i] ? __ldg(a.K + slot[i]) : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < kMvRows; i++)
+          prod[warp][i][lane + 32 * h] = rb[i] + j < re[i] ? product(p[i], x[i]) : -0.0;
+      }
+      __syncwarp();
+      if (mine >= 0)
+#pragma unroll 8
+        for (int j = 0; j < kMvChunk; j++) acc = __dadd_rn(acc, prod[warp][mine][j]);
+      __syncwarp();
+    }
+  }
+  if (in) a.y[r] = acc;
 }
 
 __global__ void linear_mpc_kernel(const LinearMpcArgs a) {
@@ -1947,7 +2055,20 @@ Solid81Kernel solid81_fn(bool mixed, int wpb) {
 
 cudaError_t prepare_device_tables() { return ensure_tables(); }
 
+namespace {
+// resident blocks per SM of each kernel and shape, + 1 (0: not asked yet); per
+// device, as the tables
+std::atomic<int> g_blocks_per_sm[kMaxTableDevices][2][3];
+}  // namespace
+
 int solid81_max_blocks_per_sm(bool mixed, int wpb) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::atomic<int>* known = dev >= 0 && dev < kMaxTableDevices
+                                ? &g_blocks_per_sm[dev][mixed][wpb == 2 ? 0 : wpb == 8 ? 2 : 1]
+                                : nullptr;
+  if (known)
+    if (const int v = known->load(std::memory_order_acquire)) return v - 1;
   const void* fn = reinterpret_cast<const void*>(solid81_fn(mixed, wpb));
   const size_t smem = solid81_smem_bytes_wpb(mixed, wpb);
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
@@ -1956,6 +2077,7 @@ int solid81_max_blocks_per_sm(bool mixed, int wpb) {
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, wpb * 32, smem) != cudaSuccess)
     return 0;
+  if (known) known->store(per_sm + 1, std::memory_order_release);
   return per_sm;
 }
 
@@ -2043,6 +2165,18 @@ cudaError_t launch_gather_bs(const GatherArgs& a, int bs, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+cudaError_t launch_gather_pair(const GatherArgs& k, const GatherArgs& f, int bs, cudaStream_t s) {
+  if (bs != 128 && bs != 256 && bs != 512 && bs != 1024) bs = 256;
+  const uint64_t nk = k.n_slots > k.s_begin ? (k.n_slots - k.s_begin + bs - 1) / bs : 0;
+  const uint64_t nf = f.n_slots > f.s_begin ? (f.n_slots - f.s_begin + bs - 1) / bs : 0;
+  if (nk + nf == 0) return cudaSuccess;
+  if (k.ids)
+    gather_pair_kernel<true><<<(unsigned)(nk + nf), bs, 0, s>>>(k, f, (uint32_t)nk);
+  else
+    gather_pair_kernel<false><<<(unsigned)(nk + nf), bs, 0, s>>>(k, f, (uint32_t)nk);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_gather(const GatherArgs& a, cudaStream_t s) { return launch_gather_bs(a, 256, s); }
 
 cudaError_t launch_segsum(const SegSumArgs& a, int bs, cudaStream_t s) {
@@ -2055,7 +2189,7 @@ cudaError_t launch_segsum(const SegSumArgs& a, int bs, cudaStream_t s) {
 
 cudaError_t launch_block_mv(const BlockMvArgs& a, cudaStream_t s) {
   if (a.n_out == 0) return cudaSuccess;
-  const int bs = 128;
+  const int bs = kMvThreads;
   block_mv_kernel<<<(unsigned)((a.n_out + bs - 1) / bs), bs, 0, s>>>(a);
   return cudaGetLastError();
 }
@@ -2093,21 +2227,46 @@ cudaError_t launch_linear(const LinearArgs& a, cudaStream_t s) {
 //   Kpp -= w / k,  Qe += B^T S w,  Fp += (J - 1 - p/k) w,
 // Dd and Dp the (XX, YY, XY) part of getDdDp_UP with C_zz = 1; K and F take
 // -Qe, -Fp and the entries in ElementPLANE41::assembleK order (PLANE41.h:54-95).
-__global__ void plane41_kernel(const Plane41Args a) {
+//
+// The FP64 pipe bounds it, so it runs the FP64 SOLID81 kernel's algebra (see
+// solid81_fp64_kernel) in two dimensions, one thread per element: covariant
+// 2 x 2 components (the third direction contributes its 1 to I1, I2 and C),
+// the characters of the four Gauss points accumulated point by point, modes
+// x, y, xy to nodes at the end.  Some 1,400 FP64 instructions per element
+// where forming B, Dd B and every Kuu entry per Gauss point took about 2,900
+// and spilled: 39,963 elements 277 -> 154 us (ncu, cold).
+struct Mode2 {
+  double x, y, xy;
+};
+
+// o[mask of b] = sigma_x Mx + sigma_y My + sigma_x sigma_y Mxy / sqrt(3)
+__device__ __forceinline__ void modes2_to_nodes(const Mode2& M, double o[4]) {
+#pragma unroll
+  for (int x = 0; x < 2; x++) {
+    const double p = fma(x ? kGaussA : -kGaussA, M.xy, M.y), m = x ? M.x : -M.x;
+    o[x] = m - p;
+    o[x + 2] = m + p;
+  }
+}
+
+__device__ __forceinline__ Mode2 corners_to_modes2(const double v[4]) {   // v by mask; not / 4
+  const double d1 = __dsub_rn(v[1], v[0]), d3 = __dsub_rn(v[3], v[2]);
+  const double e2 = __dsub_rn(v[2], v[0]), e3 = __dsub_rn(v[3], v[1]);
+  return {__dadd_rn(d1, d3), __dadd_rn(e2, e3), __dsub_rn(d3, d1)};
+}
+
+// One warp per block: with some 210 registers an SM holds nine, and warps of
+// 32 elements spread evenly over the SMs' FP64 pipes (in blocks of 128 the
+// last of them ran alone: 131 -> 125 us a call).
+constexpr int kPlaneThreads = 32;
+__global__ void __launch_bounds__(kPlaneThreads) plane41_kernel(const Plane41Args a) {
   const uint32_t e = a.e_begin + blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= a.n_elems) return;
   const uint32_t* cn = a.conn + (uint64_t)e * 4;
-  double X[4][2];
-  uint32_t eq[4][2];
-  for (int n = 0; n < 4; n++) {
-    X[n][0] = a.xyz[(uint64_t)(cn[n] - 1) * 3 + 0];
-    X[n][1] = a.xyz[(uint64_t)(cn[n] - 1) * 3 + 1];
-    eq[n][0] = a.node_eq3[(uint64_t)(cn[n] - 1) * 4 + 0];
-    eq[n][1] = a.node_eq3[(uint64_t)(cn[n] - 1) * 4 + 1];
-  }
   const uint32_t peq = a.p_eq[e];
   const double pc = a.U_cur[peq - 1];
   const double ps = a.have_state ? a.U_state[peq - 1] : 0.0;
+  const double st = a.have_state ? 1.0 : 0.0;
   int mat_id = a.mat_id;
   const double* mc = a.mc;
   double kbulk = a.kbulk;
@@ -2117,111 +2276,243 @@ __global__ void plane41_kernel(const Plane41Args a) {
     mc = mm + 1;
     kbulk = mm[6];
   }
-  double Us[8];
-  for (int n = 0; n < 4; n++)
-    for (int d = 0; d < 2; d++) Us[2 * n + d] = a.have_state ? a.U_state[eq[n][d] - 1] : 0.0;
-  const int comp[3] = {0, 3, 1};  // M_XX, M_YY, M_XY in the Voigt order xx xy xz yy yz zz
-  double Kuu[8][8] = {}, Kup[8] = {}, Qe[8] = {};
+  // positions and displacements relative to node 0, as modes
+  Mode2 Xm[2], xm[2];
+  bool rest = true;
+  {
+    double X[2][4], u[2][4] = {};
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      const uint64_t n = cn[hex_corner(b)] - 1;
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        X[i][b] = a.xyz[3 * n + i];
+        if (a.have_state) u[i][b] = a.U_state[a.node_eq3[4 * n + i] - 1];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+#pragma unroll
+      for (int b = 3; b >= 0; b--) {
+        X[i][b] -= X[i][0];
+        u[i][b] -= u[i][0];
+      }
+      const Mode2 M = corners_to_modes2(X[i]), d = corners_to_modes2(u[i]);
+      Xm[i] = {0.25 * M.x, 0.25 * M.y, 0.25 * M.xy};
+      rest = rest && d.x == 0.0 && d.y == 0.0 && d.xy == 0.0;
+      xm[i] = {fma(0.25, d.x, Xm[i].x), fma(0.25, d.y, Xm[i].y), fma(0.25, d.xy, Xm[i].xy)};
+    }
+  }
+  // sums over the Gauss points of chi_S A[ip][kq]: S = 0, 1 (xi), 2 (eta), 3.
+  // Blocks (0,0), (0,1), (1,1); of an entry p = q only the characters without
+  // coordinate p are read, and so for w F S and cof F
+  double A00[3][4] = {}, A11[3][4] = {}, A01[4][4] = {};   // sym2 / 2 p + q
+  double Pw[2][2][2] = {}, Cw[2][2][2] = {};               // [i][p]: S = 0 and the other coordinate
   double Kpp = 0.0, Fp = 0.0;
   bool bad = false;
+  const double inv_kb = 1.0 / kbulk;
+#pragma unroll 1
   for (int g = 0; g < 4; g++) {
-    // isoparametric quad, 2x2 Gauss (isoparametric.h:80-85, .cpp:13-137)
-    const double r = (g & 1) ? kGaussA : -kGaussA;
-    const double sg = (g & 2) ? kGaussA : -kGaussA;
-    const double dN[4][2] = {{-0.25 * (1.0 - sg), -0.25 * (1.0 - r)},
-                             {+0.25 * (1.0 - sg), -0.25 * (1.0 + r)},
-                             {+0.25 * (1.0 + sg), +0.25 * (1.0 + r)},
-                             {-0.25 * (1.0 + sg), +0.25 * (1.0 - r)}};
-    double Jm[2][2] = {};
-    for (int n = 0; n < 4; n++)
-      for (int i = 0; i < 2; i++)
-        for (int j = 0; j < 2; j++) Jm[i][j] += dN[n][i] * X[n][j];
-    const double det = Jm[0][0] * Jm[1][1] - Jm[0][1] * Jm[1][0];
-    if (!(det >= 1.0e-20)) bad = true;
-    const double id = 1.0 / det;
-    const double Ji[2][2] = {{Jm[1][1] * id, -Jm[0][1] * id}, {-Jm[1][0] * id, Jm[0][0] * id}};
-    double G[4][2];
-    for (int n = 0; n < 4; n++)
-      for (int i = 0; i < 2; i++) G[n][i] = Ji[i][0] * dN[n][0] + Ji[i][1] * dN[n][1];
-    const double w = 1.0 * det;
-    // state: O = B_omega U (dU/dx, dU/dy, dV/dx, dV/dy), C (xx, yy, xy)
-    double O[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int n = 0; n < 4; n++) {
-      O[0] += G[n][0] * Us[2 * n];
-      O[1] += G[n][1] * Us[2 * n];
-      O[2] += G[n][0] * Us[2 * n + 1];
-      O[3] += G[n][1] * Us[2 * n + 1];
-    }
-    const double Cxx = 1.0 + 2 * O[0] + O[0] * O[0] + O[2] * O[2];
-    const double Cyy = 1.0 + 2 * O[3] + O[3] * O[3] + O[1] * O[1];
-    const double Cxy = O[1] + O[2] + O[0] * O[1] + O[2] * O[3];
-    const double C6[6] = {Cxx, Cxy, 0.0, Cyy, 0.0, 1.0};
-    MatOut<double> mo;
-    double wD[21];
-    material<double>(mat_id, mc, C6, ps, pc, 1.0, mo, wD);  // wD = 2 Dd
-    const double S[3] = {a.have_state ? mo.S[0] : 0.0, a.have_state ? mo.S[3] : 0.0,
-                         a.have_state ? mo.S[1] : 0.0};
-    double E[3][3];
-    for (int i = 0; i < 3; i++)
-      for (int j = 0; j < 3; j++) E[i][j] = 0.5 * wD[sym6u(comp[i], comp[j])];
-    const double det2 = Cxx * Cyy - Cxy * Cxy;  // det C (C_zz = 1)
-    const double J = mo.J;
-    const double Dp[3] = {J * Cyy / det2, J * Cxx / det2, -J * Cxy / det2};
-    if (!(J > 0.0 && isfinite(J))) bad = true;
-    // B = B_L + Omega B_omega, rows (xx, yy, xy), columns (node, dof)
-    double B[3][8];
-    for (int n = 0; n < 4; n++) {
-      const double gx = G[n][0], gy = G[n][1];
-      B[0][2 * n] = gx + O[0] * gx;
-      B[0][2 * n + 1] = O[2] * gx;
-      B[1][2 * n] = O[1] * gy;
-      B[1][2 * n + 1] = gy + O[3] * gy;
-      B[2][2 * n] = gy + O[1] * gx + O[0] * gy;
-      B[2][2 * n + 1] = gx + O[3] * gx + O[2] * gy;
-    }
-    double EB[3][8];
-    for (int i = 0; i < 3; i++)
-      for (int c = 0; c < 8; c++) EB[i][c] = E[i][0] * B[0][c] + E[i][1] * B[1][c] + E[i][2] * B[2][c];
-    for (int r2 = 0; r2 < 8; r2++)
-      for (int c = r2; c < 8; c++) {
-        double v = 2.0 * (B[0][r2] * EB[0][c] + B[1][r2] * EB[1][c] + B[2][r2] * EB[2][c]);
-        // geometric term: B_omega^T S4 B_omega couples equal DoFs only
-        if ((r2 & 1) == (c & 1)) {
-          const int na = r2 >> 1, nb = c >> 1;
-          v += G[na][0] * (S[0] * G[nb][0] + S[2] * G[nb][1]) +
-               G[na][1] * (S[2] * G[nb][0] + S[1] * G[nb][1]);
-        }
-        Kuu[r2][c] += v * w;
+    const double sx = (g & 1) ? kGaussA : -kGaussA, sy = (g & 2) ? kGaussA : -kGaussA;
+    auto gradient = [&](const Mode2 m[2], double F[2][2]) {
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        F[i][0] = fma(sy, m[i].xy, m[i].x);
+        F[i][1] = fma(sx, m[i].xy, m[i].y);
       }
-    for (int c = 0; c < 8; c++) {
-      Kup[c] += (B[0][c] * Dp[0] + B[1][c] * Dp[1] + B[2][c] * Dp[2]) * w;
-      Qe[c] += (B[0][c] * S[0] + B[1][c] * S[1] + B[2][c] * S[2]) * w;
+      return minor2(F[0][0], F[1][1], F[0][1], F[1][0]);
+    };
+    double Xg[2][2], F[2][2];
+    const double w = gradient(Xm, Xg);
+    if (!(w >= 1.0e-20)) bad = true;
+    const double rw = 1.0 / w;
+    // dxi_p/dX_i, and the metric
+    const double Xi[2][2] = {{Xg[1][1] * rw, -Xg[1][0] * rw}, {-Xg[0][1] * rw, Xg[0][0] * rw}};   // [i][p]
+    double G[3];
+#pragma unroll
+    for (int p = 0; p < 2; p++)
+#pragma unroll
+      for (int r = p; r < 2; r++) G[p + r] = Xi[0][p] * Xi[0][r] + Xi[1][p] * Xi[1][r];
+    const double detF = gradient(xm, F);
+    const double dw = fabs(detF) - w;   // (J - 1) w
+    const double J = fma(dw, rw, 1.0);
+    if (!(J > 0.0 && isfinite(J))) bad = true;
+    const double kw = inv_kb * w;
+    Fp += fma(-pc, kw, dw);
+    Kpp -= kw;
+    const double rc = inv_cbrt(J), pp = rc * rc, pppp = pp * pp;
+    const double id = copysign(rw * (pp * rc), detF);
+    const double cof[2][2] = {{F[1][1], -F[1][0]}, {-F[0][1], F[0][0]}};
+    double V[2][2], FI[2][2], FA[2][2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+#pragma unroll
+      for (int p = 0; p < 2; p++) {
+        V[i][p] = cof[i][p] * id;
+        FI[i][p] = F[i][0] * G[p] + F[i][1] * G[1 + p];
+      }
     }
-    Fp += (J - 1 - pc / kbulk) * w;
-    Kpp -= 1.0 / kbulk * w;
+    const double b00 = FI[0][0] * F[0][0] + FI[0][1] * F[0][1];
+    const double b01 = FI[0][0] * F[1][0] + FI[0][1] * F[1][1];
+    const double b11 = FI[1][0] * F[1][0] + FI[1][1] * F[1][1];
+    const double tr = b00 + b11;
+    const double I1 = rest ? 3.0 : tr + 1.0;
+    const double I2 = rest ? 3.0 : fma(b00, b11, fma(-b01, b01, tr));
+    const double t13 = (1.0 / 3.0) * I1, t23 = (2.0 / 3.0) * I2;
+    // W derivatives at (I1 J^-2/3, I2 J^-4/3) (materials_hyperelastic.cpp:135-204)
+    double a1, a2 = 0.0, a11 = 0.0;
+    if (mat_id == 1) {
+      a1 = 0.5 * mc[0];
+    } else if (mat_id == 2) {
+      const double d = I1 * pp - 3.0;
+      a1 = mc[0] + 2 * mc[1] * d + 3 * mc[2] * d * d;
+      a2 = mc[3];
+      a11 = 2 * mc[1] + 6 * mc[2] * d;
+    } else {
+      a1 = mc[0];
+      a2 = mc[1];
+    }
+    const double ww = 0.0625 * w;   // the two factors 1/4 of dN/dxi
+    const double pj = pc * J, pJs = ps * J;
+    const double ko1 = st * (2 * a1 * pp), ko2 = st * (2 * a2 * pppp);
+    const double k11 = ww * (4.0 * a11 * pppp), k1 = (4.0 / 3.0) * a1 * pp,
+                 k2 = (8.0 / 3.0) * a2 * pppp;
+    const double h = -0.5 * ww * (2.0 * pj - k1 * I1 - k2 * I2);
+    const double sI = 1.5 * ww * k2, hI = 0.5 * sI;
+    const double wq = -0.25 * w;
+    const double pk = wq * ko1, pb = wq * ko2, pv = wq * pJs;
+    const double xk = -ww * k1, xb = -ww * k2, xv = 0.5 * ww * (pj - k1 * t13 - k2 * t23);
+    const double sg = detF < 0.0 ? -0.25 : 0.25;   // J C^-1 with J = |det F|
+    const double chi[2] = {(g & 1) ? 1.0 : -1.0, (g & 2) ? 1.0 : -1.0};
+    double X[2][2];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int p = 0; p < 2; p++) {
+        FA[i][p] = rest ? 0.0 : fma(-t13, V[i][p], FI[i][p]);
+        const double fc = i == 0 ? b00 * FI[0][p] + b01 * FI[1][p] : b01 * FI[0][p] + b11 * FI[1][p];
+        const double FB = rest ? 0.0 : fma(-t23, V[i][p], fma(I1, FI[i][p], -fc));
+        const double P = fma(pk, FA[i][p], fma(pb, FB, pv * V[i][p]));
+        X[i][p] = fma(xk, FA[i][p], fma(xb, FB, xv * V[i][p]));
+        Pw[i][p][0] += P;
+        Pw[i][p][1] = fma(chi[1 - p], P, Pw[i][p][1]);
+        Cw[i][p][0] = fma(sg, cof[i][p], Cw[i][p][0]);
+        Cw[i][p][1] = fma(chi[1 - p] * sg, cof[i][p], Cw[i][p][1]);
+      }
+    // S^{pq} = (ko1 + ko2 I1) g - ko2 C^{pq} + (p J - ko1 I1/3 - ko2 2 I2/3) C^-1
+    const double eg = ww * (ko1 + ko2 * I1), ecc = -ww * ko2;
+    const double ec = ww * (pJs - ko1 * t13 - ko2 * t23) + h;
+    double E[3];
+#pragma unroll
+    for (int p = 0; p < 2; p++)
+#pragma unroll
+      for (int r = p; r < 2; r++) {
+        const double CI = V[0][p] * V[0][r] + V[1][p] * V[1][r];
+        const double CC = FI[0][p] * FI[0][r] + FI[1][p] * FI[1][r];
+        E[p + r] = fma(ecc, CC, fma(ec, CI, eg * G[p + r]));
+      }
+    const bool biderman = __any_sync(__activemask(), a11 != 0.0);
+    auto entry = [&](int i, int k, int p, int r, double base) {
+      double v = fma(V[i][p], X[k][r], fma(X[i][p], V[k][r], base));
+      v = fma(h * V[i][r], V[k][p], v);
+      if (i == k) v = fma(hI * FI[i][p], FI[i][r], v);
+      else v = fma(sI * FI[i][p], FI[k][r], fma(-hI * FI[i][r], FI[k][p], v));
+      return biderman ? fma(k11 * FA[i][p], FA[k][r], v) : v;
+    };
+    auto add = [&](double acc[4], int p, int r, double v) {
+      acc[0] += v;
+      if (p == r) {
+        acc[2 - p] = fma(chi[1 - p], v, acc[2 - p]);   // the other coordinate
+      } else {
+        acc[1] = fma(chi[0], v, acc[1]);
+        acc[2] = fma(chi[1], v, acc[2]);
+        acc[3] = fma(chi[0] * chi[1], v, acc[3]);
+      }
+    };
+#pragma unroll
+    for (int p = 0; p < 2; p++)
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        if (r >= p) {
+          add(A00[p + r], p, r, entry(0, 0, p, r, fma(-hI * b00, G[p + r], E[p + r])));
+          add(A11[p + r], p, r, entry(1, 1, p, r, fma(-hI * b11, G[p + r], E[p + r])));
+        }
+        add(A01[2 * p + r], p, r, entry(0, 1, p, r, -hI * b01 * G[p + r]));
+      }
   }
   if (bad) flag_element(a.status, e + 1);
   const uint64_t kb = (uint64_t)e * 45, fb = (uint64_t)e * 9;
   auto kd = [&](uint64_t i) { return a.kpos ? (uint64_t)a.kpos[i] : i; };
   auto fd = [&](uint64_t i) { return a.fpos ? (uint64_t)a.fpos[i] : i; };
-  int t = 0;
+  // position of (i, di; j, dj), i <= j, in assembleK order
+  auto pos = [](int i, int di, int j, int dj) {
+    int t = 0;
+    for (int q = 0; q < i; q++) t += 3 + 4 * (3 - q);
+    if (i == j) return t + di * (di + 1) / 2 + dj;   // (0,0) (1,0) (1,1)
+    return t + 3 + 4 * (j - i - 1) + 2 * di + dj;
+  };
+  // block (i, k): modes of both sides to nodes; W(p, r) its four characters
+  auto block = [&](const double (*W)[4], bool sym, double K[4][4]) {
+    auto at = [&](int p, int r, int S) { return W[sym ? p + r : 2 * p + r][S]; };
+    double T[3][4];
+    // one mode of the a side: x = (0, 0), y = (1, 0), xy = (0, {1}) + (1, {0});
+    // the characters of the two sides multiply (S: xi = 1, eta = 2)
+    auto row = [&](int p, int P, Mode2& M) {
+      M.x = at(p, 0, P);
+      M.y = at(p, 1, P);
+      M.xy = at(p, 0, P ^ 2) + at(p, 1, P ^ 1);
+    };
+    Mode2 M, M2;
+    row(0, 0, M);
+    modes2_to_nodes(M, T[0]);
+    row(1, 0, M);
+    modes2_to_nodes(M, T[1]);
+    row(0, 2, M);
+    row(1, 1, M2);
+    M = {M.x + M2.x, M.y + M2.y, M.xy + M2.xy};
+    modes2_to_nodes(M, T[2]);
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      double o[4];
+      modes2_to_nodes(Mode2{T[0][b], T[1][b], T[2][b]}, o);
+#pragma unroll
+      for (int c = 0; c < 4; c++) K[hex_corner(c)][hex_corner(b)] = o[c];
+    }
+  };
+  double K[4][4];
+#pragma unroll
+  for (int d = 0; d < 2; d++) {
+    block(d == 0 ? A00 : A11, true, K);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = i; j < 4; j++) a.contribK[kd(kb + pos(i, d, j, d))] = K[i][j];
+  }
+  block(A01, false, K);
+#pragma unroll
   for (int i = 0; i < 4; i++)
-    for (int j = i; j < 4; j++)
-      for (int di = 0; di < 2; di++)
-        for (int dj = 0; dj < 2; dj++) {
-          if (i == j && dj > di) continue;
-          const int r2 = 2 * i + di, c = 2 * j + dj;
-          a.contribK[kd(kb + t++)] = r2 <= c ? Kuu[r2][c] : Kuu[c][r2];
-        }
-  for (int c = 0; c < 8; c++) a.contribK[kd(kb + 36 + c)] = Kup[c];
+#pragma unroll
+    for (int j = i; j < 4; j++) {
+      if (i != j) a.contribK[kd(kb + pos(i, 0, j, 1))] = K[i][j];
+      a.contribK[kd(kb + pos(i, 1, j, 0))] = K[j][i];
+    }
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    double o[4];
+    modes2_to_nodes(Mode2{Cw[i][0][0], Cw[i][1][0], Cw[i][0][1] + Cw[i][1][1]}, o);
+#pragma unroll
+    for (int b = 0; b < 4; b++) a.contribK[kd(kb + 36 + 2 * hex_corner(b) + i)] = o[b];
+    modes2_to_nodes(Mode2{Pw[i][0][0], Pw[i][1][0], Pw[i][0][1] + Pw[i][1][1]}, o);
+#pragma unroll
+    for (int b = 0; b < 4; b++) a.contribF[fd(fb + 2 * hex_corner(b) + i)] = o[b];
+  }
   a.contribK[kd(kb + 44)] = Kpp;
-  for (int c = 0; c < 8; c++) a.contribF[fd(fb + c)] = -Qe[c];
   a.contribF[fd(fb + 8)] = -Fp;
 }
 
 cudaError_t launch_plane41(const Plane41Args& a, cudaStream_t s) {
   if (a.n_elems <= a.e_begin) return cudaSuccess;
-  const int bs = 128;
+  const int bs = kPlaneThreads;
   plane41_kernel<<<(a.n_elems - a.e_begin + bs - 1) / bs, bs, 0, s>>>(a);
   return cudaGetLastError();
 }

@@ -12,7 +12,10 @@ constexpr int kSolidFc = 25;   // SOLID81 F contributions per element (24 Fu + 1
 
 struct ElementStatus {
   uint32_t count;  // elements flagged (J <= 0, det J <= 0, non-finite)
-  uint32_t first;  // smallest flagged 1-based element number, 0xFFFFFFFF if none
+  // ~(smallest flagged 1-based element number), 0 if none: a cleared status is
+  // all zero bytes, one memset per assembly
+  uint32_t first_inv;
+  uint32_t first() const { return ~first_inv; }
 };
 
 struct Solid81Args {
@@ -218,6 +221,9 @@ cudaError_t launch_solid81_shaped(const Solid81Args& a, bool mixed, Solid81Shape
 int solid81_max_blocks_per_sm(bool mixed, int warps_per_block);
 cudaError_t launch_gather_bs(const GatherArgs& a, int block_size, cudaStream_t s);
 cudaError_t launch_segsum(const SegSumArgs& a, int block_size, cudaStream_t s);
+// two gathers (K and F) in one launch; both with ids or both without
+cudaError_t launch_gather_pair(const GatherArgs& k, const GatherArgs& f, int block_size,
+                               cudaStream_t s);
 // kernel tables (constant memory) for the current device; call before any
 // stream capture
 cudaError_t prepare_device_tables();

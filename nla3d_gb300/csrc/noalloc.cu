@@ -149,7 +149,6 @@ extern "C" int nla3d_assemble_solid81_noalloc(const nla3d_solid81_noalloc_args* 
   // the only scratch that must start from a known value: the status word and
   // the invalid-input count
   if (cudaMemsetAsync(d->status, 0, sizeof(ElementStatus), s) != cudaSuccess ||
-      cudaMemsetAsync(&d->status->first, 0xFF, sizeof(uint32_t), s) != cudaSuccess ||
       cudaMemsetAsync(d->bad, 0, sizeof(uint32_t), s) != cudaSuccess)
     return NLA3D_ERR_CUDA;
 
