@@ -10,9 +10,8 @@
 //   1. every front is zeroed and the matrix values are scattered into it
 //      (one map entry per stored value, computed by the symbolic analysis);
 //   2. extend-add: each child's update matrix is added into its parent's
-//      front; children are taken one ordinal at a time (first children of all
-//      parents of the level, then second children, ...) so that no two
-//      threads add into one entry and the sums keep a fixed order;
+//      front, a warp per parent column taking the children in order, so that
+//      no two threads add into one entry and the sums keep a fixed order;
 //   3. partial LDL^T of the front's k pivot columns, right-looking, without
 //      pivoting (the u/p blocks are quasi-definite: K_uu > 0, K_pp < 0, and
 //      constraint rows are ordered last by the caller); a pivot below
@@ -108,24 +107,57 @@ __global__ void maxabs_final_kernel(int n, const double* __restrict__ part, doub
   if (threadIdx.x == 0) out[0] = red[0];
 }
 
-// children[blockIdx.x]: add its update matrix into its parent's front
+// Extend-add of one level in one launch: the front rows of the level are
+// contiguous in the solve vectors' order, and the lists that the forward pass
+// gathers with (per row: the children's update rows, in child order) are the
+// columns that meet in that row's column.  A warp owns a parent column and adds
+// the children's columns one after the other, four loads a lane in flight, so
+// every entry sums in child order and no two warps share one.
+// Memory bounds the wide levels (a child's triangle read, the parent's read
+// and written), dependent index loads the others.  A launch per child ordinal
+// with at most u / 32 blocks a child had too few loads in flight: 3.0 ms in
+// 100 launches of the 139k-equation bar's factor, now 1.2 in 16; 8.2 ms of the
+// 454k-equation bar's, now 4.4.  A block per column of the narrow levels, and
+// two, three or eight loads a lane, measured the same or slower.
 template <typename T>
-__global__ void extend_add_kernel(const int32_t* __restrict__ children, int n, LdltDev d,
-                                  T* __restrict__ front) {
-  const int c = children[blockIdx.x];
-  const int p = d.sn_parent[c];
-  const int64_t mc = d.row_ptr[c + 1] - d.row_ptr[c];
-  const int64_t kc = d.sn_first[c + 1] - d.sn_first[c];
+__global__ void __launch_bounds__(kThreads)
+    extend_add_kernel(uint64_t r0, uint64_t r1, const uint32_t* __restrict__ ptr,
+                      const uint32_t* __restrict__ src, const int32_t* __restrict__ row_sn,
+                      LdltDev d, T* __restrict__ front) {
+  const int lane = threadIdx.x & 31;
+  const uint64_t r = r0 + blockIdx.x * (uint64_t)(kThreads / 32) + (threadIdx.x >> 5);
+  if (r >= r1) return;
+  const uint32_t b = ptr[r], e = ptr[r + 1];
+  if (b == e) return;
+  const int p = row_sn[r];
   const int64_t mp = d.row_ptr[p + 1] - d.row_ptr[p];
-  const int64_t u = mc - kc;
-  const T* Fc = front + d.front_off[c];
-  T* Fp = front + d.front_off[p];
-  const uint32_t* rel = d.rel + d.rel_ptr[c];
-  for (int64_t j = blockIdx.y; j < u; j += gridDim.y) {
-    const int64_t pj = rel[j];
-    const T* src = Fc + (kc + j) * mc + kc;
-    T* dst = Fp + pj * mp;
-    for (int64_t i = j + threadIdx.x; i < u; i += blockDim.x) dst[rel[i]] += src[i];
+  T* dst = front + d.front_off[p] + (int64_t)(r - d.vec_off[p]) * mp;
+  for (uint32_t q = b; q < e; q++) {
+    const uint32_t sr = src[q];
+    const int c = row_sn[sr];
+    const int64_t mc = d.row_ptr[c + 1] - d.row_ptr[c];
+    const int64_t kc = d.sn_first[c + 1] - d.sn_first[c];
+    const int64_t pj = (int64_t)(sr - d.vec_off[c]);   // the child's column, in its front
+    const T* col = front + d.front_off[c] + pj * mc;
+    const uint32_t* rel = d.rel + d.rel_ptr[c];
+    constexpr int kU = 4;
+    for (int64_t i0 = pj + lane; i0 < mc; i0 += kU * 32) {
+      T v[kU], w[kU];
+      uint32_t t[kU];
+#pragma unroll
+      for (int x = 0; x < kU; x++) {
+        const int64_t i = i0 + x * 32;
+        t[x] = i < mc ? rel[i - kc] : 0u;
+        v[x] = i < mc ? col[i] : T(0);
+      }
+#pragma unroll
+      for (int x = 0; x < kU; x++)
+        if (i0 + x * 32 < mc) w[x] = dst[t[x]];
+#pragma unroll
+      for (int x = 0; x < kU; x++)
+        if (i0 + x * 32 < mc) dst[t[x]] = w[x] + v[x];
+    }
+    __syncwarp();
   }
 }
 
@@ -1805,6 +1837,7 @@ struct nla3d_ldlt {
   int32_t* d_bidx = nullptr;    // per front row (level order): its right-hand side entry or -1,
   uint32_t* d_gptr = nullptr;   // and its children's update rows
   uint32_t* d_gsrc = nullptr;
+  int32_t* d_rsn = nullptr;     // per front row: its supernode
   uint64_t* d_adest = nullptr;
   int32_t* d_perm = nullptr;
   int32_t* d_lists = nullptr;   // level lists, small lists, extend-add child lists
@@ -1826,8 +1859,7 @@ struct nla3d_ldlt {
     uint64_t vec0 = 0, vec1 = 0;                // its fronts' rows in the solve vectors
     int64_t narrow_off = 0, narrow_cnt = 0, narrow_max_u = 0;   // solves: large fronts by width
     int64_t wide_off = 0, wide_cnt = 0, wide_max_m = 0, wide_max_k = 0;
-    std::vector<int64_t> ea_off, ea_cnt;  // children of the level's parents, by ordinal
-    std::vector<uint32_t> ea_gy;          // column blocks per child (its update's size)
+    bool has_children = false;
   };
   std::vector<Level> levels;
   bool factored = false;
@@ -1886,11 +1918,10 @@ cudaError_t enqueue_factor(nla3d_ldlt* h, const double* values) {
     scatter_values_kernel<T><<<blocks, kThreads, 0, st>>>(S.nnz, h->d_adest, values, front);
   }
   for (const auto& L : h->levels) {
-    for (size_t q = 0; q < L.ea_off.size(); q++) {
-      if (!L.ea_cnt[q]) continue;
-      const dim3 grid((unsigned)L.ea_cnt[q], L.ea_gy[q]);
-      extend_add_kernel<T><<<grid, kThreads, 0, st>>>(h->d_lists + L.ea_off[q], (int)L.ea_cnt[q],
-                                                      h->dev, front);
+    if (L.has_children) {
+      constexpr uint64_t kCols = kThreads / 32;
+      extend_add_kernel<T><<<(unsigned)((L.vec1 - L.vec0 + kCols - 1) / kCols), kThreads, 0, st>>>(
+          L.vec0, L.vec1, h->d_gptr, h->d_gsrc, h->d_rsn, h->dev, front);
     }
     if (L.small_cnt) {
       const size_t smem = sizeof(T) * (size_t)L.small_max_m * (L.small_max_m + 1);
@@ -2235,25 +2266,9 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
     max_w = std::max(max_w, w);
     max_pk = std::max(max_pk, pk);
     max_large_cnt = std::max(max_large_cnt, lv.large_cnt);
-    int maxc = 0;
     for (int32_t q = S.level_ptr[L]; q < S.level_ptr[L + 1]; q++) {
       const int32_t s = S.level_list[q];
-      maxc = std::max(maxc, S.child_ptr[s + 1] - S.child_ptr[s]);
-    }
-    for (int o = 0; o < maxc; o++) {
-      lv.ea_off.push_back((int64_t)lists.size());
-      int64_t umax = 0;
-      for (int32_t q = S.level_ptr[L]; q < S.level_ptr[L + 1]; q++) {
-        const int32_t s = S.level_list[q];
-        if (S.child_ptr[s + 1] - S.child_ptr[s] > o) {
-          const int32_t c = S.child_list[S.child_ptr[s] + o];
-          lists.push_back(c);
-          umax = std::max<int64_t>(umax, S.m(c) - S.k(c));
-        }
-      }
-      lv.ea_cnt.push_back((int64_t)lists.size() - lv.ea_off.back());
-      // about 32 update columns per block, 16 .. 1024 blocks per child
-      lv.ea_gy.push_back((uint32_t)std::min<int64_t>(1024, std::max<int64_t>(16, (umax + 31) / 32)));
+      lv.has_children |= S.child_ptr[s + 1] > S.child_ptr[s];
     }
   }
   if (lists.size() >= (size_t)INT32_MAX || max_large_cnt > 65535) {
@@ -2321,6 +2336,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   LCK(upload(h, &h->d_bidx, solve_lists.b_idx));
   LCK(upload(h, &h->d_gptr, solve_lists.ptr));
   LCK(upload(h, &h->d_gsrc, solve_lists.src));
+  LCK(upload(h, &h->d_rsn, solve_lists.row_sn));
   LCK(upload(h, &h->d_inv, inv_tasks));
   LCK(upload(h, &h->d_toff, toff));
   if (precision)

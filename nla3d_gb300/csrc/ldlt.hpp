@@ -59,11 +59,13 @@ std::string ldlt_analyze(int64_t n, const uint32_t* iofeir, const uint32_t* colu
 // The solve vectors' layout: front s's m(s) rows at vec_off[s], fronts in level
 // order (a level's rows are contiguous).  Row p starts from entry b_idx[p] of
 // the right-hand side (input numbering; -1: an update row, zero) and adds the
-// children's update rows src[ptr[p] .. ptr[p+1]), in child order.
+// children's update rows src[ptr[p] .. ptr[p+1]), in child order; the same lists
+// give the columns that extend-add into row p's column.
 struct LdltSolveLists {
   std::vector<uint64_t> vec_off;    // per supernode
   std::vector<uint64_t> level_off;  // per level, + 1
   std::vector<int32_t> b_idx;
   std::vector<uint32_t> ptr, src;
+  std::vector<int32_t> row_sn;      // per row: its supernode
 };
 std::string ldlt_solve_lists(const LdltSymbolic& S, LdltSolveLists* out);

@@ -582,6 +582,7 @@ std::string ldlt_solve_lists(const LdltSymbolic& S, LdltSolveLists* out) {
   }
   out->level_off[nlev] = v;
   out->b_idx.resize(total);
+  out->row_sn.resize(total);
   out->ptr.resize(total + 1);
   out->src.resize(w);
   out->ptr[total] = (uint32_t)w;
@@ -593,6 +594,7 @@ std::string ldlt_solve_lists(const LdltSymbolic& S, LdltSolveLists* out) {
       const int64_t m = S.m(s), k = S.k(s);
       const uint64_t o = out->vec_off[s];
       for (int64_t i = 0; i < m; i++) out->b_idx[o + i] = i < k ? S.perm[S.sn_first[s] + i] : -1;
+      std::fill_n(out->row_sn.begin() + (int64_t)o, m, s);
       pos.assign(m + 1, 0);
       for (int32_t c = S.child_ptr[s]; c < S.child_ptr[s + 1]; c++) {
         const int32_t ch = S.child_list[c];
