@@ -52,6 +52,7 @@ constexpr int kSmallFront = 128;   // fronts up to this many rows: one block eac
 constexpr int kPanel = 64;         // panel width of the blocked path
 constexpr int kOuter = 256;        // outer block of the blocked path (4 panels)
 constexpr int kInv = 512;          // pivots whose triangle is kept inverted for the solves
+constexpr int kDoublings = kInv == 512 ? 3 : kInv == 256 ? 2 : kInv == 128 ? 1 : 0;
 constexpr int kNarrow = kPanel;    // fronts with up to this many pivots: one CTA per solve pass
 constexpr int kNarrowRows = 4096;  // ... and up to this many rows
 
@@ -1690,52 +1691,223 @@ __global__ void __launch_bounds__(kThreads)
   if (lane == 0) vec[d.vec_off[s] + j] -= a[0].value();
 }
 
+// x = xf in the input numbering, or x += xf; z: also the step itself
 __global__ void solve_finish_kernel(int64_t n, const int32_t* __restrict__ perm,
                                     const double* __restrict__ xf, double* __restrict__ x,
-                                    int accumulate) {
+                                    int accumulate, double* __restrict__ z) {
   const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (j >= n) return;
+  const int32_t i = perm[j];
+  const double v = xf[j];
   if (accumulate)
-    x[perm[j]] += xf[j];
+    x[i] += v;
   else
-    x[perm[j]] = xf[j];
+    x[i] = v;
+  if (z) z[i] = v;
 }
 
-// r = b - A x, A by both-triangle rows (a warp per row, fixed order); per-block
-// partial sums of r^2 and b^2 for the norms
-__global__ void residual_kernel(int64_t n, const int64_t* __restrict__ ptr,
-                                const int32_t* __restrict__ col, const uint32_t* __restrict__ slot,
-                                const double* __restrict__ A, const double* __restrict__ x,
-                                const double* __restrict__ b, double* __restrict__ r,
-                                double* __restrict__ part) {
-  __shared__ double red[2][kThreads / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t row = blockIdx.x * (int64_t)(blockDim.x / 32) + warp;
-  double rr = 0.0, bb = 0.0;
-  if (row < n) {
-    double acc = 0.0;
-    for (int64_t q = ptr[row] + lane; q < ptr[row + 1]; q += 32) acc += A[slot[q]] * x[col[q]];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (lane == 0) {
-      const double ri = b[row] - acc;
-      r[row] = ri;
-      rr = ri * ri;
-      bb = b[row] * b[row];
+// (A x)_row, A by both-triangle rows: eight lanes a row with four sums each,
+// entry q of the row in sum q % 32, and the 32 sums added pairwise as a warp a
+// row would add them, so the rounding is that of chains a 32nd of the row long.
+// The FP64 pipe bounds it (2 FMA a clock and SM): with a warp a row, the five
+// adds of the reduction cost more than the three products of a typical row of
+// 80 entries; with eight lanes a row, four rows share six adds.
+constexpr int kRowLanes = 8;
+constexpr int kRowsPerBlock = kThreads / kRowLanes;
+
+__device__ __forceinline__ double row_product(int64_t row, const int64_t* __restrict__ ptr,
+                                              const int32_t* __restrict__ col,
+                                              const uint32_t* __restrict__ slot,
+                                              const double* __restrict__ A,
+                                              const double* __restrict__ x) {
+  constexpr int kU = 32 / kRowLanes;
+  double acc[kU] = {};
+  const int64_t e = ptr[row + 1];
+  for (int64_t q = ptr[row] + threadIdx.x % kRowLanes; q < e; q += 32) {
+    double a[kU], v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+      const int64_t t = q + u * kRowLanes;
+      a[u] = t < e ? A[slot[t]] : 0.0;
+      v[u] = t < e ? x[col[t]] : 0.0;
     }
+#pragma unroll
+    for (int u = 0; u < kU; u++)
+      if (q + u * kRowLanes < e) acc[u] = fma(a[u], v[u], acc[u]);
   }
-  if (lane == 0) {
-    red[0][warp] = rr;
-    red[1][warp] = bb;
+  return (acc[0] + acc[2]) + (acc[1] + acc[3]);
+}
+
+__device__ __forceinline__ double row_sum(double acc) {   // all lanes of the warp
+#pragma unroll
+  for (int o = kRowLanes / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  return acc;
+}
+
+// r = b - A x (dr: what r fell by); per-block partial sums of r^2 and b^2 for
+// the norms.  110 -> 45 us
+// on the 139k-equation bar against a warp per row.
+__global__ void __launch_bounds__(kThreads)
+    residual_kernel(int64_t n, const int64_t* __restrict__ ptr, const int32_t* __restrict__ col,
+                    const uint32_t* __restrict__ slot, const double* __restrict__ A,
+                    const double* __restrict__ x, const double* __restrict__ b,
+                    double* __restrict__ r, double* __restrict__ part, double* __restrict__ dr) {
+  __shared__ double red[2][kRowsPerBlock];
+  const int local = threadIdx.x / kRowLanes;
+  const int64_t row = blockIdx.x * (int64_t)kRowsPerBlock + local;
+  const double ax = row_sum(row < n ? row_product(row, ptr, col, slot, A, x) : 0.0);
+  if (threadIdx.x % kRowLanes == 0) {
+    double ri = 0.0, bi = 0.0;
+    if (row < n) {
+      bi = b[row];
+      ri = bi - ax;
+      if (dr) dr[row] = r[row] - ri;
+      r[row] = ri;
+    }
+    red[0][local] = ri;
+    red[1][local] = bi;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0.0, c = 0.0;
-    for (int w = 0; w < kThreads / 32; w++) {
-      a += red[0][w];
-      c += red[1][w];
+  static_assert(kRowsPerBlock == 32, "a warp holds the block's rows");
+  if (threadIdx.x < 32) {
+    double rr = red[0][threadIdx.x] * red[0][threadIdx.x];
+    double bb = red[1][threadIdx.x] * red[1][threadIdx.x];
+    for (int o = 16; o > 0; o >>= 1) {
+      rr += __shfl_down_sync(0xffffffffu, rr, o);
+      bb += __shfl_down_sync(0xffffffffu, bb, o);
     }
-    part[2 * blockIdx.x] = a;
-    part[2 * blockIdx.x + 1] = c;
+    if (threadIdx.x == 0) {
+      part[2 * blockIdx.x] = rr;
+      part[2 * blockIdx.x + 1] = bb;
+    }
+  }
+}
+
+// the blocks' pairs of partial sums added up, in a fixed order, by one block
+// (their copy to the host took as long as the residual on large models)
+__global__ void __launch_bounds__(kThreads)
+    norms_kernel(int64_t n, const double* __restrict__ part, double* __restrict__ out) {
+  __shared__ double red[kThreads];
+  const int which = threadIdx.x & 1;   // r^2 or b^2
+  double acc = 0.0;
+#pragma unroll 8
+  for (int64_t q = threadIdx.x; q < 2 * n; q += kThreads) acc += part[q];
+  red[threadIdx.x] = acc;
+  __syncthreads();
+  for (int s = kThreads / 2; s > 1; s >>= 1) {
+    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+    __syncthreads();
+  }
+  if (threadIdx.x < 2) out[which] = red[which];
+}
+
+// ---- vector kernels of the accelerated refinement steps ----
+//
+// A refinement step z = M^-1 r leaves r - A z, and after the first steps it
+// falls by the same factor every time (0.03 a step on the 139k-equation bar,
+// 0.08 on the 454k-equation one): a few modes of I - A M^-1 dominate it.  So
+// the steps z_i and q_i = A z_i, which the next residual gives for nothing (r
+// before it less r after it), are kept, q orthonormalised, and r's components
+// along them taken out: r -= q_i <q_i, r>, x += z_i <q_i, r>, the least
+// residual in the span (GCR; Eisenstat, Elman and Schultz, SIAM J. Numer.
+// Anal. 20, 1983).  Two launches of short vectors save one or two of the six to
+// nine applications of the factor.
+constexpr int kDirs = 8;                 // steps kept; the basis starts anew when it is full
+constexpr int kDirSums = 2 * kDirs + 2;
+constexpr int kDirBlocks = 152;
+
+// partial sums of <q, Q_i>, <r, Q_i> (i < k), <q, q> and <q, r>, q = Q_k
+__global__ void __launch_bounds__(kThreads)
+    direction_sums_kernel(int64_t n, int k, const double* __restrict__ Q,
+                          const double* __restrict__ r, double* __restrict__ part) {
+  __shared__ double red[kDirSums][kThreads];
+  double acc[kDirSums] = {};
+  const double* q = Q + (int64_t)k * n;
+  for (int64_t j = blockIdx.x * (int64_t)kThreads + threadIdx.x; j < n;
+       j += (int64_t)gridDim.x * kThreads) {
+    const double qj = q[j], rj = r[j];
+#pragma unroll
+    for (int i = 0; i < kDirs; i++) {
+      if (i >= k) break;
+      const double v = Q[(int64_t)i * n + j];
+      acc[2 * i] = fma(qj, v, acc[2 * i]);
+      acc[2 * i + 1] = fma(rj, v, acc[2 * i + 1]);
+    }
+    acc[2 * kDirs] = fma(qj, qj, acc[2 * kDirs]);
+    acc[2 * kDirs + 1] = fma(qj, rj, acc[2 * kDirs + 1]);
+  }
+  // (eight threads a sum, 32 entries each: fewer FP64 adds than shuffles)
+#pragma unroll
+  for (int t = 0; t < kDirSums; t++)
+    if (t < 2 * k || t >= 2 * kDirs) red[t][threadIdx.x] = acc[t];
+  __syncthreads();
+  const int t = threadIdx.x >> 3, h = threadIdx.x & 7;
+  if (t >= kDirSums) return;   // whole groups of eight lanes
+  double v = 0.0;
+  if (t < 2 * k || t >= 2 * kDirs)
+#pragma unroll 8
+    for (int w = 0; w < kThreads / 8; w++) v += red[t][h + 8 * w];
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(__activemask(), v, o);
+  if (h == 0) part[blockIdx.x * kDirSums + t] = v;
+}
+
+// Q_k and Z_k orthonormalised from those sums, r's components along Q_0 .. Q_k
+// taken out of r and into x; partial sums of the new r^2
+__global__ void __launch_bounds__(kThreads)
+    direction_step_kernel(int64_t n, int k, double* __restrict__ Q, double* __restrict__ Z,
+                          double* __restrict__ r, double* __restrict__ x,
+                          const double* __restrict__ part, double* __restrict__ rpart) {
+  __shared__ double sum[kDirSums];
+  __shared__ double red[kThreads / 32];
+  static_assert(kDirSums * 8 <= kThreads && kDirBlocks % 8 == 0, "eight threads a sum");
+  if (threadIdx.x < kDirSums * 8) {
+    const int t = threadIdx.x >> 3, h = threadIdx.x & 7;
+    double v = 0.0;
+#pragma unroll
+    for (int b = 0; b < kDirBlocks / 8; b++) v += part[(8 * b + h) * kDirSums + t];
+    const unsigned lanes = __activemask();   // whole groups of eight
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(lanes, v, o);
+    if (h == 0) sum[t] = v;
+  }
+  __syncthreads();
+  const double qq = sum[2 * kDirs];
+  double n2 = qq, qr = sum[2 * kDirs + 1];
+  for (int i = 0; i < k; i++) {
+    n2 = fma(-sum[2 * i], sum[2 * i], n2);
+    qr = fma(-sum[2 * i], sum[2 * i + 1], qr);
+  }
+  // a step with nothing new in it is left as a null direction
+  const double inv = n2 > 1e-12 * qq ? rsqrt(n2) : 0.0;
+  const double beta = inv > 0.0 ? qr * inv : 0.0;
+  double rr = 0.0;
+  for (int64_t j = blockIdx.x * (int64_t)kThreads + threadIdx.x; j < n;
+       j += (int64_t)gridDim.x * kThreads) {
+    double q = Q[(int64_t)k * n + j], z = Z[(int64_t)k * n + j], dr = 0.0, dx = 0.0;
+#pragma unroll
+    for (int i = 0; i < kDirs; i++) {
+      if (i >= k) break;
+      const double qi = Q[(int64_t)i * n + j], zi = Z[(int64_t)i * n + j];
+      q = fma(-sum[2 * i], qi, q);
+      z = fma(-sum[2 * i], zi, z);
+      dr = fma(sum[2 * i + 1], qi, dr);
+      dx = fma(sum[2 * i + 1], zi, dx);
+    }
+    q *= inv;
+    z *= inv;
+    Q[(int64_t)k * n + j] = q;
+    Z[(int64_t)k * n + j] = z;
+    const double rj = r[j] - fma(beta, q, dr);
+    r[j] = rj;
+    x[j] += fma(beta, z, dx);
+    rr = fma(rj, rj, rr);
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int o = 16; o > 0; o >>= 1) rr += __shfl_down_sync(0xffffffffu, rr, o);
+  if (lane == 0) red[warp] = rr;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kThreads / 32; w++) rr += red[w];
+    rpart[blockIdx.x] = rr;
   }
 }
 
@@ -1774,18 +1946,14 @@ __global__ void scale_kernel(int64_t n, double alpha, const double* __restrict__
     y[i] = alpha * x[i];
 }
 
-// y = A x, A by both-triangle rows, a warp per row
-__global__ void spmv_kernel(int64_t n, const int64_t* __restrict__ ptr,
-                            const int32_t* __restrict__ col, const uint32_t* __restrict__ slot,
-                            const double* __restrict__ A, const double* __restrict__ x,
-                            double* __restrict__ y) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t row = blockIdx.x * (int64_t)(blockDim.x / 32) + warp;
-  if (row >= n) return;
-  double acc = 0.0;
-  for (int64_t q = ptr[row] + lane; q < ptr[row + 1]; q += 32) acc += A[slot[q]] * x[col[q]];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if (lane == 0) y[row] = acc;
+// y = A x
+__global__ void __launch_bounds__(kThreads)
+    spmv_kernel(int64_t n, const int64_t* __restrict__ ptr, const int32_t* __restrict__ col,
+                const uint32_t* __restrict__ slot, const double* __restrict__ A,
+                const double* __restrict__ x, double* __restrict__ y) {
+  const int64_t row = blockIdx.x * (int64_t)kRowsPerBlock + threadIdx.x / kRowLanes;
+  const double ax = row_sum(row < n ? row_product(row, ptr, col, slot, A, x) : 0.0);
+  if (row < n && threadIdx.x % kRowLanes == 0) y[row] = ax;
 }
 
 }  // namespace
@@ -1806,9 +1974,12 @@ struct nla3d_ldlt {
   double* d_xf = nullptr;
   double* d_r = nullptr;
   double* d_dx = nullptr;
-  double* d_part = nullptr;
+  double* d_part = nullptr;     // the residual's partial sums,
+  double* d_norm = nullptr;     // and their totals: r^2, b^2
   double* d_V = nullptr;        // GMRES basis, (kRestart + 1) x n, allocated on first use
   double* d_dot = nullptr;
+  double* d_dirs = nullptr;     // FP32 fronts: the refinement's Q and Z, kDirs x n each, or null
+  double* d_dirsum = nullptr;   // and their partial sums
   double* d_maxabs = nullptr;
   double* d_maxpart = nullptr;
   int* d_perturbed = nullptr;
@@ -1992,7 +2163,7 @@ cudaError_t enqueue_factor(nla3d_ldlt* h, const double* values) {
         if ((e = cudaEventRecord(h->fork, st)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(h->side, h->fork, 0)) != cudaSuccess) return e;
         forked = true;
-        for (int q = 0; q < 3; q++)
+        for (int q = 0; q < kDoublings; q++)
           for (int pass = 0; pass < 2 && L.inv_cnt[q]; pass++)
             inv_join_kernel<T><<<(unsigned)L.inv_cnt[q], kThreads, 0, h->side>>>(
                 h->d_inv + L.inv_off[q], bb, h->dev, front, h->d_toff + L.wo_off,
@@ -2072,12 +2243,13 @@ cudaError_t enqueue_solve_core(nla3d_ldlt* h, const double* b) {
   return cudaGetLastError();
 }
 
-cudaError_t enqueue_residual(nla3d_ldlt* h, const double* A, const double* x, const double* b) {
+cudaError_t enqueue_residual(nla3d_ldlt* h, const double* A, const double* x, const double* b,
+                             double* dr = nullptr) {
   const LdltSymbolic& S = h->S;
-  const int64_t rows_per_block = kThreads / 32;
-  const unsigned blocks = (unsigned)((S.n + rows_per_block - 1) / rows_per_block);
+  const unsigned blocks = (unsigned)((S.n + kRowsPerBlock - 1) / kRowsPerBlock);
   residual_kernel<<<blocks, kThreads, 0, h->stream>>>(S.n, h->d_fptr, h->d_fcol, h->d_fslot, A, x,
-                                                     b, h->d_r, h->d_part);
+                                                     b, h->d_r, h->d_part, dr);
+  norms_kernel<<<1, kThreads, 0, h->stream>>>(blocks, h->d_part, h->d_norm);
   return cudaGetLastError();
 }
 
@@ -2210,7 +2382,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
     }
     max_work = std::max(max_work, work);
     const int bt = precision ? InvTile<float>::BT : InvTile<double>::BT;
-    for (int q = 0; q < 3; q++) {
+    for (int q = 0; q < kDoublings; q++) {
       const int64_t sz = (int64_t)kPanel << q;
       lv.inv_off[q] = (int64_t)inv_tasks.size();
       for (int64_t z = 0; z < lv.large_cnt; z++) {
@@ -2350,8 +2522,15 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   LCK(dalloc(h, &h->d_rhs, S.n));
   LCK(dalloc(h, &h->d_r, S.n));
   LCK(dalloc(h, &h->d_dx, S.n));
-  LCK(dalloc(h, &h->d_part, 2 * ((S.n + 7) / 8 + 1)));
+  LCK(dalloc(h, &h->d_part, 2 * ((S.n + kRowsPerBlock - 1) / kRowsPerBlock)));
+  LCK(dalloc(h, &h->d_norm, 2));
   LCK(dalloc(h, &h->d_dot, kDotBlocks));
+  if (precision) {
+    LCK(dalloc(h, &h->d_dirsum, (size_t)kDirBlocks * kDirSums));
+    // without the memory for them the refinement takes plain steps
+    if (rc == NLA3D_OK && dalloc(h, &h->d_dirs, (size_t)2 * kDirs * S.n) != cudaSuccess)
+      cudaGetLastError();
+  }
   LCK(dalloc(h, &h->d_maxabs, 1));
   LCK(dalloc(h, &h->d_maxpart, kMaxBlocks));
   LCK(dalloc(h, &h->d_perturbed, 2));
@@ -2467,7 +2646,8 @@ unsigned vec_blocks(int64_t n) {
 // captured once into a CUDA graph reading d_rhs and leaving the factor-order
 // solution in d_xf; each solve copies its right-hand side in, replays the
 // graph and scatters (or adds) the result into `out`
-cudaError_t enqueue_solve_any(nla3d_ldlt* h, const double* rhs, double* out, int acc) {
+cudaError_t enqueue_solve_any(nla3d_ldlt* h, const double* rhs, double* out, int acc,
+                              double* z = nullptr) {
   cudaError_t e = cudaSuccess;
   // FP64 fronts have one mode; FP32 fronts: compensated FP32 products, or
   // FP64 ones in the accurate mode
@@ -2496,7 +2676,8 @@ cudaError_t enqueue_solve_any(nla3d_ldlt* h, const double* rhs, double* out, int
   if (e == cudaSuccess) e = cudaGraphLaunch(exec, h->stream);
   if (e != cudaSuccess) return e;
   const unsigned nb = (unsigned)((h->S.n + kThreads - 1) / kThreads);
-  solve_finish_kernel<<<nb, kThreads, 0, h->stream>>>(h->S.n, h->d_perm, h->d_xf, out, acc);
+  solve_finish_kernel<<<nb, kThreads, 0, h->stream>>>(h->S.n, h->d_perm, h->d_xf, out, acc,
+                                                     z);
   return cudaGetLastError();
 }
 
@@ -2514,21 +2695,31 @@ cudaError_t dot(nla3d_ldlt* h, const double* a, const double* b, double* out) {
 
 // ||b - A x|| and ||b|| (the residual kernel leaves b - A x in d_r)
 cudaError_t residual_norms(nla3d_ldlt* h, const double* values, const double* x, const double* b,
-                           double* rnorm, double* bnorm) {
-  const int64_t nblk = (h->S.n + 7) / 8;
-  std::vector<double> part(2 * nblk);
-  cudaError_t e = enqueue_residual(h, values, x, b);
+                           double* rnorm, double* bnorm, double* dr = nullptr) {
+  double sums[2] = {0.0, 0.0};
+  cudaError_t e = enqueue_residual(h, values, x, b, dr);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(part.data(), h->d_part, sizeof(double) * 2 * nblk, cudaMemcpyDeviceToHost,
-                        h->stream);
+    e = cudaMemcpyAsync(sums, h->d_norm, sizeof(sums), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  double rr = 0.0, bb = 0.0;
-  for (int64_t q = 0; q < nblk; q++) {
-    rr += part[2 * q];
-    bb += part[2 * q + 1];
-  }
+  *rnorm = std::sqrt(sums[0]);
+  *bnorm = std::sqrt(sums[1]);
+  return e;
+}
+
+// the correction after step k: x and d_r corrected; rnorm: ||r|| after it
+cudaError_t direction_step(nla3d_ldlt* h, int k, double* x, double* rnorm) {
+  const int64_t n = h->S.n;
+  double *Q = h->d_dirs, *Z = Q + (size_t)kDirs * n;
+  direction_sums_kernel<<<kDirBlocks, kThreads, 0, h->stream>>>(n, k, Q, h->d_r, h->d_dirsum);
+  direction_step_kernel<<<kDirBlocks, kThreads, 0, h->stream>>>(n, k, Q, Z, h->d_r, x, h->d_dirsum,
+                                                               h->d_dot);
+  if (!rnorm) return cudaGetLastError();
+  double part[kDirBlocks];
+  cudaError_t e = cudaMemcpyAsync(part, h->d_dot, sizeof(part), cudaMemcpyDeviceToHost, h->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  double rr = 0.0;
+  for (int q = 0; q < kDirBlocks; q++) rr += part[q];
   *rnorm = std::sqrt(rr);
-  *bnorm = std::sqrt(bb);
   return e;
 }
 
@@ -2547,7 +2738,7 @@ cudaError_t gmres_refine(nla3d_ldlt* h, const double* values, const double* b, d
     if (e != cudaSuccess) return e;
   }
   const unsigned vb = vec_blocks(n);
-  const unsigned mb = (unsigned)((n + kThreads / 32 - 1) / (kThreads / 32));
+  const unsigned mb = (unsigned)((n + kRowsPerBlock - 1) / kRowsPerBlock);
   double rnorm = 0.0, bnorm = 0.0;
   while (true) {
     e = residual_norms(h, values, x, b, &rnorm, &bnorm);
@@ -2627,16 +2818,33 @@ int nla3d_ldlt_solve(nla3d_ldlt* h, const double* values, const double* b, doubl
   h->solve_accurate = 0;
   cudaError_t e = enqueue_solve_any(h, b, x, 0);
   double rel = 0.0, prev = 0.0, rnorm = 0.0, bnorm = 0.0;
-  int it = 0;
-  // plain refinement while it converges fast; GMRES with the same factor
-  // after, its preconditioner applied with FP64 products (FP32 fronts: the
-  // compensated FP32 products carry 2^-48 per operation, which a hard
-  // system's Krylov iteration can feel)
+  int it = 0, dirs = 0;
+  const size_t n = (size_t)h->S.n;
+  if (e == cudaSuccess) e = residual_norms(h, values, x, b, &rnorm, &bnorm);
+  if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve");
+  // refinement steps while they converge fast, accelerated (FP32 fronts) from
+  // the second on; GMRES with the same factor after, its preconditioner
+  // applied with FP64 products (FP32 fronts: the compensated FP32 products
+  // carry 2^-48 per operation, which a hard system's Krylov iteration can
+  // feel).  rel is that of b - A x computed afresh, except between a step's
+  // correction and the next step
+  const double scale = bnorm > 0.0 ? bnorm : 1.0;
   for (;;) {
-    if (e == cudaSuccess) e = residual_norms(h, values, x, b, &rnorm, &bnorm);
-    if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve");
-    rel = rnorm / (bnorm > 0.0 ? bnorm : 1.0);
+    rel = rnorm / scale;
     if (!(rel > tol) || it >= max_refine) break;
+    if (dirs > 0) {
+      // the norm after the correction is read only where it can matter
+      const bool read = !(rel < 0.1 * prev) || rel < 1e4 * tol;
+      e = direction_step(h, dirs - 1, x, read ? &rnorm : nullptr);
+      if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve");
+      if (read) rel = rnorm / scale;
+      if (!(rel > tol)) {
+        e = residual_norms(h, values, x, b, &rnorm, &bnorm);
+        if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve");
+        rel = rnorm / scale;
+        if (!(rel > tol)) break;
+      }
+    }
     // (a step that cut less, but whose rate reaches tol with one more, is
     // still cheaper than GMRES, which takes two applications at least)
     if (it > 0 && !(rel < 0.1 * prev) && !(rel < prev && rel * (rel / prev) <= tol)) {
@@ -2646,7 +2854,13 @@ int nla3d_ldlt_solve(nla3d_ldlt* h, const double* values, const double* b, doubl
       break;
     }
     prev = rel;
-    e = enqueue_solve_any(h, h->d_r, x, 1);   // x += A^-1 r with the same factors
+    // x += A^-1 r with the same factors
+    if (dirs == kDirs) dirs = 0;
+    double* q = h->d_dirs ? h->d_dirs + (size_t)dirs * n : nullptr;
+    e = enqueue_solve_any(h, h->d_r, x, 1, q ? q + (size_t)kDirs * n : nullptr);
+    if (e == cudaSuccess) e = residual_norms(h, values, x, b, &rnorm, &bnorm, q);
+    if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve");
+    if (q) dirs++;
     it++;
   }
   if (steps) *steps = it;
