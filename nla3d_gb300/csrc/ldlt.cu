@@ -65,6 +65,8 @@ struct LdltDev {
   const int32_t* sn_parent;
   const int64_t* rel_ptr;
   const uint32_t* rel;
+  const int32_t* inv_first;   // per supernode: its first kInv-pivot block (large fronts)
+  float* inv_error;           // per block: the error of its joined inverse, see inv_probe_kernel
 };
 
 // ---- factorisation kernels ----
@@ -1465,11 +1467,254 @@ __global__ void __launch_bounds__(kThreads)
   if (j < k && q == 0) xf[d.sn_first[s] + j] = td[j] + x.value();
 }
 
+// ---- which joined inverses the solves may use ----
+//
+// y = X v is not a substitution: where elimination has grown (a pressure's
+// small pivot ahead of its displacements), the rounding of X, up to
+// 2^-24 |X_C| |L_CA| |X_A|, shows in v - L y although every y_i follows from
+// the ones before it within a rounding.  On the 7 x 8 x 14 block one
+// application then left up to 170 times the residual of 64-pivot substitution.
+// So each block is tried once it is joined: v = L e for signs e, y = X v, and
+// the largest |v - L y|_i / (|L| |y|)_i, the componentwise backward error
+// (Oettli and Prager, Numer. Math. 6, 1964), kept; and the same for L^T and
+// X^T.  The solves take a block whose error is above kInvError units of the
+// front type's rounding by 64-pivot substitution in one CTA (50 us for 331
+// pivots, against 6 through X).  128: sound blocks measure 0.25 to 8 units, the
+// few with small pivots 2^5 to 2^17, of which those up to 2^7 changed the
+// residual by less than a tenth and those at 2^8 by half; two of some 1,000
+// blocks of the 454k-equation bar are above, one or two of 550 of the batch of
+// 24 blocks.  The probe takes 0.1 ms of the 139k-equation bar's 11.6 ms factor.
+constexpr float kInvError = 128.0f;
+struct ProbeTask {
+  uint32_t z, j0;   // large front (index in the level's list), first pivot of the block
+};
+
+__device__ __forceinline__ float probe_abs(double x) { return (float)fabs(x); }
+__device__ __forceinline__ float probe_abs(float2 x) { return fabsf(x.x); }
+__device__ __forceinline__ double probe_sign(int j) {
+  return (__popc((uint32_t)j * 2654435761u) & 1) ? -1.0 : 1.0;
+}
+
+// One tile of 32 outputs, forward (blockIdx.z = 0) or backward (1).  phase 0:
+// v = L e, t = L^T e;  1: y = X v, x = X^T t;  2: the errors.  L[i][j] lies at
+// (i, j), X[i][j] at (j, i) of the front: L and X^T products have the outputs
+// along the contiguous index (lane = output, warps over the terms), the other
+// two the terms (a warp per output).
+template <typename T, typename D>
+__global__ void __launch_bounds__(512)
+    inv_probe_kernel(const ProbeTask* __restrict__ tasks, BigBatch b, LdltDev d,
+                     const T* __restrict__ front, double* __restrict__ work, int phase) {
+  using X = typename D::X;
+  constexpr int kW = 16;
+  __shared__ X xs[kInv];
+  __shared__ D part[kW][32];
+  __shared__ float apart[kW][32];
+  const ProbeTask t = tasks[blockIdx.x];
+  const int s = b.list[t.z];
+  const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
+  const int k = d.sn_first[s + 1] - d.sn_first[s];
+  const int n = min(k - (int)t.j0, kInv), p0 = blockIdx.y * 32;
+  if (p0 >= n) return;
+  const bool back = blockIdx.z != 0;
+  const T* F = front + d.front_off[s] + (int64_t)t.j0 * (m + 1);
+  double* vt = work + ((int64_t)blockIdx.x * 2 + blockIdx.z) * 2 * kInv;   // v or t
+  double* yx = vt + kInv;                                                  // y or x
+  for (int j = threadIdx.x; j < n; j += 512)
+    xs[j] = D::split(phase == 0 ? probe_sign(j) : phase == 1 ? vt[j] : yx[j]);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool after = back;                                 // terms q > p (else q < p)
+  const bool along = (phase == 1) == back;                 // outputs along the contiguous index
+  // outputs of this thread: along, p0 + lane, terms warp, warp + 16, ...; else
+  // p0 + warp and p0 + warp + 16, terms lane, lane + 32, ...
+  for (int h = 0; h < (along ? 1 : 2); h++) {
+    const int p = along ? p0 + lane : p0 + warp + kW * h;
+    D a[4];
+    float absum = 0.0f;
+    if (p < n) {
+      const int q0 = along ? warp : lane, dq = along ? kW : 32;
+      const T* Fp = along ? F + p : F + (int64_t)p * m;
+      const int64_t step = along ? m : 1;
+      const int lo = after ? p + 1 : 0, hi = after ? n : p;
+      for (int q = q0; q < hi; q += 4 * dq) {
+        T f[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int t4 = q + u * dq;
+          f[u] = t4 >= lo && t4 < hi ? Fp[t4 * step] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int t4 = q + u * dq;
+          if (t4 < lo || t4 >= hi) continue;
+          a[u].add(f[u], xs[t4]);
+          if (phase == 2) absum += fabsf((float)f[u] * probe_abs(xs[t4]));
+        }
+      }
+    }
+    a[0].merge(a[1]);
+    a[2].merge(a[3]);
+    a[0].merge(a[2]);
+    if (along) {
+      part[warp][lane] = a[0];
+      apart[warp][lane] = absum;
+      __syncthreads();
+      if (warp == 0)
+        for (int w = 1; w < kW; w++) {
+          a[0].merge(part[w][lane]);
+          absum += apart[w][lane];
+        }
+    } else {
+      for (int o = 16; o > 0; o >>= 1) {
+        a[0].shfl_xor(o);
+        absum += __shfl_xor_sync(0xffffffffu, absum, o);
+      }
+    }
+    if (p < n && (along ? warp : lane) == 0) {
+      const double self = phase == 0 ? probe_sign(p) : phase == 1 ? vt[p] : yx[p];
+      const double sum = self + a[0].value();   // the diagonal is one
+      if (phase < 2) {
+        (phase == 0 ? vt : yx)[p] = sum;
+      } else {
+        const float unit = std::is_same<T, double>::value ? 0x1p-53f : 0x1p-24f;
+        const float err = (float)fabs(vt[p] - sum) / (unit * (absum + (float)fabs(self)));
+        // non-negative floats order as their bits do, and a NaN above them
+        atomicMax(reinterpret_cast<int*>(d.inv_error + d.inv_first[s] + t.j0 / kInv),
+                  __float_as_int(err));
+      }
+    }
+  }
+}
+
+// the n x n block at F on its way into L2 (a substitution's steps would wait
+// for DRAM one after the other)
+template <typename T>
+__device__ __forceinline__ void prefetch_block(const T* F, int64_t m, int n) {
+  constexpr int kLine = 128 / sizeof(T);
+  const int lines = (n + kLine - 1) / kLine;
+  for (int x = threadIdx.x; x < n * lines; x += blockDim.x) {
+    const int c = x / lines, i = min((x - c * lines) * kLine, n - 1);
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(F + i + (int64_t)c * m));
+  }
+}
+
+// y from v by 64-pivot blocks of the block at F (n <= kInv pivots): the
+// blocks' own inverses, then the rows after them; one CTA of kThreads
+template <typename T, typename D>
+__device__ void fwd_substitute(const T* __restrict__ F, int64_t m, int n,
+                               const double* __restrict__ v, double* __restrict__ y) {
+  using X = typename D::X;
+  __shared__ double vs[kInv];
+  __shared__ X xs[kPanel], ys[kPanel];
+  const int t = threadIdx.x, r = t >> 2, q = t & 3;
+  prefetch_block(F, m, n);
+  for (int i = t; i < n; i += kThreads) vs[i] = v[i];
+  __syncthreads();
+  for (int b0 = 0; b0 < n; b0 += kPanel) {
+    const int nb = min(kPanel, n - b0);
+    if (t < nb) xs[t] = D::split(vs[b0 + t]);
+    __syncthreads();
+    D a;
+    const T* Xr = F + b0 + (int64_t)(b0 + r) * m;
+    if (r < nb) {
+      T f[kPanel / 4];
+#pragma unroll
+      for (int u = 0; u < kPanel / 4; u++) f[u] = q + 4 * u < r ? Xr[q + 4 * u] : T(0);
+#pragma unroll
+      for (int u = 0; u < kPanel / 4; u++)
+        if (q + 4 * u < r) a.add(f[u], xs[q + 4 * u]);
+    }
+    a.shfl_xor(1);
+    a.shfl_xor(2);
+    if (r < nb && q == 0) {
+      const double yr = vs[b0 + r] + a.value();
+      y[b0 + r] = yr;
+      ys[r] = D::split(yr);
+    }
+    __syncthreads();
+    for (int i = b0 + nb + t; i < n; i += kThreads) {
+      const T* Fi = F + i + (int64_t)b0 * m;
+      D s[4];
+      for (int c = 0; c < nb; c += 16) {
+        T f[16];
+#pragma unroll
+        for (int u = 0; u < 16; u++) f[u] = c + u < nb ? Fi[(int64_t)(c + u) * m] : T(0);
+#pragma unroll
+        for (int u = 0; u < 16; u++)
+          if (c + u < nb) s[u & 3].add(f[u], ys[c + u]);
+      }
+      s[0].merge(s[1]);
+      s[2].merge(s[3]);
+      s[0].merge(s[2]);
+      vs[i] -= s[0].value();
+    }
+    __syncthreads();
+  }
+}
+
+// x from t by 64-pivot blocks, last to first; one CTA of 1024 threads
+template <typename T, typename D>
+__device__ void bwd_substitute(const T* __restrict__ F, int64_t m, int n,
+                               const double* __restrict__ t_in, double* __restrict__ x) {
+  using X = typename D::X;
+  __shared__ double ts[kInv];
+  __shared__ X us[kPanel], xs[kPanel];
+  const int t = threadIdx.x;
+  prefetch_block(F, m, n);
+  for (int i = t; i < n; i += 1024) ts[i] = t_in[i];
+  __syncthreads();
+  for (int b0 = (n - 1) / kPanel * kPanel; b0 >= 0; b0 -= kPanel) {
+    const int nb = min(kPanel, n - b0);
+    if (t < nb) us[t] = D::split(ts[b0 + t]);
+    __syncthreads();
+    const int j = t >> 4, q = t & 15;   // 16 threads a pivot
+    D a;
+    if (j < nb) {
+      T f[kPanel / 16];
+#pragma unroll
+      for (int u = 0; u < kPanel / 16; u++) {
+        const int i = q + 16 * u;
+        f[u] = i > j && i < nb ? F[b0 + j + (int64_t)(b0 + i) * m] : T(0);
+      }
+#pragma unroll
+      for (int u = 0; u < kPanel / 16; u++) {
+        const int i = q + 16 * u;
+        if (i > j && i < nb) a.add(f[u], us[i]);
+      }
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) a.shfl_xor(o);
+    if (j < nb && q == 0) {
+      const double xj = ts[b0 + j] + a.value();
+      x[b0 + j] = xj;
+      xs[j] = D::split(xj);
+    }
+    __syncthreads();
+    for (int c0 = 0; c0 < b0; c0 += 128) {   // eight lanes a column (b0: a multiple of 64)
+      const int c = c0 + (t >> 3), h = t & 7;
+      D s;
+      if (c < b0) {
+        T f[kPanel / 8];
+#pragma unroll
+        for (int u = 0; u < kPanel / 8; u++)
+          f[u] = h + 8 * u < nb ? F[b0 + h + 8 * u + (int64_t)c * m] : T(0);
+#pragma unroll
+        for (int u = 0; u < kPanel / 8; u++)
+          if (h + 8 * u < nb) s.add(f[u], xs[h + 8 * u]);
+      }
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) s.shfl_xor(o);
+      if (c < b0 && h == 0) ts[c] -= s.value();
+    }
+    __syncthreads();
+  }
+}
+
 // forward, wide fronts, block o0: y = X v, a warp per row (a row of X is
 // contiguous; all its loads in flight)
 constexpr int kInvRows = kThreads / 32;
 template <typename T, typename D>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 4)
     fwd_inv_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
                    int64_t o0, const double* __restrict__ vec, double* __restrict__ yv) {
   using X = typename D::X;
@@ -1482,6 +1727,7 @@ __global__ void __launch_bounds__(kThreads)
   const int r0 = blockIdx.x * kInvRows;
   if (r0 >= ob) return;
   const double* v = vec + d.vec_off[s] + o0;
+  const float error = d.inv_error[d.inv_first[s] + o0 / kInv];   // looked at once X is on its way
   const int lane = threadIdx.x & 31, i = r0 + (threadIdx.x >> 5);
   T f[kInv / 32];
   if (i < ob) {
@@ -1491,6 +1737,11 @@ __global__ void __launch_bounds__(kThreads)
   }
   for (int j = threadIdx.x; j < min(ob, r0 + kInvRows); j += kThreads) xs[j] = D::split(v[j]);
   __syncthreads();
+  if (!(error <= kInvError)) {
+    if (r0 == 0)
+      fwd_substitute<T, D>(front + d.front_off[s] + o0 * (m + 1), m, ob, v, yv + d.vec_off[s] + o0);
+    return;
+  }
   if (i >= ob) return;
   D a[4];
 #pragma unroll
@@ -1637,6 +1888,7 @@ __global__ void __launch_bounds__(kColThreads)
   const int j0 = blockIdx.x * 32;
   if (j0 >= ob) return;
   const double* v = vec + d.vec_off[s] + o0;
+  const float error = d.inv_error[d.inv_first[s] + o0 / kInv];   // looked at once X is on its way
   const int j = j0 + (threadIdx.x & 31), i0 = j0 + (threadIdx.x >> 5);
   const T* Fj = front + d.front_off[s] + o0 + j + (o0 + i0) * m;   // X[i][j], i = i0 + 32 u
   T f[kInv / 32];
@@ -1645,6 +1897,11 @@ __global__ void __launch_bounds__(kColThreads)
     f[u] = i0 + 32 * u < ob && i0 + 32 * u > j ? Fj[(int64_t)(32 * u) * m] : T(0);
   for (int i = j0 + threadIdx.x; i < ob; i += kColThreads) ts[i] = D::split(v[i]);
   __syncthreads();
+  if (!(error <= kInvError)) {
+    if (j0 == 0)
+      bwd_substitute<T, D>(front + d.front_off[s] + o0 * (m + 1), m, ob, v, xf + d.sn_first[s] + o0);
+    return;
+  }
   D a[2];
 #pragma unroll
   for (int u = 0; u < kInv / 32; u++)
@@ -2002,6 +2259,9 @@ struct nla3d_ldlt {
   int n_sm = 0;
   InvTask* d_inv = nullptr;     // the inverses' joins: every level's tasks
   uint64_t* d_toff = nullptr;   // per large front: its part of the joins' workspace
+  ProbeTask* d_probe = nullptr; // the joined blocks, per level, and their vectors
+  double* d_probe_work = nullptr;
+  size_t n_inv = 0;             // kInv-pivot blocks of large fronts
   void* d_work = nullptr;
   cudaStream_t side = nullptr;  // the joins run beside the next levels
   cudaEvent_t fork = nullptr, join = nullptr;
@@ -2027,6 +2287,7 @@ struct nla3d_ldlt {
     std::vector<int64_t> tile_off, tile_cnt;  // tensor-core fronts: per outer block, its tiles
     std::vector<int64_t> itile_off, itile_cnt;  // and per panel, its in-block update's tiles
     int64_t inv_off[3] = {}, inv_cnt[3] = {};   // joins of 64-, 128-, 256-pivot blocks
+    int64_t probe_off = 0, probe_cnt = 0;       // the joined blocks
     uint64_t vec0 = 0, vec1 = 0;                // its fronts' rows in the solve vectors
     int64_t narrow_off = 0, narrow_cnt = 0, narrow_max_u = 0;   // solves: large fronts by width
     int64_t wide_off = 0, wide_cnt = 0, wide_max_m = 0, wide_max_k = 0;
@@ -2076,6 +2337,8 @@ cudaError_t enqueue_factor(nla3d_ldlt* h, const double* values) {
   cudaError_t e = cudaMemsetAsync(front, 0, sizeof(T) * h->front_entries, st);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(h->d_perturbed, 0, 2 * sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  e = cudaMemsetAsync(h->dev.inv_error, 0, sizeof(float) * h->n_inv, st);
   if (e != cudaSuccess) return e;
   bool forked = false;
   {
@@ -2168,6 +2431,9 @@ cudaError_t enqueue_factor(nla3d_ldlt* h, const double* values) {
             inv_join_kernel<T><<<(unsigned)L.inv_cnt[q], kThreads, 0, h->side>>>(
                 h->d_inv + L.inv_off[q], bb, h->dev, front, h->d_toff + L.wo_off,
                 static_cast<T*>(h->d_work), kPanel << q, pass);
+        for (int phase = 0; phase < 3; phase++)
+          inv_probe_kernel<T, Dot<T>><<<dim3((unsigned)L.probe_cnt, kInv / 32, 2), 512, 0, h->side>>>(
+              h->d_probe + L.probe_off, bb, h->dev, front, h->d_probe_work, phase);
       }
     }
   }
@@ -2312,6 +2578,10 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   }
   std::vector<InvTask> inv_tasks;
   std::vector<uint64_t> toff;
+  std::vector<ProbeTask> probes;
+  std::vector<int32_t> inv_first(ns, 0);
+  size_t n_inv = 0;
+  int64_t max_probes = 0;
   uint64_t max_work = 0;
   std::vector<uint64_t> wo, lio, pko;
   std::vector<OuterTile> tiles;
@@ -2381,6 +2651,17 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
       if (k > kPanel) work += (uint64_t)k * (kInv / 2);
     }
     max_work = std::max(max_work, work);
+    lv.probe_off = (int64_t)probes.size();
+    for (int64_t z = 0; z < lv.large_cnt; z++) {
+      const int32_t s = lists[lv.large_off + z];
+      const int64_t k = S.k(s);
+      inv_first[s] = (int32_t)n_inv;
+      n_inv += (size_t)((k + kInv - 1) / kInv);
+      for (int64_t j0 = 0; j0 + kPanel < k; j0 += kInv)
+        probes.push_back(ProbeTask{(uint32_t)z, (uint32_t)j0});
+    }
+    lv.probe_cnt = (int64_t)probes.size() - lv.probe_off;
+    max_probes = std::max(max_probes, lv.probe_cnt);
     const int bt = precision ? InvTile<float>::BT : InvTile<double>::BT;
     for (int q = 0; q < kDoublings; q++) {
       const int64_t sz = (int64_t)kPanel << q;
@@ -2511,6 +2792,9 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   LCK(upload(h, &h->d_rsn, solve_lists.row_sn));
   LCK(upload(h, &h->d_inv, inv_tasks));
   LCK(upload(h, &h->d_toff, toff));
+  LCK(upload(h, &h->d_probe, probes));
+  LCK(dalloc(h, &h->d_probe_work, (size_t)max_probes * 4 * kInv));
+  h->n_inv = n_inv;
   if (precision)
     LCK(dalloc(h, reinterpret_cast<float**>(&h->d_work), (size_t)max_work));
   else
@@ -2556,6 +2840,10 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   int64_t *rp = nullptr, *relp = nullptr;
   int32_t *rw = nullptr, *sf = nullptr, *sp = nullptr;
   uint32_t* rl = nullptr;
+  int32_t* inv_first_d = nullptr;
+  float* inv_error = nullptr;
+  LCK(upload(h, &inv_first_d, inv_first));
+  LCK(dalloc(h, &inv_error, n_inv));
   LCK(upload(h, &fo, S.front_off));
   LCK(upload(h, &vo, solve_lists.vec_off));
   LCK(upload(h, &rp, S.row_ptr));
@@ -2566,7 +2854,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   LCK(upload(h, &rl, S.rel));
   LCK(cudaStreamSynchronize(h->stream));
 #undef LCK
-  h->dev = LdltDev{fo, vo, rp, rw, sf, sp, relp, rl};
+  h->dev = LdltDev{fo, vo, rp, rw, sf, sp, relp, rl, inv_first_d, inv_error};
   if (rc != NLA3D_OK) {
     // keep the handle so that the caller can read the message, then destroy it
     *out = h;
