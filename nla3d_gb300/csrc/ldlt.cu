@@ -256,44 +256,22 @@ struct BigBatch {
 // scales its own row's entry by the pivot and updates its columns.  FP64: the
 // pivot's thread inverts it for everyone, since 256 FP64 divisions a step keep
 // the pipe busy longer than the update; FP32: every thread divides, off the
-// chain of the pivot's thread.  The inverse is formed blockwise: four 16 x 16
-// blocks by substitution (a thread per column), then X10 = -X1 (L10 X0) for 16
-// and 32.  54 -> 19 us (FP32) and 136 -> 82 us (FP64) a launch (ncu, cold)
-// against the block in shared memory, where each step's update ran as a chain
-// of dependent shared-memory accesses and the inverse row by row as another.
-constexpr int kDiagLd = kPanel + 1;
-
-// X10 = -X1 (L10 X0) for every pair of H x H diagonal blocks: a thread owns
-// H / 8 consecutive columns of one row
-template <typename T, int H>
-__device__ __forceinline__ void join_inverses(const T* Lr, T* X) {
-  constexpr int kOut = H / 8;
-  const int pr = threadIdx.x / (8 * H), i = (threadIdx.x / 8) % H, j0 = (threadIdx.x % 8) * kOut;
-  const int o = 2 * H * pr;
-  T v[kOut] = {};
-#pragma unroll 4
-  for (int q = j0; q < H; q++) {   // X0 is lower triangular
-    const T l = Lr[(o + H + i) * kDiagLd + o + q];
-#pragma unroll
-    for (int u = 0; u < kOut; u++) v[u] += l * X[(o + q) * kDiagLd + o + j0 + u];
-  }
-  T* out = X + (o + H + i) * kDiagLd + o + j0;
-#pragma unroll
-  for (int u = 0; u < kOut; u++) out[u] = v[u];   // L10 X0 in X10's place
-  __syncthreads();
-#pragma unroll
-  for (int u = 0; u < kOut; u++) v[u] = T(0);
-#pragma unroll 4
-  for (int q = 0; q <= i; q++) {   // X1 is lower triangular
-    const T x = X[(o + H + i) * kDiagLd + o + H + q];
-#pragma unroll
-    for (int u = 0; u < kOut; u++) v[u] -= x * X[(o + H + q) * kDiagLd + o + j0 + u];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int u = 0; u < kOut; u++) out[u] = v[u];
-  __syncthreads();
-}
+// chain of the pivot's thread.
+//
+// The inverse is formed by substitution, which stays accurate where pivots are
+// small (joined from inverses of 16 and 32 rows it left 0.4 instead of 1e-3 of
+// the right-hand side after one FP32 application, on a block with three pivots
+// of 1e-4).  FP64: along the way, the same row operations on the identity by
+// the column groups whose own columns are final, which costs nothing where the
+// pipe is the bound.  FP32: afterwards, four threads a column with 16 rows each
+// in registers, x_p passed on by shuffle; along the way its loads and stores
+// lengthened every step (26 us a launch).
+//
+// Against the block in shared memory, where each step's update ran as a chain
+// of dependent accesses and the inverse row by row as another: 54 -> 21 us
+// (FP32) and 136 -> 73 us (FP64) a launch.
+template <typename T>
+constexpr int kDiagLdOf = std::is_same<T, double>::value ? kPanel + 1 : kPanel + 4;
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
@@ -302,10 +280,11 @@ __global__ void __launch_bounds__(kThreads)
                         int* perturbed) {
   static_assert(kThreads == 4 * kPanel, "four column groups of 16");
   constexpr bool kShare = std::is_same<T, double>::value;
-  extern __shared__ __align__(16) unsigned char diag_smem_raw[];
-  T* Lr = reinterpret_cast<T*>(diag_smem_raw);   // Lr[r * kDiagLd + c]: unit lower factor
-  T* X = Lr + kPanel * kDiagLd;                  // X[r * kDiagLd + c]: its inverse
-  __shared__ __align__(16) T wcol[2][kPanel];
+  constexpr int kDiagLd = kDiagLdOf<T>;
+  // FP64: X[r * kDiagLd + c], to be written transposed; FP32: L, column p at p * kDiagLd
+  __shared__ __align__(16) T X[kPanel * kDiagLd];
+  __shared__ __align__(16) T wcol[2][kPanel];    // column p, unscaled
+  __shared__ __align__(16) T xrow[2][kPanel];    // row p of the inverse
   __shared__ T winv[2];
   const int s = b.list[blockIdx.x];
   const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
@@ -314,11 +293,12 @@ __global__ void __launch_bounds__(kThreads)
   const int pb = (int)(k - p0 < kPanel ? k - p0 : kPanel);
   T* F = front + d.front_off[s] + p0 + p0 * m;
   const int r = threadIdx.x & (kPanel - 1), cg = threadIdx.x / kPanel;
-  T a[16];
+  T a[16], x[16];
 #pragma unroll
   for (int j = 0; j < 16; j++) {
     const int c = 16 * cg + j;
     a[j] = r < pb && c <= r ? F[r + c * m] : (r == c ? T(1) : T(0));
+    x[j] = kShare && r == c ? T(1) : T(0);
   }
   // the pivot bound in the front's precision (the guards compare in it)
   const T tau = (T)(pivot_rel * tau_p[0]);
@@ -328,15 +308,20 @@ __global__ void __launch_bounds__(kThreads)
       const int p = 16 * blk + j;
       if (p >= pb) break;
       T* w = wcol[p & 1];
+      T* xr = xrow[p & 1];
       const bool own = cg == blk && r == p;
       if (cg == blk) w[r] = a[j];
+      if (kShare && r == p && cg <= blk) {
+#pragma unroll
+        for (int c = 0; c < 16; c++) xr[16 * cg + c] = x[c];
+      }
       if (kShare && own) {
         a[j] = guard_pivot(a[j], tau, perturbed);
         winv[p & 1] = T(1) / a[j];
       }
       __syncthreads();
       // (rows up to p are final; a warp holds 32 rows of one column group)
-      if (cg < blk || (r | 31) < p) continue;
+      if ((r | 31) < p || (!kShare && cg < blk)) continue;
       T l;
       if (kShare) {
         l = w[r] * winv[p & 1];
@@ -346,48 +331,76 @@ __global__ void __launch_bounds__(kThreads)
         if (own) a[j] = dv;
         l = w[r] / dv;
       }
-      if (cg == blk) {
-#pragma unroll
-        for (int c = j + 1; c < 16; c++) a[c] -= l * w[16 * blk + c];
-        if (r > p) a[j] = l;
-      } else {
+      if (cg > blk) {
 #pragma unroll
         for (int c = 0; c < 16; c++) a[c] -= l * w[16 * cg + c];
+      } else if (cg == blk) {
+#pragma unroll
+        for (int c = j + 1; c < 16; c++) a[c] -= l * w[16 * blk + c];
+        if (r > p) {
+          a[j] = l;
+          if (kShare) {
+#pragma unroll
+            for (int c = 0; c <= j; c++) x[c] -= l * xr[16 * blk + c];
+          }
+        }
+      } else if (r > p) {
+#pragma unroll
+        for (int c = 0; c < 16; c++) x[c] -= l * xr[16 * cg + c];
       }
     }
   }
-#pragma unroll
-  for (int j = 0; j < 16; j++) {
-    const int c = 16 * cg + j;
-    if (r < pb && c <= r) F[r + c * m] = a[j];
-    Lr[r * kDiagLd + c] = r > c && r < pb ? a[j] : T(0);
-    X[r * kDiagLd + c] = r == c ? T(1) : T(0);
-  }
-  __syncthreads();
-  if (threadIdx.x < kPanel) {
-    // columns of the four 16 x 16 diagonal blocks' inverses
-    const int o = threadIdx.x & ~15, c = threadIdx.x & 15;
-    T x[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-      T v = T(0);
-#pragma unroll
-      for (int q = 0; q < i; q++) v += Lr[(o + i) * kDiagLd + o + q] * x[q];
-      x[i] = i < c ? T(0) : (i == c ? T(1) : -v);
-      if (i > c) X[(o + i) * kDiagLd + o + c] = x[i];
-    }
-  }
-  __syncthreads();
-  join_inverses<T, 16>(Lr, X);
-  join_inverses<T, 32>(Lr, X);
   T* Li = Linv + b.li_off[blockIdx.x] + (uint64_t)(p0 / kPanel) * kPanel * kPanel;
 #pragma unroll
   for (int j = 0; j < 16; j++) {
     const int c = 16 * cg + j;
-    if (r < pb && c < pb) Li[r + c * kPanel] = X[r * kDiagLd + c];
-    // and for the solves in the front's unused upper triangle, row c of the
-    // inverse down column c (here r runs over the row's entries)
-    if (r < c && c < pb) F[r + c * m] = X[c * kDiagLd + r];
+    if (r < pb && c <= r) F[r + c * m] = a[j];
+    if (kShare) {
+      if (r < pb && c < pb) Li[r + c * kPanel] = x[j];
+      X[r * kDiagLd + c] = x[j];
+    } else {
+      X[c * kDiagLd + r] = r > c && r < pb ? a[j] : T(0);
+    }
+  }
+  __syncthreads();
+  if constexpr (kShare) {
+    // the inverse for the solves too, in the front's unused upper triangle: row
+    // c of it down column c (here r runs over the row's entries)
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+      const int c = 16 * cg + j;
+      if (r < c && c < pb) F[r + c * m] = X[c * kDiagLd + r];
+    }
+  } else {
+    // column c of the inverse, rows 16 h .. +15 in this thread: x -= L[:,p] x_p
+    const int c = threadIdx.x >> 2, h = threadIdx.x & 3, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < 16; i++) x[i] = 16 * h + i == c ? T(1) : T(0);
+    const int first = (threadIdx.x >> 5) * 8;   // the warp's first column: zeros above it
+    for (int blk = first / 16; blk < 4; blk++) {
+#pragma unroll
+      for (int j = 0; j < 16; j++) {
+        const T xp = __shfl_sync(0xffffffffu, x[j], (lane & ~3) | blk);
+        const float4* Lp = reinterpret_cast<const float4*>(X + (16 * blk + j) * kDiagLd + 16 * h);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const float4 l = Lp[u];   // zero up to row p
+          x[4 * u] -= l.x * xp;
+          x[4 * u + 1] -= l.y * xp;
+          x[4 * u + 2] -= l.z * xp;
+          x[4 * u + 3] -= l.w * xp;
+        }
+      }
+    }
+    // (Li's 64 x 64 entries are all there; past pb the unit columns)
+    float4* Lc = reinterpret_cast<float4*>(Li + c * kPanel + 16 * h);
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      Lc[u] = make_float4(x[4 * u], x[4 * u + 1], x[4 * u + 2], x[4 * u + 3]);
+    // and for the solves in the front's unused upper triangle
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+      if (c < 16 * h + i && 16 * h + i < pb) F[c + (16 * h + i) * m] = x[i];
   }
 }
 
@@ -2381,7 +2394,7 @@ cudaError_t enqueue_factor(nla3d_ldlt* h, const double* values) {
       for (int64_t o0 = 0; o0 < L.large_max_k; o0 += kOuter) {
         const int64_t o_end = std::min<int64_t>(o0 + kOuter, L.large_max_k);
         for (int64_t p0 = o0; p0 < o_end; p0 += kPanel) {
-          batched_diag_kernel<T><<<nf, kThreads, 2 * sizeof(T) * kPanel * kDiagLd, st>>>(
+          batched_diag_kernel<T><<<nf, kThreads, 0, st>>>(
               bb, h->dev, front, p0, Li, h->d_maxabs, h->pivot_rel, h->d_perturbed);
           const int64_t rest = L.large_max_m - p0 - 1;   // rows past the smallest panel
           if (rest <= 0) continue;
@@ -2766,18 +2779,12 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
     // (tensor-core fronts keep the panels' operands packed instead)
     LCK(dalloc(h, reinterpret_cast<float**>(&h->d_W), h->tc ? 1 : (size_t)max_w));
     LCK(dalloc(h, reinterpret_cast<float**>(&h->d_Linv), nlinv));
-    LCK(cudaFuncSetAttribute(batched_diag_kernel<float>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(2 * sizeof(float) * kPanel * (kPanel + 1))));
     LCK(cudaFuncSetAttribute(factor_small_kernel<float>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(sizeof(float) * kSmallFront * (kSmallFront + 1))));
   } else {
     LCK(dalloc(h, reinterpret_cast<double**>(&h->d_W), (size_t)max_w));
     LCK(dalloc(h, reinterpret_cast<double**>(&h->d_Linv), nlinv));
-    LCK(cudaFuncSetAttribute(batched_diag_kernel<double>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(2 * sizeof(double) * kPanel * (kPanel + 1))));
     LCK(cudaFuncSetAttribute(factor_small_kernel<double>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(sizeof(double) * kSmallFront * (kSmallFront + 1))));
@@ -3133,9 +3140,13 @@ int nla3d_ldlt_solve(nla3d_ldlt* h, const double* values, const double* b, doubl
         if (!(rel > tol)) break;
       }
     }
-    // (a step that cut less, but whose rate reaches tol with one more, is
-    // still cheaper than GMRES, which takes two applications at least)
-    if (it > 0 && !(rel < 0.1 * prev) && !(rel < prev && rel * (rel / prev) <= tol)) {
+    // A step that cut less, but whose rate reaches tol with one more, is still
+    // cheaper than GMRES, which takes two applications at least.  Accelerated
+    // steps may cut by as little as four: GMRES over the same Krylov space
+    // gains no more per application, and its own cost twice as much (a
+    // 454k-equation bar that once cut by 7: 8 steps in 43 ms against 9 in 81)
+    if (it > 0 && !(rel < (dirs > 0 ? 0.25 : 0.1) * prev) &&
+        !(rel < prev && rel * (rel / prev) <= tol)) {
       h->solve_accurate = 1;
       e = gmres_refine(h, values, b, x, tol, max_refine, &it, &rel);
       if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve (GMRES)");
