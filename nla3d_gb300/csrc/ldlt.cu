@@ -277,7 +277,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads)
     batched_diag_kernel(BigBatch b, LdltDev d, T* __restrict__ front, int64_t p0,
                         T* __restrict__ Linv, const double* __restrict__ tau_p, double pivot_rel,
-                        int* perturbed) {
+                        int* perturbed, int update) {
   static_assert(kThreads == 4 * kPanel, "four column groups of 16");
   constexpr bool kShare = std::is_same<T, double>::value;
   constexpr int kDiagLd = kDiagLdOf<T>;
@@ -300,6 +300,45 @@ __global__ void __launch_bounds__(kThreads)
     a[j] = r < pb && c <= r ? F[r + c * m] : (r == c ? T(1) : T(0));
     x[j] = kShare && r == c ? T(1) : T(0);
   }
+  if (!kShare && update) {
+    // the block's own part of the update that runs meanwhile: A -= L D L^T over
+    // the panel before (update 1) or the outer block before (2), 64 columns at
+    // a time through X, the next 64 on their way into registers
+    const int64_t kw = update == 1 ? kPanel : kOuter;
+    const T* Lp = front + d.front_off[s] + (p0 + r) + (p0 - kw) * m;
+    const T* Dp = front + d.front_off[s] + (p0 - kw) * (m + 1);
+#pragma unroll
+    for (int j = 0; j < 16; j++) x[j] = r < pb ? Lp[(int64_t)(16 * cg + j) * m] : T(0);
+    T dv = cg == 0 ? Dp[(int64_t)r * (m + 1)] : T(0);
+    for (int64_t c0 = 0; c0 < kw; c0 += kPanel) {
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < 16; j++) X[(16 * cg + j) * kDiagLd + r] = x[j];
+      if (cg == 0) wcol[0][r] = dv;
+      __syncthreads();
+      if (c0 + kPanel < kw) {
+#pragma unroll
+        for (int j = 0; j < 16; j++)
+          x[j] = r < pb ? Lp[(c0 + kPanel + 16 * cg + j) * m] : T(0);
+        if (cg == 0) dv = Dp[(c0 + kPanel + r) * (m + 1)];
+      }
+      if ((r | 31) < 16 * cg) continue;   // above the diagonal
+#pragma unroll 8
+      for (int c = 0; c < kPanel; c++) {
+        const T l = X[c * kDiagLd + r] * wcol[0][c];
+        const float4* w = reinterpret_cast<const float4*>(X + c * kDiagLd + 16 * cg);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const float4 v = w[u];
+          a[4 * u] -= l * v.x;
+          a[4 * u + 1] -= l * v.y;
+          a[4 * u + 2] -= l * v.z;
+          a[4 * u + 3] -= l * v.w;
+        }
+      }
+    }
+    __syncthreads();
+  }
   // the pivot bound in the front's precision (the guards compare in it)
   const T tau = (T)(pivot_rel * tau_p[0]);
   for (int blk = 0; blk < 4; blk++) {
@@ -320,8 +359,9 @@ __global__ void __launch_bounds__(kThreads)
         winv[p & 1] = T(1) / a[j];
       }
       __syncthreads();
-      // (rows up to p are final; a warp holds 32 rows of one column group)
-      if ((r | 31) < p || (!kShare && cg < blk)) continue;
+      // (rows up to p are final, rows above a group's columns not wanted; a warp
+      // holds 32 rows of one column group)
+      if ((r | 31) < p || (r | 31) < 16 * cg || (!kShare && cg < blk)) continue;
       T l;
       if (kShare) {
         l = w[r] * winv[p & 1];
@@ -547,21 +587,27 @@ __device__ __forceinline__ bool update_range(int64_t p0, int outer, int64_t k, i
   return u.jb < u.je;
 }
 
-// BT x BT tiles (blockIdx.x rows, .y columns, both from jb), front
+// the first row past the front's next diagonal block (0: no such block)
+__device__ __forceinline__ int64_t next_block_end(const UpdateRange& u, int64_t k) {
+  return u.jb < k ? u.jb + (k - u.jb < kPanel ? k - u.jb : kPanel) : 0;
+}
+
+// BT x BT tiles (blockIdx.x rows from row_tile0, .y columns, both from jb), front
 // blockIdx.z, RT x RT outputs per thread (32 / 2 for FP64: its pipe bounds the
 // kernel, one SM takes 64 us for a 64 x 64 tile of a rank-64 update, and
 // smaller tiles reach more SMs; 128 / 8 for FP32).  A thread owns rows tx + 16u and
 // columns ty + 16v: shared-memory reads are conflict-free or broadcast and
 // the stores run down the columns.  The next 16-wide slice of the operands
-// is loaded into registers while the current one is multiplied.
+// is loaded into registers while the current one is multiplied.  ahead: the
+// next diagonal block is left out (its own kernel updates it meanwhile).
 template <typename T, int BT, int RT>
 __global__ void __launch_bounds__(kThreads)
     batched_trailing_kernel(BigBatch b, LdltDev d, T* __restrict__ front, int64_t p0, int outer,
-                            const T* __restrict__ Wbuf) {
+                            const T* __restrict__ Wbuf, int row_tile0, int ahead) {
   static_assert((BT / RT) * (BT / RT) == kThreads, "one output block per thread");
   static_assert(BT / RT == 16, "16 x 16 threads");
   constexpr int LPT = 16 * BT / kThreads;   // slice elements each thread loads per operand
-  const int ti = blockIdx.x, tj = blockIdx.y;
+  const int ti = blockIdx.x + row_tile0, tj = blockIdx.y;
   if (tj > ti) return;
   const int s = b.list[blockIdx.z];
   const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
@@ -613,6 +659,7 @@ __global__ void __launch_bounds__(kThreads)
     }
     __syncthreads();
   }
+  const int64_t i_min = ahead ? next_block_end(ur, k) : 0;
 #pragma unroll
   for (int v = 0; v < RT; v++) {
     const int64_t j = j0 + ty + 16 * v;
@@ -620,7 +667,7 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
     for (int u = 0; u < RT; u++) {
       const int64_t i = i0 + tx + 16 * u;
-      if (i < m && j <= i) F[i + j * m] -= acc[u][v];
+      if (i < m && j <= i && i >= i_min) F[i + j * m] -= acc[u][v];
     }
   }
 }
@@ -859,7 +906,7 @@ struct OuterTile {
 __global__ void __launch_bounds__(kOuterThreads, 1)
     tc_packed_kernel(BigBatch b, LdltDev d, float* __restrict__ front, int64_t p0, int outer,
                      const float* __restrict__ packed, const OuterTile* __restrict__ tiles,
-                     int n_tiles, int* __restrict__ err) {
+                     int n_tiles, int* __restrict__ err, int ahead) {
   extern __shared__ __align__(1024) unsigned char pk_smem[];
   float* stage0 = reinterpret_cast<float*>(pk_smem);
   uint64_t* full = reinterpret_cast<uint64_t*>(stage0 + (size_t)kPkStages * 4 * kPkTile);
@@ -897,7 +944,7 @@ __global__ void __launch_bounds__(kOuterThreads, 1)
   };
   // the front of a tile: rows m, update range, chunks
   struct TileInfo {
-    int64_t m, jb, je, i0, j0;
+    int64_t m, jb, je, i0, j0, i_min;
     int nch;
     const float* pa;
     const float* pb;
@@ -915,6 +962,7 @@ __global__ void __launch_bounds__(kOuterThreads, 1)
     ti.m = m;
     ti.jb = ur.jb;
     ti.je = ur.je;
+    ti.i_min = ahead ? next_block_end(ur, k) : 0;
     ti.i0 = o0 + (int64_t)rI * kTcM;
     ti.j0 = o0 + (int64_t)rJ * kTcN;
     ti.nch = (int)((ur.kw + kTcKH - 1) / kTcKH);
@@ -1013,7 +1061,7 @@ __global__ void __launch_bounds__(kOuterThreads, 1)
       info(t, ti);
       const uint32_t a = it & 1u;
       const int64_t i = ti.i0 + row;
-      const bool row_in = i < ti.m;
+      const bool row_in = i < ti.m && i >= ti.i_min;
       // the front's values of the first 32 columns first: their loads overlap
       // the tile's MMAs; the second 32 load while the first are stored
       float* fp = ti.F + i + (ti.j0 + cb) * ti.m;   // (i, j0 + cb); column stride m
@@ -2278,6 +2326,8 @@ struct nla3d_ldlt {
   void* d_work = nullptr;
   cudaStream_t side = nullptr;  // the joins run beside the next levels
   cudaEvent_t fork = nullptr, join = nullptr;
+  cudaStream_t ahead = nullptr; // the next diagonal blocks run beside the updates
+  cudaEvent_t join_ahead = nullptr;
   int32_t* d_bidx = nullptr;    // per front row (level order): its right-hand side entry or -1,
   uint32_t* d_gptr = nullptr;   // and its children's update rows
   uint32_t* d_gsrc = nullptr;
@@ -2383,56 +2433,81 @@ cudaError_t enqueue_factor(nla3d_ldlt* h, const double* values) {
       const unsigned nf = (unsigned)L.large_cnt;
       constexpr int BT = TrailingShape<T>::BT, RT = TrailingShape<T>::RT;
       const bool tc = std::is_same<T, float>::value && h->tc;
-      // one FMA update launch: rows from its range's first column to the
-      // largest front's last row, `col_tiles` tiles of columns
-      auto update = [&](int64_t p, int outer, int64_t rows, unsigned col_tiles) {
+      // one FMA update launch: rows from its range's first column (and row_tile0
+      // tiles) to the largest front's last row, `col_tiles` tiles of columns
+      auto update = [&](int64_t p, int outer, int64_t rows, unsigned col_tiles, int row_tile0,
+                        int ahead) {
         const unsigned rt = (unsigned)((rows + BT - 1) / BT);
-        const dim3 grid(rt, std::min(rt, col_tiles), nf);
-        batched_trailing_kernel<T, BT, RT><<<grid, kThreads, 0, st>>>(bb, h->dev, front, p,
-                                                                       outer, W);
+        if (rt <= (unsigned)row_tile0) return;
+        const dim3 grid(rt - row_tile0, std::min(rt, col_tiles), nf);
+        batched_trailing_kernel<T, BT, RT><<<grid, kThreads, 0, st>>>(
+            bb, h->dev, front, p, outer, W, row_tile0, ahead);
       };
+      auto diag = [&](int64_t p, int upd, cudaStream_t q) {
+        batched_diag_kernel<T><<<nf, kThreads, 0, q>>>(bb, h->dev, front, p, Li, h->d_maxabs,
+                                                       h->pivot_rel, h->d_perturbed, upd);
+      };
+      // Look-ahead: the next diagonal block, a chain on one SM, is updated and
+      // factored beside the rest of the update that it would wait for.  FP32
+      // blocks take their part of the update themselves; FP64 ones have its 64
+      // rows updated first, in 16 x 16 tiles (4 us, where one SM would take 34).
+      auto look_ahead = [&](int64_t p, int outer, int64_t next) {
+        cudaError_t er = cudaEventRecord(h->fork, st);
+        if (er == cudaSuccess) er = cudaStreamWaitEvent(h->ahead, h->fork, 0);
+        if (er != cudaSuccess) return er;
+        if constexpr (std::is_same<T, double>::value)
+          batched_trailing_kernel<T, 16, 1><<<dim3(4, 4, nf), kThreads, 0, h->ahead>>>(
+              bb, h->dev, front, p, outer, W, 0, 0);
+        diag(next, std::is_same<T, double>::value ? 0 : outer + 1, h->ahead);
+        return cudaEventRecord(h->join_ahead, h->ahead);
+      };
+      constexpr int kHeadTiles = std::is_same<T, double>::value ? kPanel / BT : 0;
+      diag(0, 0, st);
       for (int64_t o0 = 0; o0 < L.large_max_k; o0 += kOuter) {
         const int64_t o_end = std::min<int64_t>(o0 + kOuter, L.large_max_k);
         for (int64_t p0 = o0; p0 < o_end; p0 += kPanel) {
-          batched_diag_kernel<T><<<nf, kThreads, 0, st>>>(
-              bb, h->dev, front, p0, Li, h->d_maxabs, h->pivot_rel, h->d_perturbed);
           const int64_t rest = L.large_max_m - p0 - 1;   // rows past the smallest panel
           if (rest <= 0) continue;
           constexpr int R = PanelRows<T>::value;
           const dim3 panel_grid((unsigned)((rest + R - 1) / R), nf);
+          const bool next = p0 + kPanel < o_end;
           if constexpr (std::is_same<T, float>::value) {
-            if (tc) {
+            if (tc)
               batched_panel_kernel<float, true><<<panel_grid, kThreads, 0, st>>>(
                   bb, h->dev, front, p0, Li, nullptr, h->d_pk);
-              // the panel's columns into the rest of its outer block
-              const int64_t pi = p0 / kPanel;
-              const int nt = (int)L.itile_cnt[pi];
-              if (nt > 0)
-                tc_packed_kernel<<<(unsigned)std::min(nt, h->n_sm), kOuterThreads, kPkSmem, st>>>(
-                    bb, h->dev, front, p0, 0, h->d_pk, h->d_tiles + L.itile_off[pi], nt, h->d_err);
-              continue;
-            }
           }
-          batched_panel_kernel<T, false><<<panel_grid, kThreads, 0, st>>>(bb, h->dev, front, p0, Li,
-                                                                         W, nullptr);
-          // (at most kOuter - kPanel columns)
-          if (p0 + kPanel < o_end)
-            update(p0, 0, rest, (unsigned)((kOuter - kPanel + BT - 1) / BT));
+          if (!tc)
+            batched_panel_kernel<T, false><<<panel_grid, kThreads, 0, st>>>(bb, h->dev, front, p0,
+                                                                           Li, W, nullptr);
+          if (next && (e = look_ahead(p0, 0, p0 + kPanel)) != cudaSuccess) return e;
+          // the panel's columns into the rest of its outer block (at most
+          // kOuter - kPanel columns)
+          if constexpr (std::is_same<T, float>::value) {
+            const int64_t pi = p0 / kPanel;
+            const int nt = tc ? (int)L.itile_cnt[pi] : 0;
+            if (nt > 0)
+              tc_packed_kernel<<<(unsigned)std::min(nt, h->n_sm), kOuterThreads, kPkSmem, st>>>(
+                  bb, h->dev, front, p0, 0, h->d_pk, h->d_tiles + L.itile_off[pi], nt, h->d_err,
+                  next);
+          }
+          if (!tc && next)
+            update(p0, 0, rest, (unsigned)((kOuter - kPanel + BT - 1) / BT), kHeadTiles, 1);
+          if (next && (e = cudaStreamWaitEvent(st, h->join_ahead, 0)) != cudaSuccess) return e;
         }
         // the outer block into every column after it
         const int64_t rest = L.large_max_m - o0 - 1;
         if (rest <= 0) continue;
+        const bool next = o_end < L.large_max_k;
+        if (next && (e = look_ahead(o0, 1, o_end)) != cudaSuccess) return e;
         if constexpr (std::is_same<T, float>::value) {
-          if (tc) {
-            const int64_t ob = o0 / kOuter;
-            const int nt = (int)L.tile_cnt[ob];
-            if (nt > 0)
-              tc_packed_kernel<<<(unsigned)std::min(nt, h->n_sm), kOuterThreads, kPkSmem, st>>>(
-                  bb, h->dev, front, o0, 1, h->d_pk, h->d_tiles + L.tile_off[ob], nt, h->d_err);
-            continue;
-          }
+          const int64_t ob = o0 / kOuter;
+          const int nt = tc ? (int)L.tile_cnt[ob] : 0;
+          if (nt > 0)
+            tc_packed_kernel<<<(unsigned)std::min(nt, h->n_sm), kOuterThreads, kPkSmem, st>>>(
+                bb, h->dev, front, o0, 1, h->d_pk, h->d_tiles + L.tile_off[ob], nt, h->d_err, next);
         }
-        update(o0, 1, rest, ~0u);
+        if (!tc) update(o0, 1, rest, ~0u, next ? kHeadTiles : 0, next);
+        if (next && (e = cudaStreamWaitEvent(st, h->join_ahead, 0)) != cudaSuccess) return e;
       }
       // the solves' inverses on the side stream
       if (L.inv_cnt[0]) {
@@ -2809,6 +2884,8 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   LCK(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
   LCK(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
   LCK(cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming));
+  LCK(cudaStreamCreateWithFlags(&h->ahead, cudaStreamNonBlocking));
+  LCK(cudaEventCreateWithFlags(&h->join_ahead, cudaEventDisableTiming));
   LCK(dalloc(h, &h->d_xf, S.n));
   LCK(dalloc(h, &h->d_rhs, S.n));
   LCK(dalloc(h, &h->d_r, S.n));
@@ -3286,10 +3363,10 @@ int nla3d_ldlt_tc_check(int m, double* out) {
     const int64_t rest = m - kb;
     const unsigned t128 = (unsigned)((rest + 127) / 128);
     batched_trailing_kernel<float, 128, 8><<<dim3(t128, t128, 1), kThreads>>>(bb, d, F1, 0, 1,
-                                                                               dW);
+                                                                               dW, 0, 0);
     e = cudaMemcpy(dP, P.data(), mp * 4, cudaMemcpyHostToDevice);
     tc_packed_kernel<<<(unsigned)std::min<int>((int)tl.size(), n_sm), kOuterThreads, kPkSmem>>>(
-        bb, d, F3, 0, 1, dP, dT, (int)tl.size(), err);
+        bb, d, F3, 0, 1, dP, dT, (int)tl.size(), err, 0);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e == cudaSuccess) e = cudaMemcpy(&tc_err, err, 4, cudaMemcpyDeviceToHost);
@@ -3323,6 +3400,8 @@ int nla3d_ldlt_destroy(nla3d_ldlt* h) {
   if (h->fork) cudaEventDestroy(h->fork);
   if (h->join) cudaEventDestroy(h->join);
   if (h->side) cudaStreamDestroy(h->side);
+  if (h->join_ahead) cudaEventDestroy(h->join_ahead);
+  if (h->ahead) cudaStreamDestroy(h->ahead);
   for (void* p : h->allocs) cudaFree(p);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
   delete h;
