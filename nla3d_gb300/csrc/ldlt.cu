@@ -2130,43 +2130,50 @@ __global__ void __launch_bounds__(kThreads)
 // residual in the span (GCR; Eisenstat, Elman and Schultz, SIAM J. Numer.
 // Anal. 20, 1983).  Two launches of short vectors save one or two of the six to
 // nine applications of the factor.
-constexpr int kDirs = 8;                 // steps kept; the basis starts anew when it is full
+constexpr int kDirs = 30;                // steps kept (GMRES's restart); then GMRES takes over
+constexpr int kStalled = 6;              // steps without a better x before that
 constexpr int kDirSums = 2 * kDirs + 2;
+constexpr int kDirChunk = 8;             // directions per block of the sums
 constexpr int kDirBlocks = 152;
 
-// partial sums of <q, Q_i>, <r, Q_i> (i < k), <q, q> and <q, r>, q = Q_k
+// partial sums of <q, Q_i>, <r, Q_i> (i < k, kDirChunk a blockIdx.y), <q, q>
+// and <q, r>, q = Q_k
 __global__ void __launch_bounds__(kThreads)
     direction_sums_kernel(int64_t n, int k, const double* __restrict__ Q,
                           const double* __restrict__ r, double* __restrict__ part) {
-  __shared__ double red[kDirSums][kThreads];
-  double acc[kDirSums] = {};
+  constexpr int kSums = 2 * kDirChunk + 2;
+  __shared__ double red[kSums][kThreads];
+  const int i0 = blockIdx.y * kDirChunk, ni = min(k - i0, kDirChunk);
+  double acc[kSums] = {};
   const double* q = Q + (int64_t)k * n;
   for (int64_t j = blockIdx.x * (int64_t)kThreads + threadIdx.x; j < n;
        j += (int64_t)gridDim.x * kThreads) {
     const double qj = q[j], rj = r[j];
 #pragma unroll
-    for (int i = 0; i < kDirs; i++) {
-      if (i >= k) break;
-      const double v = Q[(int64_t)i * n + j];
+    for (int i = 0; i < kDirChunk; i++) {
+      if (i >= ni) break;
+      const double v = Q[(int64_t)(i0 + i) * n + j];
       acc[2 * i] = fma(qj, v, acc[2 * i]);
       acc[2 * i + 1] = fma(rj, v, acc[2 * i + 1]);
     }
-    acc[2 * kDirs] = fma(qj, qj, acc[2 * kDirs]);
-    acc[2 * kDirs + 1] = fma(qj, rj, acc[2 * kDirs + 1]);
+    if (i0 == 0) {
+      acc[2 * kDirChunk] = fma(qj, qj, acc[2 * kDirChunk]);
+      acc[2 * kDirChunk + 1] = fma(qj, rj, acc[2 * kDirChunk + 1]);
+    }
   }
   // (eight threads a sum, 32 entries each: fewer FP64 adds than shuffles)
 #pragma unroll
-  for (int t = 0; t < kDirSums; t++)
-    if (t < 2 * k || t >= 2 * kDirs) red[t][threadIdx.x] = acc[t];
+  for (int t = 0; t < kSums; t++) red[t][threadIdx.x] = acc[t];
   __syncthreads();
   const int t = threadIdx.x >> 3, h = threadIdx.x & 7;
-  if (t >= kDirSums) return;   // whole groups of eight lanes
+  const bool dir = t < 2 * ni, own = i0 == 0 && t >= 2 * kDirChunk && t < kSums;
+  if (!dir && !own) return;   // whole groups of eight lanes
   double v = 0.0;
-  if (t < 2 * k || t >= 2 * kDirs)
 #pragma unroll 8
-    for (int w = 0; w < kThreads / 8; w++) v += red[t][h + 8 * w];
+  for (int w = 0; w < kThreads / 8; w++) v += red[t][h + 8 * w];
   for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(__activemask(), v, o);
-  if (h == 0) part[blockIdx.x * kDirSums + t] = v;
+  if (h == 0)
+    part[blockIdx.x * kDirSums + (dir ? 2 * i0 + t : 2 * kDirs + t - 2 * kDirChunk)] = v;
 }
 
 // Q_k and Z_k orthonormalised from those sums, r's components along Q_0 .. Q_k
@@ -2177,14 +2184,15 @@ __global__ void __launch_bounds__(kThreads)
                           const double* __restrict__ part, double* __restrict__ rpart) {
   __shared__ double sum[kDirSums];
   __shared__ double red[kThreads / 32];
-  static_assert(kDirSums * 8 <= kThreads && kDirBlocks % 8 == 0, "eight threads a sum");
-  if (threadIdx.x < kDirSums * 8) {
-    const int t = threadIdx.x >> 3, h = threadIdx.x & 7;
+  static_assert(kDirSums * 4 <= kThreads && kDirBlocks % 4 == 0, "four threads a sum");
+  if (threadIdx.x < kDirSums * 4) {
+    const int t = threadIdx.x >> 2, h = threadIdx.x & 3;
+    const unsigned lanes = __activemask();   // whole groups of four
     double v = 0.0;
+    if (t < 2 * k || t >= 2 * kDirs)
 #pragma unroll
-    for (int b = 0; b < kDirBlocks / 8; b++) v += part[(8 * b + h) * kDirSums + t];
-    const unsigned lanes = __activemask();   // whole groups of eight
-    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(lanes, v, o);
+      for (int b = 0; b < kDirBlocks / 4; b++) v += part[(4 * b + h) * kDirSums + t];
+    for (int o = 2; o > 0; o >>= 1) v += __shfl_xor_sync(lanes, v, o);
     if (h == 0) sum[t] = v;
   }
   __syncthreads();
@@ -2201,9 +2209,8 @@ __global__ void __launch_bounds__(kThreads)
   for (int64_t j = blockIdx.x * (int64_t)kThreads + threadIdx.x; j < n;
        j += (int64_t)gridDim.x * kThreads) {
     double q = Q[(int64_t)k * n + j], z = Z[(int64_t)k * n + j], dr = 0.0, dx = 0.0;
-#pragma unroll
-    for (int i = 0; i < kDirs; i++) {
-      if (i >= k) break;
+#pragma unroll 4
+    for (int i = 0; i < k; i++) {
       const double qi = Q[(int64_t)i * n + j], zi = Z[(int64_t)i * n + j];
       q = fma(-sum[2 * i], qi, q);
       z = fma(-sum[2 * i], zi, z);
@@ -2296,7 +2303,7 @@ struct nla3d_ldlt {
   double* d_norm = nullptr;     // and their totals: r^2, b^2
   double* d_V = nullptr;        // GMRES basis, (kRestart + 1) x n, allocated on first use
   double* d_dot = nullptr;
-  double* d_dirs = nullptr;     // FP32 fronts: the refinement's Q and Z, kDirs x n each, or null
+  double* d_dirs = nullptr;     // FP32 fronts: the refinement's Q and Z, kDirs x n each, and its best x, or null
   double* d_dirsum = nullptr;   // and their partial sums
   double* d_maxabs = nullptr;
   double* d_maxpart = nullptr;
@@ -2896,7 +2903,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   if (precision) {
     LCK(dalloc(h, &h->d_dirsum, (size_t)kDirBlocks * kDirSums));
     // without the memory for them the refinement takes plain steps
-    if (rc == NLA3D_OK && dalloc(h, &h->d_dirs, (size_t)2 * kDirs * S.n) != cudaSuccess)
+    if (rc == NLA3D_OK && dalloc(h, &h->d_dirs, ((size_t)2 * kDirs + 1) * S.n) != cudaSuccess)
       cudaGetLastError();
   }
   LCK(dalloc(h, &h->d_maxabs, 1));
@@ -3082,7 +3089,8 @@ cudaError_t residual_norms(nla3d_ldlt* h, const double* values, const double* x,
 cudaError_t direction_step(nla3d_ldlt* h, int k, double* x, double* rnorm) {
   const int64_t n = h->S.n;
   double *Q = h->d_dirs, *Z = Q + (size_t)kDirs * n;
-  direction_sums_kernel<<<kDirBlocks, kThreads, 0, h->stream>>>(n, k, Q, h->d_r, h->d_dirsum);
+  direction_sums_kernel<<<dim3(kDirBlocks, (unsigned)std::max(1, (k + kDirChunk - 1) / kDirChunk)),
+                          kThreads, 0, h->stream>>>(n, k, Q, h->d_r, h->d_dirsum);
   direction_step_kernel<<<kDirBlocks, kThreads, 0, h->stream>>>(n, k, Q, Z, h->d_r, x, h->d_dirsum,
                                                                h->d_dot);
   if (!rnorm) return cudaGetLastError();
@@ -3105,6 +3113,8 @@ cudaError_t gmres_refine(nla3d_ldlt* h, const double* values, const double* b, d
   const int64_t n = S.n;
   cudaStream_t st = h->stream;
   cudaError_t e = cudaSuccess;
+  static_assert(2 * kDirs >= kRestart + 1, "the refinement's directions hold the basis");
+  if (!h->d_V && h->d_dirs) h->d_V = h->d_dirs;   // done with when this is called
   if (!h->d_V) {
     e = dalloc(h, &h->d_V, (size_t)(kRestart + 1) * n);
     if (e != cudaSuccess) return e;
@@ -3194,44 +3204,69 @@ int nla3d_ldlt_solve(nla3d_ldlt* h, const double* values, const double* b, doubl
   const size_t n = (size_t)h->S.n;
   if (e == cudaSuccess) e = residual_norms(h, values, x, b, &rnorm, &bnorm);
   if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve");
-  // refinement steps while they converge fast, accelerated (FP32 fronts) from
-  // the second on; GMRES with the same factor after, its preconditioner
-  // applied with FP64 products (FP32 fronts: the compensated FP32 products
-  // carry 2^-48 per operation, which a hard system's Krylov iteration can
-  // feel).  rel is that of b - A x computed afresh, except between a step's
-  // correction and the next step
+  // Refinement steps.  Plain ones (FP64 fronts) while they converge fast;
+  // accelerated ones (FP32 fronts) from the second on, until kDirs are kept,
+  // at any rate: they take the least residual over the Krylov space as GMRES
+  // does, but x from the steps themselves, so that an inexact factor costs
+  // rate and not accuracy, and one application a step instead of FP64 products
+  // and one more for x (a 454k-equation bar whose elimination grows: 22 steps in
+  // 117 ms, against 27 in 259).  Without a better x for kStalled of them the
+  // residual is at its floor or the factor no help.
+  // GMRES with the same factor after, its preconditioner applied with FP64
+  // products (FP32 fronts: the compensated FP32 products carry 2^-48 per
+  // operation, which a hard system's Krylov iteration can feel).  rel is that
+  // of b - A x computed afresh, except between a step's correction and the next.
   const double scale = bnorm > 0.0 ? bnorm : 1.0;
+  // the best x of accelerated steps: past the attainable residual their
+  // directions are rounding errors
+  double* best_x = h->d_dirs ? h->d_dirs + (size_t)2 * kDirs * n : nullptr;
+  double best = 0.0;
+  int stalled = 0;
+  auto restore = [&] {
+    if (dirs == 0 || !(rel > best)) return cudaSuccess;
+    rel = best;
+    return cudaMemcpyAsync(x, best_x, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->stream);
+  };
   for (;;) {
     rel = rnorm / scale;
-    if (!(rel > tol) || it >= max_refine) break;
+    if (!(rel > tol)) break;
+    if (dirs > 0) {
+      stalled = dirs == 1 || rel < 0.9 * best ? 0 : stalled + 1;
+      if (dirs == 1 || rel < best) {
+        best = rel;
+        e = cudaMemcpyAsync(best_x, x, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->stream);
+        if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve");
+      }
+    }
+    if (it >= max_refine) {
+      e = restore();
+      if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve");
+      break;
+    }
     if (dirs > 0) {
       // the norm after the correction is read only where it can matter
-      const bool read = !(rel < 0.1 * prev) || rel < 1e4 * tol;
+      const bool read = rel < 1e4 * tol;
       e = direction_step(h, dirs - 1, x, read ? &rnorm : nullptr);
       if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve");
-      if (read) rel = rnorm / scale;
-      if (!(rel > tol)) {
+      if (read && !(rnorm / scale > tol)) {
         e = residual_norms(h, values, x, b, &rnorm, &bnorm);
         if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve");
         rel = rnorm / scale;
         if (!(rel > tol)) break;
       }
     }
-    // A step that cut less, but whose rate reaches tol with one more, is still
-    // cheaper than GMRES, which takes two applications at least.  Accelerated
-    // steps may cut by as little as four: GMRES over the same Krylov space
-    // gains no more per application, and its own cost twice as much (a
-    // 454k-equation bar that once cut by 7: 8 steps in 43 ms against 9 in 81)
-    if (it > 0 && !(rel < (dirs > 0 ? 0.25 : 0.1) * prev) &&
-        !(rel < prev && rel * (rel / prev) <= tol)) {
+    // (a plain step that cut less, but whose rate reaches tol with one more, is
+    // still cheaper than GMRES, which takes two applications at least)
+    if (it > 0 && (dirs > 0 ? dirs == kDirs || stalled == kStalled
+                            : !(rel < 0.1 * prev) && !(rel < prev && rel * (rel / prev) <= tol))) {
       h->solve_accurate = 1;
-      e = gmres_refine(h, values, b, x, tol, max_refine, &it, &rel);
+      e = restore();
+      if (e == cudaSuccess) e = gmres_refine(h, values, b, x, tol, max_refine, &it, &rel);
       if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve (GMRES)");
       break;
     }
     prev = rel;
     // x += A^-1 r with the same factors
-    if (dirs == kDirs) dirs = 0;
     double* q = h->d_dirs ? h->d_dirs + (size_t)dirs * n : nullptr;
     e = enqueue_solve_any(h, h->d_r, x, 1, q ? q + (size_t)kDirs * n : nullptr);
     if (e == cudaSuccess) e = residual_norms(h, values, x, b, &rnorm, &bnorm, q);
