@@ -29,9 +29,9 @@
 // Solve (multifrontal, vectors): forward by levels with the same extend-add
 // on the update vectors, D^-1, backward by levels top-down gathering the
 // solved ancestor entries; FP64 refinement r = b - A x with A's
-// both-triangle CSR in the input numbering (plain steps, then GMRES
-// preconditioned by the factor).  Factorisation and solve are captured once
-// into CUDA graphs and replayed.
+// both-triangle CSR in the input numbering (accelerated steps with FP32
+// fronts, plain ones with FP64, then GMRES preconditioned by the factor).
+// Factorisation and solve are captured once into CUDA graphs and replayed.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -186,25 +186,48 @@ __device__ __forceinline__ T guard_pivot(T dv, T tau, int* perturbed) {
 
 // one block per front (m <= kSmallFront), the front held in shared memory
 // (column-major, leading dimension m+1): right-looking LDL^T of the k pivot
-// columns, the trailing (m-k)^2 block left as the update matrix.  Threads
-// cover the trailing triangle as 32 rows x 8 columns.
+// columns, the trailing (m-k)^2 block left as the update matrix.  A warp per
+// column, lane = row.  FP64: warp 0, which updates the next pivot's column
+// first, inverts that pivot for everyone (a division per column and pivot kept
+// the FP64 pipe busy longer than the update: 311 -> 89 us for a level of the
+// 12^3 block's 46 fronts); FP32 divides (111 -> 65 us for 93 of the 139k-equation
+// bar's, the columns loaded side by side).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
     factor_small_kernel(const int32_t* __restrict__ list, LdltDev d, T* __restrict__ front,
                         const double* __restrict__ tau_p, double pivot_rel, int* perturbed) {
+  constexpr bool kShare = std::is_same<T, double>::value;
   extern __shared__ unsigned char smem_raw[];
   T* S = reinterpret_cast<T*>(smem_raw);
+  __shared__ T winv[2];
   const int s = list[blockIdx.x];
   const int m = (int)(d.row_ptr[s + 1] - d.row_ptr[s]);
   const int k = d.sn_first[s + 1] - d.sn_first[s];
   const int ld = m + 1;
   T* F = front + d.front_off[s];
-  for (int c = 0; c < m; c++)
-    for (int r = c + threadIdx.x; r < m; r += blockDim.x) S[r + c * ld] = F[r + (int64_t)c * m];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  // the lower triangle, four columns a warp in flight
+  for (int c0 = ty; c0 < m; c0 += 32)
+    for (int r0 = c0 & ~31; r0 < m; r0 += 32) {
+      T v[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int c = c0 + 8 * u, r = r0 + tx;
+        v[u] = c < m && r >= c && r < m ? F[r + (int64_t)c * m] : T(0);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int c = c0 + 8 * u, r = r0 + tx;
+        if (c < m && r >= c && r < m) S[r + c * ld] = v[u];
+      }
+    }
   __syncthreads();
   // the pivot bound in the front's precision (the guards compare in it)
   const T tau = (T)(pivot_rel * tau_p[0]);
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  if (kShare) {
+    if (threadIdx.x == 0) winv[0] = T(1) / guard_value(S[0], tau);
+    __syncthreads();
+  }
   // one barrier per pivot: the columns right of p are updated with the
   // unscaled column p (A_ij -= w_i w_j / d), which no later step writes; the
   // pivot columns are scaled after the loop
@@ -212,11 +235,13 @@ __global__ void __launch_bounds__(kThreads)
     // every thread guards the pivot itself (thread 0 counts)
     const T raw = S[p + p * ld];
     const T dv = threadIdx.x == 0 ? guard_pivot(raw, tau, perturbed) : guard_value(raw, tau);
+    const T inv = kShare ? winv[p & 1] : T(0);
     const T* colp = S + p * ld;
     for (int j = p + 1 + ty; j < m; j += 8) {
-      const T lj = colp[j] / dv;
+      const T lj = kShare ? colp[j] * inv : colp[j] / dv;
       T* col = S + j * ld;
       for (int i = j + tx; i < m; i += 32) col[i] -= colp[i] * lj;
+      if (kShare && j == p + 1 && tx == 0) winv[j & 1] = T(1) / guard_value(col[j], tau);
     }
     __syncthreads();
   }
@@ -230,8 +255,100 @@ __global__ void __launch_bounds__(kThreads)
     if (tx == 0) colp[p] = dv;
   }
   __syncthreads();
-  for (int c = 0; c < m; c++)
-    for (int r = c + threadIdx.x; r < m; r += blockDim.x) F[r + (int64_t)c * m] = S[r + c * ld];
+  for (int c = ty; c < m; c += 8)
+    for (int r = (c & ~31) + tx; r < m; r += 32)
+      if (r >= c) F[r + (int64_t)c * m] = S[r + c * ld];
+}
+
+// Small fronts of up to kTinyPivots pivots and kTinyRows rows, a warp each:
+// lane = row (kU rows a lane), the pivot columns in registers, the trailing
+// columns updated where they lie, kC in flight; the same operations in the
+// same order as a block's.  Most are leaves of one pivot and some 25 rows, for
+// which a block waited for its columns one after the other, with shared memory
+// for the level's widest front: 1104 -> 80 us for the 42,511 of the
+// 454k-equation bar, 211 -> 28 for the 17,280 of the batch.  At 128 rows a warp
+// takes longer than a block (FP64: 122 us against 89).
+constexpr int kTinyPivots = 8;
+constexpr int kTinyRows = 64;   // the factorisation's limit: past it a block is faster
+
+template <typename T, int kU, int kC>
+__device__ __forceinline__ void factor_tiny(T* __restrict__ F, int m, int k, T tau,
+                                            int* perturbed) {
+  const int lane = threadIdx.x & 31;
+  T w[kTinyPivots][kU], l[kTinyPivots][kU];   // unscaled and scaled pivot columns
+#pragma unroll
+  for (int p = 0; p < kTinyPivots; p++)
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+      const int r = lane + 32 * u;
+      w[p][u] = p < k && r >= p && r < m ? F[r + (int64_t)p * m] : T(0);
+    }
+#pragma unroll
+  for (int p = 0; p < kTinyPivots; p++) {
+    if (p >= k) break;
+    const T raw = __shfl_sync(0xffffffffu, w[p][0], p);
+    const T dv = lane == 0 ? guard_pivot(raw, tau, perturbed) : guard_value(raw, tau);
+#pragma unroll
+    for (int u = 0; u < kU; u++) l[p][u] = w[p][u] / dv;
+#pragma unroll
+    for (int q = p + 1; q < kTinyPivots; q++) {
+      if (q >= k) break;
+      const T lq = __shfl_sync(0xffffffffu, l[p][0], q);
+#pragma unroll
+      for (int u = 0; u < kU; u++) w[q][u] -= w[p][u] * lq;
+    }
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+      const int r = lane + 32 * u;
+      if (r >= p && r < m) F[r + (int64_t)p * m] = r == p ? dv : l[p][u];
+    }
+  }
+#pragma unroll
+  for (int ub = 0; ub < kU; ub++)
+    for (int jj = ub == 0 ? k / kC * kC : 0; jj < 32 && 32 * ub + jj < m; jj += kC) {
+      T c[kC][kU];
+#pragma unroll
+      for (int v = 0; v < kC; v++)
+#pragma unroll
+        for (int u = ub; u < kU; u++) {
+          const int j = 32 * ub + jj + v, r = lane + 32 * u;
+          c[v][u] = j >= k && r >= j && r < m ? F[r + (int64_t)j * m] : T(0);
+        }
+#pragma unroll
+      for (int p = 0; p < kTinyPivots; p++) {
+        if (p >= k) break;
+#pragma unroll
+        for (int v = 0; v < kC; v++) {
+          const T lj = __shfl_sync(0xffffffffu, l[p][ub], jj + v);
+#pragma unroll
+          for (int u = ub; u < kU; u++) c[v][u] -= w[p][u] * lj;
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < kC; v++)
+#pragma unroll
+        for (int u = ub; u < kU; u++) {
+          const int j = 32 * ub + jj + v, r = lane + 32 * u;
+          if (j >= k && r >= j && r < m) F[r + (int64_t)j * m] = c[v][u];
+        }
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+    factor_tiny_kernel(const int32_t* __restrict__ list, int n, LdltDev d, T* __restrict__ front,
+                       const double* __restrict__ tau_p, double pivot_rel, int* perturbed) {
+  const int q = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  if (q >= n) return;   // warp-uniform; no block barrier follows
+  const int s = list[q];
+  const int m = (int)(d.row_ptr[s + 1] - d.row_ptr[s]);
+  const int k = d.sn_first[s + 1] - d.sn_first[s];
+  T* F = front + d.front_off[s];
+  const T tau = (T)(pivot_rel * tau_p[0]);
+  if (m <= 32)
+    factor_tiny<T, 1, 8>(F, m, k, tau, perturbed);
+  else
+    factor_tiny<T, kTinyRows / 32, 4>(F, m, k, tau, perturbed);
 }
 
 // Blocked path for the fronts above kSmallFront rows, batched: every launch
@@ -269,7 +386,7 @@ struct BigBatch {
 //
 // Against the block in shared memory, where each step's update ran as a chain
 // of dependent accesses and the inverse row by row as another: 54 -> 21 us
-// (FP32) and 136 -> 73 us (FP64) a launch.
+// (FP32; 25 with its own part of an update) and 136 -> 64 us (FP64) a launch.
 template <typename T>
 constexpr int kDiagLdOf = std::is_same<T, double>::value ? kPanel + 1 : kPanel + 4;
 
@@ -455,7 +572,7 @@ __global__ void __launch_bounds__(kThreads)
 // not stored) lies transposed in the front's upper triangle, X[i][j] at
 // row j of column i: it needs no memory, no kernel of the factorisation reads
 // there, and a row of X is contiguous.  kInv = 512: the joins of the
-// 139k-equation bar take 0.9 ms of kernels beside a 14 ms factorisation; a
+// 139k-equation bar take 0.9 ms of kernels beside an 11 ms factorisation; a
 // doubling more costs four times the work of all before it.
 struct InvTask {
   uint32_t z, j0;     // large front (index in the level's list), first pivot of the pair
@@ -1327,7 +1444,6 @@ __global__ void __launch_bounds__(kThreads)
 // small fronts are leaves of one pivot and some 25 rows (10,293 in the
 // 139k-equation bar), for which a CTA each spent its time being launched;
 // with more pivots the warp's chain of columns is longer than the CTA's.
-constexpr int kTinyPivots = 8;
 constexpr int kSmallRows = kSmallFront / 32;
 
 template <typename T>
@@ -2349,7 +2465,7 @@ struct nla3d_ldlt {
   // host schedule per level
   struct Level {
     int64_t all_off = 0, all_cnt = 0;     // every supernode of the level
-    int64_t small_off = 0, small_cnt = 0, tiny_cnt = 0;   // the tiny ones come first
+    int64_t small_off = 0, small_cnt = 0, tiny_cnt = 0, warp_cnt = 0;   // see the lists
     int32_t small_max_m = 0;
     int64_t large_off = 0, large_cnt = 0; // fronts above kSmallFront rows
     int64_t wo_off = 0;                   // their W offsets in d_wo
@@ -2427,10 +2543,16 @@ cudaError_t enqueue_factor(nla3d_ldlt* h, const double* values) {
       extend_add_kernel<T><<<(unsigned)((L.vec1 - L.vec0 + kCols - 1) / kCols), kThreads, 0, st>>>(
           L.vec0, L.vec1, h->d_gptr, h->d_gsrc, h->d_rsn, h->dev, front);
     }
-    if (L.small_cnt) {
+    if (L.warp_cnt)
+      factor_tiny_kernel<T>
+          <<<(unsigned)((L.warp_cnt + kThreads / 32 - 1) / (kThreads / 32)), kThreads, 0, st>>>(
+              h->d_lists + L.small_off, (int)L.warp_cnt, h->dev, front, h->d_maxabs, h->pivot_rel,
+              h->d_perturbed);
+    if (L.small_cnt > L.warp_cnt) {
       const size_t smem = sizeof(T) * (size_t)L.small_max_m * (L.small_max_m + 1);
-      factor_small_kernel<T><<<(unsigned)L.small_cnt, kThreads, smem, st>>>(
-          h->d_lists + L.small_off, h->dev, front, h->d_maxabs, h->pivot_rel, h->d_perturbed);
+      factor_small_kernel<T><<<(unsigned)(L.small_cnt - L.warp_cnt), kThreads, smem, st>>>(
+          h->d_lists + L.small_off + L.warp_cnt, h->dev, front, h->d_maxabs, h->pivot_rel,
+          h->d_perturbed);
     }
     if (L.large_cnt) {
       const BigBatch bb{h->d_lists + L.large_off, h->d_wo + L.wo_off, h->d_lio + L.wo_off,
@@ -2689,15 +2811,18 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
     for (int32_t q = S.level_ptr[L]; q < S.level_ptr[L + 1]; q++) lists.push_back(S.level_list[q]);
     lv.all_cnt = (int64_t)lists.size() - lv.all_off;
     lv.small_off = (int64_t)lists.size();
-    for (int tiny = 1; tiny >= 0; tiny--) {
+    // up to kTinyPivots pivots first, those of up to kTinyRows rows before the others
+    for (int part = 0; part < 3; part++) {
       for (int32_t q = S.level_ptr[L]; q < S.level_ptr[L + 1]; q++) {
         const int32_t s = S.level_list[q];
-        if (S.m(s) > kSmallFront || (S.k(s) <= kTinyPivots) != (tiny != 0)) continue;
+        const int of = S.k(s) > kTinyPivots ? 2 : S.m(s) > kTinyRows ? 1 : 0;
+        if (S.m(s) > kSmallFront || of != part) continue;
         lists.push_back(s);
-        lv.small_max_m = std::max(lv.small_max_m, S.m(s));
+        if (part) lv.small_max_m = std::max(lv.small_max_m, S.m(s));
       }
       lv.small_cnt = (int64_t)lists.size() - lv.small_off;
-      if (tiny) lv.tiny_cnt = lv.small_cnt;
+      if (part == 0) lv.warp_cnt = lv.small_cnt;
+      if (part == 1) lv.tiny_cnt = lv.small_cnt;
     }
     lv.large_off = (int64_t)lists.size();
     lv.wo_off = (int64_t)wo.size();
