@@ -56,7 +56,7 @@ DRAM_BYTES_PER_ELEM_GATHER_K = (301.560064e6 + 62.591488e6) / 64000
 # FP32 2 FFMA + FADD + FMUL and FP64 2 DFMA + DADD + DMUL per element.
 MIXED_FP32_FLOP_PER_ELEM = 67044
 MIXED_FP64_FLOP_PER_ELEM = 1800
-MIXED_WARP_INSTR_PER_ELEM = 2601
+MIXED_WARP_INSTR_PER_ELEM = 2625
 METRIC = "SOLID81 assembly Melem/s"  # Newton iterations per load step (plain vs learned) in "newton"
 MIXED_DTYPE = ("f32 K_uu / f64 volumetric terms (J, J-1, p/K, K_up, K_pp, F_p) / "
                "float-pair (2^-48) F_u chain / f64 CSR sums")
@@ -614,7 +614,7 @@ def run_ours(args):
                           "the FP64 pipe of its volumetric terms the busiest unit (ncu at "
                           "64,000 elements: FP64 pipe 65%, FP32 FMA 25%, issue 43%, LSU 17%, "
                           "shared wavefronts 18%, DRAM 9%)",
-                 "profile": "profiles/solid81_mixed_fp64vol_block40_ncu.md"}
+                 "profile": "profiles/solid81_mixed_block40_ncu.md"}
         sm.close()
 
     batched = None

@@ -120,7 +120,7 @@ __global__ void maxabs_final_kernel(int n, const double* __restrict__ part, doub
 // and written), dependent index loads the others.  A launch per child ordinal
 // with at most u / 32 blocks a child had too few loads in flight: 3.0 ms in
 // 100 launches of the 139k-equation bar's factor, now 1.2 in 16; 8.2 ms of the
-// 454k-equation bar's, now 4.4.  A block per column of the narrow levels, and
+// 457k-equation bar's, now 4.4.  A block per column of the narrow levels, and
 // two, three or eight loads a lane, measured the same or slower.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(kThreads)
 // same order as a block's.  Most are leaves of one pivot and some 25 rows, for
 // which a block waited for its columns one after the other, with shared memory
 // for the level's widest front: 1104 -> 80 us for the 42,511 of the
-// 454k-equation bar, 211 -> 28 for the 17,280 of the batch.  At 128 rows a warp
+// 457k-equation bar, 211 -> 28 for the 17,280 of the batch.  At 128 rows a warp
 // takes longer than a block (FP64: 122 us against 89).
 constexpr int kTinyPivots = 8;
 constexpr int kTinyRows = 64;   // the factorisation's limit: past it a block is faster
@@ -1659,7 +1659,7 @@ __global__ void __launch_bounds__(kThreads)
 // pivots, against 6 through X).  128: sound blocks measure 0.25 to 8 units, the
 // few with small pivots 2^5 to 2^17, of which those up to 2^7 changed the
 // residual by less than a tenth and those at 2^8 by half; two of some 1,000
-// blocks of the 454k-equation bar are above, one or two of 550 of the batch of
+// blocks of the 457k-equation bar are above, one or two of 550 of the batch of
 // 24 blocks.  The probe takes 0.1 ms of the 139k-equation bar's 11.6 ms factor.
 constexpr float kInvError = 128.0f;
 struct ProbeTask {
@@ -2239,7 +2239,7 @@ __global__ void __launch_bounds__(kThreads)
 //
 // A refinement step z = M^-1 r leaves r - A z, and after the first steps it
 // falls by the same factor every time (0.03 a step on the 139k-equation bar,
-// 0.08 on the 454k-equation one): a few modes of I - A M^-1 dominate it.  So
+// 0.08 on the 457k-equation one): a few modes of I - A M^-1 dominate it.  So
 // the steps z_i and q_i = A z_i, which the next residual gives for nothing (r
 // before it less r after it), are kept, q orthonormalised, and r's components
 // along them taken out: r -= q_i <q_i, r>, x += z_i <q_i, r>, the least
@@ -3334,7 +3334,7 @@ int nla3d_ldlt_solve(nla3d_ldlt* h, const double* values, const double* b, doubl
   // at any rate: they take the least residual over the Krylov space as GMRES
   // does, but x from the steps themselves, so that an inexact factor costs
   // rate and not accuracy, and one application a step instead of FP64 products
-  // and one more for x (a 454k-equation bar whose elimination grows: 22 steps in
+  // and one more for x (a 457k-equation bar whose elimination grows: 22 steps in
   // 117 ms, against 27 in 259).  Without a better x for kStalled of them the
   // residual is at its floor or the factor no help.
   // GMRES with the same factor after, its preconditioner applied with FP64
