@@ -3028,7 +3028,9 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   if (precision) {
     LCK(dalloc(h, &h->d_dirsum, (size_t)kDirBlocks * kDirSums));
     // without the memory for them the refinement takes plain steps
-    if (rc == NLA3D_OK && dalloc(h, &h->d_dirs, ((size_t)2 * kDirs + 1) * S.n) != cudaSuccess)
+    const double dirs = 8.0 * (2 * kDirs + 1) * (double)S.n;
+    if (rc == NLA3D_OK && need + dirs <= 0.9 * (double)free_b &&
+        dalloc(h, &h->d_dirs, ((size_t)2 * kDirs + 1) * S.n) != cudaSuccess)
       cudaGetLastError();
   }
   LCK(dalloc(h, &h->d_maxabs, 1));
