@@ -1912,6 +1912,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 #pragma unroll
     for (int u = 0; u < kInv / 32; u++) f[u] = lane + 32 * u < i ? Fi[lane + 32 * u] : T(0);
   }
+  const double vi = lane == 0 && i < ob ? v[i] : 0.0;
   for (int j = threadIdx.x; j < min(ob, r0 + kInvRows); j += kThreads) xs[j] = D::split(v[j]);
   __syncthreads();
   if (!(error <= kInvError)) {
@@ -1928,7 +1929,7 @@ __global__ void __launch_bounds__(kThreads, 4)
   a[2].merge(a[3]);
   a[0].merge(a[2]);
   for (int o = 16; o > 0; o >>= 1) a[0].shfl_down(o);
-  if (lane == 0) yv[d.vec_off[s] + o0 + i] = v[i] + a[0].value();
+  if (lane == 0) yv[d.vec_off[s] + o0 + i] = vi + a[0].value();
 }
 
 // the warps' partial sums per lane, merged in a fixed order by warp 0
@@ -1953,7 +1954,10 @@ __global__ void __launch_bounds__(32 * kWarps)
     fwd_rows_kernel(const int32_t* __restrict__ list, LdltDev d, const T* __restrict__ front,
                     int64_t o0, const double* __restrict__ yv, double* __restrict__ vec) {
   using X = typename D::X;
-  __shared__ X yb[kInv];
+  struct __align__(16) Pair {
+    X a, b;
+  };
+  __shared__ __align__(16) X yb[kInv];
   __shared__ D part[kWarps][32];
   const int s = list[blockIdx.y];
   const int64_t m = d.row_ptr[s + 1] - d.row_ptr[s];
@@ -1969,17 +1973,34 @@ __global__ void __launch_bounds__(32 * kWarps)
   const int rg = warp / groups, cb = (warp - rg * groups) * 32;
   const int64_t i = r0 + 32 * rg + lane;
   const int nc = rg < row_groups && i < m ? min(ob - cb, 32) : 0;   // this warp's columns
+  const bool full = rg < row_groups && ob - cb >= 32;   // the warp's columns are all there
   T f[32];
-  const T* Fi = front + d.front_off[s] + i + (o0 + cb) * m;
+  const T* Fi = front + d.front_off[s] + (i < m ? i : m - 1) + (o0 + cb) * m;
+  if (full) {
 #pragma unroll
-  for (int u = 0; u < 32; u++) f[u] = u < nc ? Fi[(int64_t)u * m] : T(0);
+    for (int u = 0; u < 32; u++) f[u] = Fi[(int64_t)u * m];
+  } else {
+#pragma unroll
+    for (int u = 0; u < 32; u++) f[u] = u < nc ? Fi[(int64_t)u * m] : T(0);
+  }
   for (int j = threadIdx.x; j < ob; j += 32 * kWarps)
     yb[j] = D::split(yv[d.vec_off[s] + o0 + j]);
+  const double vi = cb == 0 && nc > 0 ? v[i] : 0.0;
   __syncthreads();
   D a[4];
+  if (full) {
+    const Pair* yp = reinterpret_cast<const Pair*>(yb + cb);
 #pragma unroll
-  for (int u = 0; u < 32; u++)
-    if (u < nc) a[u & 3].add(f[u], yb[cb + u]);
+    for (int u = 0; u < 32; u += 2) {
+      const Pair y = yp[u / 2];
+      a[u & 3].add(f[u], y.a);
+      a[(u + 1) & 3].add(f[u + 1], y.b);
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < 32; u++)
+      if (u < nc) a[u & 3].add(f[u], yb[cb + u]);
+  }
   a[0].merge(a[1]);
   a[2].merge(a[3]);
   a[0].merge(a[2]);
@@ -1987,7 +2008,7 @@ __global__ void __launch_bounds__(32 * kWarps)
   __syncthreads();
   if (cb == 0 && nc > 0) {
     for (int w = 1; w < groups; w++) a[0].merge(part[warp + w][lane]);
-    v[i] -= a[0].value();
+    v[i] = vi - a[0].value();
   }
 }
 
@@ -2026,6 +2047,8 @@ __global__ void __launch_bounds__(kThreads)
   const T* Fc = front + d.front_off[s] + c * m;
   double* v = vec + d.vec_off[s];
   const X* xr = reinterpret_cast<const X*>(v);
+  const double yc = lane == 0 ? yv[d.vec_off[s] + c] : 0.0;
+  const double dc = lane == 0 ? (double)Fc[c] : 1.0;
   D acc[8];
   int64_t i = k + lane;
   for (; i + 7 * 32 < m; i += 8 * 32) {
@@ -2043,7 +2066,7 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
   for (int u = 1; u < 8; u++) acc[0].merge(acc[u]);
   for (int o = 16; o > 0; o >>= 1) acc[0].shfl_down(o);
-  if (lane == 0) v[c] = yv[d.vec_off[s] + c] / (double)Fc[c] - acc[0].value();
+  if (lane == 0) v[c] = yc / dc - acc[0].value();
 }
 
 // backward, wide fronts, block o0: x = X^T t, lane = pivot j (row i of X gives
@@ -2073,6 +2096,7 @@ __global__ void __launch_bounds__(kColThreads)
   for (int u = 0; u < kInv / 32; u++)
     f[u] = i0 + 32 * u < ob && i0 + 32 * u > j ? Fj[(int64_t)(32 * u) * m] : T(0);
   for (int i = j0 + threadIdx.x; i < ob; i += kColThreads) ts[i] = D::split(v[i]);
+  const double vj = threadIdx.x < 32 && j < ob ? v[j] : 0.0;
   __syncthreads();
   if (!(error <= kInvError)) {
     if (j0 == 0)
@@ -2085,7 +2109,7 @@ __global__ void __launch_bounds__(kColThreads)
     if (i0 + 32 * u < ob && i0 + 32 * u > j) a[u & 1].add(f[u], ts[i0 + 32 * u]);
   a[0].merge(a[1]);
   if (merge_warps<kColThreads / 32>(a[0], part) && j < ob)
-    xf[d.sn_first[s] + o0 + j] = v[j] + a[0].value();
+    xf[d.sn_first[s] + o0 + j] = vj + a[0].value();
 }
 
 // backward, wide fronts, block o0: t[j] -= sum_c L[o0+c][j] x_c for the pivots
@@ -2108,6 +2132,8 @@ __global__ void __launch_bounds__(kThreads)
   if (j >= o0) return;
   const int lane = threadIdx.x & 31;
   const T* Fj = front + d.front_off[s] + o0 + j * m;
+  double* vj = vec + d.vec_off[s] + j;
+  const double v0 = lane == 0 ? *vj : 0.0;
   D a[4];
   int c = lane;
   for (; c + 7 * 32 < ob; c += 8 * 32) {
@@ -2122,7 +2148,7 @@ __global__ void __launch_bounds__(kThreads)
   a[2].merge(a[3]);
   a[0].merge(a[2]);
   for (int o = 16; o > 0; o >>= 1) a[0].shfl_down(o);
-  if (lane == 0) vec[d.vec_off[s] + j] -= a[0].value();
+  if (lane == 0) *vj = v0 - a[0].value();
 }
 
 // x = xf in the input numbering, or x += xf; z: also the step itself
