@@ -2288,7 +2288,7 @@ __global__ void __launch_bounds__(kThreads)
 // Anal. 20, 1983).  Two launches of short vectors save one or two of the six to
 // nine applications of the factor.
 constexpr int kDirs = 30;                // steps kept (GMRES's restart); then GMRES takes over
-constexpr int kStalled = 6;              // steps without a better x before that
+constexpr int kStalled = 12;             // steps without a better x before that
 constexpr int kDirSums = 2 * kDirs + 2;
 constexpr int kDirChunk = 8;             // directions per block of the sums
 constexpr int kDirBlocks = 152;
