@@ -45,6 +45,13 @@ def test_layer_and_input_gradients(batch, n_out, n_in):
     assert np.abs(dX.cpu().numpy() - (d @ w) * (1 - x * x)).max() <= tol * scale
 
 
+@pytest.mark.parametrize("n_in", [1, 66])
+@pytest.mark.parametrize("batch", [8, 9, 127, 128, 129, 256, 300])
+def test_gradients_of_a_one_output_layer(batch, n_in):
+    """One output: the batch is contiguous along both indices of dY."""
+    test_layer_and_input_gradients(batch, 1, n_in)
+
+
 def test_adam_over_many_tensors_equals_one_at_a_time():
     torch = pytest.importorskip("torch")
     from nla3d_gb300 import _lib
