@@ -766,13 +766,15 @@ __global__ void __launch_bounds__(WPB * 32)
       for (int c = 0; c < 9; c++) sm[(kFRowCof + c) * kFRow + kFElem * q + sub] = cof[c];
       // J = det F / w > 0 as sqrt(det C) gives it; an inverted element (det F
       // <= 0) is flagged
-      const double dw = fabs(detF) - w;   // (J - 1) w
-      const double J = fma(dw, rw, 1.0);
+      const double dw = fabs(detF) - fabs(w);   // (J - 1) |w|
+      const double J = fma(dw, fabs(rw), 1.0);
       const bool bad = valid && !(J > 0.0 && isfinite(J) && detF > 0.0 && w > 0.0);
       const unsigned ballot = __ballot_sync(0xFFFFFFFFu, bad);
       if (sub == 0 && ((ballot >> (q * 8)) & 0xFFu)) flag_element(a.status, e + 1);
       Kpp_part = -inv_kb * w;
-      Fp_part = fma(-pc, Kpp_part, -dw);   // -(J - 1 - p / K) w
+      // -(J - 1 - p / K) w; a mirrored element (w < 0, flagged) keeps the
+      // reference's values, J = sqrt(det C) > 0 and w signed
+      Fp_part = fma(-pc, Kpp_part, signbit(w) ? dw : -dw);
       const double rc = inv_cbrt(J);
       const double pp = rc * rc;       // J^(-2/3)
       const double id = copysign(rw * (pp * rc), detF);   // 1 / det F = 1 / (J det dX/dxi)
@@ -2356,11 +2358,11 @@ __global__ void __launch_bounds__(kPlaneThreads) plane41_kernel(const Plane41Arg
 #pragma unroll
       for (int r = p; r < 2; r++) G[p + r] = Xi[0][p] * Xi[0][r] + Xi[1][p] * Xi[1][r];
     const double detF = gradient(xm, F);
-    const double dw = fabs(detF) - w;   // (J - 1) w
-    const double J = fma(dw, rw, 1.0);
+    const double dw = fabs(detF) - fabs(w);   // (J - 1) |w|, w < 0 in a mirrored element
+    const double J = fma(dw, fabs(rw), 1.0);
     if (!(J > 0.0 && isfinite(J))) bad = true;
     const double kw = inv_kb * w;
-    Fp += fma(-pc, kw, dw);
+    Fp += fma(-pc, kw, signbit(w) ? -dw : dw);
     Kpp -= kw;
     const double rc = inv_cbrt(J), pp = rc * rc, pppp = pp * pp;
     const double id = copysign(rw * (pp * rc), detF);
@@ -2404,7 +2406,7 @@ __global__ void __launch_bounds__(kPlaneThreads) plane41_kernel(const Plane41Arg
     const double wq = -0.25 * w;
     const double pk = wq * ko1, pb = wq * ko2, pv = wq * pJs;
     const double xk = -ww * k1, xb = -ww * k2, xv = 0.5 * ww * (pj - k1 * t13 - k2 * t23);
-    const double sg = detF < 0.0 ? -0.25 : 0.25;   // J C^-1 with J = |det F|
+    const double sg = signbit(detF) != signbit(w) ? -0.25 : 0.25;   // J C^-1 with J = |det F|
     const double chi[2] = {(g & 1) ? 1.0 : -1.0, (g & 2) ? 1.0 : -1.0};
     double X[2][2];
 #pragma unroll

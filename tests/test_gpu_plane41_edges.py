@@ -35,6 +35,23 @@ def test_distorted_plates_match_the_oracle(n, material):
         assert s.element_status() == (0, 0)
 
 
+@pytest.mark.parametrize("material", sorted(MATERIALS))
+def test_mirrored_plates_keep_the_reference_values(material):
+    """Elements numbered clockwise (det dX/dxi < 0) are flagged; K and F are
+    still the reference's, which takes J = sqrt(det C) and a negative weight."""
+    mat_id, c = MATERIALS[material]
+    m = mg.plane41_plate(7, 5, 0.5, mat_id, c, clamp_y0=True)
+    m.conn = np.ascontiguousarray(m.conn[:, [3, 2, 1, 0]])
+    u, p = mg.plane_state(m, 1.2, 0.1, 0.02, seed=3)
+    s, U, K, F = assemble_state(m, u, p, "fp64")
+    _, Uo, Ko, Fo = O.solve_state(m, u, p, "port")
+    for b in K:
+        if K[b].size:
+            assert np.abs(K[b] - Ko[b]).max() <= 1e-12 * np.abs(Ko[b]).max(), b
+    assert np.abs(F - Fo).max() <= 1e-12 * np.abs(Fo).max()
+    assert s.element_status() == (m.n_elems, 1)
+
+
 @pytest.mark.parametrize("n", [(5, 6, 1), (6, 6, 2), (9, 11, 2)])
 def test_products_with_rows_above_and_below_the_long_limit(n):
     """A rigid-body end: the master's rows in K(2) hold one entry per slave

@@ -87,3 +87,19 @@ def test_two_materials_in_one_warp():
                 assert np.abs(b.mesh_K(K, i, blk) - Ko[blk]).max() <= 1e-12 * np.abs(Ko[blk]).max()
         assert np.abs(b.mesh_F(F, i) - Fo).max() <= 1e-12 * np.abs(Fo).max()
     b.close()
+
+
+@pytest.mark.parametrize("material", sorted(MATERIALS))
+def test_mirrored_elements_keep_the_reference_values(material):
+    """Elements numbered left-handed (det dX/dxi < 0) are flagged; K and F are
+    still the reference's, which takes J = sqrt(det C) and a negative weight."""
+    m = _mesh((3, 2, 1), material, seed=6)
+    m.conn = np.ascontiguousarray(m.conn[:, [3, 2, 1, 0, 7, 6, 5, 4]])
+    u, p = mg.twist_state(m, angle_deg=20.0, stretch=1.2, noise_frac=0.02, seed=4)
+    s, U, K, F = assemble_state(m, u, p, "fp64")
+    _, Uo, Ko, Fo = O.solve_state(m, u, p, "port")
+    for b in K:
+        if K[b].size:
+            assert np.abs(K[b] - Ko[b]).max() <= 1e-12 * np.abs(Ko[b]).max(), b
+    assert np.abs(F - Fo).max() <= 1e-12 * np.abs(Fo).max()
+    assert s.element_status() == (m.n_elems, 1)
