@@ -3407,7 +3407,10 @@ int nla3d_ldlt_solve(nla3d_ldlt* h, const double* values, const double* b, doubl
       }
     }
     if (it >= max_refine) {
+      // the copy has ended when the call returns, as on every other way out:
+      // the caller may read x on a stream of its own
       e = restore();
+      if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
       if (e != cudaSuccess) return cuda_fail(h, e, "ldlt_solve");
       break;
     }

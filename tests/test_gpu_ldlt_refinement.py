@@ -49,3 +49,35 @@ def test_steps_reach_the_tolerance_and_stay_there(n, cond, fronts):
     got = x.cpu().numpy()
     s.close()
     assert np.linalg.norm(got - ref) <= bound * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("fronts", ["fp32", "fp32-tc"])
+def test_x_is_whole_when_the_steps_run_out(fronts):
+    """An unattainable tolerance and every budget up to the directions that are
+    kept: once the attainable residual is reached a last step is often worse than
+    an earlier one, and the best x comes back.  Read on another stream right after
+    the call, x must have the residual that the call reports: b - A x in FP64
+    here and there differ by the rounding of n products a row, each n 2^-53 |A| |x|."""
+    torch = pytest.importorskip("torch")
+    n = 300
+    a, io, co, b = _system(n, 1e5)
+    s = ldlt.DeviceLDLT(io, co, None, fronts)
+    v, bd = torch.from_numpy(a[np.triu_indices(n)]).cuda(), torch.from_numpy(b).cuda()
+    x = torch.empty_like(bd)
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    s.factor_device(v.data_ptr())
+    spent = 0
+    for steps in range(1, 31):
+        with torch.cuda.stream(other):
+            x.fill_(float("nan"))
+            other.synchronize()
+            s.solve_device(v.data_ptr(), bd.data_ptr(), x.data_ptr(), max_refine=steps, tol=0.0,
+                           strict=False)
+            got = x.clone().cpu().numpy()
+        rounding = n * 2.0 ** -53 * np.linalg.norm(np.abs(a) @ np.abs(got)) / np.linalg.norm(b)
+        res = np.linalg.norm(b - a @ got) / np.linalg.norm(b)
+        assert abs(res - s.last_residual) <= 2 * rounding, steps
+        spent += s.last_residual > 0.0 and s.last_steps == steps   # no other way out
+    s.close()
+    assert spent > 0
