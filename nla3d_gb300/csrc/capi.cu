@@ -6,7 +6,7 @@
 // pattern, K and F (each is one reference FEStorage); on the device they are
 // concatenated so that one launch of each kernel assembles all of them:
 //
-//   geo     10 x 8E  double  element geometry, structure of arrays (FP64; mixed
+//   geo     15 x 8E  double  element geometry, structure of arrays (FP64; mixed
 //                            contexts hold Gdf, dN/dX as 24 x 8E float pairs)
 //   wdet    8E       double  Gauss weight * det J
 //   conn    8E       uint32  node ids, global (mesh node offset added)

@@ -513,11 +513,14 @@ __device__ __forceinline__ void material_mixed(int mat_id, const float2* mcd, co
 //    s = 1/sqrt(3),
 //      dN_b/dxi_p (g) = 1/8 sum_{P not containing p} s^|P| phi_{P+p}(b) chi_P(g),
 //    phi_S(b), chi_S(g) = prod_{d in S} sigma_d (P, S subsets of the three
-//    coordinates).  The material works on covariant components: with F_ip =
-//    dx_i/dxi_p, the metric g^{pq} = (dxi_p/dX . dxi_q/dX) in the place of I,
-//    V = F^-T, FI = F g, b = FI F^T:
-//      I1 = FI : F,  C^-1 -> V^T V,  J = det F / det(dX/dxi),
-//      F A = FI - I1/3 V,  F B = I1 FI - b FI - 2 I2/3 V,
+//    coordinates).  The deformation gradient F = I + O itself is formed in the
+//    global axes, O_ij = du_i/dxi_p dxi_p/dX_j, and so are J = det F, b = F F^T
+//    and the invariants; only F and cof F then take xi components, FI_ip = F_ij
+//    dxi_p/dX_j and V_ip = (F^-T)_ij dxi_p/dX_j.  (With dx_i/dxi_p and FI = dx/dxi g
+//    the condition of dX/dxi entered twice: on an element sheared by 100 K_uu lost
+//    four digits and F_u at 1e-4 strain five, for 5% fewer FP64 instructions.)
+//    With the metric g^{pq} = (dxi_p/dX . dxi_q/dX) in the place of I:
+//      C^-1 -> V^T V,  F A = FI - I1/3 V,  F B = I1 FI - b FI - 2 I2/3 V,
 //      w F S = ko1 F A + ko2 F B + p J V,  w cof(F) dN/dX -> cof(F) dN/dxi,
 //    and the tangent tensor is a sum of products of those 3 x 3 matrices
 //      A[ip][kq] = V_ip X_kq + X_ip V_kq - sIIt/2 V_iq V_kp + k11 FA_ip FA_kq
@@ -580,11 +583,8 @@ __host__ __device__ constexpr int hex_corner(int mask) {
 }
 
 // The butterfly of an element's eight lanes from corner values to shape modes
-// (lane sub holds corner hex_corner(sub), then mode sub; not divided by 8),
-// and dx_i/dxi_p at the lane's Gauss point from the seven modes m (stride ld).
-// The geometry set-up and the element kernel share them, with every rounding
-// spelled out, so that an element at rest finds det F = w bit for bit and
-// det F - w loses nothing to a small strain.
+// (lane sub holds corner hex_corner(sub), then mode sub; not divided by 8), and
+// a field's gradient in xi at the lane's Gauss point from its seven modes m.
 __device__ __forceinline__ double corners_to_mode(double v, int sub) {
   v -= __shfl_sync(0xFFFFFFFFu, v, threadIdx.x & 24);
 #pragma unroll
@@ -715,33 +715,23 @@ __global__ void __launch_bounds__(WPB * 32)
     const uint32_t ec = valid ? e : E - 1;
     const uint64_t tg = (uint64_t)ec * 8 + sub;
 
-    // ---- modal positions, lane = (element, node), then mode ----
-    double xm[3];
-    bool moved = false;   // this mode's displacement is not exactly zero
-#pragma unroll
-    for (int i = 0; i < 3; i++) xm[i] = __ldg(a.geo + (7 + i) * E8 + tg);
+    // ---- modal displacements, lane = (element, node), then mode ----
+    double um[3] = {0.0, 0.0, 0.0};
     if (a.have_state) {
       const uint32_t nid = __ldg(a.conn + (uint64_t)ec * 8 + hex_corner(sub));
       const uint4 eq = __ldg(reinterpret_cast<const uint4*>(a.node_eq3) + (nid - 1));
       const double u[3] = {a.U_state[eq.x - 1], a.U_state[eq.y - 1], a.U_state[eq.z - 1]};
 #pragma unroll
-      for (int i = 0; i < 3; i++) {
-        const double um = corners_to_mode(u[i], sub);
-        moved |= um != 0.0;
-        xm[i] = fma(0.125, um, xm[i]);   // mode 0 (the translation) is not read
-      }
+      for (int i = 0; i < 3; i++) um[i] = 0.125 * corners_to_mode(u[i], sub);
     }
-    // an element at rest (or translated): F = I, so F A = F B = 0 and I1 = 3
-    // hold exactly, as the reference finds them (and J = 1, from det F = w);
-    // rounding would leave ~eps in their place and a residual that should
-    // vanish would not
-    const bool rest = ((__ballot_sync(0xFFFFFFFFu, moved) >> (8 * q)) & 0xFFu) == 0;
 #pragma unroll
-    for (int i = 0; i < 3; i++) sm[kFModes + 32 * i + lane] = xm[i];
-    const double w = __ldg(a.wdet + tg), rw = __ldg(a.geo + 6 * E8 + tg);
-    double g[6];
+    for (int i = 0; i < 3; i++) sm[kFModes + 32 * i + lane] = um[i];   // (mode 0 is not read)
+    const double w = __ldg(a.wdet + tg);
+    double Xi[9], g[6];   // dxi_p/dX_i at 3 i + p, and the metric
 #pragma unroll
-    for (int c = 0; c < 6; c++) g[c] = __ldg(a.geo + c * E8 + tg);
+    for (int c = 0; c < 9; c++) Xi[c] = __ldg(a.geo + c * E8 + tg);
+#pragma unroll
+    for (int c = 0; c < 6; c++) g[c] = __ldg(a.geo + (9 + c) * E8 + tg);
     const double pc = a.U_cur[a.p_eq[ec] - 1];
     const double ps = a.have_state ? a.U_state[a.p_eq[ec] - 1] : 0.0;
     int mat_id = a.mat_id;
@@ -760,43 +750,52 @@ __global__ void __launch_bounds__(WPB * 32)
     {
       double F[9], cof[9];
 #pragma unroll
-      for (int i = 0; i < 3; i++) mode_gradient(sm + kFModes + 32 * i + 8 * q, sg, F + 3 * i);
-      const double detF = cofactors(F, cof);
+      for (int i = 0; i < 3; i++) {
+        double du[3];   // du_i/dxi_p
+        mode_gradient(sm + kFModes + 32 * i + 8 * q, sg, du);
 #pragma unroll
-      for (int c = 0; c < 9; c++) sm[(kFRowCof + c) * kFRow + kFElem * q + sub] = cof[c];
-      // J = det F / w > 0 as sqrt(det C) gives it; an inverted element (det F
-      // <= 0) is flagged
-      const double dw = fabs(detF) - fabs(w);   // (J - 1) |w|
-      const double J = fma(dw, fabs(rw), 1.0);
+        for (int k = 0; k < 3; k++) {
+          const double O = fma(du[2], Xi[3 * k + 2], fma(du[1], Xi[3 * k + 1], du[0] * Xi[3 * k]));
+          F[3 * i + k] = i == k ? 1.0 + O : O;
+        }
+      }
+      const double detF = cofactors(F, cof);
+      // J as sqrt(det C) gives it; an inverted element (det F <= 0, or w <= 0:
+      // numbered left-handed) is flagged and keeps the reference's values
+      const double J = fabs(detF);
       const bool bad = valid && !(J > 0.0 && isfinite(J) && detF > 0.0 && w > 0.0);
       const unsigned ballot = __ballot_sync(0xFFFFFFFFu, bad);
       if (sub == 0 && ((ballot >> (q * 8)) & 0xFFu)) flag_element(a.status, e + 1);
       Kpp_part = -inv_kb * w;
-      // -(J - 1 - p / K) w; a mirrored element (w < 0, flagged) keeps the
-      // reference's values, J = sqrt(det C) > 0 and w signed
-      Fp_part = fma(-pc, Kpp_part, signbit(w) ? dw : -dw);
+      Fp_part = fma(1.0 - J, w, -pc * Kpp_part);   // -(J - 1 - p / K) w
       const double rc = inv_cbrt(J);
       const double pp = rc * rc;       // J^(-2/3)
-      const double id = copysign(rw * (pp * rc), detF);   // 1 / det F = 1 / (J det dX/dxi)
+      // 1 / det F, the cube's three roundings taken out (F A is a difference: it
+      // shows them at small strains)
+      const double id0 = pp * rc;
+      const double id = copysign(fma(id0, fma(-J, id0, 1.0), id0), detF);
+      // F and cof F in xi components.  At rest (or translated) F = I exactly, and
+      // so V = FI, I1 = 3 and F A = F B = 0, as the reference finds them
       double V[9], FI[9];
-#pragma unroll
-      for (int c = 0; c < 9; c++) V[c] = cof[c] * id;
 #pragma unroll
       for (int i = 0; i < 3; i++)
 #pragma unroll
-        for (int p = 0; p < 3; p++)
-          FI[3 * i + p] = F[3 * i] * g[sym3(0, p)] + F[3 * i + 1] * g[sym3(1, p)] +
-                          F[3 * i + 2] * g[sym3(2, p)];
-      double I1 = FI[0] * F[0];
+        for (int p = 0; p < 3; p++) {
+          FI[3 * i + p] = fma(F[3 * i + 2], Xi[6 + p], fma(F[3 * i + 1], Xi[3 + p], F[3 * i] * Xi[p]));
+          const double c = fma(cof[3 * i + 2], Xi[6 + p],
+                               fma(cof[3 * i + 1], Xi[3 + p], cof[3 * i] * Xi[p]));
+          V[3 * i + p] = c * id;
+          sm[(kFRowCof + 3 * i + p) * kFRow + kFElem * q + sub] = w * c;
+        }
+      double I1 = F[0] * F[0];
 #pragma unroll
-      for (int c = 1; c < 9; c++) I1 = fma(FI[c], F[c], I1);
-      if (rest) I1 = 3.0;
+      for (int c = 1; c < 9; c++) I1 = fma(F[c], F[c], I1);
       const double t13 = (1.0 / 3.0) * I1;
       const double pj = pc * J, pJs = ps * J;
       const double w64 = w * 0.015625;   // the two factors 1/8 of dN/dxi
       double FA[9];
 #pragma unroll
-      for (int c = 0; c < 9; c++) FA[c] = rest ? 0.0 : fma(-t13, V[c], FI[c]);
+      for (int c = 0; c < 9; c++) FA[c] = fma(-t13, V[c], FI[c]);
       double CI[6];
 #pragma unroll
       for (int p = 0; p < 3; p++)
@@ -859,8 +858,8 @@ __global__ void __launch_bounds__(WPB * 32)
         for (int i = 0; i < 3; i++)
 #pragma unroll
           for (int k = i; k < 3; k++)
-            b[sym3(i, k)] = FI[3 * i] * F[3 * k] + FI[3 * i + 1] * F[3 * k + 1] +
-                            FI[3 * i + 2] * F[3 * k + 2];
+            b[sym3(i, k)] = F[3 * i] * F[3 * k] + F[3 * i + 1] * F[3 * k + 1] +
+                            F[3 * i + 2] * F[3 * k + 2];
         const double I2 = b[0] * b[3] + b[3] * b[5] + b[0] * b[5] - b[1] * b[1] - b[4] * b[4] -
                           b[2] * b[2];
         const double t23 = (2.0 / 3.0) * I2;
@@ -892,7 +891,7 @@ __global__ void __launch_bounds__(WPB * 32)
           const int i = c / 3, p = c % 3;
           const double fc = b[sym3(i, 0)] * FI[p] + b[sym3(i, 1)] * FI[3 + p] +
                             b[sym3(i, 2)] * FI[6 + p];
-          const double FB = rest ? 0.0 : fma(-t23, V[c], fma(I1, FI[c], -fc));
+          const double FB = fma(-t23, V[c], fma(I1, FI[c], -fc));
           sm[(kFRowP + c) * kFRow + kFElem * q + sub] = fma(pk, FA[c], fma(pb, FB, pv * V[c]));
           X[c] = fma(xk, FA[c], fma(xb, FB, xv * V[c]));
           hV[c] = h * V[c];
@@ -1430,37 +1429,51 @@ __global__ void __launch_bounds__(WPB * 32)
   }
 }
 
-// The FP64 kernel's element geometry, lane = (element, corner / mode / Gauss
-// point): shape modes of the positions (relative to node 0: no digits lost to
-// the element's distance from the origin), and at the Gauss point w = det
-// dX/dxi, 1 / w and the metric dxi_p/dX . dxi_q/dX.
+// The FP64 kernel's element geometry, one thread per Gauss point: the shape
+// modes of the positions, and from them w = det dX/dxi, dxi_p/dX_i and the metric
+// dxi_p/dX . dxi_q/dX.  The modes start from the differences along the edges: no
+// digits are lost to the element's distance from the origin, nor a thin element's
+// thickness to its length.
 __global__ void __launch_bounds__(256) solid81_geometry_kernel(const JacobianArgs a) {
   if (a.skip && *a.skip) return;
-  __shared__ double modes[3][256];
   const uint64_t E8 = (uint64_t)a.n_elems * 8;
-  const uint64_t t0 = (uint64_t)blockIdx.x * 256 + threadIdx.x;
-  const bool valid = t0 < E8;
-  const uint64_t t = valid ? t0 : E8 - 8 + (t0 & 7);   // whole elements per eight lanes
+  const uint64_t t = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+  if (t >= E8) return;
   const int sub = threadIdx.x & 7;
-  const uint32_t nid = a.conn[(t & ~7ull) + hex_corner(sub)];
-  for (int i = 0; i < 3; i++)
-    modes[i][threadIdx.x] = 0.125 * corners_to_mode(a.xyz[(uint64_t)(nid - 1) * 3 + i], sub);
-  __syncwarp();
+  const uint32_t* cn = a.conn + (t & ~7ull);
   const GaussSigns sg = gauss_signs(sub);
   double F[9], cof[9];
-  for (int i = 0; i < 3; i++) mode_gradient(&modes[i][threadIdx.x & ~7], sg, F + 3 * i);
+  for (int i = 0; i < 3; i++) {
+    double x[8], m[8], ex[4], ey[4], ez[4];   // corners by mask
+    for (int b = 0; b < 8; b++) x[b] = a.xyz[(uint64_t)(cn[hex_corner(b)] - 1) * 3 + i];
+    for (int k = 0; k < 4; k++) {
+      const int y0 = (k & 1) | (k & 2) << 1;
+      ex[k] = x[2 * k + 1] - x[2 * k];
+      ey[k] = x[y0 + 2] - x[y0];
+      ez[k] = x[k + 4] - x[k];
+    }
+    m[1] = (ex[0] + ex[1]) + (ex[2] + ex[3]);
+    m[2] = (ey[0] + ey[1]) + (ey[2] + ey[3]);
+    m[4] = (ez[0] + ez[1]) + (ez[2] + ez[3]);
+    m[3] = (ex[1] - ex[0]) + (ex[3] - ex[2]);
+    m[5] = (ex[2] - ex[0]) + (ex[3] - ex[1]);
+    m[6] = (ey[2] - ey[0]) + (ey[3] - ey[1]);
+    m[7] = (ex[3] - ex[2]) - (ex[1] - ex[0]);
+    for (int b = 1; b < 8; b++) m[b] *= 0.125;
+    mode_gradient(m, sg, F + 3 * i);
+  }
   const double det = cofactors(F, cof);
-  if (!valid) return;
   const double r = 1.0 / det;
+  for (int c = 0; c < 9; c++) {
+    cof[c] *= r;   // dxi_p/dX_i
+    a.geo[c * E8 + t] = cof[c];
+  }
   for (int p = 0; p < 3; p++)
     for (int s = p; s < 3; s++) {
-      // dxi_p/dX_i = cof_ip / det
       double v = 0.0;
-      for (int i = 0; i < 3; i++) v += (cof[3 * i + p] * r) * (cof[3 * i + s] * r);
-      a.geo[sym3(p, s) * E8 + t] = v;
+      for (int i = 0; i < 3; i++) v += cof[3 * i + p] * cof[3 * i + s];
+      a.geo[(9 + sym3(p, s)) * E8 + t] = v;
     }
-  a.geo[6 * E8 + t] = r;
-  for (int i = 0; i < 3; i++) a.geo[(7 + i) * E8 + t] = sub ? modes[i][threadIdx.x] : 0.0;
   a.wdet[t] = det;
   // isoparametric.cpp:177 logs det < 1e-20; here it is an element status
   if (!(det >= 1.0e-20) && sub == 0) flag_element(a.status, (uint32_t)(t >> 3) + 1);

@@ -7,7 +7,7 @@
 namespace nla3d_gpu {
 
 constexpr int kSolidKc = 325;  // SOLID81 K contributions per element (300 Kuu + 24 Kup + 1 Kpp)
-constexpr int kSolidGeo = 10;  // FP64 geometry values per Gauss point
+constexpr int kSolidGeo = 15;  // FP64 geometry values per Gauss point
 constexpr int kSolidFc = 25;   // SOLID81 F contributions per element (24 Fu + 1 Fp)
 
 struct ElementStatus {
@@ -20,9 +20,9 @@ struct ElementStatus {
 
 struct Solid81Args {
   uint32_t n_elems;
-  // FP64: element geometry, structure of arrays geo[c * E8 + e*8 + g]: c = 0..5
-  // the metric dxi_p/dX . dxi_q/dX (11 12 13 22 23 33) and 6 the inverse det
-  // dX/dxi at Gauss point g, 7..9 the x, y, z coefficient of shape mode g
+  // FP64: element geometry, structure of arrays geo[c * E8 + e*8 + g] at Gauss
+  // point g: c = 0..8 dxi_p/dX_i (3 i + p), 9..14 the metric dxi_p/dX . dxi_q/dX
+  // (11 12 13 22 23 33)
   const double* geo;
   const double* wdet;       // Gauss weight * det J, [e*8 + g]
   const uint32_t* conn;     // 8 node ids per element, 1-based

@@ -46,7 +46,7 @@ using namespace nla3d_gpu;
 namespace {
 
 constexpr uint64_t kScratchDoubles = NLA3D_NOALLOC_SCRATCH_BYTES / sizeof(double);
-// per element: geometry (10 x 8) + w det J (8) + K contributions (325) + F contributions (25)
+// per element: geometry (15 x 8) + w det J (8) + K contributions (325) + F contributions (25)
 constexpr uint64_t kDoublesPerElem = kSolidGeo * 8 + 8 + kSolidKc + kSolidFc;
 static_assert(NLA3D_NOALLOC_MAX_ELEMS * kDoublesPerElem <= kScratchDoubles,
               "NLA3D_NOALLOC_MAX_ELEMS does not fit the scratch array");

@@ -103,3 +103,29 @@ def test_mirrored_elements_keep_the_reference_values(material):
             assert np.abs(K[b] - Ko[b]).max() <= 1e-12 * np.abs(Ko[b]).max(), b
     assert np.abs(F - Fo).max() <= 1e-12 * np.abs(Fo).max()
     assert s.element_status() == (m.n_elems, 1)
+
+
+def _stretched(name, rng):
+    """A linear map of the mesh and a displacement gradient."""
+    small = 1e-4 * rng.uniform(-1, 1, (3, 3))
+    if name == "sheared by 100":
+        return np.array([[1.0, 100.0, 0.0], [0.0, 1.0, 0.0], [0.0, 0.0, 1.0]]), small
+    q1, _ = np.linalg.qr(rng.standard_normal((3, 3)))
+    q2, _ = np.linalg.qr(rng.standard_normal((3, 3)))
+    a = q1 @ np.diag([1.0, 0.05, 0.001]) @ q2
+    return a * np.sign(np.linalg.det(a)), small
+
+
+@pytest.mark.parametrize("name", ["sheared by 100", "thin, oblique"])
+@pytest.mark.parametrize("material", sorted(MATERIALS))
+def test_badly_shaped_elements_match_the_oracle(material, name):
+    """Elements whose dX/dxi is badly conditioned, at small strains: F is as well
+    conditioned as ever, so K and F stay within the parity bound (the oracle itself
+    is within 1e-14 of extended precision here)."""
+    mat_id, c = MATERIALS[material]
+    m = mg.solid81_block(3, 2, 2, 0.25, mat_id, c, clamp_z0=False)
+    rng = np.random.default_rng(8)
+    m.xyz = m.xyz + rng.uniform(-0.005, 0.005, m.xyz.shape)
+    a, grad = _stretched(name, rng)
+    m.xyz = np.ascontiguousarray(m.xyz @ a.T)
+    _check(m, m.xyz @ grad.T, rng.normal(0.0, 0.1, m.n_elems))
