@@ -2313,9 +2313,8 @@ __global__ void __launch_bounds__(kPlaneThreads) plane41_kernel(const Plane41Arg
     mc = mm + 1;
     kbulk = mm[6];
   }
-  // positions and displacements relative to node 0, as modes
-  Mode2 Xm[2], xm[2];
-  bool rest = true;
+  // positions and displacements as modes
+  Mode2 Xm[2], um[2];
   {
     double X[2][4], u[2][4] = {};
 #pragma unroll
@@ -2329,15 +2328,9 @@ __global__ void __launch_bounds__(kPlaneThreads) plane41_kernel(const Plane41Arg
     }
 #pragma unroll
     for (int i = 0; i < 2; i++) {
-#pragma unroll
-      for (int b = 3; b >= 0; b--) {
-        X[i][b] -= X[i][0];
-        u[i][b] -= u[i][0];
-      }
       const Mode2 M = corners_to_modes2(X[i]), d = corners_to_modes2(u[i]);
       Xm[i] = {0.25 * M.x, 0.25 * M.y, 0.25 * M.xy};
-      rest = rest && d.x == 0.0 && d.y == 0.0 && d.xy == 0.0;
-      xm[i] = {fma(0.25, d.x, Xm[i].x), fma(0.25, d.y, Xm[i].y), fma(0.25, d.xy, Xm[i].xy)};
+      um[i] = {0.25 * d.x, 0.25 * d.y, 0.25 * d.xy};
     }
   }
   // sums over the Gauss points of chi_S A[ip][kq]: S = 0, 1 (xi), 2 (eta), 3.
@@ -2357,10 +2350,10 @@ __global__ void __launch_bounds__(kPlaneThreads) plane41_kernel(const Plane41Arg
         F[i][0] = fma(sy, m[i].xy, m[i].x);
         F[i][1] = fma(sx, m[i].xy, m[i].y);
       }
-      return minor2(F[0][0], F[1][1], F[0][1], F[1][0]);
     };
-    double Xg[2][2], F[2][2];
-    const double w = gradient(Xm, Xg);
+    double Xg[2][2], du[2][2], F[2][2];
+    gradient(Xm, Xg);
+    const double w = minor2(Xg[0][0], Xg[1][1], Xg[0][1], Xg[1][0]);
     if (!(w >= 1.0e-20)) bad = true;
     const double rw = 1.0 / w;
     // dxi_p/dX_i, and the metric
@@ -2370,31 +2363,44 @@ __global__ void __launch_bounds__(kPlaneThreads) plane41_kernel(const Plane41Arg
     for (int p = 0; p < 2; p++)
 #pragma unroll
       for (int r = p; r < 2; r++) G[p + r] = Xi[0][p] * Xi[0][r] + Xi[1][p] * Xi[1][r];
-    const double detF = gradient(xm, F);
-    const double dw = fabs(detF) - fabs(w);   // (J - 1) |w|, w < 0 in a mirrored element
-    const double J = fma(dw, fabs(rw), 1.0);
+    // F = I + O in the global axes (at rest exactly I)
+    gradient(um, du);
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const double O = fma(du[i][1], Xi[k][1], du[i][0] * Xi[k][0]);
+        F[i][k] = i == k ? 1.0 + O : O;
+      }
+    const double detF = minor2(F[0][0], F[1][1], F[0][1], F[1][0]);
+    const double J = fabs(detF);
     if (!(J > 0.0 && isfinite(J))) bad = true;
     const double kw = inv_kb * w;
-    Fp += fma(-pc, kw, signbit(w) ? -dw : dw);
+    Fp += fma(J - 1.0, w, -pc * kw);
     Kpp -= kw;
     const double rc = inv_cbrt(J), pp = rc * rc, pppp = pp * pp;
-    const double id = copysign(rw * (pp * rc), detF);
-    const double cof[2][2] = {{F[1][1], -F[1][0]}, {-F[0][1], F[0][0]}};
-    double V[2][2], FI[2][2], FA[2][2];
+    const double id0 = pp * rc;
+    const double id = copysign(fma(id0, fma(-J, id0, 1.0), id0), detF);   // 1 / det F
+    // w cof F with the sign of J C^-1 (J = |det F|), a quarter of dN/dxi's factor
+    const double ws = signbit(detF) ? -0.25 * w : 0.25 * w;
+    double cof[2][2], V[2][2], FI[2][2], FA[2][2];
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
+    for (int i = 0; i < 2; i++)
 #pragma unroll
       for (int p = 0; p < 2; p++) {
-        V[i][p] = cof[i][p] * id;
-        FI[i][p] = F[i][0] * G[p] + F[i][1] * G[1 + p];
+        // cof F = (F11 -F10; -F01 F00) by rows
+        const double c = i == 0 ? fma(-F[1][0], Xi[1][p], F[1][1] * Xi[0][p])
+                                : fma(F[0][0], Xi[1][p], -F[0][1] * Xi[0][p]);
+        cof[i][p] = ws * c;
+        V[i][p] = c * id;
+        FI[i][p] = fma(F[i][1], Xi[1][p], F[i][0] * Xi[0][p]);
       }
-    }
-    const double b00 = FI[0][0] * F[0][0] + FI[0][1] * F[0][1];
-    const double b01 = FI[0][0] * F[1][0] + FI[0][1] * F[1][1];
-    const double b11 = FI[1][0] * F[1][0] + FI[1][1] * F[1][1];
+    const double b00 = F[0][0] * F[0][0] + F[0][1] * F[0][1];
+    const double b01 = F[0][0] * F[1][0] + F[0][1] * F[1][1];
+    const double b11 = F[1][0] * F[1][0] + F[1][1] * F[1][1];
     const double tr = b00 + b11;
-    const double I1 = rest ? 3.0 : tr + 1.0;
-    const double I2 = rest ? 3.0 : fma(b00, b11, fma(-b01, b01, tr));
+    const double I1 = tr + 1.0;
+    const double I2 = fma(b00, b11, fma(-b01, b01, tr));
     const double t13 = (1.0 / 3.0) * I1, t23 = (2.0 / 3.0) * I2;
     // W derivatives at (I1 J^-2/3, I2 J^-4/3) (materials_hyperelastic.cpp:135-204)
     double a1, a2 = 0.0, a11 = 0.0;
@@ -2419,22 +2425,21 @@ __global__ void __launch_bounds__(kPlaneThreads) plane41_kernel(const Plane41Arg
     const double wq = -0.25 * w;
     const double pk = wq * ko1, pb = wq * ko2, pv = wq * pJs;
     const double xk = -ww * k1, xb = -ww * k2, xv = 0.5 * ww * (pj - k1 * t13 - k2 * t23);
-    const double sg = signbit(detF) != signbit(w) ? -0.25 : 0.25;   // J C^-1 with J = |det F|
     const double chi[2] = {(g & 1) ? 1.0 : -1.0, (g & 2) ? 1.0 : -1.0};
     double X[2][2];
 #pragma unroll
     for (int i = 0; i < 2; i++)
 #pragma unroll
       for (int p = 0; p < 2; p++) {
-        FA[i][p] = rest ? 0.0 : fma(-t13, V[i][p], FI[i][p]);
+        FA[i][p] = fma(-t13, V[i][p], FI[i][p]);
         const double fc = i == 0 ? b00 * FI[0][p] + b01 * FI[1][p] : b01 * FI[0][p] + b11 * FI[1][p];
-        const double FB = rest ? 0.0 : fma(-t23, V[i][p], fma(I1, FI[i][p], -fc));
+        const double FB = fma(-t23, V[i][p], fma(I1, FI[i][p], -fc));
         const double P = fma(pk, FA[i][p], fma(pb, FB, pv * V[i][p]));
         X[i][p] = fma(xk, FA[i][p], fma(xb, FB, xv * V[i][p]));
         Pw[i][p][0] += P;
         Pw[i][p][1] = fma(chi[1 - p], P, Pw[i][p][1]);
-        Cw[i][p][0] = fma(sg, cof[i][p], Cw[i][p][0]);
-        Cw[i][p][1] = fma(chi[1 - p] * sg, cof[i][p], Cw[i][p][1]);
+        Cw[i][p][0] += cof[i][p];
+        Cw[i][p][1] = fma(chi[1 - p], cof[i][p], Cw[i][p][1]);
       }
     // S^{pq} = (ko1 + ko2 I1) g - ko2 C^{pq} + (p J - ko1 I1/3 - ko2 2 I2/3) C^-1
     const double eg = ww * (ko1 + ko2 * I1), ecc = -ww * ko2;

@@ -52,6 +52,34 @@ def test_mirrored_plates_keep_the_reference_values(material):
     assert s.element_status() == (m.n_elems, 1)
 
 
+@pytest.mark.parametrize("name", ["sheared by 100", "thin, oblique"])
+@pytest.mark.parametrize("material", sorted(MATERIALS))
+def test_badly_shaped_plates_match_the_oracle(material, name):
+    """Elements whose dX/dxi is badly conditioned, at small strains: F is as well
+    conditioned as ever, so K and F stay within the parity bound (the oracle itself
+    is within 1e-14 of extended precision here)."""
+    mat_id, c = MATERIALS[material]
+    m = mg.plane41_plate(7, 5, 0.25, mat_id, c, clamp_y0=False)
+    rng = np.random.default_rng(8)
+    m.xyz[:, :2] += rng.uniform(-0.005, 0.005, (m.n_nodes, 2))
+    a = np.array([[1.0, 100.0], [0.0, 1.0]])
+    if name == "thin, oblique":
+        t, s = np.array([0.7, 1.9])
+        a = np.array([[np.cos(t), -np.sin(t)], [np.sin(t), np.cos(t)]]) @ np.diag([1.0, 0.001]) \
+            @ np.array([[np.cos(s), -np.sin(s)], [np.sin(s), np.cos(s)]])
+    m.xyz[:, :2] = m.xyz[:, :2] @ a.T
+    u = np.zeros((m.n_nodes, 3))
+    u[:, :2] = m.xyz[:, :2] @ (1e-4 * rng.uniform(-1, 1, (2, 2))).T
+    p = rng.normal(0.0, 0.1, m.n_elems)
+    s, U, K, F = assemble_state(m, u, p, "fp64")
+    _, Uo, Ko, Fo = O.solve_state(m, u, p, "port")
+    for b in K:
+        if K[b].size:
+            assert np.abs(K[b] - Ko[b]).max() <= 1e-12 * np.abs(Ko[b]).max(), b
+    assert np.abs(F - Fo).max() <= 1e-12 * np.abs(Fo).max()
+    assert s.element_status() == (0, 0)
+
+
 @pytest.mark.parametrize("n", [(5, 6, 1), (6, 6, 2), (9, 11, 2)])
 def test_products_with_rows_above_and_below_the_long_limit(n):
     """A rigid-body end: the master's rows in K(2) hold one entry per slave
