@@ -2844,7 +2844,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   std::vector<uint64_t> wo, lio, pko;
   std::vector<OuterTile> tiles;
   int64_t max_w = 0, max_large_cnt = 0, max_pk = 0;
-  uint64_t li_total = 0;
+  uint64_t max_li = 0;
   h->levels.resize(nlev);
   for (int L = 0; L < nlev; L++) {
     auto& lv = h->levels[L];
@@ -2868,6 +2868,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
     lv.large_off = (int64_t)lists.size();
     lv.wo_off = (int64_t)wo.size();
     int64_t w = 0, pk = 0;
+    uint64_t li = 0;
     for (int32_t q = S.level_ptr[L]; q < S.level_ptr[L + 1]; q++) {
       const int32_t s = S.level_list[q];
       if (S.m(s) > kSmallFront) {
@@ -2875,10 +2876,10 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
         wo.push_back((uint64_t)w);
         w += (int64_t)S.m(s) *
              std::min<int64_t>(kOuter, ((int64_t)S.k(s) + kPanel - 1) / kPanel * kPanel);
-        lio.push_back(li_total);
+        lio.push_back(li);
         pko.push_back((uint64_t)pk);
         pk += ((int64_t)S.m(s) + kTcM - 1) / kTcM * (int64_t)kPkBlock;
-        li_total += (uint64_t)((S.k(s) + kPanel - 1) / kPanel) * kPanel * kPanel;
+        li += (uint64_t)((S.k(s) + kPanel - 1) / kPanel) * kPanel * kPanel;
         lv.large_max_m = std::max<int64_t>(lv.large_max_m, S.m(s));
         lv.large_max_k = std::max<int64_t>(lv.large_max_k, S.k(s));
       }
@@ -2978,6 +2979,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
       }
     }
     max_w = std::max(max_w, w);
+    max_li = std::max(max_li, li);
     max_pk = std::max(max_pk, pk);
     max_large_cnt = std::max(max_large_cnt, lv.large_cnt);
     for (int32_t q = S.level_ptr[L]; q < S.level_ptr[L + 1]; q++) {
@@ -3004,8 +3006,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   e = cudaMemGetInfo(&free_b, &total_b);
   const size_t tsize = precision ? sizeof(float) : sizeof(double);
   const double need = (double)h->front_entries * tsize + (double)S.nnz * 8 + (double)S.n * 64 +
-                      (double)S.full_col.size() * 8 + (double)S.rows.size() * 24 +
-                      (double)max_work * tsize;
+                      (double)S.full_col.size() * 8 + (double)S.rows.size() * 8;
   int rc = NLA3D_OK;
   if (e != cudaSuccess)
     rc = cuda_fail(h, e, "cudaMemGetInfo");
@@ -3022,7 +3023,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
     LCK(dalloc(h, reinterpret_cast<float**>(&h->d_front), h->front_entries));
   else
     LCK(dalloc(h, reinterpret_cast<double**>(&h->d_front), h->front_entries));
-  const size_t nlinv = (size_t)std::max<uint64_t>(li_total, 1);
+  const size_t nlinv = (size_t)max_li;   // the panels of one level read them, nothing later
   if (precision) {
     // (tensor-core fronts keep the panels' operands packed instead)
     LCK(dalloc(h, reinterpret_cast<float**>(&h->d_W), h->tc ? 1 : (size_t)max_w));
@@ -3066,14 +3067,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   LCK(dalloc(h, &h->d_part, 2 * ((S.n + kRowsPerBlock - 1) / kRowsPerBlock)));
   LCK(dalloc(h, &h->d_norm, 2));
   LCK(dalloc(h, &h->d_dot, kDotBlocks));
-  if (precision) {
-    LCK(dalloc(h, &h->d_dirsum, (size_t)kDirBlocks * kDirSums));
-    // without the memory for them the refinement takes plain steps
-    const double dirs = 8.0 * (2 * kDirs + 1) * (double)S.n;
-    if (rc == NLA3D_OK && need + dirs <= 0.9 * (double)free_b &&
-        dalloc(h, &h->d_dirs, ((size_t)2 * kDirs + 1) * S.n) != cudaSuccess)
-      cudaGetLastError();
-  }
+  if (precision) LCK(dalloc(h, &h->d_dirsum, (size_t)kDirBlocks * kDirSums));
   LCK(dalloc(h, &h->d_maxabs, 1));
   LCK(dalloc(h, &h->d_maxpart, kMaxBlocks));
   LCK(dalloc(h, &h->d_perturbed, 2));
@@ -3111,11 +3105,23 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   LCK(upload(h, &sp, S.sn_parent));
   LCK(upload(h, &relp, S.rel_ptr));
   LCK(upload(h, &rl, S.rel));
+  if (precision) {
+    // the refinement's directions last, of what the rest has left and with the
+    // tenth that `need` leaves free: without them the refinement takes plain steps
+    size_t left = 0;
+    LCK(cudaMemGetInfo(&left, &total_b));
+    const double dirs = 8.0 * (2 * kDirs + 1) * (double)S.n;
+    if (rc == NLA3D_OK && dirs <= (double)left - 0.1 * (double)free_b &&
+        dalloc(h, &h->d_dirs, ((size_t)2 * kDirs + 1) * S.n) != cudaSuccess)
+      cudaGetLastError();
+  }
   LCK(cudaStreamSynchronize(h->stream));
 #undef LCK
   h->dev = LdltDev{fo, vo, rp, rw, sf, sp, relp, rl, inv_first_d, inv_error};
   if (rc != NLA3D_OK) {
-    // keep the handle so that the caller can read the message, then destroy it
+    // keep the handle so that the caller can read the message, then destroy it;
+    // what it holds so far is never run
+    h->d_front = nullptr;
     *out = h;
     return rc;
   }
