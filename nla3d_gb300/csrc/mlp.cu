@@ -34,8 +34,8 @@ namespace {
 // have released it, and a chunk's loads are issued before that wait.  The
 // epilogue reads TMEM (warp w: lanes 32 (w % 4) .. +31 = rows, columns
 // 8 (w / 4) .. +7), adds the bias, applies the activation and stores FP32.
-// Every wait is bounded: on a timeout the tile's outputs are set to NaN and
-// g_mlp_timeouts is incremented.
+// Every wait is bounded: on a timeout the tile's outputs, its row sums among
+// them, are set to NaN and g_mlp_timeouts is incremented.
 //
 // The network's products (batch x 256 x 256) are far below the chip: what
 // bounds one is the latency of its serial chunks.  128 x 128 tiles with
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kThreads)
     float* part = reinterpret_cast<float*>(smem);
     int r, k;
     unit_of<kTcM>(threadIdx.x, false, r, k);
-    part[(threadIdx.x / kTcM) * kTcM + r] = row_sum;
+    part[(threadIdx.x / kTcM) * kTcM + r] = ok ? row_sum : __uint_as_float(0x7FC00000u);
     __syncthreads();
     if (threadIdx.x < kTcM && m0 + threadIdx.x < M)
       a_sum[m0 + threadIdx.x] = (part[threadIdx.x] + part[kTcM + threadIdx.x]) +
