@@ -330,8 +330,7 @@ cudaError_t enqueue_elements(nla3d_ctx* c, uint32_t e0, uint32_t e1) {
     a.have_state = c->have_state ? 1 : 0;
     a.mat_id = m0.mat_id;
     for (int i = 0; i < 5; i++) a.mc[i] = m0.mat_c[i];
-    a.kbulk = bulk_of(m0);
-    a.inv_kb = 1.0 / a.kbulk;
+    a.inv_kb = 1.0 / bulk_of(m0);
     a.elem_mesh = c->uniform_material ? nullptr : c->d_elem_mesh;
     a.mesh_mat = c->uniform_material ? nullptr : c->d_mesh_mat;
     a.kpos = c->layout ? c->d_kpos : nullptr;
@@ -343,7 +342,6 @@ cudaError_t enqueue_elements(nla3d_ctx* c, uint32_t e0, uint32_t e1) {
       a.Gdf = c->d_Gdf;
       a.wdf = c->d_wdf;
       for (int i = 0; i < 5; i++) a.mcd[i] = split_pair(m0.mat_c[i]);
-      a.inv_kbd = split_pair(1.0 / a.kbulk);
       a.mesh_mat_df = c->uniform_material ? nullptr : c->d_mesh_mat_df;
     }
     e = launch_solid81_shaped(a, c->precision == NLA3D_PREC_MIXED, c->shape, c->stream);

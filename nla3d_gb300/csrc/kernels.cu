@@ -94,86 +94,6 @@ __device__ __forceinline__ void flag_element(ElementStatus* st, uint32_t el1) {
   atomicMax(&st->first_inv, ~el1);
 }
 
-template <typename TT>
-__device__ __forceinline__ void tangent_from_coefficients(const TT At[6], const TT Bt[6],
-                                                          const TT Ct[6], TT wk11, TT wk1,
-                                                          TT wk2, TT wc0, TT sIIt, TT sI,
-                                                          TT wD[21]);
-
-// Material response at one Gauss point (materials_hyperelastic.cpp:30-129).
-// Inputs: C (Voigt), p_state (for S), p_cur (for Dd).  Outputs: S, J and the
-// coefficient form of w*2*Dd:
-//   wD = A (x) P + B (x) Q + Ci (x) R + sIIt * IIt + sI * (I (x) I - II)
-template <typename TT>
-struct MatOut {
-  double S[6];
-  double J;
-};
-
-template <typename TT>
-__device__ __forceinline__ void material(int mat_id, const double* mc, const double C[6],
-                                         double p_state, double p_cur, double w, MatOut<TT>& o,
-                                         TT wD[21]) {
-  const double I1 = C[0] + C[3] + C[5];
-  const double I2 = C[0] * C[3] + C[3] * C[5] + C[0] * C[5] - C[1] * C[1] - C[4] * C[4] -
-                    C[2] * C[2];
-  const double detC = C[0] * (C[3] * C[5] - C[4] * C[4]) - C[1] * (C[1] * C[5] - C[4] * C[2]) +
-                      C[2] * (C[1] * C[4] - C[3] * C[2]);
-  const double J = sqrt(detC);
-  const double rc = rcbrt(J);
-  const double pp = rc * rc;       // J^(-2/3)
-  const double pppp = pp * pp;     // J^(-4/3)
-  const double oo = 1.0 / (J * J);
-  double Ci[6];
-  Ci[0] = oo * (C[3] * C[5] - C[4] * C[4]);
-  Ci[1] = oo * (C[2] * C[4] - C[1] * C[5]);
-  Ci[2] = oo * (C[1] * C[4] - C[2] * C[3]);
-  Ci[3] = oo * (C[0] * C[5] - C[2] * C[2]);
-  Ci[4] = oo * (C[1] * C[2] - C[0] * C[4]);
-  Ci[5] = oo * (C[0] * C[3] - C[1] * C[1]);
-  const double t13 = (1.0 / 3.0) * I1, t23 = (2.0 / 3.0) * I2;
-  // W derivatives at (I1 J^-2/3, I2 J^-4/3) (materials_hyperelastic.cpp:135-204)
-  double a1, a2 = 0.0, a11 = 0.0;
-  if (mat_id == 1) {
-    a1 = 0.5 * mc[0];
-  } else if (mat_id == 2) {
-    const double d = I1 * pp - 3.0;
-    a1 = mc[0] + 2 * mc[1] * d + 3 * mc[2] * d * d;
-    a2 = mc[3];
-    a11 = 2 * mc[1] + 6 * mc[2] * d;
-  } else {
-    a1 = mc[0];
-    a2 = mc[1];
-  }
-  const double I6[6] = {1.0, 0.0, 0.0, 1.0, 0.0, 1.0};
-  double A[6], B[6];
-#pragma unroll
-  for (int i = 0; i < 6; i++) {
-    A[i] = I6[i] - t13 * Ci[i];
-    B[i] = I1 * I6[i] - C[i] - t23 * Ci[i];
-  }
-  const double ko1 = 2 * a1 * pp, ko2 = 2 * a2 * pppp, pJs = p_state * J;
-#pragma unroll
-  for (int i = 0; i < 6; i++) o.S[i] = ko1 * A[i] + ko2 * B[i] + pJs * Ci[i];
-  o.J = J;
-  // tangent coefficients (Dd before the reference's /2, times w)
-  const double k11 = 4.0 * a11 * pppp, k1 = (4.0 / 3.0) * a1 * pp, k2 = (8.0 / 3.0) * a2 * pppp;
-  const double pj = p_cur * J;
-  const double c0 = pj - k1 * t13 - k2 * t23;
-  const TT sIIt = (TT)(w * (2.0 * pj - k1 * I1 - k2 * I2));
-  const TT sI = (TT)(w * 1.5 * k2);
-  // scalar coefficients in FP64, the 6-vectors P, Q, R in the tangent type
-  const TT wk11 = (TT)(w * k11), wk1 = (TT)(w * k1), wk2 = (TT)(w * k2), wc0 = (TT)(w * c0);
-  TT At[6], Bt[6], Ct[6];
-#pragma unroll
-  for (int i = 0; i < 6; i++) {
-    At[i] = (TT)A[i];
-    Bt[i] = (TT)B[i];
-    Ct[i] = (TT)Ci[i];
-  }
-  tangent_from_coefficients<TT>(At, Bt, Ct, wk11, wk1, wk2, wc0, sIIt, sI, wD);
-}
-
 // w * 2 Dd, packed upper Voigt, from the coefficient form
 //   A (x) P + B (x) Q + Ci (x) R + sIIt * IIt + sI * (I (x) I - II)
 // with P = wk11 A - wk1 Ci, Q = -wk2 Ci, R = -wk1 A - wk2 B + wc0 Ci
@@ -397,9 +317,9 @@ __device__ __forceinline__ dw dw_diff_prod(dw a, dw b, dw c, dw d) {
   return acc_val(t);
 }
 
-// The material response of material<TT> with the state (S, J) in pairs and
-// the tangent coefficients rounded to float (materials_hyperelastic.cpp:30-129,
-// 135-204).
+// Material response at one Gauss point (materials_hyperelastic.cpp:30-129,
+// 135-204) from C (Voigt), p_state (for S) and p_cur (for the tangent): the state
+// (S, J) in pairs, the tangent coefficients rounded to float.
 __device__ __forceinline__ void material_mixed(int mat_id, const float2* mcd, const dw C[6],
                                                dw p_state, dw p_cur, dw w, dw S[6], dw& Jout,
                                                float wD[21]) {
@@ -2077,8 +1997,6 @@ cudaError_t ensure_tables() {
 size_t solid81_smem_bytes_wpb(bool mixed, int wpb) {
   return mixed ? kDposBytes + wpb * sizeof(MixedSmem) : kHead64Bytes + wpb * kFWarp * sizeof(double);
 }
-
-size_t solid81_smem_bytes(bool mixed) { return solid81_smem_bytes_wpb(mixed, kWarpsPerBlock); }
 
 using Solid81Kernel = void (*)(Solid81Args);
 

@@ -33,10 +33,9 @@ struct Solid81Args {
   int have_state;           // 0: state of Element::pre() (C = I, S = 0, O = 0)
   int mat_id;
   double mc[5];
-  double kbulk;
   // optional per-element material (several meshes in one launch): when
   // elem_mesh != nullptr, element e uses mesh_mat[8 * elem_mesh[e] + ...] =
-  // (mat_id, c0..c4, K, 1/K) instead of mat_id / mc / kbulk
+  // (mat_id, c0..c4, K, 1/K) instead of mat_id / mc / inv_kb
   const uint32_t* elem_mesh;
   const double* mesh_mat;
   // optional slot-ordered output: contribution c of element e goes to
@@ -57,7 +56,6 @@ struct Solid81Args {
   const float2* Gdf;
   const float2* wdf;        // w det J
   float2 mcd[5];            // material constants
-  float2 inv_kbd;           // 1 / K
   double inv_kb;            // 1 / K in FP64
   const float2* mesh_mat_df;  // per mesh: 8 pairs (-, c0..c4, K, 1/K) when elem_mesh != nullptr
   // optional: a device word; when non-null and non-zero the launch does
@@ -240,7 +238,6 @@ cudaError_t launch_linear_mpc(const LinearMpcArgs& a, cudaStream_t s);
 cudaError_t launch_linear(const LinearArgs& a, cudaStream_t s);
 cudaError_t launch_plane41(const Plane41Args& a, cudaStream_t s);
 cudaError_t launch_lines(const LineArgs& a, cudaStream_t s);
-size_t solid81_smem_bytes(bool mixed);
 cudaError_t probe_fma_peak(bool fp64, double* flops);
 
 }  // namespace nla3d_gpu

@@ -62,7 +62,6 @@ struct LdltDev {
   const int64_t* row_ptr;
   const int32_t* rows;
   const int32_t* sn_first;
-  const int32_t* sn_parent;
   const int64_t* rel_ptr;
   const uint32_t* rel;
   const int32_t* inv_first;   // per supernode: its first kInv-pivot block (large fronts)
@@ -2498,14 +2497,13 @@ struct nla3d_ldlt {
   int32_t* d_rsn = nullptr;     // per front row: its supernode
   uint64_t* d_adest = nullptr;
   int32_t* d_perm = nullptr;
-  int32_t* d_lists = nullptr;   // level lists, small lists, extend-add child lists
+  int32_t* d_lists = nullptr;   // per level: small, large, narrow and wide fronts
   int64_t* d_fptr = nullptr;
   int32_t* d_fcol = nullptr;
   uint32_t* d_fslot = nullptr;
   LdltDev dev{};
   // host schedule per level
   struct Level {
-    int64_t all_off = 0, all_cnt = 0;     // every supernode of the level
     int64_t small_off = 0, small_cnt = 0, tiny_cnt = 0, warp_cnt = 0;   // see the lists
     int32_t small_max_m = 0;
     int64_t large_off = 0, large_cnt = 0; // fronts above kSmallFront rows
@@ -2825,7 +2823,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   }
   const LdltSymbolic& S = h->S;
   h->front_entries = S.front_off.back();
-  // the schedule: per level, all / small / large supernodes, children by ordinal
+  // the schedule: per level, its small and large fronts
   const int64_t ns = S.n_sn();
   const int nlev = (int)S.level_ptr.size() - 1;
   std::vector<int32_t> lists;
@@ -2848,9 +2846,6 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   h->levels.resize(nlev);
   for (int L = 0; L < nlev; L++) {
     auto& lv = h->levels[L];
-    lv.all_off = (int64_t)lists.size();
-    for (int32_t q = S.level_ptr[L]; q < S.level_ptr[L + 1]; q++) lists.push_back(S.level_list[q]);
-    lv.all_cnt = (int64_t)lists.size() - lv.all_off;
     lv.small_off = (int64_t)lists.size();
     // up to kTinyPivots pivots first, those of up to kTinyRows rows before the others
     for (int part = 0; part < 3; part++) {
@@ -3091,7 +3086,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   LCK(upload(h, &h->d_fslot, S.full_slot));
   uint64_t *fo = nullptr, *vo = nullptr;
   int64_t *rp = nullptr, *relp = nullptr;
-  int32_t *rw = nullptr, *sf = nullptr, *sp = nullptr;
+  int32_t *rw = nullptr, *sf = nullptr;
   uint32_t* rl = nullptr;
   int32_t* inv_first_d = nullptr;
   float* inv_error = nullptr;
@@ -3102,7 +3097,6 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   LCK(upload(h, &rp, S.row_ptr));
   LCK(upload(h, &rw, S.rows));
   LCK(upload(h, &sf, S.sn_first));
-  LCK(upload(h, &sp, S.sn_parent));
   LCK(upload(h, &relp, S.rel_ptr));
   LCK(upload(h, &rl, S.rel));
   if (precision) {
@@ -3117,7 +3111,7 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   }
   LCK(cudaStreamSynchronize(h->stream));
 #undef LCK
-  h->dev = LdltDev{fo, vo, rp, rw, sf, sp, relp, rl, inv_first_d, inv_error};
+  h->dev = LdltDev{fo, vo, rp, rw, sf, relp, rl, inv_first_d, inv_error};
   if (rc != NLA3D_OK) {
     // keep the handle so that the caller can read the message, then destroy it;
     // what it holds so far is never run

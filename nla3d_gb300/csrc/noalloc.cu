@@ -171,10 +171,9 @@ extern "C" int nla3d_assemble_solid81_noalloc(const nla3d_solid81_noalloc_args* 
   ea.have_state = 1;
   ea.mat_id = a->mat_id;
   for (int i = 0; i < 5; i++) ea.mc[i] = a->mat_c[i];
-  ea.kbulk = a->mat_id == NLA3D_MAT_NEO_HOOKEAN ? a->mat_c[1]
-                                                : (a->mat_id == NLA3D_MAT_BIDERMAN ? a->mat_c[4]
-                                                                                   : a->mat_c[2]);
-  ea.inv_kb = 1.0 / ea.kbulk;
+  ea.inv_kb = 1.0 / (a->mat_id == NLA3D_MAT_NEO_HOOKEAN ? a->mat_c[1]
+                     : a->mat_id == NLA3D_MAT_BIDERMAN  ? a->mat_c[4]
+                                                        : a->mat_c[2]);
   ea.contribK = contribK;
   ea.contribF = contribF;
   ea.status = d->status;
