@@ -81,3 +81,28 @@ def test_x_is_whole_when_the_steps_run_out(fronts):
         spent += s.last_residual > 0.0 and s.last_steps == steps   # no other way out
     s.close()
     assert spent > 0
+
+
+@pytest.mark.parametrize("fronts", ["fp32", "fp32-tc"])
+def test_gmres_after_the_steps_and_a_solve_after_it(fronts):
+    """An unattainable tolerance with more steps than the accelerated ones take:
+    GMRES goes on from the best x, its basis in the directions' memory.  The
+    residual it ends with is rounding (n products a row, each 2^-53 |A| |x|), and
+    the next solve on the handle repeats the first bit for bit."""
+    torch = pytest.importorskip("torch")
+    n = 300
+    a, io, co, b = _system(n, 1e5)
+    s = ldlt.DeviceLDLT(io, co, None, fronts)
+    v, bd = torch.from_numpy(a[np.triu_indices(n)]).cuda(), torch.from_numpy(b).cuda()
+    x, y = torch.empty_like(bd), torch.empty_like(bd)
+    torch.cuda.synchronize()
+    s.factor_device(v.data_ptr())
+    s.solve_device(v.data_ptr(), bd.data_ptr(), x.data_ptr(), max_refine=40, tol=1e-12)
+    first = x.cpu().numpy()
+    s.solve_device(v.data_ptr(), bd.data_ptr(), y.data_ptr(), max_refine=45, tol=0.0, strict=False)
+    got = y.cpu().numpy()
+    rounding = n * 2.0 ** -53 * np.linalg.norm(np.abs(a) @ np.abs(got))
+    assert np.linalg.norm(b - a @ got) <= rounding
+    s.solve_device(v.data_ptr(), bd.data_ptr(), x.data_ptr(), max_refine=40, tol=1e-12)
+    assert np.array_equal(x.cpu().numpy(), first)
+    s.close()
