@@ -34,22 +34,22 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 # FP64 flop per SOLID81 element the FP64 kernel executes (Mooney-Rivlin;
-# 4,688 DFMA + 3,044 DADD + 1,464 DMUL thread instructions per element in one
-# ncu capture; 2 DFMA + DADD + DMUL).  The kernel works in the element's
-# reference coordinates and sums over the Gauss points by Walsh-Hadamard
+# 4,968 DFMA + 3,076 DADD + 1,688 DMUL thread instructions per element in one
+# ncu capture; 2 DFMA + DADD + DMUL).  The kernel forms the tangent in the
+# element's reference coordinates and sums over the Gauss points by Walsh-Hadamard
 # transforms; the Bh^T D Bh formulation costs 69,072 (8 x 8634) for the same
 # element.
-FLOP_PER_ELEM = 13884
+FLOP_PER_ELEM = 14700
 FLOP_PER_ELEM_BTDB = 69072
 # FP64 instructions per element in the same capture: a DMUL or DADD takes the
 # pipe as long as a DFMA for half the flops, so the pipe's instruction rate is
 # the tighter ceiling.
-FP64_INSTR_PER_ELEM = 9196
+FP64_INSTR_PER_ELEM = 9732
 # DRAM bytes per element of solid81_fp64_kernel and of the K gather in one
 # ncu capture of a 40^3 block (64,000 elements, 9,675,406 K slots), used to
 # scale the traffic to the measured launch; the element kernel's writes are a
 # lower bound there (L2 still held part of them when the kernel ended).
-DRAM_BYTES_PER_ELEM_SOLID81 = (51.446784e6 + 118.781952e6) / 64000
+DRAM_BYTES_PER_ELEM_SOLID81 = (71.906560e6 + 119.612160e6) / 64000
 DRAM_BYTES_PER_ELEM_GATHER_K = (301.560064e6 + 62.591488e6) / 64000
 # Executed arithmetic per element of solid81_mixed_kernel, from the
 # instruction counters of one ncu capture of a 40^3 block (64,000 elements):
@@ -610,10 +610,9 @@ def run_ours(args):
                  "K_rel_err_vs_fp64": float(np.abs(K32 - K64).max() / np.abs(K64).max()),
                  "F_rel_err_vs_fp64": float(np.abs(F32 - F64).max() / np.abs(F64).max()),
                  "dtype": MIXED_DTYPE,
-                 "bound": "latency of the element kernel (short-scoreboard stalls first), "
-                          "the FP64 pipe of its volumetric terms the busiest unit (ncu at "
-                          "64,000 elements: FP64 pipe 65%, FP32 FMA 25%, issue 43%, LSU 17%, "
-                          "shared wavefronts 18%, DRAM 9%)",
+                 "bound": "latency and issue of the element kernel at 16 warps per SM (ncu at "
+                          "64,000 elements: issue 48%, FP64 pipe 46%; stalls: wait, then "
+                          "short scoreboard)",
                  "profile": "profiles/solid81_mixed_block40_ncu.md"}
         sm.close()
 

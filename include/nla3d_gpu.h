@@ -327,7 +327,8 @@ int nla3d_probe_fma_peak(int fp64, double* flops);
  *   nla3d_mlp_adam    Adam step on FP32 master weights (step >= 1), refreshing
  *                     the BF16 copy w_bf16 when non-NULL
  *   nla3d_mlp_layer_grads  dW[o,i] = sum_b dY[b,o] X[b,i] and db[o] = sum_b
- *                     dY[b,o] in one launch (row-major, contiguous)
+ *                     dY[b,o] in one launch, two with one output (row-major,
+ *                     contiguous)
  *   nla3d_mlp_input_grad   dX[b,i] = (sum_o dY[b,o] W[o,i]) (1 - Y[b,i]^2), W
  *                     BF16 (n_out x n_in), Y the layer's tanh input (NULL:
  *                     without the factor)
@@ -470,9 +471,13 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
 int nla3d_ldlt_factor(nla3d_ldlt* h, const double* values);
 /* EquationSolver::substituteEquations: x = K(2)^-1 b on device vectors, then
  * refinement until ||b - K x|| <= tol ||b|| with at most max_refine further
- * applications of the factor: steps x += K^-1 (b - K x) while each cuts the
- * residual tenfold (or one more at its rate reaches tol), then restarted
- * GMRES(30) preconditioned by the factor
+ * applications of the factor.  FP64 fronts: steps x += K^-1 (b - K x) while
+ * each cuts the residual tenfold (or one more at its rate reaches tol).  FP32
+ * fronts: accelerated steps, which take the least residual over the steps so
+ * far, at any rate, up to 30 or 12 in a row without a better x; the best x is
+ * returned when max_refine runs out (without device memory for their 61 vectors
+ * of n, the FP64 fronts' steps).  Then restarted GMRES(30) preconditioned by the
+ * factor.  x is complete when the call returns
  * (values: the same K as factored, or a nearby one).  NLA3D_ERR_RANGE when
  * tol is not reached; steps and rel_residual may be NULL. */
 int nla3d_ldlt_solve(nla3d_ldlt* h, const double* values, const double* b, double* x,

@@ -456,10 +456,10 @@ __device__ __forceinline__ void material_mixed(int mat_id, const float2* mcd, co
 //    sides: for each of the 7 modes P+p, seven sums over the modes Q+q and
 //    their butterfly to the 8 nodes b (22 adds / FMA), then for each b the
 //    butterfly over the modes to the 8 nodes a.
-//  9,196 FP64 instructions per element (Mooney-Rivlin, counted by ncu) where
+//  9,732 FP64 instructions per element (Mooney-Rivlin, counted by ncu) where
 //  the form with h_a and 231 accumulated entries took 16,723.  Element launch
-//  at 1e6 elements, Mooney-Rivlin: 28.0 -> 17.3 ms; at 216,000: 3.96 ms, and
-//  3.05 ms Neo-Hookean.  The FP64 pipe is 87% busy; what is left is the two
+//  at 1e6 elements, Mooney-Rivlin: 28.9 -> 19.1 ms; at 216,000: 4.18 ms, and
+//  3.27 ms Neo-Hookean.  The FP64 pipe is 87% busy; what is left is the two
 //  warps per scheduler that shared memory allows waiting at the exchanges
 //  (short scoreboard).
 //
@@ -2184,12 +2184,14 @@ cudaError_t launch_linear(const LinearArgs& a, cudaStream_t s) {
 // -Qe, -Fp and the entries in ElementPLANE41::assembleK order (PLANE41.h:54-95).
 //
 // The FP64 pipe bounds it, so it runs the FP64 SOLID81 kernel's algebra (see
-// solid81_fp64_kernel) in two dimensions, one thread per element: covariant
-// 2 x 2 components (the third direction contributes its 1 to I1, I2 and C),
+// solid81_fp64_kernel) in two dimensions, one thread per element: 2 x 2
+// components (the third direction contributes its 1 to I1, I2 and C),
 // the characters of the four Gauss points accumulated point by point, modes
-// x, y, xy to nodes at the end.  Some 1,400 FP64 instructions per element
+// x, y, xy to nodes at the end.  Some 1,500 FP64 instructions per element
 // where forming B, Dd B and every Kuu entry per Gauss point took about 2,900
-// and spilled: 39,963 elements 277 -> 154 us (ncu, cold).
+// and spilled: 39,963 elements 277 -> 164 us (ncu, cold).  As there, F is formed
+// in the global axes: with F from dx/dxi (4% faster) K_uu of an element sheared
+// by 100 lost four digits.
 struct Mode2 {
   double x, y, xy;
 };

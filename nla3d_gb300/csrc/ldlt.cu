@@ -2287,7 +2287,14 @@ __global__ void __launch_bounds__(kThreads)
 // Anal. 20, 1983).  Two launches of short vectors save one or two of the six to
 // nine applications of the factor.
 constexpr int kDirs = 30;                // steps kept (GMRES's restart); then GMRES takes over
-constexpr int kStalled = 12;             // steps without a better x before that
+// Steps without a better x before that: the residual can stay level until the
+// space holds the factor's bad modes, and a new basis with GMRES gives the steps
+// away.  Twelve against six on 288 made systems (200 to 500 rows, every fourth to
+// seventh pivot 1e-2 to 1e-5): 1,173 ms against 1,418, one solve of 54 instead of
+// 70 steps among them; a Newton solve of the 457k-equation bar 89 steps where six
+// did not reach 1e-10 in 100.  A factor of no help at all costs as much either way
+// (2,095 and 2,207 ms a solve of the 1.07M-equation bar, 100 steps).
+constexpr int kStalled = 12;
 constexpr int kDirSums = 2 * kDirs + 2;
 constexpr int kDirChunk = 8;             // directions per block of the sums
 constexpr int kDirBlocks = 152;
@@ -3379,11 +3386,13 @@ int nla3d_ldlt_solve(nla3d_ldlt* h, const double* values, const double* b, doubl
   // rate and not accuracy, and one application a step instead of FP64 products
   // and one more for x (a 457k-equation bar whose elimination grows: 22 steps in
   // 117 ms, against 27 in 259).  Without a better x for kStalled of them the
-  // residual is at its floor or the factor no help.
+  // residual is at its floor or the factor no help.  They apply the factor with
+  // the compensated FP32 products (2^-48 per operation): on the same factors FP64
+  // products took the same steps to the same residual in each of 1,050 Newton
+  // solves of bars of 139k to 1.07M equations, at twice the time a step.
   // GMRES with the same factor after, its preconditioner applied with FP64
-  // products (FP32 fronts: the compensated FP32 products carry 2^-48 per
-  // operation, which a hard system's Krylov iteration can feel).  rel is that
-  // of b - A x computed afresh, except between a step's correction and the next.
+  // products.  rel is that of b - A x computed afresh, except between a step's
+  // correction and the next.
   const double scale = bnorm > 0.0 ? bnorm : 1.0;
   // the best x of accelerated steps: past the attainable residual their
   // directions are rounding errors
