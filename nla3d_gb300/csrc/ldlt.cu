@@ -1351,7 +1351,11 @@ struct DotWide {
 };
 
 // Solves of the small fronts: one CTA per front, FP64 products whatever the
-// fronts' type (FP32 entries widened by integer operations).
+// fronts' type.  FP32 entries take the conversion instruction: these chains wait
+// for latency, and widening by integer operations only lengthens them (a pass:
+// 100,000 tridiagonal equations in one chain 121.6 instead of 104.1 ms, a band of
+// 40 39.8 instead of 33.1, the 139k-equation bar 1.74 instead of 1.69, the batch
+// 1.25 instead of 1.21).
 // forward: v[0:k] <- D^-1 L11^-1 v[0:k], v[k:m] <- v[k:m] - L21 (L11^-1 v[0:k]);
 // blocks of 64 pivots: the block's unit triangle in shared memory, then one
 // pass over the rows below it
@@ -1371,18 +1375,18 @@ __global__ void __launch_bounds__(kThreads)
     __syncthreads();
     for (int c = 0; c < cb; c++) {
       const int t = threadIdx.x;
-      if (t > c && t < cb) yb[t] -= widen(F[(c0 + t) + (c0 + c) * m]) * yb[c];
+      if (t > c && t < cb) yb[t] -= (double)F[(c0 + t) + (c0 + c) * m] * yb[c];
       __syncthreads();
     }
     if (threadIdx.x < cb) v[c0 + threadIdx.x] = yb[threadIdx.x];
     for (int64_t i = c0 + cb + threadIdx.x; i < m; i += blockDim.x) {
       double acc = 0.0;
-      for (int c = 0; c < cb; c++) acc += widen(F[i + (c0 + c) * m]) * yb[c];
+      for (int c = 0; c < cb; c++) acc += (double)F[i + (c0 + c) * m] * yb[c];
       v[i] -= acc;
     }
     __syncthreads();
   }
-  for (int64_t c = threadIdx.x; c < k; c += blockDim.x) v[c] /= widen(F[c + c * m]);
+  for (int64_t c = threadIdx.x; c < k; c += blockDim.x) v[c] /= (double)F[c + c * m];
 }
 
 // backward: x[0:k] = L11^-T (v[0:k] - L21^T x_rest), x_rest gathered from the
@@ -1406,10 +1410,10 @@ __global__ void __launch_bounds__(kThreads)
     double acc = 0.0, acc2 = 0.0;
     int64_t i = k + lane;
     for (; i + 32 < m; i += 64) {
-      acc += widen(F[i + c * m]) * xf[rows[i]];
-      acc2 += widen(F[i + 32 + c * m]) * xf[rows[i + 32]];
+      acc += (double)F[i + c * m] * xf[rows[i]];
+      acc2 += (double)F[i + 32 + c * m] * xf[rows[i + 32]];
     }
-    if (i < m) acc += widen(F[i + c * m]) * xf[rows[i]];
+    if (i < m) acc += (double)F[i + c * m] * xf[rows[i]];
     acc += acc2;
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     if (lane == 0) v[c] -= acc;
@@ -1419,14 +1423,14 @@ __global__ void __launch_bounds__(kThreads)
     const int cb = (int)(k - c0 < kPanel ? k - c0 : kPanel);
     for (int c = warp; c < cb; c += nwarps) {
       double acc = 0.0;
-      for (int64_t i = c0 + cb + lane; i < k; i += 32) acc += widen(F[i + (c0 + c) * m]) * v[i];
+      for (int64_t i = c0 + cb + lane; i < k; i += 32) acc += (double)F[i + (c0 + c) * m] * v[i];
       for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
       if (lane == 0) xb[c] = v[c0 + c] - acc;
     }
     __syncthreads();
     for (int c = cb - 1; c >= 0; c--) {
       const int t = threadIdx.x;
-      if (t < c) xb[t] -= widen(F[(c0 + c) + (c0 + t) * m]) * xb[c];
+      if (t < c) xb[t] -= (double)F[(c0 + c) + (c0 + t) * m] * xb[c];
       __syncthreads();
     }
     if (threadIdx.x < cb) v[c0 + threadIdx.x] = xb[threadIdx.x];
