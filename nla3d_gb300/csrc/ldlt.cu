@@ -2222,15 +2222,21 @@ __device__ __forceinline__ double row_sum(double acc) {   // all lanes of the wa
   return acc;
 }
 
-// r = b - A x (dr: what r fell by); per-block partial sums of r^2 and b^2 for
-// the norms.  110 -> 45 us
-// on the 139k-equation bar against a warp per row.
+// r = b - A x (dr: what r fell by) and the sums of r^2 and b^2 in `norms`: partial
+// sums per block, added up in a fixed order by the block that finishes last (a
+// launch of its own for them was 3 us of a small system's pass; copying the pairs
+// to the host took as long as the residual on large ones).  `done` counts the
+// blocks and returns to zero.  110 -> 45 us on the 139k-equation bar against a warp
+// per row.
 __global__ void __launch_bounds__(kThreads)
     residual_kernel(int64_t n, const int64_t* __restrict__ ptr, const int32_t* __restrict__ col,
                     const uint32_t* __restrict__ slot, const double* __restrict__ A,
                     const double* __restrict__ x, const double* __restrict__ b,
-                    double* __restrict__ r, double* __restrict__ part, double* __restrict__ dr) {
+                    double* __restrict__ r, double* __restrict__ part, double* __restrict__ dr,
+                    unsigned* __restrict__ done, double* __restrict__ norms) {
   __shared__ double red[2][kRowsPerBlock];
+  __shared__ double sum[kThreads];
+  __shared__ bool last;
   const int local = threadIdx.x / kRowLanes;
   const int64_t row = blockIdx.x * (int64_t)kRowsPerBlock + local;
   const double ax = row_sum(row < n ? row_product(row, ptr, col, slot, A, x) : 0.0);
@@ -2257,26 +2263,24 @@ __global__ void __launch_bounds__(kThreads)
     if (threadIdx.x == 0) {
       part[2 * blockIdx.x] = rr;
       part[2 * blockIdx.x + 1] = bb;
+      __threadfence();
+      last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;
     }
   }
-}
-
-// the blocks' pairs of partial sums added up, in a fixed order, by one block
-// (their copy to the host took as long as the residual on large models)
-__global__ void __launch_bounds__(kThreads)
-    norms_kernel(int64_t n, const double* __restrict__ part, double* __restrict__ out) {
-  __shared__ double red[kThreads];
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
   const int which = threadIdx.x & 1;   // r^2 or b^2
   double acc = 0.0;
 #pragma unroll 8
-  for (int64_t q = threadIdx.x; q < 2 * n; q += kThreads) acc += part[q];
-  red[threadIdx.x] = acc;
+  for (int64_t q = threadIdx.x; q < 2 * (int64_t)gridDim.x; q += kThreads) acc += __ldcg(part + q);
+  sum[threadIdx.x] = acc;
   __syncthreads();
   for (int s = kThreads / 2; s > 1; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+    if (threadIdx.x < s) sum[threadIdx.x] += sum[threadIdx.x + s];
     __syncthreads();
   }
-  if (threadIdx.x < 2) out[which] = red[which];
+  if (threadIdx.x < 2) norms[which] = sum[which];
 }
 
 // ---- vector kernels of the accelerated refinement steps ----
@@ -2467,7 +2471,8 @@ struct nla3d_ldlt {
   double* d_r = nullptr;
   double* d_dx = nullptr;
   double* d_part = nullptr;     // the residual's partial sums,
-  double* d_norm = nullptr;     // and their totals: r^2, b^2
+  double* d_norm = nullptr;     // their totals: r^2, b^2,
+  unsigned* d_done = nullptr;   // and the blocks that have written theirs
   double* d_V = nullptr;        // GMRES basis, (kRestart + 1) x n, allocated on first use
   double* d_dot = nullptr;
   double* d_dirs = nullptr;     // FP32 fronts: the refinement's Q and Z, kDirs x n each, and its best x, or null
@@ -2781,8 +2786,8 @@ cudaError_t enqueue_residual(nla3d_ldlt* h, const double* A, const double* x, co
   const LdltSymbolic& S = h->S;
   const unsigned blocks = (unsigned)((S.n + kRowsPerBlock - 1) / kRowsPerBlock);
   residual_kernel<<<blocks, kThreads, 0, h->stream>>>(S.n, h->d_fptr, h->d_fcol, h->d_fslot, A, x,
-                                                     b, h->d_r, h->d_part, dr);
-  norms_kernel<<<1, kThreads, 0, h->stream>>>(blocks, h->d_part, h->d_norm);
+                                                     b, h->d_r, h->d_part, dr, h->d_done,
+                                                     h->d_norm);
   return cudaGetLastError();
 }
 
@@ -3072,6 +3077,8 @@ int nla3d_ldlt_create(int64_t n, const uint32_t* iofeir, const uint32_t* columns
   LCK(dalloc(h, &h->d_dx, S.n));
   LCK(dalloc(h, &h->d_part, 2 * ((S.n + kRowsPerBlock - 1) / kRowsPerBlock)));
   LCK(dalloc(h, &h->d_norm, 2));
+  LCK(dalloc(h, &h->d_done, 1));
+  LCK(cudaMemsetAsync(h->d_done, 0, sizeof(unsigned), h->stream));
   LCK(dalloc(h, &h->d_dot, kDotBlocks));
   if (precision) LCK(dalloc(h, &h->d_dirsum, (size_t)kDirBlocks * kDirSums));
   LCK(dalloc(h, &h->d_maxabs, 1));
